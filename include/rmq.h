@@ -259,7 +259,7 @@ int rmq_probe_gather(const rmq_handle_t *h, const int32_t *d_queries, int64_t q,
  *       superset lay inside [l, r]
  *   [1] settled by a narrower probe plus one per-element entry
  *   [2] the three-part decomposition (two entries, probe of the middle)
- *   [3] inside one micro-block: one thread scans it
+ *   [3] inside one micro-block: its line of values is scanned
  *   [4] inside one block without the sub-block level: an edge entry
  *   [5] inside one block without the sub-block level: warp scan
  *   [6] per-element entries read (random 8-byte HBM lookups)

@@ -101,16 +101,15 @@ struct BatchParams {
     uint32_t phases;  // bit 0 build, bit 1 table levels, bit 2 queries
 };
 
-// Dynamic shared memory of a light batch CTA: the warps' miss queues, then
-// every thread's line slot (kLineChunks 16-byte chunks).
-constexpr size_t kLightQueueBytes = sizeof(MissQueue) * (kBatchThreads / 32);
-constexpr size_t kLightSmemBytes =
-    kLightQueueBytes + sizeof(uint4) * kLineChunks * static_cast<size_t>(kBatchThreads);
-static_assert(kLightQueueBytes % 16 == 0, "line slots start 16-byte aligned");
-// minima per buffer of a light tile (two buffers)
-constexpr uint32_t kTileEntries = static_cast<uint32_t>(kLightSmemBytes / (2 * sizeof(Entry)));
-static_assert(kTileEntries >= kMicroTile + 1023 && kTileEntries >= kMicroTileSmall + 2047,
-              "tiles of 2048 up to bs 32768 and of 1024 at bs 65536 fit");
+// minima per buffer of a light tile (two buffers): a tile of 2048 and its
+// halo up to bs 32768, one of 1024 at bs 65536
+constexpr uint32_t kTileEntries = kMicroTile + 1023u;
+static_assert(kTileEntries >= kMicroTileSmall + 2047u, "small tiles fit");
+// Dynamic shared memory of a light batch CTA: the tiles' buffers in phase A,
+// the warps' miss queues in phase C.
+constexpr size_t kLightSmemBytes = 2 * sizeof(Entry) * kTileEntries;
+static_assert(sizeof(MissQueue<kBatchQPT>) * (kBatchThreads / 32) <= kLightSmemBytes,
+              "miss queues fit");
 
 // Light kernels (batch_light.cu): the instantiation for (aligned, key mode),
 // its dynamic shared memory and CTAs per SM (the dynamic-memory limit set).
@@ -351,7 +350,7 @@ __device__ __forceinline__ void table_steps(const BatchParams &P, cg::grid_group
 
 // Phase C: the query items, in the queued form.
 template <bool ALIGNED, bool LIGHT, uint32_t MODE>
-__device__ __forceinline__ void query_items(const BatchParams &P, MissQueue &mq, uint4 *lines) {
+__device__ __forceinline__ void query_items(const BatchParams &P, MissQueue<kBatchQPT> &mq) {
     for (int32_t it = (P.phases & 4u) ? blockIdx.x : P.nqitems; it < P.nqitems; it += gridDim.x) {
         const uint4 w = P.qitems[it];
         const BatchArray a = P.arrays[w.x];
@@ -363,7 +362,7 @@ __device__ __forceinline__ void query_items(const BatchParams &P, MissQueue &mq,
         o.invalid = P.invalid;
         o.span = P.total_q - a.qoff;
         answer_range_queued<ALIGNED, LIGHT, LIGHT, MODE, kBatchThreads, kBatchQPT>(
-            v, o, w.y, static_cast<int64_t>(w.y) + w.z, mq, lines);
+            v, o, w.y, static_cast<int64_t>(w.y) + w.z, mq);
     }
 }
 
@@ -384,14 +383,14 @@ __global__ void __launch_bounds__(kBatchThreads, RMQ_BATCH_MINB) batch_kernel(Ba
     grid.sync();
     table_steps<false>(P, grid);
     // C: the warps' miss queues live in the staging memory of phase A
-    static_assert(sizeof(MissQueue) * (kBatchThreads / 32) <= sizeof(Entry) * kStageEntries,
+    static_assert(sizeof(MissQueue<kBatchQPT>) * (kBatchThreads / 32) <= sizeof(Entry) * kStageEntries,
                   "miss queues fit the staging memory");
-    MissQueue &mq = reinterpret_cast<MissQueue *>(stage)[threadIdx.x >> 5];
-    query_items<ALIGNED, false, MODE>(P, mq, nullptr);
+    query_items<ALIGNED, false, MODE>(
+        P, reinterpret_cast<MissQueue<kBatchQPT> *>(stage)[threadIdx.x >> 5]);
 }
 
-// Light index: block and micro-block tables only. Dynamic shared memory
-// (kLightSmemBytes): miss queues, then the threads' line slots.
+// Light index: block and micro-block tables only, kLightSmemBytes of dynamic
+// shared memory.
 template <bool ALIGNED, uint32_t MODE>
 __global__ void __launch_bounds__(kBatchThreads, RMQ_BATCH_LIGHT_MINB)
 batch_kernel_light(BatchParams P) {
@@ -412,9 +411,8 @@ batch_kernel_light(BatchParams P) {
     }
     grid.sync();
     table_steps<true>(P, grid);
-    MissQueue &mq = reinterpret_cast<MissQueue *>(s_light)[threadIdx.x >> 5];
-    uint4 *lines = reinterpret_cast<uint4 *>(s_light + kLightQueueBytes);
-    query_items<ALIGNED, true, MODE>(P, mq, lines);
+    query_items<ALIGNED, true, MODE>(
+        P, reinterpret_cast<MissQueue<kBatchQPT> *>(s_light)[threadIdx.x >> 5]);
 }
 
 }  // namespace

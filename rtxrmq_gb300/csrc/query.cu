@@ -21,10 +21,7 @@ constexpr int kThreads = 256;
 #endif
 constexpr int kQPT = RMQ_QUERY_QPT;
 #ifndef RMQ_QUERY_MINB
-#define RMQ_QUERY_MINB 1  // CTAs per SM the query kernel is compiled for (a register bound)
-#endif
-#ifndef RMQ_QUERY_LIGHT_MINB
-#define RMQ_QUERY_LIGHT_MINB 3  // the same for the light-index instantiations (68 registers)
+#define RMQ_QUERY_MINB 4  // CTAs per SM the query kernel is compiled for (a register bound)
 #endif
 
 // Queries base + t + k * kThreads (k < kQPT) of a full step, no bounds checks.
@@ -42,14 +39,9 @@ __device__ __forceinline__ void load_full(const QueryOut &o, int64_t base, int2 
 // measurement instantiation (rmq_query_stats), which also counts how each
 // query was settled and what it read into stats[kStatCount].
 template <bool ALIGNED, bool MICRO, bool LIGHT, uint32_t MODE, bool STATS>
-__global__ void __launch_bounds__(kThreads, LIGHT ? RMQ_QUERY_LIGHT_MINB : RMQ_QUERY_MINB)
+__global__ void __launch_bounds__(kThreads, RMQ_QUERY_MINB)
 query_kernel(V1View v, QueryOut o, int64_t q, unsigned long long *stats) {
-    __shared__ MissQueue s_mq[kThreads / 32];
-    // light index only: each thread's slot for the line copies of its
-    // misses (dynamic shared memory; none is given to other launches, so
-    // they keep the whole L1)
-    extern __shared__ uint4 s_lines[];
-    uint4 *const lines = LIGHT ? s_lines : nullptr;
+    __shared__ MissQueue<kQPT> s_mq[kThreads / 32];
     constexpr int64_t chunk = static_cast<int64_t>(kThreads) * kQPT;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * chunk;
     int64_t c0 = static_cast<int64_t>(blockIdx.x) * chunk;
@@ -58,14 +50,15 @@ query_kernel(V1View v, QueryOut o, int64_t q, unsigned long long *stats) {
     QStats s;
     if constexpr (STATS)
         for (int c = 0; c < kStatCount; ++c) s.c[c] = 0u;
-    MissQueue &mq = s_mq[threadIdx.x >> 5];
+    MissQueue<kQPT> &mq = s_mq[threadIdx.x >> 5];
     uint32_t waiting = 0;  // the warp's queue length (warp-uniform)
     int2 cur[kQPT];
     if (c0 <= last_full)
         load_full(o, c0, cur);
     else
         load_queries<kQPT>(o, c0, q, cur);
-    for (; c0 < q; c0 += stride) {
+    const StepMap map{c0, stride};
+    for (uint32_t id0 = 0; c0 < q; c0 += stride, id0 += static_cast<uint32_t>(chunk)) {
         const int64_t c1 = c0 + stride;
         int2 nxt[kQPT];
         if (c1 <= last_full)
@@ -74,14 +67,18 @@ query_kernel(V1View v, QueryOut o, int64_t q, unsigned long long *stats) {
             load_queries<kQPT>(o, c1, q, nxt);
         if (c0 <= last_full)
             answer_step_queued<ALIGNED, MICRO, LIGHT, MODE, kThreads, kQPT, STATS, true>(
-                v, o, c0, static_cast<uint32_t>(chunk), cur, s, mq, waiting, lines);
+                v, o, c0, static_cast<uint32_t>(chunk), id0, cur, s, mq, waiting);
         else
             answer_step_queued<ALIGNED, MICRO, LIGHT, MODE, kThreads, kQPT, STATS, false>(
-                v, o, c0, static_cast<uint32_t>(q - c0), cur, s, mq, waiting, lines);
+                v, o, c0, static_cast<uint32_t>(q - c0), id0, cur, s, mq, waiting);
+        // one site for the drain: its code is large, and every copy of it
+        // costs instruction fetches
+        while (waiting >= (c1 >= q ? 1u : 32u))
+            drain_misses<ALIGNED, MICRO, LIGHT, MODE, STATS, kThreads, kQPT>(
+                v, o, map, mq, waiting, l2_keep_policy(), s);
 #pragma unroll
         for (int k = 0; k < kQPT; ++k) cur[k] = nxt[k];
     }
-    if (waiting) drain_misses<ALIGNED, MICRO, LIGHT, MODE, STATS>(v, o, mq, waiting, l2_keep_policy(), s, lines);
     if constexpr (STATS) flush_stats(s, stats);
 }
 
@@ -182,6 +179,10 @@ cudaError_t occupancy(K kernel, std::atomic<int> *cache, int *per_sm) {
     return err;
 }
 
+// `bytes` of shared memory per SM (the runtime's 1 KB per CTA included) as a
+// percentage of the largest carve-out, 228 KB.
+int carveout_percent(size_t bytes) { return static_cast<int>((bytes * 100 + 228 * 1024 - 1) / (228 * 1024)); }
+
 uint32_t grid_size(int64_t q, int64_t per_block, int per_sm, const DeviceInfo &dev) {
     const int64_t need = (q + per_block - 1) / per_block;
     const int64_t cap = static_cast<int64_t>(dev.sms) * per_sm;
@@ -215,29 +216,26 @@ V1View view_of(const BuildPlan &p) {
     return v;
 }
 
-constexpr size_t kLineBytes = sizeof(uint4) * kLineChunks * kThreads;  // light launches
-
 template <bool ALIGNED, bool MICRO, bool LIGHT, uint32_t MODE, bool STATS>
 cudaError_t launch_query_t(const V1View &v, const QueryOut &o, int64_t q,
                            unsigned long long *stats, const DeviceInfo &dev, cudaStream_t s) {
     static std::atomic<int> per_sm_cache{0};
     auto kern = query_kernel<ALIGNED, MICRO, LIGHT, MODE, STATS>;
-    const size_t smem = LIGHT ? kLineBytes : 0;
     int per_sm = per_sm_cache.load(std::memory_order_relaxed);
     if (per_sm == 0) {
-        cudaError_t err;
-        if (LIGHT) {
-            // the line slots exceed the 48 KB default of dynamic shared memory
-            err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem));
-            if (err != cudaSuccess) return err;
-        }
-        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem);
+        cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, 0);
         if (err != cudaSuccess) return err;
         if (per_sm < 1) per_sm = 1;
+        // Shared memory no larger than the resident CTAs' queues need: the
+        // rest stays L1, where the block table's upper levels hit. The
+        // default split gives 100 KB for the 41 KB used (lr=-2, bs 4096,
+        // n = 1e8: 0.52 ms, with this 0.48).
+        err = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                   carveout_percent(per_sm * (sizeof(MissQueue<kQPT>) * (kThreads / 32) + 1024)));
+        if (err != cudaSuccess) return err;
         per_sm_cache.store(per_sm, std::memory_order_relaxed);
     }
-    kern<<<grid_size(q, kThreads * kQPT, per_sm, dev), kThreads, smem, s>>>(v, o, q, stats);
+    kern<<<grid_size(q, kThreads * kQPT, per_sm, dev), kThreads, 0, s>>>(v, o, q, stats);
     return cudaGetLastError();
 }
 

@@ -14,8 +14,8 @@
 // touches (blocks lB..rB, or with the sub-block level the 32-element
 // micro-blocks l/32..r/32), and when the leftmost best of that superset
 // lies inside [l, r] it is the answer without any per-element lookup. A
-// query inside one micro-block is settled by one thread's scan of that
-// 128-byte line; without the sub-block level a query inside one block that
+// query inside one micro-block is settled by a scan of that 128-byte line,
+// 8 lanes per query; without the sub-block level a query inside one block that
 // the probe does not settle reads pre / suf at a block edge, or is scanned
 // by the whole warp (__reduce_min_sync over the composites). All
 // comparisons are unsigned minima of the composites of common.cuh; only the
@@ -130,43 +130,6 @@ __device__ __forceinline__ uint64_t ld_moff_word(const V1View &v, uint64_t i, ui
     return r;
 }
 
-// Leftmost minimum of local A[a..b] (b - a < 32) computed by one thread.
-// ALIGNED: 16-byte loads of the chunks covering [a, b] (at most 9), two per
-// round, so that few registers are live.
-template <bool ALIGNED>
-__device__ __forceinline__ Entry thread_range_min(const V1View &v, uint32_t a, uint32_t b,
-                                                  uint32_t mode) {
-    const int64_t aa = v.off + a, ab = v.off + b;
-    Entry best = kEntryNone;
-    if (ALIGNED) {
-#pragma unroll 2
-        for (int64_t p = aa & ~int64_t(3); p <= ab; p += 4) {
-            uint32_t w[4];
-            if (p + 3 < v.limit) {
-                const uint4 f = ld_elem4(v, p);
-                w[0] = f.x;
-                w[1] = f.y;
-                w[2] = f.z;
-                w[3] = f.w;
-            } else {
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    w[c] = (p + c <= ab) ? ld_elem(v, p + c) : 0u;
-            }
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int64_t g = p + c;
-                if (g >= aa && g <= ab)
-                    best = better(best, make_entry(w[c], static_cast<uint32_t>(g - v.off), mode));
-            }
-        }
-    } else {
-        for (int64_t g = aa; g <= ab; ++g)
-            best = better(best, make_entry(ld_elem(v, g), static_cast<uint32_t>(g - v.off), mode));
-    }
-    return best;
-}
-
 struct QueryOut {
     const int2 *Q;        // queries of this array (local l, r)
     float *val;           // outputs aligned with Q, may be null
@@ -274,7 +237,7 @@ enum QStat : int {
     kStatFirst = 0,   // settled by the superset probe
     kStatSecond,      // settled by the second probe and one per-element entry
     kStatFull,        // three-part decomposition: two entries and a middle probe
-    kStatMicroScan,   // inside one micro-block: one thread scans its line
+    kStatMicroScan,   // inside one micro-block: its line of values is scanned
     kStatBlockEdge,   // one block, no sub-block level: pre / suf at a block edge
     kStatWarpScan,    // one block, no sub-block level: warp-cooperative scan
     kStatEntries,     // per-element entries read (pre, suf, mpre, msuf)
@@ -351,13 +314,6 @@ __device__ __forceinline__ uint32_t range_sectors(const V1View &v, uint32_t a, u
     return static_cast<uint32_t>(((v.off + b) >> 3) - ((v.off + a) >> 3) + 1);
 }
 
-// the probe that served a queued query (its code's low bits)
-enum : uint32_t {
-    kPathTable = 1,       // superset probe over blocks lB..rB
-    kPathMicroTable = 2,  // superset probe over micro-blocks ml..mr
-    kPathBlock = 4,       // one block, no sub-block level (an edge entry settles it)
-};
-
 // ---- the queued form (query_kernel, batch_kernel's query phase) -------------
 //
 // Settling a query that its probe leaves open inside the same step would
@@ -365,102 +321,132 @@ enum : uint32_t {
 // narrower probe, then maybe the rest). The queued form is specialised at
 // compile time on the key mode and on whether the index has the sub-block
 // level, and its main pass does only the superset probe: a query the probe
-// settles is stored at once; one it leaves open goes into a per-warp queue
-// in shared memory, and whenever 32 are waiting the warp settles them
-// together, one per lane (finish_miss).
+// settles is stored at once; one it leaves open, or that lies inside one
+// micro-block, goes into a per-warp queue in shared memory, and whenever 32
+// are waiting the warp settles them together (drain_misses).
 
-// code of a queued query: its path, and kMissLeft when the probe's best
-// lay left of l (else right of r)
-constexpr uint32_t kMissLeft = 8u;
+// ---- lines of values, settled by the warp ---------------------------------
+//
+// A query inside one micro-block, and a miss of the light index, needs the
+// best of part of one 32-element line. Scanned by the lane that owns the
+// query, a load instruction touches up to 32 different 128-byte lines, one
+// L1 tag lookup each, for up to 9 instructions, and a warp waits for its
+// longest scan. Here 8 lanes take one request, 16 bytes each: a load
+// instruction touches 4 lines and each line is looked up once. What bounds
+// it is the random lines' DRAM traffic. Measured (2^26 queries, ms): ranges
+// of 32 over n = 1e8 2.78 -> 1.81; light index, uniform 0.527 -> 0.346, short
+// (lr=-3) 1.18 -> 1.09, ranges of 32 4.99 -> 3.2 (those took 40 KB of shared
+// memory per CTA for the lines besides, and ran 3 CTAs per SM).
 
-// Shared-memory slot of one thread for a line of values: up to 9 16-byte
-// chunks (a 32-element micro-block not starting on a chunk boundary).
-constexpr int kLineChunks = 10;
-
-// Leftmost best of local A[lo..hi] (inside one micro-block) through an
-// asynchronous copy of the 16-byte chunks that cover it into the calling
-// thread's slot (cp.async.cg, bypassing L1), then a scan of the slot: one
-// memory round trip, few registers. The values base must be 16-byte
-// aligned; chunks past the end of the buffer are not read.
+// The best of one lane's chunk b[0..3] among the elements whose bit of `nib`
+// is set, in key mode MODE: its key, and its position | (-0.0 flag << 2).
+// With no element set, or every set element at the largest key, the key is
+// the largest one (the caller then takes the request's first element).
 template <uint32_t MODE>
-__device__ __forceinline__ Entry line_min_async(const V1View &v, uint32_t lo, uint32_t hi,
-                                                uint4 *slot) {
-    const int64_t glo = v.off + lo, ghi = v.off + hi;
-    const int64_t p0 = glo & ~int64_t(3);
-    const int nc = static_cast<int>(((ghi & ~int64_t(3)) - p0) / 4) + 1;
-    const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(slot));
-    const float *base = v.A + p0;  // 16-byte aligned
-    const int64_t room = v.limit - p0;  // elements from base to the end of the buffer
-    if (room >= 4 * nc) {
-#pragma unroll 1
-        for (int c = 0; c < nc; ++c)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
-                         :: "r"(sbase + 16u * c), "l"(base + 4 * c) : "memory");
+__device__ __forceinline__ void chunk_best(const uint32_t (&b)[4], uint32_t nib, uint32_t &key,
+                                           uint32_t &info) {
+    if constexpr (MODE == kFloatMin || MODE == kFloatMax) {
+        // the IEEE minimum (maximum) skips NaN, which orders last; the first
+        // value equal to it is the leftmost best and gives the key
+        float x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            x[k] = __uint_as_float((nib >> k) & 1u ? b[k] : 0x7fc00000u);
+        const float m = MODE == kFloatMin ? fminf(fminf(x[0], x[1]), fminf(x[2], x[3]))
+                                          : fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
+        const uint32_t p = x[0] == m ? 0u : x[1] == m ? 1u : x[2] == m ? 2u : 3u;
+        const uint32_t wb = p == 0u ? b[0] : p == 1u ? b[1] : p == 2u ? b[2] : b[3];
+        key = m == m ? key_of(wb, MODE) : 0xffffffffu;
+        info = p | (negzero_of(wb, MODE) << 2);
     } else {
-        // the buffer ends inside the line: copy what lies inside it
-#pragma unroll 1
-        for (int c = 0; c < nc; ++c) {
-            const int64_t avail = room - 4 * c;  // elements of the chunk inside the buffer
-            const uint32_t bytes = avail >= 4 ? 16u : static_cast<uint32_t>(avail > 0 ? avail * 4 : 0);
-            if (rmq_chk(p0 >= 0 && bytes > 0u))
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
-                             :: "r"(sbase + 16u * c), "l"(base + 4 * c), "r"(bytes) : "memory");
-        }
-    }
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-    // 32-bit keys first, one composite at the end: the smallest key and the
-    // first local index holding it (strict <, in index order) is the
-    // leftmost best; if every key is the largest, that is element lo.
-    const int32_t l0 = static_cast<int32_t>(p0 - v.off);  // local index of slot[0].x
-    uint32_t km = 0xffffffffu, pos = lo, nz = 0u;
-#pragma unroll 1
-    for (int c = 0; c < nc; ++c) {
-        const uint4 f = slot[c];
-        const uint32_t w[4] = {f.x, f.y, f.z, f.w};
-        const int32_t c0 = l0 + 4 * c;  // local index of w[0]
-        if constexpr (MODE == kFloatMin || MODE == kFloatMax) {
-            // the chunk's IEEE minimum (maximum) over its values in [lo, hi]
-            // (others as NaN, which it skips), the first value equal to it,
-            // and one key from that value's bits
-            float x[4];
+        key = 0xffffffffu;
+        info = 0u;
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                x[k] = __uint_as_float(
-                    static_cast<uint32_t>(c0 + k - static_cast<int32_t>(lo)) <= hi - lo
-                        ? w[k] : 0x7fc00000u);
-            const float m = MODE == kFloatMin ? fminf(fminf(x[0], x[1]), fminf(x[2], x[3]))
-                                              : fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
-            const uint32_t p = x[0] == m ? 0u : x[1] == m ? 1u : x[2] == m ? 2u : x[3] == m ? 3u : 0u;
-            const uint32_t wb = __float_as_uint(p == 0u ? x[0] : p == 1u ? x[1] : p == 2u ? x[2] : x[3]);
-            const uint32_t kk = key_of(wb, MODE);
-            if (kk < km) {
-                km = kk;
-                pos = static_cast<uint32_t>(c0) + p;
-                nz = negzero_of(wb, MODE);
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int32_t li = c0 + k;
-                const uint32_t kk = key_of(w[k], MODE);
-                if (static_cast<uint32_t>(li - static_cast<int32_t>(lo)) <= hi - lo && kk < km) {
-                    km = kk;
-                    pos = static_cast<uint32_t>(li);
-                    nz = negzero_of(w[k], MODE);
-                }
+        for (int k = 3; k >= 0; --k) {
+            const uint32_t kk = (nib >> k) & 1u ? key_of(b[k], MODE) : 0xffffffffu;
+            if (kk <= key) {
+                key = kk;
+                info = static_cast<uint32_t>(k);
             }
         }
     }
-    return (static_cast<uint64_t>(km) << 32) | (pos << 1) | nz;
 }
 
-// Leftmost best of local A[lo..hi] inside one micro-block for a miss: the
-// asynchronous line copy when the thread has a slot and the values are
-// aligned, else the thread's own scan.
+// One chunk of values: elements 4 sub .. 4 sub + 3 of the 32-element line
+// `line` (array-relative), of which only those set in `nib` are read when the
+// 16-byte load is not possible (values not 16-byte aligned, or the chunk
+// passes the end of the buffer).
+template <bool ALIGNED>
+__device__ __forceinline__ void load_chunk(const V1View &v, uint32_t line, uint32_t sub,
+                                           uint32_t nib, uint32_t (&b)[4]) {
+    const int64_t g = v.off + static_cast<int64_t>(line) * 32 + 4 * sub;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) b[k] = 0u;
+    if (nib == 0u) return;
+    if (ALIGNED && (v.off & 3) == 0 && g + 4 <= v.limit) {
+        const uint4 f = ld_elem4(v, g);
+        b[0] = f.x;
+        b[1] = f.y;
+        b[2] = f.z;
+        b[3] = f.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if ((nib >> k) & 1u) b[k] = ld_elem(v, g + k);
+    }
+}
+
+// Rounds of 4 requests whose loads are in flight together. Two: four cost 9
+// to 16 more registers in the main pass they share a kernel with (uniform
+// lengths, n = 1e8, q = 2^26: 0.309 ms with two, 0.341 with four) and settle
+// misses no faster.
+constexpr int kLineRounds = 2;
+
+// Leftmost best of the elements of line `line` whose bits are set in `bits`,
+// for every lane with bits != 0, kEntryNone for the others; the whole warp
+// calls it.
 template <bool ALIGNED, uint32_t MODE>
-__device__ __forceinline__ Entry line_min(const V1View &v, uint32_t lo, uint32_t hi, uint4 *slot) {
-    if (ALIGNED && slot) return line_min_async<MODE>(v, lo, hi, slot);
-    return thread_range_min<ALIGNED>(v, lo, hi, MODE);
+__device__ __forceinline__ Entry warp_lines(const V1View &v, uint32_t line, uint32_t bits) {
+    const uint32_t lane = threadIdx.x & 31u, sub = lane & 7u, grp = lane >> 3;
+    const uint32_t act = __ballot_sync(0xffffffffu, bits != 0u);
+    Entry out = kEntryNone;
+#pragma unroll 1
+    for (uint32_t h = 0; h < 32u; h += 4u * kLineRounds) {
+        if (((act >> h) & ((1u << (4 * kLineRounds)) - 1u)) == 0u) continue;  // warp-uniform
+        uint32_t b[kLineRounds][4];
+#pragma unroll
+        for (int t = 0; t < kLineRounds; ++t) {
+            const uint32_t ln = __shfl_sync(0xffffffffu, line, h + 4u * t + grp);
+            const uint32_t m = __shfl_sync(0xffffffffu, bits, h + 4u * t + grp);
+            load_chunk<ALIGNED>(v, ln, sub, (m >> (4u * sub)) & 15u, b[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < kLineRounds; ++t) {
+            const uint32_t m = __shfl_sync(0xffffffffu, bits, h + 4u * t + grp);
+            uint32_t gk, info;
+            chunk_best<MODE>(b[t], (m >> (4u * sub)) & 15u, gk, info);
+            const uint32_t key = gk;
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) gk = min(gk, __shfl_xor_sync(0xffffffffu, gk, o, 8));
+            const uint32_t own = (__ballot_sync(0xffffffffu, key == gk) >> (8u * grp)) & 0xffu;
+            const uint32_t w = __ffs(own) - 1u;
+            info = __shfl_sync(0xffffffffu, info, 8u * grp + w);
+            // every set element at the largest key: the first of them
+            const uint32_t pos = gk == 0xffffffffu ? __ffs(m) - 1u : 4u * w + (info & 3u);
+            const uint32_t nz = gk == 0xffffffffu ? 0u : info >> 2;
+            // to the lane that asked: h + 4 t + its group
+            const uint32_t rk = __shfl_sync(0xffffffffu, gk, 8u * (lane & 3u));
+            const uint32_t rl = __shfl_sync(0xffffffffu, (pos << 1) | nz, 8u * (lane & 3u));
+            if (bits != 0u && (lane >> 2) == (h >> 2) + t)
+                out = (static_cast<uint64_t>(rk) << 32) | ((line << 6) + rl);
+        }
+    }
+    return out;
+}
+
+// Bits lo .. hi (inclusive, 0 <= lo <= hi <= 31)
+__device__ __forceinline__ uint32_t bit_range(uint32_t lo, uint32_t hi) {
+    return (0xffffffffu >> (31u - hi)) & (0xffffffffu << lo);
 }
 
 // With per-element entries, the part of a query in its end unit on the
@@ -476,118 +462,139 @@ __device__ __forceinline__ Entry right_part(const V1View &v, bool micro, uint32_
 }
 
 // Light index: the query's part in its end unit on one side, [l, end of
-// l's unit] (left) or [start of r's unit, r] (right): one line of values
-// inside the end micro-block, plus for a block unit the micro table over
-// the block's whole micro-blocks on that side. The side is a value, not a
-// branch, so lanes settling left and right parts run the same code.
-template <bool ALIGNED, uint32_t MODE, bool STATS>
-__device__ __forceinline__ Entry light_part(const V1View &v, bool micro, bool left, uint32_t a,
+// l's unit] (left) or [start of r's unit, r] (right): part of one line of
+// values inside the end micro-block (its line and element bits), plus for a
+// block unit the best of the block's whole micro-blocks on that side. The
+// side is a value, not a branch, so that lanes settling left and right parts
+// run the same code.
+template <bool STATS>
+__device__ __forceinline__ Entry light_rest(const V1View &v, bool micro, bool left, uint32_t a,
                                             uint32_t b, uint32_t l, uint32_t r, uint64_t pol,
-                                            QStats &s, uint4 *slot) {
-    const uint32_t lo = left ? l : (r & ~31u);
-    const uint32_t hi = left ? min(l | 31u, v.n - 1u) : r;
-    const Entry line = line_min<ALIGNED, MODE>(v, lo, hi, slot);
-    if constexpr (STATS) s.c[kStatSectors] += range_sectors(v, lo, hi);
-    if (micro) return line;
+                                            QStats &s, uint32_t &line, uint32_t &bits) {
+    line = (left ? l : r) >> 5;
+    // the left end's unit lies before the right end's, so its line is whole
+    bits = left ? 0xffffffffu << (l & 31u) : 0xffffffffu >> (31u - (r & 31u));
+    if constexpr (STATS) s.c[kStatSectors] += range_sectors(v, left ? l : (r & ~31u), left ? l | 31u : r);
+    if (micro) return kEntryNone;
     // block a is full when a < b: its last micro-block ends inside the array
     const uint32_t ml = l >> 5, me = (((a + 1u) * v.bs) >> 5) - 1u;
     const uint32_t mr = r >> 5, ms = (b * v.bs) >> 5;
     const bool has = left ? ml < me : ms < mr;
-    if (!has) return line;
-    return better(line, micro_probe<STATS>(v, left ? ml + 1u : ms, left ? me : mr - 1u, pol, s));
+    if (!has) return kEntryNone;
+    return micro_probe<STATS>(v, left ? ml + 1u : ms, left ? me : mr - 1u, pol, s);
 }
 
 // Settles one query whose superset best lay outside [l, r] (or, without
-// the sub-block level, inside one block at an edge): the query's part in
-// the end unit on that side and a narrower probe, loaded together, then
-// only if needed the other end's part and the middle units.
-template <bool ALIGNED, bool MICRO, bool LIGHT, uint32_t MODE, bool STATS>
-__device__ __forceinline__ Entry finish_miss(const V1View &v, uint32_t l, uint32_t r,
-                                             uint32_t code, uint64_t pol, QStats &s,
-                                             uint4 *slot) {
-    const uint32_t path = code & 7u;
-    if constexpr (LIGHT) {
-        // one copy of the part's code: the second pass (the other end, after
-        // the middle units) runs only for the rare query the narrower probe
-        // does not settle
-        const bool micro = path == kPathMicroTable;
-        const uint32_t a = micro ? (l >> 5) : div31(l, v.dv);
-        const uint32_t b = micro ? (r >> 5) : div31(r, v.dv);
-        bool left = (code & kMissLeft) != 0u;
-        const Entry e2 = unit_probe<STATS>(v, micro, left ? a + 1u : a, left ? b : b - 1u, pol, s);
-        Entry res = kEntryNone;
-#pragma unroll 1
-        for (int pass = 0; pass < 2; ++pass) {
-            res = better(res, light_part<ALIGNED, MODE, STATS>(v, micro, left, a, b, l, r, pol, s,
-                                                               slot));
-            if (pass == 1) break;
-            const uint32_t m2 = entry_idx(e2);
-            if (left ? m2 <= r : m2 >= l) {
-                if constexpr (STATS) s.c[kStatSecond] += 1u;
-                return better(res, e2);
-            }
-            if constexpr (STATS) s.c[kStatFull] += 1u;
-            if (b - a >= 2u) res = better(res, unit_probe<STATS>(v, micro, a + 1u, b - 1u, pol, s));
-            left = !left;
-        }
-        return res;
-    } else {
-        if (path == kPathBlock) {
-            if constexpr (STATS) s.c[kStatBlockEdge] += 1u;
-            const uint32_t bstart = div31(l, v.dv) * v.bs;
-            const uint32_t bend = min(bstart + v.bs, v.n) - 1u;
-            return r == bend ? left_entry<STATS>(v, false, l, s) : right_entry<STATS>(v, false, r, s);
-        }
-        const bool micro = path == kPathMicroTable;
-        const uint32_t a = micro ? (l >> 5) : div31(l, v.dv);
-        const uint32_t b = micro ? (r >> 5) : div31(r, v.dv);
-        const bool left = (code & kMissLeft) != 0u;
-        // the narrower probe first: its loads are in flight while the part's
-        // entry is loaded
-        const Entry e2 = left ? unit_probe<STATS>(v, micro, a + 1u, b, pol, s)
-                              : unit_probe<STATS>(v, micro, a, b - 1u, pol, s);
-        const Entry e1 = left ? left_part<STATS>(v, micro, l, s) : right_part<STATS>(v, micro, r, s);
-        const uint32_t m2 = entry_idx(e2);
-        if (left ? m2 <= r : m2 >= l) {
-            if constexpr (STATS) s.c[kStatSecond] += 1u;
-            return better(e1, e2);
-        }
-        if constexpr (STATS) s.c[kStatFull] += 1u;
-        const Entry mid = (b - a >= 2u) ? unit_probe<STATS>(v, micro, a + 1u, b - 1u, pol, s)
-                                        : kEntryNone;
-        const Entry other = left ? right_part<STATS>(v, micro, r, s) : left_part<STATS>(v, micro, l, s);
-        return better(better(e1, other), mid);
+// the sub-block level, inside one block at an edge) from the per-element
+// entries: the query's part in the end unit on that side and a narrower
+// probe, loaded together, then only if needed the other end's part and the
+// middle units.
+template <bool STATS>
+__device__ __forceinline__ Entry finish_miss(const V1View &v, bool micro, bool left, uint32_t l,
+                                             uint32_t r, uint64_t pol, QStats &s) {
+    const uint32_t a = micro ? (l >> 5) : div31(l, v.dv);
+    const uint32_t b = micro ? (r >> 5) : div31(r, v.dv);
+    if (a == b) {
+        // one block, without the sub-block level: the query touches an edge
+        if constexpr (STATS) s.c[kStatBlockEdge] += 1u;
+        const uint32_t bend = min(a * v.bs + v.bs, v.n) - 1u;
+        return r == bend ? left_entry<STATS>(v, false, l, s) : right_entry<STATS>(v, false, r, s);
     }
+    // the narrower probe first: its loads are in flight while the part's
+    // entry is loaded
+    const Entry e2 = left ? unit_probe<STATS>(v, micro, a + 1u, b, pol, s)
+                          : unit_probe<STATS>(v, micro, a, b - 1u, pol, s);
+    const Entry e1 = left ? left_part<STATS>(v, micro, l, s) : right_part<STATS>(v, micro, r, s);
+    const uint32_t m2 = entry_idx(e2);
+    if (left ? m2 <= r : m2 >= l) {
+        if constexpr (STATS) s.c[kStatSecond] += 1u;
+        return better(e1, e2);
+    }
+    if constexpr (STATS) s.c[kStatFull] += 1u;
+    const Entry mid = (b - a >= 2u) ? unit_probe<STATS>(v, micro, a + 1u, b - 1u, pol, s)
+                                    : kEntryNone;
+    const Entry other = left ? right_part<STATS>(v, micro, r, s) : left_part<STATS>(v, micro, l, s);
+    return better(better(e1, other), mid);
 }
 
-// One warp's queue: up to 31 waiting queries plus the 32 that one query
-// slot of a step can add.
+// One warp's queue: up to 31 waiting queries plus the 32 that each query
+// slot of a step can add, 12 bytes each (what it takes from the L1 matters:
+// the block table's upper levels live there). `id` numbers the queries of
+// the CTA in the order it takes them: step * step size + place in the step.
+template <int QPT>
 struct MissQueue {
-    static constexpr int kCap = 64;
-    int64_t qi[kCap];
-    uint32_t l[kCap];
+    static constexpr int kCap = 32 * (QPT + 1);
+    uint32_t l[kCap];   // kMissLeft set: the probe's best lay left of l
     uint32_t r[kCap];
-    uint8_t code[kCap];
+    uint32_t id[kCap];
+};
+constexpr uint32_t kMissLeft = 0x80000000u;  // above every index
+
+// The queries a CTA takes: steps of `chunk` consecutive ones, `stride` apart.
+struct StepMap {
+    int64_t first;
+    int64_t stride;
+    __device__ __forceinline__ int64_t query(uint32_t id, uint32_t chunk) const {
+        return first + static_cast<int64_t>(id / chunk) * stride + id % chunk;
+    }
 };
 
 // Settles the last min(count, 32) queued queries, one per lane; the whole
-// warp calls it (count is warp-uniform).
-// `lines`: kLineChunks chunks of shared memory per thread of the CTA for
-// the light index's line copies, or null.
-template <bool ALIGNED, bool MICRO, bool LIGHT, uint32_t MODE, bool STATS>
-__device__ __forceinline__ void drain_misses(const V1View &v, const QueryOut &o, MissQueue &mq,
-                                             uint32_t &count, uint64_t pol, QStats &s,
-                                             uint4 *lines) {
+// warp calls it (count is warp-uniform). Queries inside one micro-block, and
+// the light index's misses, read lines of values, the warp together.
+template <bool ALIGNED, bool MICRO, bool LIGHT, uint32_t MODE, bool STATS, int THREADS, int QPT>
+__device__ __forceinline__ void drain_misses(const V1View &v, const QueryOut &o,
+                                             const StepMap &map, MissQueue<QPT> &mq,
+                                             uint32_t &count, uint64_t pol, QStats &s) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t take = count < 32u ? count : 32u;
     __syncwarp();
-    if (lane < take) {
-        const uint32_t e = count - take + lane;
-        const Entry r = finish_miss<ALIGNED, MICRO, LIGHT, MODE, STATS>(
-            v, mq.l[e], mq.r[e], mq.code[e], pol, s,
-            lines ? lines + threadIdx.x * kLineChunks : nullptr);
-        put_result(o, mq.qi[e], r, MODE);
+    const uint32_t e = count - take + lane;
+    const bool act = lane < take;
+    const uint32_t lq = act ? mq.l[e] : 0u, r = act ? mq.r[e] : 0u;
+    const uint32_t l = lq & ~kMissLeft;
+    const bool left = (lq & kMissLeft) != 0u;
+    const bool micro = MICRO && (r >> 5) - (l >> 5) < v.micro_span;
+    const bool scan = MICRO && act && (l >> 5) == (r >> 5);
+    const bool miss = act && !scan;
+    Entry res = kEntryNone;
+    uint32_t line = l >> 5, bits = scan ? bit_range(l & 31u, r & 31u) : 0u;
+    if constexpr (!LIGHT) {
+        if (MICRO && __any_sync(0xffffffffu, scan)) res = warp_lines<ALIGNED, MODE>(v, line, bits);
+        if (miss) res = finish_miss<STATS>(v, micro, left, l, r, pol, s);
+    } else {
+        const uint32_t a = micro ? (l >> 5) : div31(l, v.dv);
+        const uint32_t b = micro ? (r >> 5) : div31(r, v.dv);
+        Entry e2 = kEntryNone;
+        if (miss) {
+            e2 = unit_probe<STATS>(v, micro, left ? a + 1u : a, left ? b : b - 1u, pol, s);
+            res = light_rest<STATS>(v, micro, left, a, b, l, r, pol, s, line, bits);
+        }
+        // one copy of the line scan's code: the second pass (the other end,
+        // after the middle units) runs only for the rare query the narrower
+        // probe does not settle
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+            res = better(res, warp_lines<ALIGNED, MODE>(v, line, bits));
+            if (pass == 1) break;
+            bits = 0u;
+            bool more = false;
+            if (miss) {
+                const uint32_t m2 = entry_idx(e2);
+                more = left ? m2 > r : m2 < l;
+                if constexpr (STATS) s.c[more ? kStatFull : kStatSecond] += 1u;
+                if (!more) {
+                    res = better(res, e2);
+                } else {
+                    if (b - a >= 2u)
+                        res = better(res, unit_probe<STATS>(v, micro, a + 1u, b - 1u, pol, s));
+                    res = better(res, light_rest<STATS>(v, micro, !left, a, b, l, r, pol, s, line, bits));
+                }
+            }
+            if (!__any_sync(0xffffffffu, more)) break;
+        }
     }
+    if (act) put_result(o, map.query(mq.id[e], THREADS * QPT), res, MODE);
     __syncwarp();
     count -= take;
 }
@@ -654,21 +661,21 @@ __device__ __forceinline__ Entry superset_probe(const V1View &v, uint32_t l, uin
     return better(e1, e2);
 }
 
-// One step of the queued form over queries [base, base + cnt) (cnt <=
+// One step of the queued form over `cnt` queries from `base` on (cnt <=
 // THREADS * QPT): thread t handles base + t + k * THREADS, already loaded
 // into qq. FULL: cnt == THREADS * QPT, so no query needs a bounds check.
 // MICRO: the index has the sub-block level (then every query inside one
 // block spans few enough micro-blocks for the micro table, and only the
 // block table serves longer ones). LIGHT: a light index (no per-element
-// entries; `lines` holds the threads' line slots). `count` carries the warp's queue length
-// from step to step; the caller drains the rest.
+// entries). Queries left open join the warp's queue, whose length `count`
+// carries from step to step; `id0` is the step's first query in the CTA's
+// numbering. The caller drains the queue.
 template <bool ALIGNED, bool MICRO, bool LIGHT, uint32_t MODE, int THREADS, int QPT, bool STATS,
           bool FULL>
 __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryOut &o,
-                                                   int64_t base, uint32_t cnt,
+                                                   int64_t base, uint32_t cnt, uint32_t id0,
                                                    const int2 (&qq)[QPT], QStats &s,
-                                                   MissQueue &mq, uint32_t &count,
-                                                   uint4 *lines = nullptr) {
+                                                   MissQueue<QPT> &mq, uint32_t &count) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t pol = l2_keep_policy();
     float *const vs = o.val ? o.val + base : nullptr;
@@ -699,17 +706,18 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
             }
             continue;
         }
-        if (MICRO && scan[k]) {
-            res[k] = thread_range_min<ALIGNED>(v, l, r, MODE);
-            if constexpr (STATS) {
+        // a query inside one micro-block still holds kEntryNone here, whose
+        // index lies outside [l, r]
+        miss[k] = entry_idx(res[k]) - l > r - l;
+        any_miss |= miss[k];
+        if constexpr (STATS) {
+            if (MICRO && scan[k]) {
                 s.c[kStatMicroScan] += 1u;
                 s.c[kStatSectors] += range_sectors(v, l, r);
+            } else {
+                s.c[kStatFirst] += miss[k] ? 0u : 1u;
             }
-        } else {
-            miss[k] = entry_idx(res[k]) - l > r - l;
-            if constexpr (STATS) s.c[kStatFirst] += miss[k] ? 0u : 1u;
         }
-        any_miss |= miss[k];
         // the probe's answer is stored even for a query it leaves open: the
         // drain (same warp, after __syncwarp) or the warp scan (same thread)
         // overwrites it, and whole-warp stores keep the output lines whole
@@ -721,7 +729,6 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
 #pragma unroll
     for (int k = 0; k < QPT; ++k) {
         const uint32_t l = static_cast<uint32_t>(qq[k].x), r = static_cast<uint32_t>(qq[k].y);
-        uint32_t code = mic[k] ? kPathMicroTable : kPathTable;
         wscan[k] = false;
         if (!MICRO && miss[k]) {
             const uint32_t lB = div31(l, v.dv);
@@ -730,7 +737,6 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
                 // query touches the block's edge, else the warp scans it
                 const uint32_t bstart = lB * v.bs;
                 const uint32_t bend = min(bstart + v.bs, v.n) - 1u;
-                code = kPathBlock;
                 if (r != bend && l != bstart) {
                     miss[k] = false;
                     wscan[k] = true;
@@ -740,14 +746,11 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
         const unsigned mask = __ballot_sync(0xffffffffu, miss[k]);
         if (miss[k]) {
             const uint32_t e = count + __popc(mask & ((1u << lane) - 1u));
-            if (code != kPathBlock && entry_idx(res[k]) < l) code |= kMissLeft;
-            mq.qi[e] = base + threadIdx.x + k * THREADS;
-            mq.l[e] = l;
+            mq.l[e] = l | (entry_idx(res[k]) < l ? kMissLeft : 0u);
             mq.r[e] = r;
-            mq.code[e] = static_cast<uint8_t>(code);
+            mq.id[e] = id0 + threadIdx.x + k * THREADS;
         }
         count += __popc(mask);
-        if (count >= 32u) drain_misses<ALIGNED, MICRO, LIGHT, MODE, STATS>(v, o, mq, count, pol, s, lines);
     }
     if constexpr (!MICRO) {
 #pragma unroll
@@ -785,28 +788,29 @@ __device__ __forceinline__ void flush_stats(const QStats &s, unsigned long long 
 
 // Answer queries [q0, q1) of one array with the whole CTA (THREADS
 // threads) in the queued form, QPT queries per thread per step; `mq` is the
-// calling warp's queue, empty on entry and on return. LIGHT: a light index,
-// `lines` the CTA's line slots (kLineChunks chunks per thread).
+// calling warp's queue, empty on entry and on return. LIGHT: a light index.
 template <bool ALIGNED, bool MICRO, bool LIGHT, uint32_t MODE, int THREADS, int QPT>
 __device__ __forceinline__ void answer_range_queued(const V1View &v, const QueryOut &o,
-                                                    int64_t q0, int64_t q1, MissQueue &mq,
-                                                    uint4 *lines) {
+                                                    int64_t q0, int64_t q1, MissQueue<QPT> &mq) {
     constexpr int64_t step = static_cast<int64_t>(THREADS) * QPT;
+    const StepMap map{q0, step};
     QStats s;
-    uint32_t waiting = 0;
-    for (int64_t base = q0; base < q1; base += step) {
+    uint32_t waiting = 0, id0 = 0;
+    for (int64_t base = q0; base < q1; base += step, id0 += step) {
         int2 qq[QPT];
         load_queries<QPT>(o, base, q1, qq);
         if (base + step <= q1)
             answer_step_queued<ALIGNED, MICRO, LIGHT, MODE, THREADS, QPT, false, true>(
-                v, o, base, static_cast<uint32_t>(step), qq, s, mq, waiting, lines);
+                v, o, base, static_cast<uint32_t>(step), id0, qq, s, mq, waiting);
         else
             answer_step_queued<ALIGNED, MICRO, LIGHT, MODE, THREADS, QPT, false, false>(
-                v, o, base, static_cast<uint32_t>(q1 - base), qq, s, mq, waiting, lines);
+                v, o, base, static_cast<uint32_t>(q1 - base), id0, qq, s, mq, waiting);
+        // one site for the drain: its code is large, and every copy of it
+        // costs instruction fetches
+        while (waiting >= (base + step >= q1 ? 1u : 32u))
+            drain_misses<ALIGNED, MICRO, LIGHT, MODE, false, THREADS, QPT>(v, o, map, mq, waiting,
+                                                                           l2_keep_policy(), s);
     }
-    if (waiting)
-        drain_misses<ALIGNED, MICRO, LIGHT, MODE, false>(v, o, mq, waiting, l2_keep_policy(), s,
-                                                         lines);
 }
 
 }  // namespace rmq
