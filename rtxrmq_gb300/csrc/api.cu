@@ -13,6 +13,7 @@
 
 #include "../../include/rmq.h"
 #include "engine.h"
+#include "tables_impl.cuh"
 
 struct rmq_handle {
     rmq::BuildPlan plan;
@@ -21,6 +22,11 @@ struct rmq_handle {
     size_t mem_bytes;
     unsigned long long *invalid;    // device counter of rejected queries
     int64_t table_bytes;
+    // rmq_probe_gather on a table index: the per-element entries it looks up
+    // (pre, suf, then block minima), allocated and built by its first call
+    // under host_mu
+    void *entries;
+    bool entries_built;
     // rmq_query_host pipeline, created on its first call: device staging for
     // kHostStreams chunks (queries in, values and indices out), its streams
     // and events, and a lock that keeps concurrent calls from interleaving
@@ -267,6 +273,41 @@ int rmq_query(const rmq_handle_t *h, const int32_t *d_queries, int64_t q, float 
     return RMQ_OK;
 }
 
+// The plan of a handle with pre / suf present. A table index has none: the
+// first call allocates and builds them on `stream` and waits for that. While
+// the stream is capturing, waiting is not possible, so the build is captured
+// with the probe instead (and allocation, which belongs to the handle and not
+// to the graph, goes through with the capture checks relaxed).
+static int plan_with_entries(rmq_handle_t *h, const DeviceInfo &dev, cudaStream_t stream,
+                             BuildPlan *plan) {
+    *plan = h->plan;
+    if (!h->plan.micro) return RMQ_OK;
+    std::lock_guard<std::mutex> lock(*h->host_mu);
+    const size_t n = plan->n, nb = (n + plan->bs - 1) / plan->bs;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaError_t err = cudaStreamIsCapturing(stream, &cap);
+    if (err == cudaSuccess && !h->entries) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        const bool relax = cap != cudaStreamCaptureStatusNone;
+        if (relax) err = cudaThreadExchangeStreamCaptureMode(&mode);
+        if (err == cudaSuccess) err = dev_malloc(&h->entries, sizeof(Entry) * (2 * n + nb));
+        if (relax) cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    if (err != cudaSuccess) return cuda_fail(err, "rmq_probe_gather: entries");
+    plan->pre = static_cast<Entry *>(h->entries);
+    plan->suf = plan->pre + n;
+    plan->st = plan->suf + n;  // the builder's block minima
+    if (!h->entries_built) {
+        err = launch_build_entries(*plan, dev, stream);
+        if (err == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+            err = cudaStreamSynchronize(stream);
+            h->entries_built = err == cudaSuccess;
+        }
+        if (err != cudaSuccess) return cuda_fail(err, "rmq_probe_gather: entries");
+    }
+    return RMQ_OK;
+}
+
 int rmq_probe_gather(const rmq_handle_t *h, const int32_t *d_queries, int64_t q, float *d_val,
                      int32_t *d_idx, rmq_stream_t stream) {
     NvtxRange nvtx_range("rmq_probe_gather");
@@ -292,7 +333,10 @@ int rmq_probe_gather(const rmq_handle_t *h, const int32_t *d_queries, int64_t q,
     a.val = d_val;
     a.idx = d_idx;
     a.invalid = nullptr;
-    cudaError_t err = launch_probe_gather(h->plan, a, dev, stream);
+    BuildPlan plan;
+    rc = plan_with_entries(const_cast<rmq_handle_t *>(h), dev, stream, &plan);
+    if (rc) return rc;
+    cudaError_t err = launch_probe_gather(plan, a, dev, stream);
     if (err != cudaSuccess) return cuda_fail(err, "rmq_probe_gather: launch");
     return RMQ_OK;
 }
@@ -552,6 +596,8 @@ int rmq_free(rmq_handle_t *h) {
     cudaError_t err = release_staging(h);
     cudaError_t e2 = cudaFree(h->mem);
     if (err == cudaSuccess) err = e2;
+    e2 = cudaFree(h->entries);
+    if (err == cudaSuccess) err = e2;
     delete h->host_mu;
     delete h;
     if (err != cudaSuccess) return cuda_fail(err, "rmq_free: cudaFree");
@@ -563,17 +609,20 @@ int rmq_info(const rmq_handle_t *h, rmq_info_t *info) {
     if (!h || !info) return set_error(RMQ_EINVAL, "rmq_info: NULL argument");
     info->n = h->plan.n;
     info->bs = h->plan.bs;
-    info->nb = h->plan.nb;
-    info->levels = static_cast<int32_t>(h->plan.levels);
+    const uint32_t nb = (h->plan.n + h->plan.bs - 1) / h->plan.bs;
+    info->nb = nb;
+    info->levels = static_cast<int32_t>(st_levels(nb));
     info->aligned = h->plan.aligned ? 1 : 0;
     info->table_bytes = h->table_bytes;
     info->struct_bytes = static_cast<int64_t>(h->mem_bytes);
-    info->micro_levels = static_cast<int32_t>(h->plan.mlevels);
+    info->micro_levels = h->plan.micro ? static_cast<int32_t>(micro_levels(
+                                             h->plan.bs < 64u ? 64u : h->plan.bs)) : 0;
     info->light = h->plan.light ? 1 : 0;
     info->micro_table_bytes =
         h->plan.micro ? static_cast<int64_t>(static_cast<size_t>(h->plan.nmicro) *
-                                             (sizeof(Entry) + static_cast<size_t>(h->plan.moff_bytes) *
-                                                                  (h->plan.mlevels - 1)))
+                                             (sizeof(Entry) + (wide_masks(h->plan.nmicro) ? 8 : 4) +
+                                              h->plan.moff_bytes *
+                                                  moff_rows(h->plan.mlevels, wide_masks(h->plan.nmicro))))
                       : 0;
     info->is_max = (h->plan.kmode & 1u) ? 1 : 0;
     info->is_int32 = (h->plan.kmode >= kIntMin) ? 1 : 0;

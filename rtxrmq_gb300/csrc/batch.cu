@@ -56,11 +56,10 @@ cudaError_t full_kernel_t(uint32_t mode, const void **fn, int *per_sm) {
     }
 }
 
-// The kernel a run of this plan launches, its dynamic shared memory and CTAs per SM.
+// The kernel a run of this plan launches and its CTAs per SM.
 cudaError_t batch_kernel_for(bool light, bool aligned, uint32_t mode, const void **fn,
-                             size_t *smem, int *per_sm) {
+                             size_t smem, int *per_sm) {
     if (light) return batch_light_kernel(aligned, mode, fn, smem, per_sm);
-    *smem = 0;
     return aligned ? full_kernel_t<true>(mode, fn, per_sm) : full_kernel_t<false>(mode, fn, per_sm);
 }
 
@@ -299,6 +298,7 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
     std::vector<std::vector<uint4>> lvl(kMaxLevels);
     int64_t ws_entries = 0;
     int32_t maxlev = 1;
+    uint32_t halo = 0;  // the longest of the plan's tables
     b->h_arrays.resize(narrays);
     // table item: (array, kind << 16 | level, first, count) at table step `step`
     auto add_items = [&](int step, uint32_t i, uint32_t kind, uint32_t k, uint32_t cnt,
@@ -331,8 +331,8 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
         a.off = s;
         a.qoff = qs;
         a.n = static_cast<uint32_t>(n);
-        a.bs = static_cast<uint32_t>(bs);
-        a.nb = static_cast<uint32_t>((n + bs - 1) / bs);
+        a.bs = light && n > 0 ? table_block(static_cast<uint32_t>(bs)) : static_cast<uint32_t>(bs);
+        a.nb = static_cast<uint32_t>((n + a.bs - 1) / a.bs);
         a.levels = a.nb > 0 ? st_levels(a.nb) : 0u;
         a.U = make_unit_layout(a.bs, a.nb);
         a.dv = make_div31(a.bs);
@@ -344,10 +344,10 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
             a.moff_bytes = a.mlevels ? micro_offset_bytes(a.mlevels) : 0u;
             a.mst = ws_entries;
             ws_entries += a.nmicro;
+            a.mask = ws_entries = (ws_entries + 1) / 2 * 2;  // 16-byte aligned
+            ws_entries += a.nmicro;
             a.moff = ws_entries;
-            const int64_t moff_bytes = a.mlevels > 1 ? static_cast<int64_t>(a.moff_bytes) * a.nmicro *
-                                                           (a.mlevels - 1) : 0;
-            ws_entries += (moff_bytes + 7) / 8;
+            ws_entries += (static_cast<int64_t>(a.moff_bytes) * a.nmicro * moff_rows(a.mlevels, wide_masks(a.nmicro)) + 7) / 8;
             a.pre = -1;
         } else {
             a.pre = ws_entries;
@@ -357,26 +357,14 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
         b->limit = std::max(b->limit, s + n);
         b->total_q = std::max(b->total_q, qs + qc);
         if (light && a.nmicro > 0) {
-            // A: tiles (micro-block minima, every micro-table level and, when
-            // the blocks' micro-blocks divide a tile, the block minima, from
-            // one read of the values) if the micro table's halo fits a
-            // tile, else chunks of micro-block minima followed by one table
-            // item per micro level. B: block minima from the micro-block
+            // A: tiles (micro-block minima, micro table and, when the
+            // blocks' micro-blocks divide a tile, the block minima, from one
+            // read of the values). B: block minima from the micro-block
             // minima unless the tiles wrote them, then block level k.
             const uint32_t pb = a.bs / kMicro;
-            const uint32_t halo = (1u << (a.mlevels - 1)) - 1u;
-            const uint32_t tile = halo + kMicroTile <= kTileEntries        ? kMicroTile
-                                  : halo + kMicroTileSmall <= kTileEntries ? kMicroTileSmall
-                                                                           : 0u;
-            if (tile) {
-                a.light_flags = kLightTiled | (tile % pb == 0 ? kLightTileBmin : 0u) |
-                                (tile == kMicroTileSmall ? kLightSmallTile : 0u);
-                for (uint32_t t = 0; t * tile < a.nmicro; ++t) build.push_back(make_uint2(i, t));
-            } else {
-                for (uint32_t c = 0; c * kLightChunk < a.nmicro; ++c) build.push_back(make_uint2(i, c));
-                for (uint32_t k = 1; k < a.mlevels && (1u << k) <= a.nmicro; ++k)
-                    add_items(k, i, kItemMicroLevel, k, a.nmicro - (1u << k) + 1, lchunk);
-            }
+            halo = std::max(halo, table_halo(a.mlevels));
+            a.light_flags = kMicroTile % pb == 0 ? kLightTileBmin : 0u;
+            for (uint32_t t = 0; t * kMicroTile < a.nmicro; ++t) build.push_back(make_uint2(i, t));
             const int bstep = (a.light_flags & kLightTileBmin) ? 0 : 1;  // step of block level 0
             if (bstep == 1)
                 add_items(1, i, kItemBlockMinima, 0, a.nb, std::max<uint32_t>(1u, lchunk / pb));
@@ -411,6 +399,7 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
     P.nbuild = static_cast<int32_t>(build.size());
     P.nqitems = static_cast<int32_t>(b->h_qitems.size());
     P.total_q = b->total_q;
+    P.tile_cap = tile_entries(halo);
 
     // one allocation: arrays | build | lvl | qitems | counter | workspace
     const size_t o_arr = 0;
@@ -491,9 +480,9 @@ static int launch_batch(rmq_batch_t *b, const float *d_vals, const int32_t *d_qu
     P.phases = phases;
     const bool aligned = reinterpret_cast<uintptr_t>(d_vals) % 16 == 0;
     const void *kern = nullptr;
-    size_t smem = 0;
+    const size_t smem = b->light ? light_smem(P.tile_cap) : 0;
     int per_sm = 0;
-    cudaError_t err = batch_kernel_for(b->light, aligned, b->kmode, &kern, &smem, &per_sm);
+    cudaError_t err = batch_kernel_for(b->light, aligned, b->kmode, &kern, smem, &per_sm);
     if (err != cudaSuccess) return cuda_fail(err, who);
     // a cooperative launch needs every CTA resident
     if (per_sm < 1) return set_error(RMQ_ENOTSUP, "%s: kernel cannot be resident", who);
@@ -549,6 +538,7 @@ int rmq_batch_run_per_array(rmq_batch_t *b, const float *d_vals, const int32_t *
         p.A = d_vals + a.off;
         p.n = a.n;
         p.bs = a.bs;
+        p.tbs = a.bs;
         p.nb = a.nb;
         p.levels = a.levels;
         p.aligned = reinterpret_cast<uintptr_t>(p.A) % 16 == 0;
@@ -557,10 +547,11 @@ int rmq_batch_run_per_array(rmq_batch_t *b, const float *d_vals, const int32_t *
         p.light = b->light;
         if (b->light) {
             // the plain light index over the plan's own workspace layout
-            p.micro = a.mlevels > 0;
+            p.micro = true;
             p.nmicro = a.nmicro;
             p.mlevels = a.mlevels;
             p.mst = ws + a.mst;
+            p.mask = ws + a.mask;
             p.moff = ws + a.moff;
             p.moff_bytes = a.moff_bytes;
         } else {

@@ -25,6 +25,7 @@
 #include "build_impl.cuh"
 #include "engine.h"
 #include "query_impl.cuh"
+#include "tables_impl.cuh"
 
 // CTAs per SM the persistent batch kernels are compiled for (a register bound).
 #ifndef RMQ_BATCH_MINB
@@ -43,30 +44,20 @@ constexpr int kBatchQPT = 2;
 constexpr uint32_t kQueryChunk = 2048;
 constexpr uint32_t kLevelChunk = 4096;
 constexpr int kMaxLevels = 32;
-// micro-blocks per light build item: 16 per warp of the CTA
-constexpr uint32_t kLightChunk = kMicroPerWarp * (kBatchThreads / 32);
 
 // kinds of table items (bits 16.. of the item's second word; bits 0..15
 // hold the level)
 enum : uint32_t {
     kItemBlockLevel = 0,   // block-table level k from level k - 1
     kItemBlockMinima = 1,  // block-table level 0 from the micro-block minima
-    kItemMicroLevel = 2,   // micro-table level k from level k - 1
 };
-// Light tiles (phase A items of a light array whose micro table is shallow
-// enough): kMicroTile (or kMicroTileSmall) micro-blocks whose minima, every
-// micro-table level and the minima of the blocks inside come from one read
-// of the tile's values plus a halo of 2^(mlevels - 1) - 1 micro-blocks. The
-// levels are built in two shared-memory buffers of kTileEntries minima each,
-// so tile + halo <= kTileEntries: tiles of 2048 up to bs 32768, of 1024 at
-// bs 65536. Other light arrays take chunks in phase A and one table item
-// per level.
+// Light tiles (phase A items of a light array): kMicroTile micro-blocks whose
+// minima, micro table and the minima of the blocks inside come from one read
+// of the tile's values plus a halo of table_halo(mlevels) micro-blocks. The
+// table is built in shared memory (tables_impl.cuh).
 constexpr uint32_t kMicroTile = 2048;
-constexpr uint32_t kMicroTileSmall = 1024;
 // BatchArray::light_flags
-constexpr uint32_t kLightTiled = 1;       // phase A items are tiles
-constexpr uint32_t kLightTileBmin = 2;    // tiles also write the block minima (bs / 32 divides the tile)
-constexpr uint32_t kLightSmallTile = 4;   // tiles of kMicroTileSmall
+constexpr uint32_t kLightTileBmin = 1;    // tiles also write the block minima (bs / 32 divides the tile)
 
 struct BatchArray {
     int64_t off;    // first value in the buffer
@@ -74,7 +65,8 @@ struct BatchArray {
     int64_t pre;    // workspace entry offset of pre[]; suf[] follows at pre + n (full)
     int64_t st;     // workspace entry offset of the sparse table
     int64_t mst;    // workspace entry offset of the micro-block minima (light)
-    int64_t moff;   // workspace entry offset of the micro-table offsets (light)
+    int64_t mask;   // workspace entry offset of the micro table's masks (light)
+    int64_t moff;   // workspace entry offset of its offset rows (light)
     uint32_t n, bs, nb, levels;
     uint32_t nmicro, mlevels, moff_bytes, light_flags;
     UnitLayout U;
@@ -98,22 +90,24 @@ struct BatchParams {
     const uint4 *qitems;
     int32_t nqitems;
     int64_t total_q;  // one past the last query any array owns
+    uint32_t tile_cap;  // light: minima per tile buffer
     uint32_t phases;  // bit 0 build, bit 1 table levels, bit 2 queries
 };
 
-// minima per buffer of a light tile (two buffers): a tile of 2048 and its
-// halo up to bs 32768, one of 1024 at bs 65536
-constexpr uint32_t kTileEntries = kMicroTile + 1023u;
-static_assert(kTileEntries >= kMicroTileSmall + 2047u, "small tiles fit");
-// Dynamic shared memory of a light batch CTA: the tiles' buffers in phase A,
-// the warps' miss queues in phase C.
-constexpr size_t kLightSmemBytes = 2 * sizeof(Entry) * kTileEntries;
-static_assert(sizeof(MissQueue<kBatchQPT>) * (kBatchThreads / 32) <= kLightSmemBytes,
+// Minima of a tile and its halo: the longest (blocks of 2^15), and of a plan
+// whose largest halo is `halo` (BatchParams::tile_cap).
+constexpr uint32_t kTileEntries = kMicroTile + 1024u;
+inline uint32_t tile_entries(uint32_t halo) { return (kMicroTile + halo + 1u) & ~1u; }
+// Dynamic shared memory of a light batch CTA: the tile's buffers in phase A,
+// the warps' miss queues in phase C. A plan asks for what its own tiles need:
+// the rest is L1 for its queries.
+inline size_t light_smem(uint32_t tile_cap) { return table_smem(tile_cap); }
+static_assert(sizeof(MissQueue<true>) * (kBatchThreads / 32) <= table_smem(kMicroTile),
               "miss queues fit");
 
 // Light kernels (batch_light.cu): the instantiation for (aligned, key mode),
-// its dynamic shared memory and CTAs per SM (the dynamic-memory limit set).
-cudaError_t batch_light_kernel(bool aligned, uint32_t mode, const void **fn, size_t *smem,
+// CTAs per SM with `smem` bytes of dynamic shared memory (the limit set).
+cudaError_t batch_light_kernel(bool aligned, uint32_t mode, const void **fn, size_t smem,
                                int *per_sm);
 
 namespace {
@@ -133,12 +127,13 @@ __device__ __forceinline__ V1View batch_view(const BatchParams &P, const BatchAr
     v.st = P.ws + a.st;
     v.kmode = MODE;
     v.levels = a.levels;
-    v.mpre = nullptr;
-    v.msuf = nullptr;
+    v.light = LIGHT;
     if (LIGHT) {
         v.pre = nullptr;
         v.suf = nullptr;
         v.mst = P.ws + a.mst;
+        v.mask = P.ws + a.mask;
+        v.wide = wide_masks(a.nmicro);
         v.moff = P.ws + a.moff;
         v.moff_bytes = a.moff_bytes;
         v.nmicro = a.nmicro;
@@ -149,6 +144,8 @@ __device__ __forceinline__ V1View batch_view(const BatchParams &P, const BatchAr
         v.pre = P.ws + a.pre;
         v.suf = P.ws + a.pre + a.n;
         v.mst = nullptr;
+        v.mask = nullptr;
+        v.wide = false;
         v.moff = nullptr;
         v.moff_bytes = 0u;
         v.nmicro = 0;
@@ -175,22 +172,6 @@ __device__ __forceinline__ UnitJob unit_job(const BatchParams &P, uint32_t array
     J.kmode = MODE;
     J.nb = a.nb;
     return J;
-}
-
-// Light phase A: minima of micro-blocks [c * kLightChunk, ...) of one array,
-// kMicroPerWarp per warp.
-template <bool ALIGNED, uint32_t MODE>
-__device__ __forceinline__ void light_chunk(const BatchParams &P, const BatchArray &a,
-                                            uint32_t c) {
-    const uint32_t j0 = c * kLightChunk + (threadIdx.x >> 5) * kMicroPerWarp;
-    if (j0 >= a.nmicro) return;  // whole warp
-    const float *A = P.A + a.off;
-    Entry m[4];
-    // whole rows inside the array, 16-byte aligned
-    if (ALIGNED && a.off % 4 == 0 && (j0 + kMicroPerWarp) * kMicroElems <= a.n)
-        micro_min_warp<MODE, true>(A, a.n, j0, a.nmicro, P.ws + a.mst, 0u, m);
-    else
-        micro_min_warp<MODE, false>(A, a.n, j0, a.nmicro, P.ws + a.mst, 0u, m);
 }
 
 // Light table step, kind kItemBlockMinima: block minima of blocks [first,
@@ -221,60 +202,21 @@ __device__ __forceinline__ void light_block_minima(const BatchParams &P, const B
     }
 }
 
-template <class O>
-__device__ __forceinline__ void light_micro_level_w(const BatchParams &P, const BatchArray &a,
-                                                    uint32_t k, uint32_t first, uint32_t count) {
-    O *off = reinterpret_cast<O *>(P.ws + a.moff);
-    O *__restrict__ cur = off + static_cast<size_t>(k - 1) * a.nmicro;
-    const O *__restrict__ prev = off + static_cast<size_t>(k >= 2 ? k - 2 : 0) * a.nmicro;
-    for (uint32_t i = first + threadIdx.x; i < first + count; i += kBatchThreads)
-        micro_level_at(P.ws + a.mst, cur, prev, a.nmicro, k, i);
-}
-
-// Every level 1 .. mlevels - 1 of the micro table at positions [t0, t0 +
-// count) from the minima src[0 .. e) of micro-blocks [t0, t0 + e) in shared
-// memory. Level k holds the best minimum of every window of 2^k micro-blocks
-// whose window lies in the loaded range (the better of the level below's two
-// halves), written to the other buffer; the offset stored is that minimum's
-// micro-block (its element index / 32) minus the window's first. One barrier
-// per level.
-template <class O>
-__device__ __forceinline__ void micro_tile_levels(const BatchParams &P, const BatchArray &a,
-                                                  uint32_t t0, uint32_t count, uint32_t e,
-                                                  Entry *src, Entry *dst) {
-    O *off = reinterpret_cast<O *>(P.ws + a.moff);
-    for (uint32_t k = 1; k < a.mlevels && (1u << k) <= e; ++k) {
-        const uint32_t half = 1u << (k - 1);
-        const uint32_t valid = e - (1u << k) + 1;  // windows inside the loaded range
-        O *__restrict__ row = off + static_cast<size_t>(k - 1) * a.nmicro + t0;
-        for (uint32_t i = threadIdx.x; i < valid; i += kBatchThreads) {
-            const Entry m = better(src[i], src[i + half]);
-            dst[i] = m;
-            if (i < count) row[i] = static_cast<O>((entry_idx(m) >> 5) - (t0 + i));
-        }
-        __syncthreads();
-        Entry *t = src;
-        src = dst;
-        dst = t;
-    }
-}
-
-// Light phase A, one tile (kLightTiled arrays): the minima of micro-blocks
-// [t0, t0 + count + halo) from the values into shared memory (8 rows of 512
-// bytes per warp step, all loads in flight), the tile's own minima to the
-// micro-block minima table, the minima of the blocks inside the tile
-// (kLightTileBmin), and every micro-table level at [t0, t0 + count). The
-// halo's minima are computed again by the next tile.
-template <bool ALIGNED, uint32_t MODE, class O>
+// Light phase A, one tile: the minima of micro-blocks [t0, t0 + count + halo)
+// from the values into shared memory (8 rows of 512 bytes per warp step, all
+// loads in flight), the tile's own minima to the micro-block minima table,
+// the minima of the blocks inside the tile (kLightTileBmin), and the micro
+// table at [t0, t0 + count). The halo's minima are computed again by the
+// next tile.
+template <bool ALIGNED, uint32_t MODE>
 __device__ __forceinline__ void light_tile(const BatchParams &P, const BatchArray &a, uint32_t t,
                                            unsigned char *smem) {
     Entry *key = reinterpret_cast<Entry *>(smem);
-    const uint32_t tile = (a.light_flags & kLightSmallTile) ? kMicroTileSmall : kMicroTile;
-    const uint32_t t0 = t * tile;
-    const uint32_t count = min(tile, a.nmicro - t0);
-    const uint32_t halo = (1u << (a.mlevels - 1)) - 1u;
-    const uint32_t jend = min(t0 + count + halo, a.nmicro);
-    const uint32_t e = jend - t0;  // minima held in shared memory (<= kTileEntries)
+    uint32_t *keys = reinterpret_cast<uint32_t *>(key + 2 * P.tile_cap);
+    const uint32_t t0 = t * kMicroTile;
+    const uint32_t count = min(kMicroTile, a.nmicro - t0);
+    const uint32_t jend = min(t0 + count + table_halo(a.mlevels), a.nmicro);
+    const uint32_t e = jend - t0;  // minima held in shared memory (<= P.tile_cap)
     const float *A = P.A + a.off;
     const bool vec = ALIGNED && a.off % 4 == 0;
     // 8 rows (32 micro-blocks, 4 KB) per warp step: 96 KB of loads in flight per SM
@@ -313,10 +255,20 @@ __device__ __forceinline__ void light_tile(const BatchParams &P, const BatchArra
             }
         }
     }
-    // the levels write only the second buffer first; the block minima and
-    // the table copy above read the first
-    micro_tile_levels<O>(P, a, t0, count, e, key, key + kTileEntries);
-    __syncthreads();  // the next tile overwrites both buffers
+    tile_keys<kBatchThreads>(key, e, keys);
+    __syncthreads();
+    MicroTable T;
+    T.mst = mst;
+    T.mask = P.ws + a.mask;
+    T.moff = P.ws + a.moff;
+    T.moff_bytes = a.moff_bytes;
+    T.nmicro = a.nmicro;
+    T.mlevels = a.mlevels;
+    // its rows overwrite `key` only behind a barrier, after the block minima
+    // and the table copy above have read it
+    table_tile<kBatchThreads>(T, t0, count, e, key, key + P.tile_cap, keys,
+                              keys + key_words(P.tile_cap));
+    __syncthreads();  // the next tile overwrites the buffers
 }
 
 // Phase B: table steps 1 .. maxlev - 1, a grid barrier after each.
@@ -329,13 +281,6 @@ __device__ __forceinline__ void table_steps(const BatchParams &P, cg::grid_group
             const uint32_t kind = w.y >> 16, k = w.y & 0xffffu;
             if (LIGHT && kind == kItemBlockMinima) {
                 light_block_minima(P, a, w.z, w.w);
-            } else if (LIGHT && kind == kItemMicroLevel) {
-                if (a.moff_bytes == 1u)
-                    light_micro_level_w<uint8_t>(P, a, k, w.z, w.w);
-                else if (a.moff_bytes == 2u)
-                    light_micro_level_w<uint16_t>(P, a, k, w.z, w.w);
-                else
-                    light_micro_level_w<uint32_t>(P, a, k, w.z, w.w);
             } else {
                 const Entry *__restrict__ prev = P.ws + a.st + static_cast<int64_t>(k - 1) * a.nb;
                 Entry *__restrict__ cur = P.ws + a.st + static_cast<int64_t>(k) * a.nb;
@@ -350,7 +295,7 @@ __device__ __forceinline__ void table_steps(const BatchParams &P, cg::grid_group
 
 // Phase C: the query items, in the queued form.
 template <bool ALIGNED, bool LIGHT, uint32_t MODE>
-__device__ __forceinline__ void query_items(const BatchParams &P, MissQueue<kBatchQPT> &mq) {
+__device__ __forceinline__ void query_items(const BatchParams &P, MissQueue<LIGHT> &mq) {
     for (int32_t it = (P.phases & 4u) ? blockIdx.x : P.nqitems; it < P.nqitems; it += gridDim.x) {
         const uint4 w = P.qitems[it];
         const BatchArray a = P.arrays[w.x];
@@ -361,7 +306,7 @@ __device__ __forceinline__ void query_items(const BatchParams &P, MissQueue<kBat
         o.idx = P.idx ? P.idx + a.qoff : nullptr;
         o.invalid = P.invalid;
         o.span = P.total_q - a.qoff;
-        answer_range_queued<ALIGNED, LIGHT, LIGHT, MODE, kBatchThreads, kBatchQPT>(
+        answer_range_queued<ALIGNED, LIGHT, MODE, kBatchThreads, kBatchQPT>(
             v, o, w.y, static_cast<int64_t>(w.y) + w.z, mq);
     }
 }
@@ -370,7 +315,7 @@ __device__ __forceinline__ void query_items(const BatchParams &P, MissQueue<kBat
 // inside one block.
 template <bool ALIGNED, uint32_t MODE>
 __global__ void __launch_bounds__(kBatchThreads, RMQ_BATCH_MINB) batch_kernel(BatchParams P) {
-    __shared__ Entry stage[kStageEntries];
+    __shared__ __align__(16) Entry stage[kStageEntries];
     __shared__ uint64_t s_warp[kWarpSlots];
     __shared__ uint32_t s_flag[2 * kBuildWarps];
     cg::grid_group grid = cg::this_grid();
@@ -383,36 +328,29 @@ __global__ void __launch_bounds__(kBatchThreads, RMQ_BATCH_MINB) batch_kernel(Ba
     grid.sync();
     table_steps<false>(P, grid);
     // C: the warps' miss queues live in the staging memory of phase A
-    static_assert(sizeof(MissQueue<kBatchQPT>) * (kBatchThreads / 32) <= sizeof(Entry) * kStageEntries,
+    static_assert(sizeof(MissQueue<false>) * (kBatchThreads / 32) <= sizeof(Entry) * kStageEntries,
                   "miss queues fit the staging memory");
     query_items<ALIGNED, false, MODE>(
-        P, reinterpret_cast<MissQueue<kBatchQPT> *>(stage)[threadIdx.x >> 5]);
+        P, reinterpret_cast<MissQueue<false> *>(stage)[threadIdx.x >> 5]);
 }
 
-// Light index: block and micro-block tables only, kLightSmemBytes of dynamic
-// shared memory.
+// Light index: block and micro-block tables only, light_smem() bytes of
+// dynamic shared memory.
 template <bool ALIGNED, uint32_t MODE>
 __global__ void __launch_bounds__(kBatchThreads, RMQ_BATCH_LIGHT_MINB)
 batch_kernel_light(BatchParams P) {
-    extern __shared__ __align__(16) unsigned char s_light[];
+    extern __shared__ __align__(128) unsigned char s_light[];
     cg::grid_group grid = cg::this_grid();
 
-    // A: tiles (micro-block minima, micro table, block minima) or chunks
-    // (micro-block minima only)
+    // A: tiles (micro-block minima, micro table, block minima)
     for (int32_t it = (P.phases & 1u) ? blockIdx.x : P.nbuild; it < P.nbuild; it += gridDim.x) {
         const uint2 w = P.build[it];
-        const BatchArray &a = P.arrays[w.x];
-        if (!(a.light_flags & kLightTiled))
-            light_chunk<ALIGNED, MODE>(P, a, w.y);
-        else if (a.moff_bytes == 1u)
-            light_tile<ALIGNED, MODE, uint8_t>(P, a, w.y, s_light);
-        else
-            light_tile<ALIGNED, MODE, uint16_t>(P, a, w.y, s_light);
+        light_tile<ALIGNED, MODE>(P, P.arrays[w.x], w.y, s_light);
     }
     grid.sync();
     table_steps<true>(P, grid);
     query_items<ALIGNED, true, MODE>(
-        P, reinterpret_cast<MissQueue<kBatchQPT> *>(s_light)[threadIdx.x >> 5]);
+        P, reinterpret_cast<MissQueue<true> *>(s_light)[threadIdx.x >> 5]);
 }
 
 }  // namespace

@@ -9,25 +9,26 @@
 namespace rmq {
 namespace {
 
-std::atomic<int> g_light_per_sm[8];  // (aligned, key mode)
+std::atomic<bool> g_light_ready[8];  // (aligned, key mode)
 
 template <bool ALIGNED, uint32_t MODE>
-cudaError_t pick_light(const void **fn, size_t *smem, int *per_sm) {
+cudaError_t pick_light(const void **fn, size_t smem, int *per_sm) {
     auto kern = batch_kernel_light<ALIGNED, MODE>;
-    std::atomic<int> &slot = g_light_per_sm[(ALIGNED ? 4 : 0) + MODE];
-    if (slot.load(std::memory_order_relaxed) == 0) {
+    std::atomic<bool> &slot = g_light_ready[(ALIGNED ? 4 : 0) + MODE];
+    if (!slot.load(std::memory_order_relaxed)) {
         // above the default 48 KB of dynamic shared memory
-        const cudaError_t err = cudaFuncSetAttribute(
-            kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLightSmemBytes));
+        const cudaError_t err =
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(light_smem(kTileEntries)));
         if (err != cudaSuccess) return err;
+        slot.store(true, std::memory_order_relaxed);
     }
     *fn = reinterpret_cast<const void *>(kern);
-    *smem = kLightSmemBytes;
-    return occupancy_cached(kern, kBatchThreads, slot, *per_sm, kLightSmemBytes);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern, kBatchThreads, smem);
 }
 
 template <bool ALIGNED>
-cudaError_t light_kernel_t(uint32_t mode, const void **fn, size_t *smem, int *per_sm) {
+cudaError_t light_kernel_t(uint32_t mode, const void **fn, size_t smem, int *per_sm) {
     switch (mode) {
     case kFloatMax: return pick_light<ALIGNED, kFloatMax>(fn, smem, per_sm);
     case kIntMin: return pick_light<ALIGNED, kIntMin>(fn, smem, per_sm);
@@ -38,7 +39,7 @@ cudaError_t light_kernel_t(uint32_t mode, const void **fn, size_t *smem, int *pe
 
 }  // namespace
 
-cudaError_t batch_light_kernel(bool aligned, uint32_t mode, const void **fn, size_t *smem,
+cudaError_t batch_light_kernel(bool aligned, uint32_t mode, const void **fn, size_t smem,
                                int *per_sm) {
     return aligned ? light_kernel_t<true>(mode, fn, smem, per_sm)
                    : light_kernel_t<false>(mode, fn, smem, per_sm);

@@ -9,6 +9,7 @@
 //   st[k][j] = leftmost minimum of blocks j .. j + 2^k - 1 (k = 0: block minima)
 #include "build_impl.cuh"
 #include "engine.h"
+#include "tables_impl.cuh"
 
 // CTAs per SM the unit kernel is compiled for (a register bound).
 #ifndef RMQ_BUILD_MINB
@@ -48,93 +49,18 @@ __global__ void st_level_kernel(Entry *st, uint32_t nb, uint32_t k) {
         if (rmq_chk(j + half < nb)) cur[j] = better(prev[j], prev[j + half]);
 }
 
-// Level k >= 1 of the micro table as offsets (micro_level_at).
-template <class O>
-__global__ void micro_level_kernel(const Entry *__restrict__ mst0, O *off, uint32_t nmicro,
-                                   uint32_t k) {
-    const uint32_t cnt = nmicro - (1u << k) + 1;
-    O *cur = off + static_cast<size_t>(k - 1) * nmicro;
-    const O *prev = off + static_cast<size_t>(k >= 2 ? k - 2 : 0) * nmicro;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt;
-         i += gridDim.x * blockDim.x)
-        micro_level_at(mst0, cur, prev, nmicro, k, i);
+constexpr int kTableThreads = 256;
+
+// The micro table (masks and offset rows) from the micro-block minima, one
+// tile of consecutive positions per CTA.
+__global__ void __launch_bounds__(kTableThreads)
+table_kernel(MicroTable T, uint32_t tile) {
+    extern __shared__ __align__(16) unsigned char s_tile[];
+    const uint32_t t0 = blockIdx.x * tile;
+    table_tile_global<kTableThreads>(T, t0, min(tile, T.nmicro - t0), s_tile);
 }
 
-// Sub-block level: 8 lanes per 32-element micro-block, 4 consecutive
-// elements per lane (one 16-byte load), 4 micro-blocks per warp. Each lane
-// scans its 4 elements both ways, then the 8 lanes of a micro-block scan
-// their totals with width-8 shuffles; results are written as two 16-byte
-// stores per lane and array, and the micro-block minimum (suffix minimum at
-// its first element) as level 0 of the micro table.
-template <uint32_t MODE>
-__global__ void __launch_bounds__(256)
-micro_scan_kernel(const float *__restrict__ A, uint32_t n, uint32_t nmicro, Entry *mpre,
-                  Entry *msuf, Entry *mst0, bool aligned) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t sub = lane & 7u;        // lane within its micro-block
-    const uint32_t grp = lane >> 3;        // micro-block within the warp
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w * 4u < nmicro;
-         w += warps) {
-        const uint32_t j = w * 4u + grp;
-        const uint32_t g0 = j * kMicro + sub * 4u;   // may pass n (then nothing is valid)
-        uint32_t b[4];
-        if (aligned && g0 + 3u < n) {
-            const uint4 f = ld_u4(A + g0);
-            b[0] = f.x;
-            b[1] = f.y;
-            b[2] = f.z;
-            b[3] = f.w;
-        } else {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) b[k] = (g0 + k < n) ? ld_u1(A + g0 + k) : 0u;
-        }
-        Entry p[4], q[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) p[k] = (g0 + k < n) ? make_entry(b[k], g0 + k, MODE) : kEntryNone;
-        q[3] = p[3];
-#pragma unroll
-        for (int k = 2; k >= 0; --k) q[k] = better(p[k], q[k + 1]);
-#pragma unroll
-        for (int k = 1; k < 4; ++k) p[k] = better(p[k - 1], p[k]);
-        // lane totals scanned across the 8 lanes of the micro-block
-        Entry ip = p[3], is = q[0];
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-            const Entry tp = __shfl_up_sync(0xffffffffu, ip, o, 8);
-            const Entry ts = __shfl_down_sync(0xffffffffu, is, o, 8);
-            if (sub >= static_cast<uint32_t>(o)) ip = better(ip, tp);
-            if (sub + o < 8u) is = better(is, ts);
-        }
-        Entry ep = __shfl_up_sync(0xffffffffu, ip, 1, 8);
-        Entry es = __shfl_down_sync(0xffffffffu, is, 1, 8);
-        if (sub == 0u) ep = kEntryNone;
-        if (sub == 7u) es = kEntryNone;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            p[k] = better(ep, p[k]);
-            q[k] = better(es, q[k]);
-        }
-        if (j < nmicro) {
-            if (g0 + 3u < n) {
-                __stcs(reinterpret_cast<ulonglong2 *>(mpre + g0), make_ulonglong2(p[0], p[1]));
-                __stcs(reinterpret_cast<ulonglong2 *>(mpre + g0 + 2), make_ulonglong2(p[2], p[3]));
-                __stcs(reinterpret_cast<ulonglong2 *>(msuf + g0), make_ulonglong2(q[0], q[1]));
-                __stcs(reinterpret_cast<ulonglong2 *>(msuf + g0 + 2), make_ulonglong2(q[2], q[3]));
-            } else {
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (g0 + k < n) {
-                        st_entry(mpre + g0 + k, p[k]);
-                        st_entry(msuf + g0 + k, q[k]);
-                    }
-            }
-            if (sub == 0u) mst0[j] = q[0];
-        }
-    }
-}
-
-// Light index, one pass over the values: the minimum of every 32-element
+// One pass over the values: the minimum of every 32-element
 // micro-block (level 0 of the micro table) and, folded in with a 64-bit
 // atomic minimum, of every block (level 0 of the block table, filled with
 // all-ones before; bs a multiple of 32, so every micro-block lies in one
@@ -201,28 +127,34 @@ cudaError_t launch_levels(Entry *st, uint32_t nb, uint32_t levels, const DeviceI
     return cudaSuccess;
 }
 
-template <class O>
-cudaError_t launch_micro_levels_w(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s) {
-    // bs <= n keeps every window inside the array (2^k <= nmicro); the
-    // bound is checked here as well
-    for (uint32_t k = 1; k < p.mlevels && (1u << k) <= p.nmicro; ++k) {
-        const uint32_t cnt = p.nmicro - (1u << k) + 1;
-        uint32_t g = (cnt + 255) / 256;
-        const uint32_t cap = static_cast<uint32_t>(dev.sms) * 8u;
-        if (g > cap) g = cap;
-        micro_level_kernel<O><<<g, 256, 0, s>>>(p.mst, static_cast<O *>(p.moff), p.nmicro, k);
-        cudaError_t err = cudaGetLastError();
-        if (err != cudaSuccess) return err;
-    }
-    return cudaSuccess;
+// Positions per table tile: 1024, 2048 where the halo is about as long (rows
+// up to level 9 and 10), 256 while a tile per SM is not to be had.
+uint32_t table_tile_size(const BuildPlan &p, const DeviceInfo &dev) {
+    if (p.mlevels >= 10) return 2048u;
+    return p.nmicro >= 1024u * static_cast<uint32_t>(dev.sms) ? 1024u : 256u;
 }
 
-cudaError_t launch_micro_levels(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s) {
-    switch (p.moff_bytes) {
-    case 1: return launch_micro_levels_w<uint8_t>(p, dev, s);
-    case 2: return launch_micro_levels_w<uint16_t>(p, dev, s);
-    default: return launch_micro_levels_w<uint32_t>(p, dev, s);
+cudaError_t launch_table(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s) {
+    MicroTable T;
+    T.mst = p.mst;
+    T.mask = p.mask;
+    T.moff = p.moff;
+    T.moff_bytes = p.moff_bytes;
+    T.nmicro = p.nmicro;
+    T.mlevels = p.mlevels;
+    const uint32_t tile = table_tile_size(p, dev);
+    const size_t smem = table_smem((tile + table_halo(p.mlevels) + 1u) & ~1u);
+    static std::atomic<bool> ready{false};
+    if (!ready.load(std::memory_order_relaxed)) {
+        // the largest tile: 2048 positions and a halo of 1023
+        const cudaError_t err = cudaFuncSetAttribute(
+            table_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            static_cast<int>(table_smem(2048u + 1024u)));
+        if (err != cudaSuccess) return err;
+        ready.store(true, std::memory_order_relaxed);
     }
+    table_kernel<<<(p.nmicro + tile - 1) / tile, kTableThreads, smem, s>>>(T, tile);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -232,30 +164,29 @@ uint32_t st_levels(uint32_t nb) { return nb ? static_cast<uint32_t>(ilog2(nb)) +
 namespace {
 size_t a256(size_t x) { return (x + 255) / 256 * 256; }
 struct Offsets {
-    size_t pre, suf, st, mst, moff, mpre, msuf, counter, total;
+    size_t pre, suf, st, mst, mask, moff, counter, total;
 };
 Offsets offsets_of(const BuildPlan &p) {
     Offsets o;
-    const size_t nent = p.light ? 0 : a256(sizeof(Entry) * static_cast<size_t>(p.n));
+    const size_t nent = p.micro ? 0 : a256(sizeof(Entry) * static_cast<size_t>(p.n));
     o.pre = 0;
     o.suf = nent;
     o.st = 2 * nent;
     o.mst = o.st + a256(sizeof(Entry) * static_cast<size_t>(p.nb) * p.levels);
-    o.moff = o.mst + (p.micro ? a256(sizeof(Entry) * static_cast<size_t>(p.nmicro)) : 0);
-    o.mpre = o.moff + (p.micro ? a256(static_cast<size_t>(p.moff_bytes) * p.nmicro *
-                                      (p.mlevels - 1)) : 0);
-    o.msuf = o.mpre + (p.micro ? nent : 0);
-    o.counter = o.msuf + (p.micro ? nent : 0);
+    o.mask = o.mst + a256(sizeof(Entry) * static_cast<size_t>(p.nmicro));
+    o.moff = o.mask + a256((wide_masks(p.nmicro) ? 8 : 4) * static_cast<size_t>(p.nmicro));
+    o.counter = o.moff + a256(static_cast<size_t>(p.moff_bytes) * p.nmicro * moff_rows(p.mlevels, wide_masks(p.nmicro)));
     o.total = o.counter + 256;
     return o;
 }
 }  // namespace
 
 size_t plan_index(BuildPlan &p, bool no_micro) {
-    p.nb = (p.n + p.bs - 1) / p.bs;
+    p.micro = !no_micro;
+    p.tbs = p.micro ? table_block(p.bs) : p.bs;
+    p.nb = (p.n + p.tbs - 1) / p.tbs;
     p.levels = st_levels(p.nb);
-    p.mlevels = no_micro ? 0u : micro_levels(p.bs);
-    p.micro = p.mlevels > 0;
+    p.mlevels = p.micro ? micro_levels(p.tbs) : 0u;
     p.nmicro = p.micro ? (p.n + kMicro - 1) / kMicro : 0u;
     p.moff_bytes = p.micro ? micro_offset_bytes(p.mlevels) : 0u;
     p.aligned = reinterpret_cast<uintptr_t>(p.A) % 16 == 0;
@@ -265,37 +196,50 @@ size_t plan_index(BuildPlan &p, bool no_micro) {
 unsigned long long *place_index(BuildPlan &p, void *base_v) {
     char *base = static_cast<char *>(base_v);
     const Offsets o = offsets_of(p);
-    p.pre = p.light ? nullptr : reinterpret_cast<Entry *>(base + o.pre);
-    p.suf = p.light ? nullptr : reinterpret_cast<Entry *>(base + o.suf);
+    p.pre = p.micro ? nullptr : reinterpret_cast<Entry *>(base + o.pre);
+    p.suf = p.micro ? nullptr : reinterpret_cast<Entry *>(base + o.suf);
     p.st = reinterpret_cast<Entry *>(base + o.st);
     p.mst = p.micro ? reinterpret_cast<Entry *>(base + o.mst) : nullptr;
+    p.mask = p.micro ? static_cast<void *>(base + o.mask) : nullptr;
     p.moff = p.micro ? static_cast<void *>(base + o.moff) : nullptr;
-    p.mpre = p.micro && !p.light ? reinterpret_cast<Entry *>(base + o.mpre) : nullptr;
-    p.msuf = p.micro && !p.light ? reinterpret_cast<Entry *>(base + o.msuf) : nullptr;
     return reinterpret_cast<unsigned long long *>(base + o.counter);
 }
 
-// The sub-block level works on 32-element micro-blocks aligned in the
-// array, whatever the block size. A query first probes the micro table over
-// every micro-block it touches (a superset of [l, r]; two windows of 2^k
-// micro-blocks cover up to 2^(k+1) - 1 of them), so the table holds windows
-// long enough for any query inside one block: a block touches bs/32
-// micro-blocks when blocks start on micro-block boundaries (bs a multiple
-// of 32), at most floor((bs + 30) / 32) + 1 otherwise.
+size_t layout_v5(uint32_t n, uint32_t bs, bool light, bool no_micro, LayoutV5 *out) {
+    out->nb = (n + bs - 1) / bs;
+    out->levels = st_levels(out->nb);
+    out->mlevels = no_micro ? 0u : micro_levels(bs);
+    out->nmicro = out->mlevels ? (n + kMicro - 1) / kMicro : 0u;
+    const size_t nent = light ? 0 : a256(sizeof(Entry) * static_cast<size_t>(n));
+    size_t total = 2 * nent + a256(sizeof(Entry) * static_cast<size_t>(out->nb) * out->levels) + 256;
+    if (out->mlevels)
+        total += a256(sizeof(Entry) * static_cast<size_t>(out->nmicro)) + 2 * nent +
+                 a256(static_cast<size_t>(micro_offset_bytes(out->mlevels)) * out->nmicro *
+                      (out->mlevels - 1));
+    return total;
+}
+
+// The micro table works on 32-element micro-blocks aligned in the array,
+// whatever the block size. A query first probes it over every micro-block it
+// touches (a superset of [l, r]; two windows of 2^k micro-blocks cover up to
+// 2^(k+1) - 1 of them), so it holds windows long enough for any query inside
+// one block: a block touches bs/32 micro-blocks when blocks start on
+// micro-block boundaries (bs a multiple of 32, as in every table index), at
+// most floor((bs + 30) / 32) + 1 otherwise.
 uint32_t micro_levels(uint32_t bs) {
     if (bs < 2 * kMicro) return 0;
     const uint32_t touched = (bs % kMicro == 0) ? bs / kMicro : (bs + kMicro - 2) / kMicro + 1;
     return st_levels(touched);
 }
 
-cudaError_t launch_build_light(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s) {
+static cudaError_t launch_build_tables(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s) {
     cudaError_t err = cudaMemsetAsync(p.st, 0xff, sizeof(Entry) * static_cast<size_t>(p.nb), s);
     if (err != cudaSuccess) return err;
     // 8 warps per CTA, kMicroPerWarp micro-blocks per warp step
     uint32_t g = (p.nmicro + 8 * kMicroPerWarp - 1) / (8 * kMicroPerWarp);
     const uint32_t cap = static_cast<uint32_t>(dev.sms) * 8u;
     if (g > cap) g = cap;
-    const uint32_t per_block = p.bs / kMicro;
+    const uint32_t per_block = p.tbs / kMicro;
     switch (p.kmode) {
     case kFloatMax:
         micro_min_kernel<kFloatMax><<<g, 256, 0, s>>>(p.A, p.n, p.nmicro, per_block, p.mst, p.st,
@@ -318,26 +262,25 @@ cudaError_t launch_build_light(const BuildPlan &p, const DeviceInfo &dev, cudaSt
     if (err != cudaSuccess) return err;
     err = launch_levels(p.st, p.nb, p.levels, dev, s);
     if (err != cudaSuccess) return err;
-    return launch_micro_levels(p, dev, s);
+    return launch_table(p, dev, s);
 }
 
-cudaError_t launch_build(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s) {
-    if (p.n == 0) return cudaSuccess;
-    if (p.light) return launch_build_light(p, dev, s);
+cudaError_t launch_build_entries(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s) {
     UnitJob J;
     J.A = p.A;
     J.off = 0;
     J.limit = p.n;
     J.n = p.n;
     J.bs = p.bs;
-    J.U = make_unit_layout(p.bs, p.nb);
+    const uint32_t nb = (p.n + p.bs - 1) / p.bs;
+    J.U = make_unit_layout(p.bs, nb);
     J.dv = make_div31(p.bs);
     J.pre = p.pre;
     J.suf = p.suf;
     J.bmin = p.st;
     J.kmode = p.kmode;
-    J.nb = p.nb;
-    const uint32_t nunits = unit_count(p.nb, J.U);
+    J.nb = nb;
+    const uint32_t nunits = unit_count(nb, J.U);
 
     // every key mode compiles to the same resources; the float-min
     // instantiation stands for all four
@@ -355,35 +298,15 @@ cudaError_t launch_build(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t
         launch_units<true>(J, nunits, grid, s);
     else
         launch_units<false>(J, nunits, grid, s);
-    err = cudaGetLastError();
-    if (err != cudaSuccess) return err;
-    err = launch_levels(p.st, p.nb, p.levels, dev, s);
-    if (err != cudaSuccess || !p.micro) return err;
+    return cudaGetLastError();
+}
 
-    uint32_t g = (p.nmicro + 31) / 32;  // 8 warps per CTA, 4 micro-blocks per warp
-    const uint32_t cap = static_cast<uint32_t>(dev.sms) * 8u;
-    if (g > cap) g = cap;
-    switch (p.kmode) {
-    case kFloatMax:
-        micro_scan_kernel<kFloatMax><<<g, 256, 0, s>>>(p.A, p.n, p.nmicro, p.mpre, p.msuf, p.mst,
-                                                       p.aligned);
-        break;
-    case kIntMin:
-        micro_scan_kernel<kIntMin><<<g, 256, 0, s>>>(p.A, p.n, p.nmicro, p.mpre, p.msuf, p.mst,
-                                                     p.aligned);
-        break;
-    case kIntMax:
-        micro_scan_kernel<kIntMax><<<g, 256, 0, s>>>(p.A, p.n, p.nmicro, p.mpre, p.msuf, p.mst,
-                                                     p.aligned);
-        break;
-    default:
-        micro_scan_kernel<kFloatMin><<<g, 256, 0, s>>>(p.A, p.n, p.nmicro, p.mpre, p.msuf, p.mst,
-                                                       p.aligned);
-        break;
-    }
-    err = cudaGetLastError();
+cudaError_t launch_build(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s) {
+    if (p.n == 0) return cudaSuccess;
+    if (p.micro) return launch_build_tables(p, dev, s);
+    const cudaError_t err = launch_build_entries(p, dev, s);
     if (err != cudaSuccess) return err;
-    return launch_micro_levels(p, dev, s);
+    return launch_levels(p.st, p.nb, p.levels, dev, s);
 }
 
 RMQ_VIOLATIONS_READER(violations_build)

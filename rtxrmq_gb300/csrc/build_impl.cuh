@@ -735,7 +735,7 @@ __device__ __forceinline__ void build_unit(const UnitJob &J, uint32_t u, Entry *
     }
 }
 
-// ---- light index: micro-block minima and the micro table's levels ----
+// ---- table index: micro-block minima ----
 
 constexpr uint32_t kMicroElems = 32;    // elements per micro-block
 constexpr uint32_t kMicroPerWarp = 16;  // micro-blocks a warp reduces per step
@@ -763,26 +763,6 @@ __device__ __forceinline__ Entry micro_row_min(const uint32_t (&b)[4], uint32_t 
     if (!FULL && base >= n) return kEntryNone;
     const uint32_t idx = base + 4u * w + (winfo & 3u);
     return (static_cast<uint64_t>(gk) << 32) | (idx << 1) | (winfo >> 2);
-}
-
-// One offset of level k >= 1 of the micro table (as offsets): the window of
-// 2^k micro-blocks at i is the windows of 2^(k-1) at i and i + 2^(k-1); each
-// half's best micro-block comes from the level below (`prev`, level k - 1;
-// level 0 = the minima themselves), the better of the two is kept as its
-// offset from i in `cur`. Unsigned comparison of composites keeps the
-// leftmost of equal minima.
-template <class O>
-__device__ __forceinline__ void micro_level_at(const Entry *__restrict__ mst0, O *cur,
-                                               const O *prev, uint32_t nmicro, uint32_t k,
-                                               uint32_t i) {
-    const uint32_t half = 1u << (k - 1);
-    uint32_t a = i, b = i + half;
-    if (k >= 2) {
-        a += prev[i];
-        b += prev[i + half];
-    }
-    if (rmq_chk(a < nmicro && b < nmicro && a - i < half && b - i < 2 * half))
-        cur[i] = static_cast<O>((mst0[b] < mst0[a] ? b : a) - i);
 }
 
 // Micro-block minima of micro-blocks [j0, j0 + 16) of one array (values

@@ -137,11 +137,12 @@ __device__ __forceinline__ bool rmq_chk(bool) { return true; }
 // With e = m*d - 2^(31+s) < d <= 2^s and x < 2^31 the error term
 // x*e / (d * 2^(31+s)) stays below 1/d, so the floor is exact
 // (Granlund & Montgomery, PLDI 1994, round-up variant).
+// For d = 2^s, s >= 1, m = 2^(32 - s) and no shift give the same.
 struct Div31 {
     uint32_t d;
-    uint32_t m;      // multiplier (unused for powers of two)
-    uint32_t shift;  // s - 1 after the high multiply, or log2 d for pow2
-    uint32_t pow2;
+    uint32_t m;      // multiplier (unused for d == 1)
+    uint32_t shift;  // after the high multiply
+    uint32_t one;    // d == 1
 };
 
 inline Div31 make_div31(uint32_t d) {
@@ -150,11 +151,11 @@ inline Div31 make_div31(uint32_t d) {
     uint32_t s = 0;
     while ((1ull << s) < d) ++s;
     if ((1u << s) == d) {
-        r.pow2 = 1;
-        r.m = 0;
-        r.shift = s;
+        r.one = d == 1;
+        r.m = d == 1 ? 0u : 1u << (32 - s);
+        r.shift = 0;
     } else {
-        r.pow2 = 0;
+        r.one = 0;
         const uint64_t num = 1ull << (31 + s);
         r.m = static_cast<uint32_t>((num + d - 1) / d);
         r.shift = s - 1;
@@ -162,14 +163,16 @@ inline Div31 make_div31(uint32_t d) {
     return r;
 }
 
-RMQ_HD uint32_t div31(uint32_t x, const Div31 &D) {
-    if (D.pow2) return x >> D.shift;
+// d >= 2 (every block of a table index): no branch
+RMQ_HD uint32_t div31_ge2(uint32_t x, const Div31 &D) {
 #ifdef __CUDA_ARCH__
     return __umulhi(x, D.m) >> D.shift;
 #else
     return static_cast<uint32_t>((static_cast<uint64_t>(x) * D.m) >> 32) >> D.shift;
 #endif
 }
+
+RMQ_HD uint32_t div31(uint32_t x, const Div31 &D) { return D.one ? x : div31_ge2(x, D); }
 
 // floor(log2 x) for x >= 1
 RMQ_HD int ilog2(uint32_t x) {

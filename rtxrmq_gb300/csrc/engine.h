@@ -77,44 +77,50 @@ unsigned long long violations_persist();
 struct BuildPlan {
     const float *A;
     uint32_t n;
-    uint32_t bs;
-    uint32_t nb;
-    uint32_t levels;
+    uint32_t bs;      // block size asked for
     bool aligned;
-    Entry *pre;   // [n]
-    Entry *suf;   // [n]
-    Entry *st;    // [levels * nb], level 0 = block minima
-    // sub-block level (every bs >= 64): minima of the 32-element
-    // micro-blocks and a sparse table over them truncated to the window
-    // lengths a same-block query can need. Level 0 holds the micro-block
-    // minima as entries; level k >= 1 holds, for the window of 2^k
-    // micro-blocks starting at j, the offset (< 2^k) of its leftmost best
-    // micro-block in moff_bytes = 1, 2 or 4 bytes: 1/8 to 1/2 of the bytes
-    // of entries, so that the table stays in L2
+    uint32_t kmode;   // KeyMode: float32 / int32 elements, minimum / maximum
+    // the table index (every index but RMQ_BUILD_NO_MICRO ones): minima of
+    // the 32-element micro-blocks, the micro table over them (masks and
+    // offset rows, tables_impl.cuh) and a sparse table over the minima of
+    // blocks of tbs elements. Without it: pre / suf per element and the
+    // sparse table over blocks of bs (tbs == bs)
     bool micro;
-    uint32_t nmicro;   // ceil(n / 32)
+    bool light;       // RMQ_BUILD_LIGHT was given (reported, same structure)
+    uint32_t tbs;
+    uint32_t nb;      // blocks of tbs elements
+    uint32_t levels;
+    Entry *st;        // [levels * nb], level 0 = block minima
+    uint32_t nmicro;  // ceil(n / 32)
     uint32_t mlevels;
-    Entry *mst;        // [nmicro] micro-block minima (table level 0)
-    void *moff;        // [(mlevels - 1) * nmicro] offsets of levels 1 ..
     uint32_t moff_bytes;
-    Entry *mpre;       // [n] leftmost minimum of A[microstart(i) .. i]
-    Entry *msuf;       // [n] leftmost minimum of A[i .. microend(i)]
-    uint32_t kmode;    // KeyMode: float32 / int32 elements, minimum / maximum
-    // light index (RMQ_BUILD_LIGHT): the tables only, no per-element entries
-    // (pre, suf, mpre, msuf are null); needs the sub-block level and blocks
-    // on micro-block boundaries (bs a multiple of 32)
-    bool light;
+    Entry *mst;       // [nmicro] micro-block minima
+    void *mask;       // [nmicro] (tables_impl.cuh)
+    void *moff;       // [moff_rows * nmicro]
+    Entry *pre;       // [n]
+    Entry *suf;       // [n]
 };
 constexpr uint32_t kMicro = 32;
-// levels of the micro table for block size bs (0 when not applicable)
+// levels of a micro table that answers every query inside one block of bs
+// elements (0 below 64)
 uint32_t micro_levels(uint32_t bs);
 // bytes of one micro-table offset for a table of `mlevels` levels: the
 // largest offset is 2^(mlevels - 1) - 1
 inline uint32_t micro_offset_bytes(uint32_t mlevels) {
     return mlevels <= 9 ? 1u : (mlevels <= 17 ? 2u : 4u);
 }
+// Block size of the block table of a table index asked for with block size
+// bs. Multiples of 32 (blocks hold whole micro-blocks), at least 64. Above
+// 2^15 the micro table would be 13 rows and more of 2-byte offsets, too large
+// for L2 and read twice per query: queries inside such blocks go through
+// blocks of 4096 instead (n = 1e8, 2^26 queries, lr=-2, bs 195312: 0.83 ms
+// with the rows, 0.48 with blocks of 4096).
+inline uint32_t table_block(uint32_t bs) {
+    if (bs > (1u << 15)) return 4096u;
+    return bs <= 64u ? 64u : (bs + 31u) / 32u * 32u;
+}
 
-// Fill the size fields of a plan (A, n, bs and light given; micro level on
+// Fill the size fields of a plan (A, n, bs and light given; the table index
 // unless `no_micro`); returns the bytes of the single allocation holding the
 // index and its invalid-query counter.
 size_t plan_index(BuildPlan &p, bool no_micro);
@@ -122,6 +128,15 @@ size_t plan_index(BuildPlan &p, bool no_micro);
 unsigned long long *place_index(BuildPlan &p, void *base);
 uint32_t st_levels(uint32_t nb);
 cudaError_t launch_build(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s);
+// Per-element prefix / suffix minima over blocks of p.bs elements into p.pre
+// and p.suf, block minima into p.st[0 .. ceil(n / bs)).
+cudaError_t launch_build_entries(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s);
+// Size fields of index files of version 5, whose full indexes held four
+// entries per element; returns the bytes of their payload.
+struct LayoutV5 {
+    uint32_t nb, levels, nmicro, mlevels;
+};
+size_t layout_v5(uint32_t n, uint32_t bs, bool light, bool no_micro, LayoutV5 *out);
 
 // ---- handles (api.cu) ----
 }  // namespace rmq

@@ -121,9 +121,13 @@ extern "C" int rmq_query_noalloc(const float *d_vals, int64_t n, int64_t bs,
     p.A = d_vals;
     p.n = static_cast<uint32_t>(n);
     p.bs = static_cast<uint32_t>(bs);
-    // the sub-block level when it fits, otherwise the plain index (same results)
-    size_t need = plan_index(p, false);
-    if (need > kNoallocScratchBytes) need = plan_index(p, true);
+    // the sizes accepted are those of a full index with four entries per
+    // element, or two without the sub-block level; the table index built
+    // below is smaller than either
+    LayoutV5 full;
+    size_t need = layout_v5(p.n, p.bs, false, false, &full);
+    if (need > kNoallocScratchBytes) need = layout_v5(p.n, p.bs, false, true, &full);
+    if (need <= kNoallocScratchBytes) need = plan_index(p, false);
     if (need > kNoallocScratchBytes)
         return set_error(RMQ_EINVAL,
                          "rmq_query_noalloc: n=%lld with bs=%lld needs %zu bytes of scratch; the "

@@ -21,8 +21,13 @@ namespace {
 constexpr char kMagic[16] = "RTXRMQ-GB300-IX";
 // 2: entries are comparison composites; 3: sub-block level for every
 // bs >= 64; 4: micro-table levels 1.. stored as offsets; 5: micro table
-// deep enough for every micro-block a block touches, light indexes
-constexpr uint32_t kVersion = 5;
+// deep enough for every micro-block a block touches, light indexes; 6: table
+// indexes hold no per-element entries, micro table as masks and offset rows.
+// Files of version 5 are read too: their layout is checked, their payload
+// (whose tables are laid out otherwise) skipped, and the index is built from
+// the values.
+constexpr uint32_t kVersion = 6;
+constexpr uint32_t kVersionRebuilt = 5;
 constexpr size_t kIoChunk = size_t(64) << 20;
 
 struct FileHeader {
@@ -171,7 +176,7 @@ int rmq_load(const float *d_vals, int64_t n, const char *path, rmq_stream_t stre
     if (!fp) return set_error(RMQ_EINVAL, "rmq_load: cannot open %s", path);
     FileHeader hd;
     if (std::fread(&hd, sizeof(hd), 1, fp) != 1 || std::memcmp(hd.magic, kMagic, sizeof(kMagic)) ||
-        hd.version != kVersion || hd.header_check != header_hash(hd)) {
+        (hd.version != kVersion && hd.version != kVersionRebuilt) || hd.header_check != header_hash(hd)) {
         std::fclose(fp);
         return set_error(RMQ_EINVAL, "rmq_load: %s is not an index file of this version", path);
     }
@@ -189,10 +194,14 @@ int rmq_load(const float *d_vals, int64_t n, const char *path, rmq_stream_t stre
     p.light = (hd.flags & RMQ_BUILD_LIGHT) != 0;
     // a light index may round a block size above n up to a multiple of 32
     const uint64_t bs_max = p.light ? (hd.n + 31) / 32 * 32 : hd.n;
-    const size_t bytes = (hd.bs >= 1 && hd.bs <= bs_max)
-                             ? plan_index(p, (hd.flags & RMQ_BUILD_NO_MICRO) != 0) : 0;
-    if (!bytes || bytes != hd.bytes || p.nb != hd.nb || p.levels != hd.levels ||
-        p.nmicro != hd.nmicro || p.mlevels != hd.mlevels) {
+    const bool old = hd.version == kVersionRebuilt;
+    const bool no_micro = (hd.flags & RMQ_BUILD_NO_MICRO) != 0;
+    const bool bs_ok = hd.bs >= 1 && hd.bs <= bs_max;
+    const size_t bytes = bs_ok ? plan_index(p, no_micro) : 0;
+    LayoutV5 v5{p.nb, p.levels, p.nmicro, p.mlevels};
+    const size_t payload = bs_ok && old ? layout_v5(p.n, p.bs, p.light, no_micro, &v5) : bytes;
+    if (!bytes || payload != hd.bytes || v5.nb != hd.nb || v5.levels != hd.levels ||
+        v5.nmicro != hd.nmicro || v5.mlevels != hd.mlevels) {
         std::fclose(fp);
         return set_error(RMQ_EINVAL, "rmq_load: %s has an inconsistent layout", path);
     }
@@ -216,19 +225,20 @@ int rmq_load(const float *d_vals, int64_t n, const char *path, rmq_stream_t stre
     }
     std::vector<char> buf;
     try {
-        buf.resize(bytes < kIoChunk ? bytes : kIoChunk);
+        buf.resize(payload < kIoChunk ? payload : kIoChunk);
     } catch (...) {
         std::fclose(fp);
         cudaFree(mem);
         return set_error(RMQ_ENOMEM, "rmq_load: host buffer");
     }
-    for (size_t off = 0; off < bytes; off += buf.size()) {
-        const size_t m = bytes - off < buf.size() ? bytes - off : buf.size();
+    for (size_t off = 0; off < payload; off += buf.size()) {
+        const size_t m = payload - off < buf.size() ? payload - off : buf.size();
         if (std::fread(buf.data(), 1, m, fp) != m) {
             std::fclose(fp);
             cudaFree(mem);
             return set_error(RMQ_EINVAL, "rmq_load: %s is truncated", path);
         }
+        if (old) continue;
         err = cudaMemcpyAsync(static_cast<char *>(mem) + off, buf.data(), m,
                               cudaMemcpyHostToDevice, stream);
         if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
@@ -239,6 +249,20 @@ int rmq_load(const float *d_vals, int64_t n, const char *path, rmq_stream_t stre
         }
     }
     std::fclose(fp);
+    if (old) {
+        DeviceInfo dev;
+        rc = device_info(&dev);
+        if (rc == RMQ_OK) {
+            place_index(p, mem);
+            err = launch_build(p, dev, stream);
+            if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
+            if (err != cudaSuccess) rc = cuda_fail(err, "rmq_load: build");
+        }
+        if (rc) {
+            cudaFree(mem);
+            return rc;
+        }
+    }
     rc = handle_adopt(p, mem, bytes, stream, out);
     if (rc) cudaFree(mem);
     return rc;

@@ -38,10 +38,10 @@ __device__ __forceinline__ void load_full(const QueryOut &o, int64_t base, int2 
 // key mode and on whether the index has the sub-block level. STATS: the
 // measurement instantiation (rmq_query_stats), which also counts how each
 // query was settled and what it read into stats[kStatCount].
-template <bool ALIGNED, bool MICRO, bool LIGHT, uint32_t MODE, bool STATS>
+template <bool ALIGNED, bool MICRO, uint32_t MODE, bool STATS>
 __global__ void __launch_bounds__(kThreads, RMQ_QUERY_MINB)
 query_kernel(V1View v, QueryOut o, int64_t q, unsigned long long *stats) {
-    __shared__ MissQueue<kQPT> s_mq[kThreads / 32];
+    __shared__ __align__(128) MissQueue<MICRO> s_mq[kThreads / 32];
     constexpr int64_t chunk = static_cast<int64_t>(kThreads) * kQPT;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * chunk;
     int64_t c0 = static_cast<int64_t>(blockIdx.x) * chunk;
@@ -50,7 +50,7 @@ query_kernel(V1View v, QueryOut o, int64_t q, unsigned long long *stats) {
     QStats s;
     if constexpr (STATS)
         for (int c = 0; c < kStatCount; ++c) s.c[c] = 0u;
-    MissQueue<kQPT> &mq = s_mq[threadIdx.x >> 5];
+    MissQueue<MICRO> &mq = s_mq[threadIdx.x >> 5];
     uint32_t waiting = 0;  // the warp's queue length (warp-uniform)
     int2 cur[kQPT];
     if (c0 <= last_full)
@@ -65,17 +65,8 @@ query_kernel(V1View v, QueryOut o, int64_t q, unsigned long long *stats) {
             load_full(o, c1, nxt);
         else if (c1 < q)
             load_queries<kQPT>(o, c1, q, nxt);
-        if (c0 <= last_full)
-            answer_step_queued<ALIGNED, MICRO, LIGHT, MODE, kThreads, kQPT, STATS, true>(
-                v, o, c0, static_cast<uint32_t>(chunk), id0, cur, s, mq, waiting);
-        else
-            answer_step_queued<ALIGNED, MICRO, LIGHT, MODE, kThreads, kQPT, STATS, false>(
-                v, o, c0, static_cast<uint32_t>(q - c0), id0, cur, s, mq, waiting);
-        // one site for the drain: its code is large, and every copy of it
-        // costs instruction fetches
-        while (waiting >= (c1 >= q ? 1u : 32u))
-            drain_misses<ALIGNED, MICRO, LIGHT, MODE, STATS, kThreads, kQPT>(
-                v, o, map, mq, waiting, l2_keep_policy(), s);
+        answer_step_queued<ALIGNED, MICRO, MODE, kThreads, kQPT, STATS>(
+            v, o, map, c0, static_cast<uint32_t>(min(chunk, q - c0)), id0, c1 >= q, cur, s, mq, waiting);
 #pragma unroll
         for (int k = 0; k < kQPT; ++k) cur[k] = nxt[k];
     }
@@ -197,30 +188,31 @@ V1View view_of(const BuildPlan &p) {
     v.off = 0;
     v.limit = p.n;
     v.n = p.n;
-    v.bs = p.bs;
+    v.bs = p.tbs;
     v.nb = p.nb;
-    v.dv = make_div31(p.bs);
+    v.dv = make_div31(p.tbs);
+    v.st = p.st;
+    v.mst = p.mst;
+    v.mask = p.mask;
+    v.wide = wide_masks(p.nmicro);
+    v.moff = p.moff;
+    v.moff_bytes = p.moff_bytes;
+    v.nmicro = p.nmicro;
     v.pre = p.pre;
     v.suf = p.suf;
-    v.st = p.st;
-    v.mst = p.micro ? p.mst : nullptr;
-    v.moff = p.micro ? p.moff : nullptr;
-    v.moff_bytes = p.micro ? p.moff_bytes : 0u;
-    v.nmicro = p.micro ? p.nmicro : 0u;
-    v.mpre = p.micro ? p.mpre : nullptr;
-    v.msuf = p.micro ? p.msuf : nullptr;
     v.kmode = p.kmode;
     v.levels = p.levels;
-    v.mlevels = p.micro ? p.mlevels : 0u;
+    v.mlevels = p.mlevels;
     v.micro_span = p.micro ? (1u << p.mlevels) - 1u : 0u;
+    v.light = p.light;
     return v;
 }
 
-template <bool ALIGNED, bool MICRO, bool LIGHT, uint32_t MODE, bool STATS>
+template <bool ALIGNED, bool MICRO, uint32_t MODE, bool STATS>
 cudaError_t launch_query_t(const V1View &v, const QueryOut &o, int64_t q,
                            unsigned long long *stats, const DeviceInfo &dev, cudaStream_t s) {
     static std::atomic<int> per_sm_cache{0};
-    auto kern = query_kernel<ALIGNED, MICRO, LIGHT, MODE, STATS>;
+    auto kern = query_kernel<ALIGNED, MICRO, MODE, STATS>;
     int per_sm = per_sm_cache.load(std::memory_order_relaxed);
     if (per_sm == 0) {
         cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, 0);
@@ -231,7 +223,7 @@ cudaError_t launch_query_t(const V1View &v, const QueryOut &o, int64_t q,
         // default split gives 100 KB for the 41 KB used (lr=-2, bs 4096,
         // n = 1e8: 0.52 ms, with this 0.48).
         err = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                   carveout_percent(per_sm * (sizeof(MissQueue<kQPT>) * (kThreads / 32) + 1024)));
+                                   carveout_percent(per_sm * (sizeof(MissQueue<MICRO>) * (kThreads / 32) + 1024)));
         if (err != cudaSuccess) return err;
         per_sm_cache.store(per_sm, std::memory_order_relaxed);
     }
@@ -239,29 +231,25 @@ cudaError_t launch_query_t(const V1View &v, const QueryOut &o, int64_t q,
     return cudaGetLastError();
 }
 
-template <bool ALIGNED, bool MICRO, bool LIGHT, bool STATS>
+template <bool ALIGNED, bool MICRO, bool STATS>
 cudaError_t launch_query_m(const V1View &v, const QueryOut &o, int64_t q,
                            unsigned long long *stats, const DeviceInfo &dev, cudaStream_t s) {
     switch (v.kmode) {
-    case kFloatMax: return launch_query_t<ALIGNED, MICRO, LIGHT, kFloatMax, STATS>(v, o, q, stats, dev, s);
-    case kIntMin: return launch_query_t<ALIGNED, MICRO, LIGHT, kIntMin, STATS>(v, o, q, stats, dev, s);
-    case kIntMax: return launch_query_t<ALIGNED, MICRO, LIGHT, kIntMax, STATS>(v, o, q, stats, dev, s);
-    default: return launch_query_t<ALIGNED, MICRO, LIGHT, kFloatMin, STATS>(v, o, q, stats, dev, s);
+    case kFloatMax: return launch_query_t<ALIGNED, MICRO, kFloatMax, STATS>(v, o, q, stats, dev, s);
+    case kIntMin: return launch_query_t<ALIGNED, MICRO, kIntMin, STATS>(v, o, q, stats, dev, s);
+    case kIntMax: return launch_query_t<ALIGNED, MICRO, kIntMax, STATS>(v, o, q, stats, dev, s);
+    default: return launch_query_t<ALIGNED, MICRO, kFloatMin, STATS>(v, o, q, stats, dev, s);
     }
 }
 
 template <bool STATS>
 cudaError_t launch_query_s(const BuildPlan &p, const V1View &v, const QueryOut &o, int64_t q,
                            unsigned long long *stats, const DeviceInfo &dev, cudaStream_t s) {
-    const bool micro = v.mst != nullptr;
-    if (micro && p.light)
-        return p.aligned ? launch_query_m<true, true, true, STATS>(v, o, q, stats, dev, s)
-                         : launch_query_m<false, true, true, STATS>(v, o, q, stats, dev, s);
     if (p.aligned)
-        return micro ? launch_query_m<true, true, false, STATS>(v, o, q, stats, dev, s)
-                     : launch_query_m<true, false, false, STATS>(v, o, q, stats, dev, s);
-    return micro ? launch_query_m<false, true, false, STATS>(v, o, q, stats, dev, s)
-                 : launch_query_m<false, false, false, STATS>(v, o, q, stats, dev, s);
+        return p.micro ? launch_query_m<true, true, STATS>(v, o, q, stats, dev, s)
+                       : launch_query_m<true, false, STATS>(v, o, q, stats, dev, s);
+    return p.micro ? launch_query_m<false, true, STATS>(v, o, q, stats, dev, s)
+                   : launch_query_m<false, false, STATS>(v, o, q, stats, dev, s);
 }
 
 cudaError_t launch_query(const BuildPlan &p, const QueryArgs &a, const DeviceInfo &dev,

@@ -30,6 +30,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "tables_impl.cuh"
 
 namespace rmq {
 
@@ -43,21 +44,23 @@ struct V1View {
     uint32_t bs;
     uint32_t nb;
     Div31 dv;
-    const Entry *pre;
-    const Entry *suf;
     const Entry *st;
-    // sub-block level: 32-element micro-blocks (local index / 32), whatever
-    // the block size; null when the index has none (same-block queries then
-    // use the warp-cooperative scan)
-    const Entry *mst;   // micro-block minima (micro-table level 0)
-    const void *moff;   // levels 1..: offsets of each window's best micro-block
+    // table index: 32-element micro-blocks (local index / 32) and the micro
+    // table over their minima (tables_impl.cuh); blocks hold whole
+    // micro-blocks. Null when the index has none: per-element entries then
+    // (same-block queries use the warp-cooperative scan)
+    const Entry *mst;      // micro-block minima
+    const void *mask;
+    bool wide;             // 64-bit masks, else 32-bit
+    const void *moff;
     uint32_t moff_bytes;
     uint32_t nmicro;
-    const Entry *mpre;  // in-micro-block prefix / suffix minima
-    const Entry *msuf;
+    const Entry *pre;
+    const Entry *suf;
     uint32_t kmode;     // KeyMode: element type and minimum / maximum
     uint32_t levels;    // sparse-table levels (st holds levels * nb entries)
-    uint32_t mlevels;   // micro-table levels (moff holds mlevels - 1 rows of nmicro)
+    uint32_t mlevels;   // micro-table levels (moff holds moff_rows(mlevels) rows of nmicro)
+    bool light;         // counting launches: how the end parts are counted
     // 2^mlevels - 1: a query whose end micro-blocks ml < mr have
     // mr - ml < micro_span is probed through the micro table (0: no micro level)
     uint32_t micro_span;
@@ -73,14 +76,6 @@ __device__ __forceinline__ uint4 ld_elem4(const V1View &v, int64_t g) {
 }
 __device__ __forceinline__ Entry ld_entry(const Entry *t, uint64_t i, uint64_t size) {
     return rmq_chk(i < size) ? t[i] : kEntryNone;
-}
-
-// The same, as a streaming load (evict-first in L1 and L2), for the random
-// per-element sub-block entries: they are read once, and the micro table
-// they would otherwise evict is read by every same-block query.
-__device__ __forceinline__ Entry ld_entry_cs(const Entry *t, uint64_t i, uint64_t size) {
-    return rmq_chk(i < size) ? __ldcs(reinterpret_cast<const unsigned long long *>(t) + i)
-                             : kEntryNone;
 }
 
 // The small tables every query probes (the sparse table over block minima,
@@ -101,32 +96,30 @@ __device__ __forceinline__ Entry ld_entry_keep(const Entry *t, uint64_t i, uint6
     return v;
 }
 
-// Offset i of the micro table's levels 1.. (moff_bytes wide, the same for
-// every query of an index, so the branch does not diverge).
+// Mask of micro-block j, and offset i of the micro table's rows. Width is the
+// same for every query of an index, so the branches on it do not diverge.
+__device__ __forceinline__ uint64_t ld_mask(const V1View &v, uint32_t j, uint64_t pol) {
+    if (!rmq_chk(j < v.nmicro)) return 1u;
+    if (v.wide) {
+        unsigned long long r;
+        asm volatile("ld.global.L2::cache_hint.u64 %0, [%1], %2;"
+                     : "=l"(r) : "l"(static_cast<const uint64_t *>(v.mask) + j), "l"(pol));
+        return r;
+    }
+    uint32_t r;
+    asm volatile("ld.global.L2::cache_hint.u32 %0, [%1], %2;"
+                 : "=r"(r) : "l"(static_cast<const uint32_t *>(v.mask) + j), "l"(pol));
+    return r;
+}
 __device__ __forceinline__ uint32_t ld_moff(const V1View &v, uint64_t i, uint64_t pol) {
-    if (!rmq_chk(i < static_cast<uint64_t>(v.mlevels - 1u) * v.nmicro)) return 0u;
+    if (!rmq_chk(i < static_cast<uint64_t>(moff_rows(v.mlevels, v.wide)) * v.nmicro)) return 0u;
     uint32_t r;
     if (v.moff_bytes == 1u)
         asm volatile("ld.global.L2::cache_hint.u8 %0, [%1], %2;"
                      : "=r"(r) : "l"(static_cast<const uint8_t *>(v.moff) + i), "l"(pol));
-    else if (v.moff_bytes == 2u)
+    else
         asm volatile("ld.global.L2::cache_hint.u16 %0, [%1], %2;"
                      : "=r"(r) : "l"(static_cast<const uint16_t *>(v.moff) + i), "l"(pol));
-    else
-        asm volatile("ld.global.L2::cache_hint.u32 %0, [%1], %2;"
-                     : "=r"(r) : "l"(static_cast<const uint32_t *>(v.moff) + i), "l"(pol));
-    return r;
-}
-
-// The aligned 8-byte word of the 1-byte micro-table offsets that holds
-// offset i (the table starts 256-byte aligned; its tail is padded to 256
-// bytes, so the word never passes the allocation).
-__device__ __forceinline__ uint64_t ld_moff_word(const V1View &v, uint64_t i, uint64_t pol) {
-    const uint64_t w = i >> 3;
-    if (!rmq_chk(w < (static_cast<uint64_t>(v.mlevels - 1u) * v.nmicro + 7) / 8)) return 0u;
-    uint64_t r;
-    asm volatile("ld.global.L2::cache_hint.u64 %0, [%1], %2;"
-                 : "=l"(r) : "l"(static_cast<const uint64_t *>(v.moff) + w), "l"(pol));
     return r;
 }
 
@@ -205,14 +198,14 @@ __device__ __forceinline__ Entry warp_scan_range(const V1View &v, uint32_t l, ui
 // Queries base + threadIdx.x + k * blockDim.x (k < QPT) of [.., q1), loaded
 // ahead of use (the query stream may come from host memory over the host
 // link, so a caller can issue the next step's loads before answering the
-// current step).
+// current step). A query past q1 is an invalid one.
 template <int QPT>
 __device__ __forceinline__ void load_queries(const QueryOut &o, int64_t base, int64_t q1,
                                              int2 (&qq)[QPT]) {
 #pragma unroll
     for (int k = 0; k < QPT; ++k) {
         const int64_t i = base + threadIdx.x + static_cast<int64_t>(k) * blockDim.x;
-        qq[k] = make_int2(0, 0);
+        qq[k] = make_int2(-1, -1);
         if (i < q1 && rmq_chk(i < o.span)) qq[k] = __ldcs(o.Q + i);
     }
 }
@@ -266,47 +259,56 @@ __device__ __forceinline__ Entry st_probe(const V1View &v, uint32_t a, uint32_t 
     return better(x, y);
 }
 
-// Leftmost best of micro-blocks a..b (a <= b, b - a + 1 < 2^mlevels): the
-// offsets of the two windows' best micro-blocks, then their minima.
+// Leftmost best of micro-blocks a..b (a <= b, b - a + 1 < 2^mlevels): from
+// the mask of a for up to 32 (64) of them, else the better of the two windows
+// of 2^k that cover them (the lowest such k from the masks' highest bits, then
+// offset rows).
 template <bool STATS>
 __device__ __forceinline__ Entry micro_probe(const V1View &v, uint32_t a, uint32_t b, uint64_t pol,
                                              QStats &s) {
-    const int lev = ilog2(b - a + 1u);
+    const uint32_t w = b - a + 1u;
+    if (w <= (v.wide ? 64u : 32u)) {
+        uint32_t x = a;
+        if (w > 1u) {
+            if (v.wide)
+                x += 63u - __clzll(ld_mask(v, a, pol) & (~0ull >> (64u - w)));
+            else
+                x += 31u - __clz(static_cast<uint32_t>(ld_mask(v, a, pol)) & (0xffffffffu >> (32u - w)));
+        }
+        if constexpr (STATS) s.c[kStatTable] += w > 1u ? 2u : 1u;
+        return ld_entry_keep(v.mst, x, v.nmicro, pol);
+    }
+    const uint32_t lev = ilog2(w);
     uint32_t x = a, y = b + 1u - (1u << lev);
-    if (lev > 0) {
-        const uint64_t row = static_cast<uint64_t>(lev - 1) * v.nmicro;
-        const bool two = y != x;
-        const uint32_t ox = ld_moff(v, row + x, pol);
-        const uint32_t oy = two ? ld_moff(v, row + y, pol) : ox;
-        if constexpr (STATS) s.c[kStatTable] += two ? 2u : 1u;
+    const uint32_t row0 = mask_levels(v.wide);
+    if (lev < row0) {
+        const uint64_t mx = ld_mask(v, x, pol), my = ld_mask(v, y, pol);
+        x += 63u - __clzll(mx);
+        y += 63u - __clzll(my);
+    } else {
+        const uint64_t row = static_cast<uint64_t>(lev - row0) * v.nmicro;
+        const uint32_t ox = ld_moff(v, row + x, pol), oy = ld_moff(v, row + y, pol);
         x += ox;
         y += oy;
     }
     const Entry ex = ld_entry_keep(v.mst, x, v.nmicro, pol);
     Entry ey = ex;
     if (y != x) ey = ld_entry_keep(v.mst, y, v.nmicro, pol);
-    if constexpr (STATS) s.c[kStatTable] += (y != x) ? 2u : 1u;
+    if constexpr (STATS) s.c[kStatTable] += y != x ? 4u : 3u;
     return better(ex, ey);
 }
 
+// Without the sub-block level: suf[l] (best of A[l .. end of l's block]),
+// pre[r] (best of A[start of r's block .. r]).
 template <bool STATS>
-__device__ __forceinline__ Entry unit_probe(const V1View &v, bool micro, uint32_t a, uint32_t b,
-                                            uint64_t pol, QStats &s) {
-    return micro ? micro_probe<STATS>(v, a, b, pol, s) : st_probe<STATS>(v, a, b, pol, s);
-}
-
-// S[l]: best of A[l .. end of l's unit]; P[r]: best of A[start of r's unit .. r].
-// The micro-level entries are read with streaming loads (they are read once,
-// and would otherwise push the micro table out of L2).
-template <bool STATS>
-__device__ __forceinline__ Entry left_entry(const V1View &v, bool micro, uint32_t l, QStats &s) {
+__device__ __forceinline__ Entry left_entry(const V1View &v, uint32_t l, QStats &s) {
     if constexpr (STATS) s.c[kStatEntries] += 1u;
-    return micro ? ld_entry_cs(v.msuf, l, v.n) : ld_entry(v.suf, l, v.n);
+    return ld_entry(v.suf, l, v.n);
 }
 template <bool STATS>
-__device__ __forceinline__ Entry right_entry(const V1View &v, bool micro, uint32_t r, QStats &s) {
+__device__ __forceinline__ Entry right_entry(const V1View &v, uint32_t r, QStats &s) {
     if constexpr (STATS) s.c[kStatEntries] += 1u;
-    return micro ? ld_entry_cs(v.mpre, r, v.n) : ld_entry(v.pre, r, v.n);
+    return ld_entry(v.pre, r, v.n);
 }
 
 // 32-byte sectors of the local range A[a..b]
@@ -327,121 +329,173 @@ __device__ __forceinline__ uint32_t range_sectors(const V1View &v, uint32_t a, u
 
 // ---- lines of values, settled by the warp ---------------------------------
 //
-// A query inside one micro-block, and a miss of the light index, needs the
-// best of part of one 32-element line. Scanned by the lane that owns the
-// query, a load instruction touches up to 32 different 128-byte lines, one
-// L1 tag lookup each, for up to 9 instructions, and a warp waits for its
-// longest scan. Here 8 lanes take one request, 16 bytes each: a load
-// instruction touches 4 lines and each line is looked up once. What bounds
-// it is the random lines' DRAM traffic. Measured (2^26 queries, ms): ranges
-// of 32 over n = 1e8 2.78 -> 1.81; light index, uniform 0.527 -> 0.346, short
-// (lr=-3) 1.18 -> 1.09, ranges of 32 4.99 -> 3.2 (those took 40 KB of shared
-// memory per CTA for the lines besides, and ran 3 CTAs per SM).
+// A query inside one micro-block, and the end part of a query whose probe did
+// not settle it, is the best of part of one 32-element line. Scanned by the
+// lane that owns the query straight from memory, a load instruction touches
+// up to 32 different 128-byte lines, one L1 tag lookup each, for up to 9
+// instructions. Here the warp first copies the lines of its requests into
+// shared memory, 8 lanes per line and 16 bytes each (one tag lookup per line,
+// all copies in flight together, no registers held), and the probes of the
+// same drain run while they arrive; then every lane reduces lines without
+// bank conflicts (chunks XOR-swizzled by the line's slot).
 
-// The best of one lane's chunk b[0..3] among the elements whose bit of `nib`
-// is set, in key mode MODE: its key, and its position | (-0.0 flag << 2).
-// With no element set, or every set element at the largest key, the key is
-// the largest one (the caller then takes the request's first element).
+// Lines a warp stages at a time: 16 (2 KB per warp, two lanes per line). 32
+// need fewer instructions but twice the shared memory, taken from the L1 that
+// block tables live in (n = 1e8, 2^26 queries, uniform lengths, bs 2^15:
+// 0.33 ms with 16, 0.57 with 32; ranges of 32: 1.60 and 1.81).
+constexpr int kStageLines = 16;
+constexpr int kLanesPerLine = 32 / kStageLines;
+constexpr int kChunksPerLane = 8 / kLanesPerLine;
+
+// What a key mode compares: IEEE minimum / maximum, which skips NaN (ordered
+// last) and equates the zeros, or signed minimum / maximum. `fill` stands for
+// an element outside the request: it never beats one inside.
 template <uint32_t MODE>
-__device__ __forceinline__ void chunk_best(const uint32_t (&b)[4], uint32_t nib, uint32_t &key,
-                                           uint32_t &info) {
-    if constexpr (MODE == kFloatMin || MODE == kFloatMax) {
-        // the IEEE minimum (maximum) skips NaN, which orders last; the first
-        // value equal to it is the leftmost best and gives the key
-        float x[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            x[k] = __uint_as_float((nib >> k) & 1u ? b[k] : 0x7fc00000u);
-        const float m = MODE == kFloatMin ? fminf(fminf(x[0], x[1]), fminf(x[2], x[3]))
-                                          : fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
-        const uint32_t p = x[0] == m ? 0u : x[1] == m ? 1u : x[2] == m ? 2u : 3u;
-        const uint32_t wb = p == 0u ? b[0] : p == 1u ? b[1] : p == 2u ? b[2] : b[3];
-        key = m == m ? key_of(wb, MODE) : 0xffffffffu;
-        info = p | (negzero_of(wb, MODE) << 2);
-    } else {
-        key = 0xffffffffu;
-        info = 0u;
-#pragma unroll
-        for (int k = 3; k >= 0; --k) {
-            const uint32_t kk = (nib >> k) & 1u ? key_of(b[k], MODE) : 0xffffffffu;
-            if (kk <= key) {
-                key = kk;
-                info = static_cast<uint32_t>(k);
-            }
-        }
-    }
+struct Best {
+    using T = float;
+    static __device__ __forceinline__ T of(uint32_t b) { return __uint_as_float(b); }
+    static __device__ __forceinline__ uint32_t bits(T x) { return __float_as_uint(x); }
+    static __device__ __forceinline__ T fill() { return __uint_as_float(0x7fc00000u); }
+    static __device__ __forceinline__ T best(T a, T b) { return MODE == kFloatMin ? fminf(a, b) : fmaxf(a, b); }
+};
+template <>
+struct Best<kIntMin> {
+    using T = int32_t;
+    static __device__ __forceinline__ T of(uint32_t b) { return static_cast<int32_t>(b); }
+    static __device__ __forceinline__ uint32_t bits(T x) { return static_cast<uint32_t>(x); }
+    static __device__ __forceinline__ T fill() { return 0x7fffffff; }
+    static __device__ __forceinline__ T best(T a, T b) { return min(a, b); }
+};
+template <>
+struct Best<kIntMax> {
+    using T = int32_t;
+    static __device__ __forceinline__ T of(uint32_t b) { return static_cast<int32_t>(b); }
+    static __device__ __forceinline__ uint32_t bits(T x) { return static_cast<uint32_t>(x); }
+    static __device__ __forceinline__ T fill() { return -0x7fffffff - 1; }
+    static __device__ __forceinline__ T best(T a, T b) { return max(a, b); }
+};
+
+// Shared-memory address of chunk 0 of a staged line; chunk c is at ^ (c << 4).
+__device__ __forceinline__ uint32_t staged_line(uint32_t stage, uint32_t slot) {
+    return stage + slot * 128u + ((slot & 7u) << 4);
+}
+__device__ __forceinline__ uint4 lds_chunk(uint32_t addr) {
+    uint4 f;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(f.x), "=r"(f.y), "=r"(f.z), "=r"(f.w) : "r"(addr));
+    return f;
 }
 
-// One chunk of values: elements 4 sub .. 4 sub + 3 of the 32-element line
-// `line` (array-relative), of which only those set in `nib` are read when the
-// 16-byte load is not possible (values not 16-byte aligned, or the chunk
-// passes the end of the buffer).
+// Starts copying the chunks holding a set bit of the requests of lanes
+// h .. h + kStageLines - 1 into the warp's stage. Bytes past the end of the
+// buffer are not read.
 template <bool ALIGNED>
-__device__ __forceinline__ void load_chunk(const V1View &v, uint32_t line, uint32_t sub,
-                                           uint32_t nib, uint32_t (&b)[4]) {
-    const int64_t g = v.off + static_cast<int64_t>(line) * 32 + 4 * sub;
+__device__ __forceinline__ void stage_lines(const V1View &v, uint32_t line, uint32_t bits,
+                                            uint32_t stage, uint32_t h) {
+    const uint32_t lane = threadIdx.x & 31u, sub = lane & 7u, grp = lane >> 3;
+    // whole chunks by 16-byte copies when every requested line lies inside
+    // the buffer and on a 16-byte boundary
+    const int64_t end = v.off + static_cast<int64_t>(line) * 32 + 32;
+    const bool whole = ALIGNED && (v.off & 3) == 0 &&
+                       !__any_sync(0xffffffffu, bits != 0u && end > v.limit);
+    const float *const base = v.A + v.off + 4 * sub;
+    if (whole) {
+        // slot 4 t + grp: its swizzle depends on t's parity alone
+        const uint32_t d0 = staged_line(stage, grp) ^ (sub << 4);
+        const uint32_t d1 = staged_line(stage, 4u + grp) ^ (sub << 4);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) b[k] = 0u;
-    if (nib == 0u) return;
-    if (ALIGNED && (v.off & 3) == 0 && g + 4 <= v.limit) {
-        const uint4 f = ld_elem4(v, g);
-        b[0] = f.x;
-        b[1] = f.y;
-        b[2] = f.z;
-        b[3] = f.w;
+        for (uint32_t t = 0; t < kStageLines / 4; ++t) {
+            const uint32_t ln = __shfl_sync(0xffffffffu, line, h + 4u * t + grp);
+            const uint32_t bt = __shfl_sync(0xffffffffu, bits, h + 4u * t + grp);
+            const float *src = base + static_cast<size_t>(ln) * 32;
+            const uint32_t dst = ((t & 1u) ? d1 : d0) + (t / 2u) * 1024u;
+            if ((bt >> (4u * sub)) & 15u && rmq_chk(v.off + static_cast<int64_t>(ln) * 32 + 32 <= v.limit))
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
+        }
     } else {
+#pragma unroll 1
+        for (uint32_t t = 0; t < kStageLines / 4; ++t) {
+            const uint32_t slot = 4u * t + grp;
+            const uint32_t ln = __shfl_sync(0xffffffffu, line, h + slot);
+            const uint32_t nib = (__shfl_sync(0xffffffffu, bits, h + slot) >> (4u * sub)) & 15u;
+            const uint32_t dst = staged_line(stage, slot) ^ (sub << 4);
+            const float *src = base + static_cast<size_t>(ln) * 32;
+            const int64_t g = v.off + static_cast<int64_t>(ln) * 32 + 4 * sub;
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if ((nib >> k) & 1u) b[k] = ld_elem(v, g + k);
+            for (int k = 0; k < 4; ++k)
+                if ((nib >> k) & 1u && rmq_chk(g >= 0 && g + k < v.limit))
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;"
+                                 :: "r"(dst + 4u * k), "l"(src + k) : "memory");
+        }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-// Rounds of 4 requests whose loads are in flight together. Two: four cost 9
-// to 16 more registers in the main pass they share a kernel with (uniform
-// lengths, n = 1e8, q = 2^26: 0.309 ms with two, 0.341 with four) and settle
-// misses no faster.
-constexpr int kLineRounds = 2;
-
-// Leftmost best of the elements of line `line` whose bits are set in `bits`,
-// for every lane with bits != 0, kEntryNone for the others; the whole warp
-// calls it.
-template <bool ALIGNED, uint32_t MODE>
-__device__ __forceinline__ Entry warp_lines(const V1View &v, uint32_t line, uint32_t bits) {
-    const uint32_t lane = threadIdx.x & 31u, sub = lane & 7u, grp = lane >> 3;
-    const uint32_t act = __ballot_sync(0xffffffffu, bits != 0u);
-    Entry out = kEntryNone;
-#pragma unroll 1
-    for (uint32_t h = 0; h < 32u; h += 4u * kLineRounds) {
-        if (((act >> h) & ((1u << (4 * kLineRounds)) - 1u)) == 0u) continue;  // warp-uniform
-        uint32_t b[kLineRounds][4];
+// Waits for the staged lines and returns, on lanes h .. h + kStageLines - 1
+// with bits != 0, the leftmost best of their requests; kEntryNone elsewhere.
+// The set bits of a request are consecutive.
+template <uint32_t MODE>
+__device__ __forceinline__ Entry reduce_lines(uint32_t line, uint32_t bits, uint32_t stage,
+                                              uint32_t h) {
+    using B = Best<MODE>;
+    constexpr uint32_t kBits = 4u * kChunksPerLane;
+    const uint32_t lane = threadIdx.x & 31u;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+    // kLanesPerLine lanes per line, kChunksPerLane consecutive chunks each
+    const uint32_t slot = lane / kLanesPerLine, c0 = (lane % kLanesPerLine) * kChunksPerLane;
+    const uint32_t all = kLanesPerLine == 1 ? bits : __shfl_sync(0xffffffffu, bits, h + slot);
+    const uint32_t mine = kBits == 32u ? all : (all >> (4u * c0)) & ((1u << (kBits % 32u)) - 1u);
+    const uint32_t base = staged_line(stage, slot) ^ (c0 << 4);
+    // the elements outside the request in its first and last chunk are
+    // overwritten with the fill, so that only whole chunks are selected below
+    const uint32_t first = mine ? __ffs(mine) - 1u : 0u, end = 31u - __clz(mine | 1u);
+    const uint32_t fill = B::bits(B::fill());
 #pragma unroll
-        for (int t = 0; t < kLineRounds; ++t) {
-            const uint32_t ln = __shfl_sync(0xffffffffu, line, h + 4u * t + grp);
-            const uint32_t m = __shfl_sync(0xffffffffu, bits, h + 4u * t + grp);
-            load_chunk<ALIGNED>(v, ln, sub, (m >> (4u * sub)) & 15u, b[t]);
-        }
-#pragma unroll
-        for (int t = 0; t < kLineRounds; ++t) {
-            const uint32_t m = __shfl_sync(0xffffffffu, bits, h + 4u * t + grp);
-            uint32_t gk, info;
-            chunk_best<MODE>(b[t], (m >> (4u * sub)) & 15u, gk, info);
-            const uint32_t key = gk;
-#pragma unroll
-            for (int o = 4; o > 0; o >>= 1) gk = min(gk, __shfl_xor_sync(0xffffffffu, gk, o, 8));
-            const uint32_t own = (__ballot_sync(0xffffffffu, key == gk) >> (8u * grp)) & 0xffu;
-            const uint32_t w = __ffs(own) - 1u;
-            info = __shfl_sync(0xffffffffu, info, 8u * grp + w);
-            // every set element at the largest key: the first of them
-            const uint32_t pos = gk == 0xffffffffu ? __ffs(m) - 1u : 4u * w + (info & 3u);
-            const uint32_t nz = gk == 0xffffffffu ? 0u : info >> 2;
-            // to the lane that asked: h + 4 t + its group
-            const uint32_t rk = __shfl_sync(0xffffffffu, gk, 8u * (lane & 3u));
-            const uint32_t rl = __shfl_sync(0xffffffffu, (pos << 1) | nz, 8u * (lane & 3u));
-            if (bits != 0u && (lane >> 2) == (h >> 2) + t)
-                out = (static_cast<uint64_t>(rk) << 32) | ((line << 6) + rl);
-        }
+    for (uint32_t k = 0; k < 3; ++k) {
+        if (k < (first & 3u))
+            asm volatile("st.shared.u32 [%0], %1;" :: "r"((base ^ ((first >> 2) << 4)) + 4u * k), "r"(fill) : "memory");
+        if (3u - k > (end & 3u))
+            asm volatile("st.shared.u32 [%0], %1;" :: "r"((base ^ ((end >> 2) << 4)) + 12u - 4u * k), "r"(fill) : "memory");
     }
-    return out;
+    typename B::T m[kChunksPerLane];
+#pragma unroll
+    for (int c = 0; c < kChunksPerLane; ++c) {
+        const uint4 f = lds_chunk(base ^ (c << 4));
+        m[c] = B::best(B::best(B::best(B::of(f.x), B::of(f.y)), B::of(f.z)), B::of(f.w));
+        m[c] = mine & (15u << (4 * c)) ? m[c] : B::fill();
+    }
+    typename B::T mm = m[0];
+#pragma unroll
+    for (int c = 1; c < kChunksPerLane; ++c) mm = B::best(mm, m[c]);
+    // the first chunk holding it, and in that chunk the first element
+    uint32_t cs = 0u;
+#pragma unroll
+    for (int c = kChunksPerLane - 1; c >= 0; --c) cs = m[c] == mm ? c : cs;
+    const uint4 f = lds_chunk(base ^ (cs << 4));
+    uint32_t pos = 3u, wb = f.w;
+    if (B::of(f.z) == mm) pos = 2u, wb = f.z;
+    if (B::of(f.y) == mm) pos = 1u, wb = f.y;
+    if (B::of(f.x) == mm) pos = 0u, wb = f.x;
+    // no number, or nothing above the fill: every element of the request has
+    // the largest key, and the first of them is the best
+    const bool last = !(mm == mm) || mm == B::fill();
+    uint32_t hi = last ? 0xffffffffu : key_of(wb, MODE);
+    uint32_t lo = (4u * c0 + (last ? first : 4u * cs + pos)) << 1 | (last ? 0u : negzero_of(wb, MODE));
+    if (kLanesPerLine > 1) {
+        if (mine == 0u) lo = 0xffffffffu;
+#pragma unroll
+        for (int o = 1; o < kLanesPerLine; o <<= 1) {
+            const uint32_t th = __shfl_xor_sync(0xffffffffu, hi, o), tl = __shfl_xor_sync(0xffffffffu, lo, o);
+            if (th < hi || (th == hi && tl < lo)) hi = th, lo = tl;
+        }
+        const uint32_t from = ((lane - h) * kLanesPerLine) & 31u;
+        hi = __shfl_sync(0xffffffffu, hi, from);
+        lo = __shfl_sync(0xffffffffu, lo, from);
+    }
+    __syncwarp();  // the stage may be written again
+    return bits != 0u && lane - h < kStageLines
+               ? (static_cast<uint64_t>(hi) << 32) | ((line << 6) + lo) : kEntryNone;
 }
 
 // Bits lo .. hi (inclusive, 0 <= lo <= hi <= 31)
@@ -449,85 +503,75 @@ __device__ __forceinline__ uint32_t bit_range(uint32_t lo, uint32_t hi) {
     return (0xffffffffu >> (31u - hi)) & (0xffffffffu << lo);
 }
 
-// With per-element entries, the part of a query in its end unit on the
-// left, [l, end of l's unit] (micro-block, or block), and on the right,
-// [start of r's unit, r]: one entry each.
+// Table index: of the query's part in its end unit on one side, [l, end of
+// l's unit] (left) or [start of r's unit, r] (right), what lies outside the
+// line of its end: for a block, the best of the block's whole micro-blocks on
+// that side. The side is a value, not a branch, so that lanes settling left
+// and right parts run the same code.
 template <bool STATS>
-__device__ __forceinline__ Entry left_part(const V1View &v, bool micro, uint32_t l, QStats &s) {
-    return left_entry<STATS>(v, micro, l, s);
-}
-template <bool STATS>
-__device__ __forceinline__ Entry right_part(const V1View &v, bool micro, uint32_t r, QStats &s) {
-    return right_entry<STATS>(v, micro, r, s);
-}
-
-// Light index: the query's part in its end unit on one side, [l, end of
-// l's unit] (left) or [start of r's unit, r] (right): part of one line of
-// values inside the end micro-block (its line and element bits), plus for a
-// block unit the best of the block's whole micro-blocks on that side. The
-// side is a value, not a branch, so that lanes settling left and right parts
-// run the same code.
-template <bool STATS>
-__device__ __forceinline__ Entry light_rest(const V1View &v, bool micro, bool left, uint32_t a,
-                                            uint32_t b, uint32_t l, uint32_t r, uint64_t pol,
-                                            QStats &s, uint32_t &line, uint32_t &bits) {
-    line = (left ? l : r) >> 5;
-    // the left end's unit lies before the right end's, so its line is whole
-    bits = left ? 0xffffffffu << (l & 31u) : 0xffffffffu >> (31u - (r & 31u));
-    if constexpr (STATS) s.c[kStatSectors] += range_sectors(v, left ? l : (r & ~31u), left ? l | 31u : r);
+__device__ __forceinline__ Entry end_rest(const V1View &v, bool micro, bool left, uint32_t a,
+                                          uint32_t b, uint32_t l, uint32_t r, uint64_t pol,
+                                          QStats &s) {
+    if constexpr (STATS) {
+        if (v.light)
+            s.c[kStatSectors] += range_sectors(v, left ? l : (r & ~31u), left ? l | 31u : r);
+        else
+            s.c[kStatEntries] += 1u;
+    }
     if (micro) return kEntryNone;
     // block a is full when a < b: its last micro-block ends inside the array
-    const uint32_t ml = l >> 5, me = (((a + 1u) * v.bs) >> 5) - 1u;
-    const uint32_t mr = r >> 5, ms = (b * v.bs) >> 5;
+    const uint32_t pb = v.bs >> 5;
+    const uint32_t ml = l >> 5, me = (a + 1u) * pb - 1u;
+    const uint32_t mr = r >> 5, ms = b * pb;
     const bool has = left ? ml < me : ms < mr;
     if (!has) return kEntryNone;
     return micro_probe<STATS>(v, left ? ml + 1u : ms, left ? me : mr - 1u, pol, s);
 }
 
-// Settles one query whose superset best lay outside [l, r] (or, without
-// the sub-block level, inside one block at an edge) from the per-element
-// entries: the query's part in the end unit on that side and a narrower
+// Without the sub-block level: settles one query whose superset best lay
+// outside [l, r], or inside one block at an edge, from the per-element
+// entries: the query's part in the end block on that side and a narrower
 // probe, loaded together, then only if needed the other end's part and the
-// middle units.
+// middle blocks.
 template <bool STATS>
-__device__ __forceinline__ Entry finish_miss(const V1View &v, bool micro, bool left, uint32_t l,
-                                             uint32_t r, uint64_t pol, QStats &s) {
-    const uint32_t a = micro ? (l >> 5) : div31(l, v.dv);
-    const uint32_t b = micro ? (r >> 5) : div31(r, v.dv);
+__device__ __forceinline__ Entry finish_entries(const V1View &v, bool left, uint32_t l, uint32_t r,
+                                                uint64_t pol, QStats &s) {
+    const uint32_t a = div31(l, v.dv), b = div31(r, v.dv);
     if (a == b) {
-        // one block, without the sub-block level: the query touches an edge
         if constexpr (STATS) s.c[kStatBlockEdge] += 1u;
         const uint32_t bend = min(a * v.bs + v.bs, v.n) - 1u;
-        return r == bend ? left_entry<STATS>(v, false, l, s) : right_entry<STATS>(v, false, r, s);
+        return r == bend ? left_entry<STATS>(v, l, s) : right_entry<STATS>(v, r, s);
     }
     // the narrower probe first: its loads are in flight while the part's
     // entry is loaded
-    const Entry e2 = left ? unit_probe<STATS>(v, micro, a + 1u, b, pol, s)
-                          : unit_probe<STATS>(v, micro, a, b - 1u, pol, s);
-    const Entry e1 = left ? left_part<STATS>(v, micro, l, s) : right_part<STATS>(v, micro, r, s);
+    const Entry e2 = st_probe<STATS>(v, left ? a + 1u : a, left ? b : b - 1u, pol, s);
+    const Entry e1 = left ? left_entry<STATS>(v, l, s) : right_entry<STATS>(v, r, s);
     const uint32_t m2 = entry_idx(e2);
     if (left ? m2 <= r : m2 >= l) {
         if constexpr (STATS) s.c[kStatSecond] += 1u;
         return better(e1, e2);
     }
     if constexpr (STATS) s.c[kStatFull] += 1u;
-    const Entry mid = (b - a >= 2u) ? unit_probe<STATS>(v, micro, a + 1u, b - 1u, pol, s)
-                                    : kEntryNone;
-    const Entry other = left ? right_part<STATS>(v, micro, r, s) : left_part<STATS>(v, micro, l, s);
+    const Entry mid = (b - a >= 2u) ? st_probe<STATS>(v, a + 1u, b - 1u, pol, s) : kEntryNone;
+    const Entry other = left ? right_entry<STATS>(v, r, s) : left_entry<STATS>(v, l, s);
     return better(better(e1, other), mid);
 }
 
-// One warp's queue: up to 31 waiting queries plus the 32 that each query
-// slot of a step can add, 12 bytes each (what it takes from the L1 matters:
-// the block table's upper levels live there). `id` numbers the queries of
-// the CTA in the order it takes them: step * step size + place in the step.
-template <int QPT>
+// One warp's queue (up to 31 waiting queries plus the 32 that one query slot
+// of a step can add, 12 bytes each) and its line stage: what they take from
+// the L1 matters, the block table's upper levels live there. `id` numbers the
+// queries of the CTA in the order it takes them: step * step size + place in
+// the step.
+template <bool MICRO>
 struct MissQueue {
-    static constexpr int kCap = 32 * (QPT + 1);
+    static constexpr int kCap = 64;
+    uint4 stage[MICRO ? kStageLines * 8 : 1];
+    Entry part[MICRO ? kCap : 1];  // kSecond: the best of what is settled so far
     uint32_t l[kCap];   // kMissLeft set: the probe's best lay left of l
-    uint32_t r[kCap];
+    uint32_t r[kCap];   // kSecond set: back for its other end
     uint32_t id[kCap];
 };
+constexpr uint32_t kSecond = 0x80000000u;  // above every index
 constexpr uint32_t kMissLeft = 0x80000000u;  // above every index
 
 // The queries a CTA takes: steps of `chunk` consecutive ones, `stride` apart.
@@ -540,63 +584,79 @@ struct StepMap {
 };
 
 // Settles the last min(count, 32) queued queries, one per lane; the whole
-// warp calls it (count is warp-uniform). Queries inside one micro-block, and
-// the light index's misses, read lines of values, the warp together.
-template <bool ALIGNED, bool MICRO, bool LIGHT, uint32_t MODE, bool STATS, int THREADS, int QPT>
+// warp calls it (count is warp-uniform). With the sub-block level, a query
+// inside one micro-block is one line of values. A query whose probe's best
+// lay outside needs the units without the end unit that held it (e2) and its
+// part in that end unit; e2 settles it when it lies inside [l, r]. Else,
+// rarely, it joins the queue again, for the units between both ends and its
+// part at the other end: few lanes in a warp need that, so doing it at once
+// would cost every drain a second pass.
+template <bool ALIGNED, bool MICRO, uint32_t MODE, bool STATS, int THREADS, int QPT>
 __device__ __forceinline__ void drain_misses(const V1View &v, const QueryOut &o,
-                                             const StepMap &map, MissQueue<QPT> &mq,
+                                             const StepMap &map, MissQueue<MICRO> &mq,
                                              uint32_t &count, uint64_t pol, QStats &s) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t take = count < 32u ? count : 32u;
     __syncwarp();
-    const uint32_t e = count - take + lane;
+    count -= take;
+    const uint32_t e = count + lane;
     const bool act = lane < take;
-    const uint32_t lq = act ? mq.l[e] : 0u, r = act ? mq.r[e] : 0u;
-    const uint32_t l = lq & ~kMissLeft;
+    const uint32_t lq = act ? mq.l[e] : 0u, rq = act ? mq.r[e] : 0u;
+    const uint32_t id = act ? mq.id[e] : 0u;
+    const uint32_t l = lq & ~kMissLeft, r = rq & ~kSecond;
     const bool left = (lq & kMissLeft) != 0u;
-    const bool micro = MICRO && (r >> 5) - (l >> 5) < v.micro_span;
-    const bool scan = MICRO && act && (l >> 5) == (r >> 5);
-    const bool miss = act && !scan;
     Entry res = kEntryNone;
-    uint32_t line = l >> 5, bits = scan ? bit_range(l & 31u, r & 31u) : 0u;
-    if constexpr (!LIGHT) {
-        if (MICRO && __any_sync(0xffffffffu, scan)) res = warp_lines<ALIGNED, MODE>(v, line, bits);
-        if (miss) res = finish_miss<STATS>(v, micro, left, l, r, pol, s);
+    bool again = false;
+    if constexpr (!MICRO) {
+        if (act) res = finish_entries<STATS>(v, left, l, r, pol, s);
     } else {
-        const uint32_t a = micro ? (l >> 5) : div31(l, v.dv);
-        const uint32_t b = micro ? (r >> 5) : div31(r, v.dv);
+        const uint32_t stage = static_cast<uint32_t>(__cvta_generic_to_shared(mq.stage));
+        const bool second = (rq & kSecond) != 0u;
+        const bool side = left != second;  // the end whose line is wanted
+        const bool scan = (l >> 5) == (r >> 5);
+        const uint32_t line = (side ? l : r) >> 5;
+        // the left end's unit lies before the right end's, so its line is whole
+        uint32_t bits = scan ? bit_range(l & 31u, r & 31u)
+                        : side ? 0xffffffffu << (l & 31u) : 0xffffffffu >> (31u - (r & 31u));
+        if (!act) bits = 0u;
+        stage_lines<ALIGNED>(v, line, bits, stage, 0u);
+        if (second) res = mq.part[e];
+        // the probes run while the lines arrive
         Entry e2 = kEntryNone;
-        if (miss) {
-            e2 = unit_probe<STATS>(v, micro, left ? a + 1u : a, left ? b : b - 1u, pol, s);
-            res = light_rest<STATS>(v, micro, left, a, b, l, r, pol, s, line, bits);
+        if (act && !scan) {
+            const bool micro = (r >> 5) - (l >> 5) < v.micro_span;
+            const uint32_t a = micro ? (l >> 5) : div31_ge2(l, v.dv);
+            const uint32_t b = micro ? (r >> 5) : div31_ge2(r, v.dv);
+            const uint32_t lo = a + (left || second), hi = b - (!left || second);
+            if (lo <= hi)
+                e2 = micro ? micro_probe<STATS>(v, lo, hi, pol, s) : st_probe<STATS>(v, lo, hi, pol, s);
+            res = better(res, end_rest<STATS>(v, micro, side, a, b, l, r, pol, s));
+            const uint32_t m2 = entry_idx(e2);
+            again = !second && (left ? m2 > r : m2 < l);
+            if (!again) res = better(res, e2);
+            if constexpr (STATS)
+                if (!second) s.c[again ? kStatFull : kStatSecond] += 1u;
         }
-        // one copy of the line scan's code: the second pass (the other end,
-        // after the middle units) runs only for the rare query the narrower
-        // probe does not settle
+        res = better(res, reduce_lines<MODE>(line, bits, stage, 0u));
 #pragma unroll 1
-        for (int pass = 0; pass < 2; ++pass) {
-            res = better(res, warp_lines<ALIGNED, MODE>(v, line, bits));
-            if (pass == 1) break;
-            bits = 0u;
-            bool more = false;
-            if (miss) {
-                const uint32_t m2 = entry_idx(e2);
-                more = left ? m2 > r : m2 < l;
-                if constexpr (STATS) s.c[more ? kStatFull : kStatSecond] += 1u;
-                if (!more) {
-                    res = better(res, e2);
-                } else {
-                    if (b - a >= 2u)
-                        res = better(res, unit_probe<STATS>(v, micro, a + 1u, b - 1u, pol, s));
-                    res = better(res, light_rest<STATS>(v, micro, !left, a, b, l, r, pol, s, line, bits));
-                }
-            }
-            if (!__any_sync(0xffffffffu, more)) break;
+        for (uint32_t h = kStageLines; h < 32u; h += kStageLines) {
+            stage_lines<ALIGNED>(v, line, bits, stage, h);
+            res = better(res, reduce_lines<MODE>(line, bits, stage, h));
         }
     }
-    if (act) put_result(o, map.query(mq.id[e], THREADS * QPT), res, MODE);
+    if (act && !again) put_result(o, map.query(id, THREADS * QPT), res, MODE);
+    if constexpr (MICRO) {
+        const unsigned mask = __ballot_sync(0xffffffffu, again);
+        if (again) {
+            const uint32_t w = count + __popc(mask & ((1u << lane) - 1u));
+            mq.l[w] = lq;
+            mq.r[w] = r | kSecond;
+            mq.id[w] = id;
+            mq.part[w] = res;
+        }
+        count += __popc(mask);
+    }
     __syncwarp();
-    count -= take;
 }
 
 // The bits of an entry's element for key mode MODE, without branches
@@ -624,73 +684,53 @@ __device__ __forceinline__ uint32_t decode_bits(Entry e) {
 // sequence).
 template <bool MICRO, bool STATS>
 __device__ __forceinline__ Entry superset_probe(const V1View &v, uint32_t l, uint32_t r,
-                                                uint64_t pol, QStats &s, bool &mic) {
+                                                uint64_t pol, QStats &s) {
     const uint32_t ml = l >> 5, mr = r >> 5;
-    mic = MICRO && mr - ml < v.micro_span;
-    const uint32_t a = mic ? ml : div31(l, v.dv);
-    const uint32_t b = mic ? mr : div31(r, v.dv);
+    if (MICRO && mr - ml < v.micro_span) return micro_probe<STATS>(v, ml, mr, pol, s);
+    const uint32_t a = MICRO ? div31_ge2(l, v.dv) : div31(l, v.dv);
+    const uint32_t b = MICRO ? div31_ge2(r, v.dv) : div31(r, v.dv);
     const int lev = ilog2(b - a + 1u);
-    uint32_t x = a, y = b + 1u - (1u << lev);
-    if (MICRO && mic) {
-        // lev >= 1: the query spans at least two micro-blocks. The two
-        // windows overlap, so 1-byte offsets often share an aligned 8-byte
-        // word (one load), and both windows often point at the same best
-        // micro-block (one minimum load).
-        const uint64_t row = static_cast<uint64_t>(lev - 1) * v.nmicro;
-        if (v.moff_bytes == 1u && ((row + x) >> 3) == ((row + y) >> 3)) {
-            const uint64_t w = ld_moff_word(v, row + x, pol);
-            x += static_cast<uint32_t>(w >> (8 * ((row + x) & 7))) & 0xffu;
-            y += static_cast<uint32_t>(w >> (8 * ((row + y) & 7))) & 0xffu;
-            if constexpr (STATS) s.c[kStatTable] += 1u;
-        } else {
-            x += ld_moff(v, row + x, pol);
-            y += ld_moff(v, row + y, pol);
-            if constexpr (STATS) s.c[kStatTable] += 2u;
-        }
-        const Entry e1 = ld_entry_keep(v.mst, x, v.nmicro, pol);
-        Entry e2 = e1;
-        if (x != y) e2 = ld_entry_keep(v.mst, y, v.nmicro, pol);
-        if constexpr (STATS) s.c[kStatTable] += x != y ? 2u : 1u;
-        return better(e1, e2);
-    }
     const Entry *t = v.st + static_cast<uint64_t>(lev) * v.nb;
     const uint64_t size = static_cast<uint64_t>(v.levels - lev) * v.nb;
-    const Entry e1 = ld_entry_keep(t, x, size, pol);
-    const Entry e2 = ld_entry_keep(t, y, size, pol);
+    const Entry e1 = ld_entry_keep(t, a, size, pol);
+    const Entry e2 = ld_entry_keep(t, b + 1u - (1u << lev), size, pol);
     if constexpr (STATS) s.c[kStatTable] += 2u;
     return better(e1, e2);
 }
 
 // One step of the queued form over `cnt` queries from `base` on (cnt <=
 // THREADS * QPT): thread t handles base + t + k * THREADS, already loaded
-// into qq. FULL: cnt == THREADS * QPT, so no query needs a bounds check.
+// into qq (invalid from base + cnt on, so that only the rare path of invalid
+// queries compares with cnt).
 // MICRO: the index has the sub-block level (then every query inside one
 // block spans few enough micro-blocks for the micro table, and only the
-// block table serves longer ones). LIGHT: a light index (no per-element
-// entries). Queries left open join the warp's queue, whose length `count`
-// carries from step to step; `id0` is the step's first query in the CTA's
-// numbering. The caller drains the queue.
-template <bool ALIGNED, bool MICRO, bool LIGHT, uint32_t MODE, int THREADS, int QPT, bool STATS,
-          bool FULL>
+// block table serves longer ones). Queries left open join the warp's queue, whose length `count`
+// carries from step to step (`last` empties it); `id0` is the step's first
+// query in the CTA's numbering.
+template <bool ALIGNED, bool MICRO, uint32_t MODE, int THREADS, int QPT, bool STATS>
 __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryOut &o,
-                                                   int64_t base, uint32_t cnt, uint32_t id0,
+                                                   const StepMap &map, int64_t base, uint32_t cnt,
+                                                   uint32_t id0, bool last,
                                                    const int2 (&qq)[QPT], QStats &s,
-                                                   MissQueue<QPT> &mq, uint32_t &count) {
+                                                   MissQueue<MICRO> &mq, uint32_t &count) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t pol = l2_keep_policy();
     float *const vs = o.val ? o.val + base : nullptr;
     int32_t *const is = o.idx ? o.idx + base : nullptr;
     Entry res[QPT];
-    bool ok[QPT], scan[QPT], mic[QPT];
+    bool ok[QPT], scan[QPT];
 #pragma unroll
     for (int k = 0; k < QPT; ++k) {
-        const uint32_t j = threadIdx.x + k * THREADS;
         const uint32_t l = static_cast<uint32_t>(qq[k].x), r = static_cast<uint32_t>(qq[k].y);
-        ok[k] = (FULL || j < cnt) && qq[k].x >= 0 && l <= r && r < v.n;
+        ok[k] = qq[k].x >= 0 && l <= r && r < v.n;
         scan[k] = MICRO && (l >> 5) == (r >> 5);
-        mic[k] = false;
         res[k] = kEntryNone;
-        if (ok[k] && !scan[k]) res[k] = superset_probe<MICRO, STATS>(v, l, r, pol, s, mic[k]);
+        if (ok[k]) {
+            if (!scan[k])
+                res[k] = superset_probe<MICRO, STATS>(v, l, r, pol, s);
+            else if (l == r)
+                res[k] = make_entry(ld_elem(v, v.off + l), l, MODE);
+        }
     }
     bool miss[QPT];
     bool any_miss = false;
@@ -700,14 +740,14 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
         const uint32_t l = static_cast<uint32_t>(qq[k].x), r = static_cast<uint32_t>(qq[k].y);
         miss[k] = false;
         if (!ok[k]) {
-            if (FULL || j < cnt) {
+            if (j < cnt) {
                 put_invalid(o, base + j);
                 if constexpr (STATS) s.c[kStatInvalid] += 1u;
             }
             continue;
         }
-        // a query inside one micro-block still holds kEntryNone here, whose
-        // index lies outside [l, r]
+        // a query inside one micro-block (of more than one element) still
+        // holds kEntryNone here, whose index lies outside [l, r]
         miss[k] = entry_idx(res[k]) - l > r - l;
         any_miss |= miss[k];
         if constexpr (STATS) {
@@ -724,38 +764,21 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
         if (vs) __stcs(reinterpret_cast<unsigned int *>(vs) + j, decode_bits<MODE>(res[k]));
         if (is) __stcs(is + j, static_cast<int32_t>(entry_idx(res[k])));
     }
-    if (!__any_sync(0xffffffffu, any_miss)) return;
-    bool wscan[QPT];
-#pragma unroll
-    for (int k = 0; k < QPT; ++k) {
-        const uint32_t l = static_cast<uint32_t>(qq[k].x), r = static_cast<uint32_t>(qq[k].y);
-        wscan[k] = false;
-        if (!MICRO && miss[k]) {
-            const uint32_t lB = div31(l, v.dv);
-            if (lB == div31(r, v.dv)) {
-                // one block without the sub-block level: an edge entry when the
-                // query touches the block's edge, else the warp scans it
-                const uint32_t bstart = lB * v.bs;
-                const uint32_t bend = min(bstart + v.bs, v.n) - 1u;
-                if (r != bend && l != bstart) {
-                    miss[k] = false;
-                    wscan[k] = true;
-                }
-            }
-        }
-        const unsigned mask = __ballot_sync(0xffffffffu, miss[k]);
-        if (miss[k]) {
-            const uint32_t e = count + __popc(mask & ((1u << lane) - 1u));
-            mq.l[e] = l | (entry_idx(res[k]) < l ? kMissLeft : 0u);
-            mq.r[e] = r;
-            mq.id[e] = id0 + threadIdx.x + k * THREADS;
-        }
-        count += __popc(mask);
-    }
     if constexpr (!MICRO) {
 #pragma unroll
         for (int k = 0; k < QPT; ++k) {
-            unsigned mask = __ballot_sync(0xffffffffu, wscan[k]);
+            // one block without the sub-block level: an edge entry when the
+            // query touches the block's edge, else the warp scans it
+            bool wscan = false;
+            if (miss[k]) {
+                const uint32_t l = static_cast<uint32_t>(qq[k].x), r = static_cast<uint32_t>(qq[k].y);
+                const uint32_t lB = div31(l, v.dv);
+                const uint32_t bstart = lB * v.bs;
+                const uint32_t bend = min(bstart + v.bs, v.n) - 1u;
+                wscan = lB == div31(r, v.dv) && r != bend && l != bstart;
+                if (wscan) miss[k] = false;
+            }
+            unsigned mask = __ballot_sync(0xffffffffu, wscan);
             while (mask) {
                 const int src = __ffs(mask) - 1;
                 mask &= mask - 1u;
@@ -771,6 +794,35 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
                 }
             }
         }
+    }
+    // queue what is open, slot by slot, and drain: one copy of the drain's
+    // code (every copy costs instruction fetches)
+    if (!last && !__any_sync(0xffffffffu, any_miss)) return;
+#pragma unroll 1
+    for (int k = 0; k < QPT; ++k) {
+        int2 lr = qq[0];
+        bool open = miss[0];
+        uint32_t at = entry_idx(res[0]);
+#pragma unroll
+        for (int j = 1; j < QPT; ++j)
+            if (k == j) {
+                lr = qq[j];
+                open = miss[j];
+                at = entry_idx(res[j]);
+            }
+        const unsigned mask = __ballot_sync(0xffffffffu, open);
+        if (open) {
+            const uint32_t l = static_cast<uint32_t>(lr.x);
+            const uint32_t e = count + __popc(mask & ((1u << lane) - 1u));
+            mq.l[e] = l | (at < l ? kMissLeft : 0u);
+            mq.r[e] = static_cast<uint32_t>(lr.y);
+            mq.id[e] = id0 + threadIdx.x + k * THREADS;
+        }
+        count += __popc(mask);
+        const uint32_t drain_at = last && k == QPT - 1 ? 1u : 32u;
+#pragma unroll 1
+        while (count >= drain_at)
+            drain_misses<ALIGNED, MICRO, MODE, STATS, THREADS, QPT>(v, o, map, mq, count, pol, s);
     }
 }
 
@@ -788,10 +840,10 @@ __device__ __forceinline__ void flush_stats(const QStats &s, unsigned long long 
 
 // Answer queries [q0, q1) of one array with the whole CTA (THREADS
 // threads) in the queued form, QPT queries per thread per step; `mq` is the
-// calling warp's queue, empty on entry and on return. LIGHT: a light index.
-template <bool ALIGNED, bool MICRO, bool LIGHT, uint32_t MODE, int THREADS, int QPT>
+// calling warp's queue, empty on entry and on return.
+template <bool ALIGNED, bool MICRO, uint32_t MODE, int THREADS, int QPT>
 __device__ __forceinline__ void answer_range_queued(const V1View &v, const QueryOut &o,
-                                                    int64_t q0, int64_t q1, MissQueue<QPT> &mq) {
+                                                    int64_t q0, int64_t q1, MissQueue<MICRO> &mq) {
     constexpr int64_t step = static_cast<int64_t>(THREADS) * QPT;
     const StepMap map{q0, step};
     QStats s;
@@ -799,17 +851,9 @@ __device__ __forceinline__ void answer_range_queued(const V1View &v, const Query
     for (int64_t base = q0; base < q1; base += step, id0 += step) {
         int2 qq[QPT];
         load_queries<QPT>(o, base, q1, qq);
-        if (base + step <= q1)
-            answer_step_queued<ALIGNED, MICRO, LIGHT, MODE, THREADS, QPT, false, true>(
-                v, o, base, static_cast<uint32_t>(step), id0, qq, s, mq, waiting);
-        else
-            answer_step_queued<ALIGNED, MICRO, LIGHT, MODE, THREADS, QPT, false, false>(
-                v, o, base, static_cast<uint32_t>(q1 - base), id0, qq, s, mq, waiting);
-        // one site for the drain: its code is large, and every copy of it
-        // costs instruction fetches
-        while (waiting >= (base + step >= q1 ? 1u : 32u))
-            drain_misses<ALIGNED, MICRO, LIGHT, MODE, false, THREADS, QPT>(v, o, map, mq, waiting,
-                                                                           l2_keep_policy(), s);
+        answer_step_queued<ALIGNED, MICRO, MODE, THREADS, QPT, false>(
+            v, o, map, base, static_cast<uint32_t>(min(step, q1 - base)), id0, base + step >= q1, qq,
+            s, mq, waiting);
     }
 }
 
