@@ -2,8 +2,8 @@
 // answered by one persistent, cooperative launch (build + query), the same
 // work as one plain build/query launch sequence per array, the gradient
 // scatter of the differentiable range-min, and the per-size-bucket
-// autotuner. The kernels are in batch_impl.cuh; this unit instantiates the
-// full-index kernels, batch_light.cu the light-index ones.
+// autotuner. The kernel is in batch_impl.cuh; this unit instantiates it for
+// 16-byte aligned values, batch_unaligned.cu for others.
 //
 // The reference has no batched form: rtx_rmq<T> (src/rtx.h:24-177) builds one
 // structure for one array and launches one optixLaunch per batch of queries.
@@ -27,8 +27,8 @@ scatter_grad_kernel(const BatchArray *arrays, const uint4 *qitems, int32_t nqite
     for (int32_t it = blockIdx.x; it < nqitems; it += gridDim.x) {
         const uint4 w = qitems[it];
         const int64_t qoff = arrays[w.x].qoff + w.y;
-        const int64_t off = arrays[w.x].off;
-        const uint32_t n = arrays[w.x].n;
+        const int64_t off = arrays[w.x].off + arrays[w.x].lead;
+        const uint32_t n = arrays[w.x].n - arrays[w.x].lead;
         for (uint32_t j = threadIdx.x; j < w.z; j += kThreads) {
             // argmins outside the array (-1 for invalid queries) add nothing
             const int32_t li = idx[qoff + j];
@@ -37,35 +37,14 @@ scatter_grad_kernel(const BatchArray *arrays, const uint4 *qitems, int32_t nqite
     }
 }
 
-std::atomic<int> g_batch_per_sm[8];  // full kernels: (aligned, key mode)
-
-template <bool ALIGNED, uint32_t MODE>
-cudaError_t pick_full(const void **fn, int *per_sm) {
-    *fn = reinterpret_cast<const void *>(batch_kernel<ALIGNED, MODE>);
-    return occupancy_cached(batch_kernel<ALIGNED, MODE>, kThreads,
-                            g_batch_per_sm[(ALIGNED ? 4 : 0) + MODE], *per_sm);
-}
-
-template <bool ALIGNED>
-cudaError_t full_kernel_t(uint32_t mode, const void **fn, int *per_sm) {
-    switch (mode) {
-    case kFloatMax: return pick_full<ALIGNED, kFloatMax>(fn, per_sm);
-    case kIntMin: return pick_full<ALIGNED, kIntMin>(fn, per_sm);
-    case kIntMax: return pick_full<ALIGNED, kIntMax>(fn, per_sm);
-    default: return pick_full<ALIGNED, kFloatMin>(fn, per_sm);
-    }
-}
-
-// The kernel a run of this plan launches and its CTAs per SM.
-cudaError_t batch_kernel_for(bool light, bool aligned, uint32_t mode, const void **fn,
-                             size_t smem, int *per_sm) {
-    if (light) return batch_light_kernel(aligned, mode, fn, smem, per_sm);
-    return aligned ? full_kernel_t<true>(mode, fn, per_sm) : full_kernel_t<false>(mode, fn, per_sm);
-}
-
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 }  // namespace
+
+cudaError_t batch_kernel_aligned(uint32_t mode, const void **fn, int *per_sm) {
+    return batch_kernel_t<true>(mode, fn, per_sm);
+}
+
 RMQ_VIOLATIONS_READER(violations_batch)
 
 }  // namespace rmq
@@ -85,7 +64,8 @@ struct rmq_batch {
     BatchParams P;       // device pointers filled, per-run fields left empty
     uint32_t flags;      // RMQ_BUILD_INT32 / RMQ_BUILD_MAX / RMQ_BUILD_LIGHT
     uint32_t kmode;      // KeyMode of every array
-    bool light;          // light index (block and micro-block tables only)
+    int32_t max_levels;  // of the arrays' block tables
+    bool unaligned;      // an array too long for a lead: never the aligned kernel
     int32_t bucket_bs[RMQ_BATCH_BUCKETS];
     rmq_batch_tile_t tiles[RMQ_BATCH_BUCKETS];  // block size and tile schedule per bucket
     const float *built_vals;  // values of the last build enqueued on this plan
@@ -95,18 +75,11 @@ namespace {
 
 int bucket_of(int64_t n) { return n <= 1 ? 0 : ilog2(static_cast<uint32_t>(n)); }
 
-int64_t default_bs(int64_t n, bool light) {
-    // Without autotuning, full index: small blocks, so that a query inside
-    // one block is a short warp scan (the full batched index has no
-    // sub-block level) and the sparse table does the rest; 64 below 2^17
-    // elements, 256 above (what the autotuner picks for the ragged
-    // benchmark, within 5% of it there). Light index: the micro table
-    // answers queries inside a block and settles more of them than the
-    // block table does for queries across blocks, so blocks of 4096 (the
-    // ragged benchmark's queries: 3.1 ms against 8.8 ms at 1024).
-    if (light) return 4096;
-    return n < (1 << 17) ? 64 : 256;
-}
+// Without autotuning: the micro table answers queries inside a block and
+// settles more of them than the block table does for queries across blocks,
+// and its rows grow with the block; 4096 (the ragged benchmark's queries took
+// 3.1 ms at 4096 and 8.8 ms at 1024 with an earlier kernel).
+constexpr int64_t kDefaultBatchBs = 4096;
 
 }  // namespace
 
@@ -158,8 +131,7 @@ int autotune_buckets(int32_t narrays, const int64_t *h_starts, const int64_t *h_
         if (h_lengths[i] > 0) members[bucket_of(h_lengths[i])].push_back(i);  // empty: no structure
     }
     static const int32_t bs_cands[] = {64, 256, 1024, 4096, 16384, 65536};
-    // light plans: small blocks send short queries through the coarser block
-    // probe, so only these, starting from the default; another is taken only
+    // light plans: only these, starting from the default; another is taken only
     // when it is more than 3% faster (per-bucket timings are short and noisy)
     static const int32_t light_cands[] = {4096, 1024, 16384};
     const bool light = (flags & RMQ_BUILD_LIGHT) != 0;
@@ -283,7 +255,7 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
     b->total_q = 0;
     b->mem = nullptr;
     b->flags = flags;
-    b->light = light;
+    b->unaligned = false;
     b->kmode = ((flags & RMQ_BUILD_INT32) ? kIntMin : kFloatMin) + ((flags & RMQ_BUILD_MAX) ? 1u : 0u);
     for (int i = 0; i < RMQ_BATCH_BUCKETS; ++i) {
         const rmq_batch_tile_t t = h_bucket_tiles ? h_bucket_tiles[i] : rmq_batch_tile_t{0, 0, 0, 0};
@@ -294,18 +266,16 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
         b->tiles[i].reserved = 0;
     }
 
-    std::vector<uint2> build;
-    std::vector<std::vector<uint4>> lvl(kMaxLevels);
+    std::vector<uint4> runs;
+    std::vector<std::vector<uint4>> steps(kMaxSteps);
     int64_t ws_entries = 0;
-    int32_t maxlev = 1;
-    uint32_t halo = 0;  // the longest of the plan's tables
+    b->max_levels = 1;
     b->h_arrays.resize(narrays);
     // table item: (array, kind << 16 | level, first, count) at table step `step`
     auto add_items = [&](int step, uint32_t i, uint32_t kind, uint32_t k, uint32_t cnt,
                          uint32_t chunk) {
         for (uint32_t j = 0; j < cnt; j += chunk)
-            lvl[step].push_back(make_uint4(i, (kind << 16) | k, j, std::min(chunk, cnt - j)));
-        maxlev = std::max<int32_t>(maxlev, step + 1);
+            steps[step].push_back(make_uint4(i, (kind << 16) | k, j, std::min(chunk, cnt - j)));
     };
     for (int32_t i = 0; i < narrays; ++i) {
         const int64_t n = h_lengths[i], s = h_starts[i];
@@ -320,62 +290,55 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
         // an empty array has no structure; its queries (if any) are invalid
         const int bk = n > 0 ? bucket_of(n) : 0;
         int64_t bs = n > 0 ? b->bucket_bs[bk] : 1;
-        if (bs <= 0) bs = default_bs(n, light);
+        if (bs <= 0) bs = kDefaultBatchBs;
         const uint32_t qchunk = static_cast<uint32_t>(b->tiles[bk].query_chunk);
         const uint32_t lchunk = static_cast<uint32_t>(b->tiles[bk].level_chunk);
-        // light: blocks on micro-block boundaries, one block of at least 64
-        // for an array shorter than bs
-        if (bs > n) bs = n == 0 ? 1 : (light ? std::max<int64_t>(64, (n + 31) / 32 * 32) : n);
         BatchArray &a = b->h_arrays[i];
         std::memset(&a, 0, sizeof(a));
-        a.off = s;
+        // from the 128-byte boundary before its first element, unless that
+        // takes the positions past 2^31 - 1
+        uint32_t lead = n > 0 ? static_cast<uint32_t>(s & 31) : 0u;
+        if (n + lead > 0x7fffffffLL) {
+            lead = 0;
+            b->unaligned = b->unaligned || s % 4 != 0;
+        }
+        a.off = s - lead;
         a.qoff = qs;
-        a.n = static_cast<uint32_t>(n);
-        a.bs = light && n > 0 ? table_block(static_cast<uint32_t>(bs)) : static_cast<uint32_t>(bs);
-        a.nb = static_cast<uint32_t>((n + a.bs - 1) / a.bs);
+        a.n = static_cast<uint32_t>(n) + lead;
+        a.lead = lead;
+        a.bs = table_block(static_cast<uint32_t>(std::min<int64_t>(bs, std::max<int64_t>(n, 1))));
+        a.nb = (a.n + a.bs - 1) / a.bs;
         a.levels = a.nb > 0 ? st_levels(a.nb) : 0u;
-        a.U = make_unit_layout(a.bs, a.nb);
         a.dv = make_div31(a.bs);
+        a.nmicro = (a.n + kMicro - 1) / kMicro;
+        a.mlevels = a.n > 0 ? micro_levels(a.bs) : 0u;
+        a.moff_bytes = a.mlevels ? micro_offset_bytes(a.mlevels) : 0u;
         a.st = ws_entries;
         ws_entries += static_cast<int64_t>(a.nb) * a.levels;
-        if (light) {
-            a.nmicro = static_cast<uint32_t>((n + kMicro - 1) / kMicro);
-            a.mlevels = n > 0 ? micro_levels(a.bs) : 0u;
-            a.moff_bytes = a.mlevels ? micro_offset_bytes(a.mlevels) : 0u;
-            a.mst = ws_entries;
-            ws_entries += a.nmicro;
-            a.mask = ws_entries = (ws_entries + 1) / 2 * 2;  // 16-byte aligned
-            ws_entries += a.nmicro;
-            a.moff = ws_entries;
-            ws_entries += (static_cast<int64_t>(a.moff_bytes) * a.nmicro * moff_rows(a.mlevels, wide_masks(a.nmicro)) + 7) / 8;
-            a.pre = -1;
-        } else {
-            a.pre = ws_entries;
-            ws_entries += 2 * n;
-        }
+        a.mst = ws_entries;
+        ws_entries += a.nmicro;
+        a.mask = ws_entries;
+        ws_entries += a.nmicro;
+        a.moff = ws_entries;
+        ws_entries += (static_cast<int64_t>(a.moff_bytes) * a.nmicro * moff_rows(a.mlevels, false) + 7) / 8;
         ws_entries = (ws_entries + 31) & ~int64_t(31);  // 256-byte alignment per array
         b->limit = std::max(b->limit, s + n);
         b->total_q = std::max(b->total_q, qs + qc);
-        if (light && a.nmicro > 0) {
-            // A: tiles (micro-block minima, micro table and, when the
-            // blocks' micro-blocks divide a tile, the block minima, from one
-            // read of the values). B: block minima from the micro-block
-            // minima unless the tiles wrote them, then block level k.
-            const uint32_t pb = a.bs / kMicro;
-            halo = std::max(halo, table_halo(a.mlevels));
-            a.light_flags = kMicroTile % pb == 0 ? kLightTileBmin : 0u;
-            for (uint32_t t = 0; t * kMicroTile < a.nmicro; ++t) build.push_back(make_uint2(i, t));
-            const int bstep = (a.light_flags & kLightTileBmin) ? 0 : 1;  // step of block level 0
-            if (bstep == 1)
-                add_items(1, i, kItemBlockMinima, 0, a.nb, std::max<uint32_t>(1u, lchunk / pb));
-            for (uint32_t k = 1; k < a.levels; ++k)
-                add_items(static_cast<int>(k) + bstep, i, kItemBlockLevel, k, a.nb - (1u << k) + 1,
-                          lchunk);
-        } else if (!light) {
-            const uint32_t nunits = unit_count(a.nb, a.U);
-            for (uint32_t u = 0; u < nunits; ++u) build.push_back(make_uint2(i, u));
-            for (uint32_t k = 1; k < a.levels; ++k)
-                add_items(k, i, kItemBlockLevel, k, a.nb - (1u << k) + 1, lchunk);
+        b->max_levels = std::max<int32_t>(b->max_levels, static_cast<int32_t>(a.levels));
+        if (a.n > 0) {
+            // A: runs of units. B, step 1: block minima, rows made apart;
+            // then the block table's levels
+            const uint32_t units = (a.nmicro + kUnit - 1) / kUnit;
+            for (uint32_t u = 0; u < units; u += kRunUnits)
+                runs.push_back(make_uint4(i, u, std::min(kRunUnits, units - u), 0));
+            add_items(1, i, kItemBlockMinima, 0, a.nb, std::max<uint32_t>(8u, lchunk / (a.bs / kMicro)));
+            if (split_rows(a.mlevels)) add_items(1, i, kItemRows, 0, a.nmicro, kBatchRowTile);
+            if (a.nb <= kOneItemTable) {
+                if (a.levels > 1) add_items(2, i, kItemTable, 0, a.nb, a.nb);
+            } else {
+                for (uint32_t k = 0; k + 1 < a.levels; k += kLevelGroup)
+                    add_items(2 + static_cast<int>(k / kLevelGroup), i, kItemLevels, k, a.nb, lchunk);
+            }
         }
         for (int64_t j = 0; j < qc; j += qchunk)
             b->h_qitems.push_back(make_uint4(i, static_cast<uint32_t>(j),
@@ -385,27 +348,25 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
         delete b;
         return set_error(RMQ_EINVAL, "rmq_batch_create: value span too large");
     }
-    std::vector<uint4> lvl_flat;
+    std::vector<uint4> tables;
     BatchParams &P = b->P;
     std::memset(&P, 0, sizeof(P));
-    P.maxlev = maxlev;
-    for (int k = 0; k <= kMaxLevels; ++k) P.lvl_start[k] = 0;
-    for (int k = 1; k < kMaxLevels; ++k) {
-        P.lvl_start[k] = static_cast<int32_t>(lvl_flat.size());
-        lvl_flat.insert(lvl_flat.end(), lvl[k].begin(), lvl[k].end());
+    P.steps = 1;
+    for (int k = 0; k < kMaxSteps; ++k) {
+        P.step_start[k] = static_cast<int32_t>(tables.size());
+        tables.insert(tables.end(), steps[k].begin(), steps[k].end());
+        if (!steps[k].empty()) P.steps = k + 1;
     }
-    P.lvl_start[kMaxLevels] = static_cast<int32_t>(lvl_flat.size());
-    for (int k = maxlev; k < kMaxLevels; ++k) P.lvl_start[k] = P.lvl_start[kMaxLevels];
-    P.nbuild = static_cast<int32_t>(build.size());
+    P.step_start[kMaxSteps] = static_cast<int32_t>(tables.size());
+    P.nruns = static_cast<int32_t>(runs.size());
     P.nqitems = static_cast<int32_t>(b->h_qitems.size());
     P.total_q = b->total_q;
-    P.tile_cap = tile_entries(halo);
 
-    // one allocation: arrays | build | lvl | qitems | counter | workspace
+    // one allocation: arrays | runs | tables | qitems | counter | workspace
     const size_t o_arr = 0;
-    const size_t o_build = align_up(o_arr + sizeof(BatchArray) * narrays, 256);
-    const size_t o_lvl = align_up(o_build + sizeof(uint2) * build.size(), 256);
-    const size_t o_q = align_up(o_lvl + sizeof(uint4) * lvl_flat.size(), 256);
+    const size_t o_runs = align_up(o_arr + sizeof(BatchArray) * narrays, 256);
+    const size_t o_tables = align_up(o_runs + sizeof(uint4) * runs.size(), 256);
+    const size_t o_q = align_up(o_tables + sizeof(uint4) * tables.size(), 256);
     const size_t o_cnt = align_up(o_q + sizeof(uint4) * b->h_qitems.size(), 256);
     const size_t o_ws = align_up(o_cnt + 256, 256);
     b->ws_bytes = sizeof(Entry) * static_cast<size_t>(ws_entries);
@@ -420,11 +381,11 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
     char *base = static_cast<char *>(b->mem);
     err = cudaMemcpy(base + o_arr, b->h_arrays.data(), sizeof(BatchArray) * narrays,
                      cudaMemcpyHostToDevice);
-    if (err == cudaSuccess && !build.empty())
-        err = cudaMemcpy(base + o_build, build.data(), sizeof(uint2) * build.size(),
+    if (err == cudaSuccess && !runs.empty())
+        err = cudaMemcpy(base + o_runs, runs.data(), sizeof(uint4) * runs.size(),
                          cudaMemcpyHostToDevice);
-    if (err == cudaSuccess && !lvl_flat.empty())
-        err = cudaMemcpy(base + o_lvl, lvl_flat.data(), sizeof(uint4) * lvl_flat.size(),
+    if (err == cudaSuccess && !tables.empty())
+        err = cudaMemcpy(base + o_tables, tables.data(), sizeof(uint4) * tables.size(),
                          cudaMemcpyHostToDevice);
     if (err == cudaSuccess && !b->h_qitems.empty())
         err = cudaMemcpy(base + o_q, b->h_qitems.data(), sizeof(uint4) * b->h_qitems.size(),
@@ -437,8 +398,8 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
         return rc;
     }
     P.arrays = reinterpret_cast<const BatchArray *>(base + o_arr);
-    P.build = reinterpret_cast<const uint2 *>(base + o_build);
-    P.lvl = reinterpret_cast<const uint4 *>(base + o_lvl);
+    P.runs = reinterpret_cast<const uint4 *>(base + o_runs);
+    P.tables = reinterpret_cast<const uint4 *>(base + o_tables);
     P.qitems = reinterpret_cast<const uint4 *>(base + o_q);
     P.invalid = reinterpret_cast<unsigned long long *>(base + o_cnt);
     P.ws = reinterpret_cast<Entry *>(base + o_ws);
@@ -478,17 +439,17 @@ static int launch_batch(rmq_batch_t *b, const float *d_vals, const int32_t *d_qu
     P.val = d_val;
     P.idx = d_idx;
     P.phases = phases;
-    const bool aligned = reinterpret_cast<uintptr_t>(d_vals) % 16 == 0;
+    const bool aligned = reinterpret_cast<uintptr_t>(d_vals) % 16 == 0 && !b->unaligned;
     const void *kern = nullptr;
-    const size_t smem = b->light ? light_smem(P.tile_cap) : 0;
     int per_sm = 0;
-    cudaError_t err = batch_kernel_for(b->light, aligned, b->kmode, &kern, smem, &per_sm);
+    cudaError_t err = aligned ? batch_kernel_aligned(b->kmode, &kern, &per_sm)
+                              : batch_kernel_unaligned(b->kmode, &kern, &per_sm);
     if (err != cudaSuccess) return cuda_fail(err, who);
     // a cooperative launch needs every CTA resident
     if (per_sm < 1) return set_error(RMQ_ENOTSUP, "%s: kernel cannot be resident", who);
     const unsigned grid = static_cast<unsigned>(dev.sms * per_sm);
     void *args[] = {&P};
-    err = cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kThreads), args, smem, stream);
+    err = cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kThreads), args, kBatchSmem, stream);
     if (err != cudaSuccess) return cuda_fail(err, who);
     if (phases & 1u) b->built_vals = d_vals;
     return RMQ_OK;
@@ -535,29 +496,26 @@ int rmq_batch_run_per_array(rmq_batch_t *b, const float *d_vals, const int32_t *
         const BatchArray &a = b->h_arrays[i];
         BuildPlan p;
         std::memset(&p, 0, sizeof(p));
-        p.A = d_vals + a.off;
+        p.A = d_vals;
+        p.off = a.off;
+        p.limit = b->limit;
+        p.lead = a.lead;
         p.n = a.n;
         p.bs = a.bs;
         p.tbs = a.bs;
         p.nb = a.nb;
         p.levels = a.levels;
-        p.aligned = reinterpret_cast<uintptr_t>(p.A) % 16 == 0;
-        p.st = ws + a.st;
+        p.aligned = reinterpret_cast<uintptr_t>(d_vals) % 16 == 0 && a.off % 4 == 0;
         p.kmode = b->kmode;
-        p.light = b->light;
-        if (b->light) {
-            // the plain light index over the plan's own workspace layout
-            p.micro = true;
-            p.nmicro = a.nmicro;
-            p.mlevels = a.mlevels;
-            p.mst = ws + a.mst;
-            p.mask = ws + a.mask;
-            p.moff = ws + a.moff;
-            p.moff_bytes = a.moff_bytes;
-        } else {
-            p.pre = ws + a.pre;
-            p.suf = ws + a.pre + a.n;
-        }
+        p.light = true;
+        p.micro = true;
+        p.nmicro = a.nmicro;
+        p.mlevels = a.mlevels;
+        p.moff_bytes = a.moff_bytes;
+        p.st = ws + a.st;
+        p.mst = ws + a.mst;
+        p.mask = ws + a.mask;
+        p.moff = ws + a.moff;
         cudaError_t err = launch_build(p, dev, stream);
         if (err != cudaSuccess) return cuda_fail(err, "rmq_batch_run_per_array: build");
         if (qcount[i] == 0) continue;
@@ -604,9 +562,9 @@ int rmq_batch_info(const rmq_batch_t *b, rmq_batch_info_t *info) {
     info->queries_span = b->total_q;
     info->workspace_bytes = static_cast<int64_t>(b->ws_bytes);
     info->device_bytes = static_cast<int64_t>(b->mem_bytes);
-    info->build_items = b->P.nbuild;
+    info->build_items = b->P.nruns;
     info->query_items = b->P.nqitems;
-    info->max_levels = b->P.maxlev;
+    info->max_levels = b->max_levels;
     info->flags = static_cast<int32_t>(b->flags);
     for (int i = 0; i < RMQ_BATCH_BUCKETS; ++i) info->bucket_bs[i] = b->bucket_bs[i];
     return RMQ_OK;

@@ -1,75 +1,70 @@
-// batch_impl.cuh -- the persistent batch kernels, shared by batch.cu (full
-// index: per-element prefix / suffix entries) and batch_light.cu (light
-// index: block and micro-block tables only). Each translation unit
-// instantiates only its own kernels.
+// batch_impl.cuh -- the persistent batch kernel, instantiated by batch.cu
+// (16-byte aligned values) and batch_unaligned.cu.
 //
-// Persistent kernel, three phases separated by grid-wide barriers of a
-// cooperative launch (all CTAs are co-resident, guaranteed by the launch):
-//   A  build items. Full: (array, unit) prefix/suffix minima + block minima,
-//      the plain builder's CTA body (build_impl.cuh). Light: (array, tile)
-//      micro-block minima, every micro-table level and the block minima of
-//      a tile, from one read of its values (light_tile); for block sizes
-//      above 65536, (array, chunk) micro-block minima only;
-//   B  table items (array, kind | level, first entry, count), one step per
-//      barrier: block-table level k at step k (at step k + 1 when step 1
-//      computes the block minima from the micro-block minima), and for
-//      untiled light arrays micro-table level k at step k;
-//   C  query items (array, first query, count), query_impl.cuh's queued
-//      form (light: misses settle from value lines, no entries).
+// Persistent kernel, phases separated by grid-wide barriers of a cooperative
+// launch (all CTAs are co-resident, guaranteed by the launch):
+//   A  run items (array, first unit, units): micro-block minima and micro
+//      table, the plain builder's CTA body (build_run, tables_impl.cuh);
+//   B  table items (array, kind | level, first, count), one step per barrier:
+//      the block minima and the rows made apart from the masks at step 1, the
+//      block table's levels after them;
+//   C  query items (array, first query, count), query_impl.cuh's queued form.
 // Work lists are built on the host once per plan, so a run allocates nothing
 // and can be captured in a CUDA graph.
+//
+// An array is built from the 128-byte boundary (32 values) at or before its
+// first element on: its micro-blocks are whole 128-byte lines whatever its
+// offset, so rows stored back to back take 16-byte copies too.
 #pragma once
 
 #include <cooperative_groups.h>
 
-#include "build_impl.cuh"
 #include "engine.h"
 #include "query_impl.cuh"
 #include "tables_impl.cuh"
 
-// CTAs per SM the persistent batch kernels are compiled for (a register bound).
+// CTAs per SM the persistent batch kernel is compiled for (a register bound).
 #ifndef RMQ_BATCH_MINB
 #define RMQ_BATCH_MINB 4
-#endif
-#ifndef RMQ_BATCH_LIGHT_MINB
-#define RMQ_BATCH_LIGHT_MINB 3  // the light-index kernels
 #endif
 
 namespace rmq {
 
-constexpr int kBatchThreads = kBuildThreads;  // phase A runs the unit builder
+constexpr int kBatchThreads = kUnit;  // phase A runs the table builder
 constexpr int kBatchQPT = 2;
 // default tile schedule: queries per query item, table entries per level
 // item (a plan can set both per size bucket, rmq_batch_create_ex)
 constexpr uint32_t kQueryChunk = 2048;
 constexpr uint32_t kLevelChunk = 4096;
-constexpr int kMaxLevels = 32;
+constexpr int kMaxSteps = 16;
+// units (of 256 micro-blocks) per run item: 512 KB of values, so that the 63
+// to 255 micro-blocks a run reads beyond its end stay below a few percent
+constexpr uint32_t kRunUnits = 16;
+// positions per item of rows made apart, and the largest block table that one
+// item takes through all its levels: both fit the run's shared memory
+constexpr uint32_t kBatchRowTile = 1024;
+constexpr uint32_t kOneItemTable = 2048;
 
-// kinds of table items (bits 16.. of the item's second word; bits 0..15
-// hold the level)
+// kinds of table items (bits 16.. of the item's second word; bits 0..15 hold
+// the level)
 enum : uint32_t {
-    kItemBlockLevel = 0,   // block-table level k from level k - 1
-    kItemBlockMinima = 1,  // block-table level 0 from the micro-block minima
+    kItemBlockMinima = 0,  // block minima from the micro-block minima
+    kItemRows = 1,         // offset rows (split_rows)
+    kItemTable = 2,        // every level of a small block table
+    kItemLevels = 3,       // levels k + 1 .. k + kLevelGroup of a larger one
 };
-// Light tiles (phase A items of a light array): kMicroTile micro-blocks whose
-// minima, micro table and the minima of the blocks inside come from one read
-// of the tile's values plus a halo of table_halo(mlevels) micro-blocks. The
-// table is built in shared memory (tables_impl.cuh).
-constexpr uint32_t kMicroTile = 2048;
-// BatchArray::light_flags
-constexpr uint32_t kLightTileBmin = 1;    // tiles also write the block minima (bs / 32 divides the tile)
 
 struct BatchArray {
-    int64_t off;    // first value in the buffer
+    int64_t off;    // the 128-byte boundary its index starts at (values)
     int64_t qoff;   // first query
-    int64_t pre;    // workspace entry offset of pre[]; suf[] follows at pre + n (full)
-    int64_t st;     // workspace entry offset of the sparse table
-    int64_t mst;    // workspace entry offset of the micro-block minima (light)
-    int64_t mask;   // workspace entry offset of the micro table's masks (light)
-    int64_t moff;   // workspace entry offset of its offset rows (light)
-    uint32_t n, bs, nb, levels;
-    uint32_t nmicro, mlevels, moff_bytes, light_flags;
-    UnitLayout U;
+    int64_t st;     // workspace entry offset of the block table
+    int64_t mst;    // ... of the micro-block minima
+    int64_t mask;   // ... of the micro table's masks
+    int64_t moff;   // ... of its offset rows
+    uint32_t n;     // elements from off on
+    uint32_t lead;  // of which the first `lead` are not the array's
+    uint32_t bs, nb, levels;
+    uint32_t nmicro, mlevels, moff_bytes;
     Div31 dv;
 };
 
@@ -82,275 +77,150 @@ struct BatchParams {
     unsigned long long *invalid;
     Entry *ws;
     const BatchArray *arrays;
-    const uint2 *build;
-    int32_t nbuild;
-    const uint4 *lvl;
-    int32_t maxlev;   // table steps run: 1 .. maxlev - 1
-    int32_t lvl_start[kMaxLevels + 1];
+    const uint4 *runs;
+    int32_t nruns;
+    const uint4 *tables;
+    int32_t steps;        // table steps run: 1 .. steps - 1
+    int32_t step_start[kMaxSteps + 1];
     const uint4 *qitems;
     int32_t nqitems;
-    int64_t total_q;  // one past the last query any array owns
-    uint32_t tile_cap;  // light: minima per tile buffer
-    uint32_t phases;  // bit 0 build, bit 1 table levels, bit 2 queries
+    int64_t total_q;      // one past the last query any array owns
+    uint32_t phases;      // bit 0 runs, bit 1 table steps, bit 2 queries
 };
 
-// Minima of a tile and its halo: the longest (blocks of 2^15), and of a plan
-// whose largest halo is `halo` (BatchParams::tile_cap).
-constexpr uint32_t kTileEntries = kMicroTile + 1024u;
-inline uint32_t tile_entries(uint32_t halo) { return (kMicroTile + halo + 1u) & ~1u; }
-// Dynamic shared memory of a light batch CTA: the tile's buffers in phase A,
-// the warps' miss queues in phase C. A plan asks for what its own tiles need:
-// the rest is L1 for its queries.
-inline size_t light_smem(uint32_t tile_cap) { return table_smem(tile_cap); }
-static_assert(sizeof(MissQueue<true>) * (kBatchThreads / 32) <= table_smem(kMicroTile),
-              "miss queues fit");
+// Dynamic shared memory of a CTA: the run's buffers in phase A, buffers of
+// two halves in phase B, the warps' miss queues in phase C.
+constexpr size_t kBatchSmem = sizeof(TableSmem);
+static_assert(2 * sizeof(Entry) * (kBatchRowTile + 1024) <= kBatchSmem, "row tiles fit");
+static_assert(2 * sizeof(Entry) * kOneItemTable <= kBatchSmem, "small tables fit");
+static_assert(sizeof(MissQueue<true>) * (kBatchThreads / 32) <= kBatchSmem, "miss queues fit");
 
-// Light kernels (batch_light.cu): the instantiation for (aligned, key mode),
-// CTAs per SM with `smem` bytes of dynamic shared memory (the limit set).
-cudaError_t batch_light_kernel(bool aligned, uint32_t mode, const void **fn, size_t smem,
-                               int *per_sm);
+// The instantiation for (aligned, key mode) and its CTAs per SM (its limit of
+// dynamic shared memory set).
+cudaError_t batch_kernel_aligned(uint32_t mode, const void **fn, int *per_sm);
+cudaError_t batch_kernel_unaligned(uint32_t mode, const void **fn, int *per_sm);
 
 namespace {
 
 namespace cg = cooperative_groups;
 
-template <bool LIGHT, uint32_t MODE>
+template <uint32_t MODE>
 __device__ __forceinline__ V1View batch_view(const BatchParams &P, const BatchArray &a) {
     V1View v;
     v.A = P.A;
     v.off = a.off;
     v.limit = P.limit;
     v.n = a.n;
+    v.lead = a.lead;
     v.bs = a.bs;
     v.nb = a.nb;
     v.dv = a.dv;
     v.st = P.ws + a.st;
+    v.mst = P.ws + a.mst;
+    v.mask = P.ws + a.mask;
+    v.wide = wide_masks(a.nmicro);
+    v.moff = P.ws + a.moff;
+    v.moff_bytes = a.moff_bytes;
+    v.nmicro = a.nmicro;
+    v.pre = nullptr;
+    v.suf = nullptr;
     v.kmode = MODE;
     v.levels = a.levels;
-    v.light = LIGHT;
-    if (LIGHT) {
-        v.pre = nullptr;
-        v.suf = nullptr;
-        v.mst = P.ws + a.mst;
-        v.mask = P.ws + a.mask;
-        v.wide = wide_masks(a.nmicro);
-        v.moff = P.ws + a.moff;
-        v.moff_bytes = a.moff_bytes;
-        v.nmicro = a.nmicro;
-        v.mlevels = a.mlevels;
-        v.micro_span = (1u << a.mlevels) - 1u;
-    } else {
-        // full batched arrays answer same-block queries with warp scans
-        v.pre = P.ws + a.pre;
-        v.suf = P.ws + a.pre + a.n;
-        v.mst = nullptr;
-        v.mask = nullptr;
-        v.wide = false;
-        v.moff = nullptr;
-        v.moff_bytes = 0u;
-        v.nmicro = 0;
-        v.mlevels = 0u;
-        v.micro_span = 0u;
-    }
+    v.mlevels = a.mlevels;
+    v.micro_span = (1u << a.mlevels) - 1u;
+    v.light = true;
     return v;
 }
 
-template <uint32_t MODE>
-__device__ __forceinline__ UnitJob unit_job(const BatchParams &P, uint32_t array) {
-    const BatchArray a = P.arrays[array];
-    UnitJob J;
-    J.A = P.A;
-    J.off = a.off;
-    J.limit = P.limit;
-    J.n = a.n;
-    J.bs = a.bs;
-    J.U = a.U;
-    J.dv = a.dv;
-    J.pre = P.ws + a.pre;
-    J.suf = P.ws + a.pre + a.n;
-    J.bmin = P.ws + a.st;
-    J.kmode = MODE;
-    J.nb = a.nb;
-    return J;
-}
-
-// Light table step, kind kItemBlockMinima: block minima of blocks [first,
-// first + count) from the micro-block minima (bs / 32 per block): a thread
-// per block for small blocks, a warp per block otherwise.
-__device__ __forceinline__ void light_block_minima(const BatchParams &P, const BatchArray &a,
-                                                   uint32_t first, uint32_t count) {
-    const Entry *mst = P.ws + a.mst;
-    Entry *bmin = P.ws + a.st;
-    const uint32_t pb = a.bs / kMicroElems;
-    if (pb <= 16u) {
-        for (uint32_t b = first + threadIdx.x; b < first + count; b += kBatchThreads) {
-            Entry m = kEntryNone;
-            const uint32_t j1 = min(b * pb + pb, a.nmicro);
-            for (uint32_t j = b * pb; j < j1; ++j) m = better(m, mst[j]);
-            if (rmq_chk(b < a.nb)) bmin[b] = m;
-        }
-        return;
-    }
-    const uint32_t lane = threadIdx.x & 31u;
-    for (uint32_t b = first + (threadIdx.x >> 5); b < first + count; b += kBatchThreads / 32) {
-        Entry m = kEntryNone;
-        const uint32_t j1 = min(b * pb + pb, a.nmicro);
-        for (uint32_t j = b * pb + lane; j < j1; j += 32u) m = better(m, mst[j]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = better(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (lane == 0u && rmq_chk(b < a.nb)) bmin[b] = m;
-    }
-}
-
-// Light phase A, one tile: the minima of micro-blocks [t0, t0 + count + halo)
-// from the values into shared memory (8 rows of 512 bytes per warp step, all
-// loads in flight), the tile's own minima to the micro-block minima table,
-// the minima of the blocks inside the tile (kLightTileBmin), and the micro
-// table at [t0, t0 + count). The halo's minima are computed again by the
-// next tile.
-template <bool ALIGNED, uint32_t MODE>
-__device__ __forceinline__ void light_tile(const BatchParams &P, const BatchArray &a, uint32_t t,
-                                           unsigned char *smem) {
-    Entry *key = reinterpret_cast<Entry *>(smem);
-    uint32_t *keys = reinterpret_cast<uint32_t *>(key + 2 * P.tile_cap);
-    const uint32_t t0 = t * kMicroTile;
-    const uint32_t count = min(kMicroTile, a.nmicro - t0);
-    const uint32_t jend = min(t0 + count + table_halo(a.mlevels), a.nmicro);
-    const uint32_t e = jend - t0;  // minima held in shared memory (<= P.tile_cap)
-    const float *A = P.A + a.off;
-    const bool vec = ALIGNED && a.off % 4 == 0;
-    // 8 rows (32 micro-blocks, 4 KB) per warp step: 96 KB of loads in flight per SM
-    constexpr uint32_t kRows = 8, kPerWarp = 4 * kRows;
-    for (uint32_t j0 = t0 + (threadIdx.x >> 5) * kPerWarp; j0 < jend;
-         j0 += kPerWarp * (kBatchThreads / 32)) {
-        if (vec && (j0 + kPerWarp) * kMicroElems <= a.n)
-            micro_min_rows<MODE, true, kRows>(A, a.n, j0, jend, key, t0);
-        else
-            micro_min_rows<MODE, false, kRows>(A, a.n, j0, jend, key, t0);
-    }
-    __syncthreads();
-    Entry *mst = P.ws + a.mst;
-    for (uint32_t i = threadIdx.x; i < count; i += kBatchThreads) mst[t0 + i] = key[i];
-    if (a.light_flags & kLightTileBmin) {
-        // blocks [t0 / pb, (t0 + count - 1) / pb], all inside the tile
-        const uint32_t pb = a.bs / kMicroElems;
-        const uint32_t b0 = t0 / pb, nbt = (count + pb - 1) / pb;
-        Entry *bmin = P.ws + a.st;
-        if (pb <= 16u) {
-            for (uint32_t x = threadIdx.x; x < nbt; x += kBatchThreads) {
-                Entry mm = kEntryNone;
-                const uint32_t j1 = min(x * pb + pb, count);
-                for (uint32_t j = x * pb; j < j1; ++j) mm = better(mm, key[j]);
-                if (rmq_chk(b0 + x < a.nb)) bmin[b0 + x] = mm;
-            }
-        } else {
-            const uint32_t lane = threadIdx.x & 31u;
-            for (uint32_t x = threadIdx.x >> 5; x < nbt; x += kBatchThreads / 32) {
-                Entry mm = kEntryNone;
-                const uint32_t j1 = min(x * pb + pb, count);
-                for (uint32_t j = x * pb + lane; j < j1; j += 32u) mm = better(mm, key[j]);
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) mm = better(mm, __shfl_xor_sync(0xffffffffu, mm, o));
-                if (lane == 0u && rmq_chk(b0 + x < a.nb)) bmin[b0 + x] = mm;
-            }
-        }
-    }
-    tile_keys<kBatchThreads>(key, e, keys);
-    __syncthreads();
+__device__ __forceinline__ MicroTable batch_table(const BatchParams &P, const BatchArray &a) {
     MicroTable T;
-    T.mst = mst;
+    T.mst = P.ws + a.mst;
     T.mask = P.ws + a.mask;
     T.moff = P.ws + a.moff;
     T.moff_bytes = a.moff_bytes;
     T.nmicro = a.nmicro;
     T.mlevels = a.mlevels;
-    // its rows overwrite `key` only behind a barrier, after the block minima
-    // and the table copy above have read it
-    table_tile<kBatchThreads>(T, t0, count, e, key, key + P.tile_cap, keys,
-                              keys + key_words(P.tile_cap));
-    __syncthreads();  // the next tile overwrites the buffers
+    return T;
 }
 
-// Phase B: table steps 1 .. maxlev - 1, a grid barrier after each.
-template <bool LIGHT>
-__device__ __forceinline__ void table_steps(const BatchParams &P, cg::grid_group &grid) {
-    for (int s = 1; (P.phases & 2u) && s < P.maxlev; ++s) {
-        for (int32_t it = P.lvl_start[s] + blockIdx.x; it < P.lvl_start[s + 1]; it += gridDim.x) {
-            const uint4 w = P.lvl[it];
+// Phase B: table steps 1 .. steps - 1, a grid barrier after each.
+__device__ __forceinline__ void table_steps(const BatchParams &P, cg::grid_group &grid,
+                                            unsigned char *smem) {
+    for (int s = 1; (P.phases & 2u) && s < P.steps; ++s) {
+        for (int32_t it = P.step_start[s] + blockIdx.x; it < P.step_start[s + 1]; it += gridDim.x) {
+            const uint4 w = P.tables[it];
             const BatchArray &a = P.arrays[w.x];
             const uint32_t kind = w.y >> 16, k = w.y & 0xffffu;
-            if (LIGHT && kind == kItemBlockMinima) {
-                light_block_minima(P, a, w.z, w.w);
-            } else {
-                const Entry *__restrict__ prev = P.ws + a.st + static_cast<int64_t>(k - 1) * a.nb;
-                Entry *__restrict__ cur = P.ws + a.st + static_cast<int64_t>(k) * a.nb;
-                const uint32_t half = 1u << (k - 1);
-                for (uint32_t j = w.z + threadIdx.x; j < w.z + w.w; j += kBatchThreads)
-                    if (rmq_chk(j + half < a.nb)) cur[j] = better(prev[j], prev[j + half]);
-            }
+            Entry *st = P.ws + a.st;
+            if (kind == kItemBlockMinima)
+                block_minima<kBatchThreads>(P.ws + a.mst, a.nmicro, a.bs / 32u, w.z, w.z + w.w, a.nb, st);
+            else if (kind == kItemRows)
+                rows_tile_global<kBatchThreads>(batch_table(P, a), w.z, w.w, smem);
+            else if (kind == kItemTable)
+                all_levels<kBatchThreads>(st, a.nb, a.levels, reinterpret_cast<Entry *>(smem));
+            else
+                level_group<kBatchThreads>(st, a.nb, k, min(kLevelGroup, a.levels - 1u - k), w.z, w.w);
         }
         grid.sync();
     }
 }
 
 // Phase C: the query items, in the queued form.
-template <bool ALIGNED, bool LIGHT, uint32_t MODE>
-__device__ __forceinline__ void query_items(const BatchParams &P, MissQueue<LIGHT> &mq) {
+template <bool ALIGNED, uint32_t MODE>
+__device__ __forceinline__ void query_items(const BatchParams &P, MissQueue<true> &mq) {
     for (int32_t it = (P.phases & 4u) ? blockIdx.x : P.nqitems; it < P.nqitems; it += gridDim.x) {
         const uint4 w = P.qitems[it];
         const BatchArray a = P.arrays[w.x];
-        const V1View v = batch_view<LIGHT, MODE>(P, a);
+        const V1View v = batch_view<MODE>(P, a);
         QueryOut o;
         o.Q = P.Q + a.qoff;
         o.val = P.val ? P.val + a.qoff : nullptr;
         o.idx = P.idx ? P.idx + a.qoff : nullptr;
         o.invalid = P.invalid;
         o.span = P.total_q - a.qoff;
-        answer_range_queued<ALIGNED, LIGHT, MODE, kBatchThreads, kBatchQPT>(
+        answer_range_queued<ALIGNED, true, MODE, true, kBatchThreads, kBatchQPT>(
             v, o, w.y, static_cast<int64_t>(w.y) + w.z, mq);
     }
 }
 
-// Full index: prefix / suffix entries per element, warp scans for queries
-// inside one block.
 template <bool ALIGNED, uint32_t MODE>
 __global__ void __launch_bounds__(kBatchThreads, RMQ_BATCH_MINB) batch_kernel(BatchParams P) {
-    __shared__ __align__(16) Entry stage[kStageEntries];
-    __shared__ uint64_t s_warp[kWarpSlots];
-    __shared__ uint32_t s_flag[2 * kBuildWarps];
+    extern __shared__ __align__(1024) unsigned char s_batch[];
     cg::grid_group grid = cg::this_grid();
-
-    // A: units
-    for (int32_t it = (P.phases & 1u) ? blockIdx.x : P.nbuild; it < P.nbuild; it += gridDim.x) {
-        const uint2 w = P.build[it];
-        build_unit<ALIGNED, MODE>(unit_job<MODE>(P, w.x), w.y, stage, s_warp, s_flag);
+    for (int32_t it = (P.phases & 1u) ? blockIdx.x : P.nruns; it < P.nruns; it += gridDim.x) {
+        const uint4 w = P.runs[it];
+        const BatchArray &a = P.arrays[w.x];
+        const uint32_t lo = w.y * kUnit;
+        build_run<ALIGNED, MODE>(P.A, P.limit, a.off, a.n, a.lead, P.ws + a.mst, batch_table(P, a), lo,
+                                 min(lo + w.z * kUnit, a.nmicro), *reinterpret_cast<TableSmem *>(s_batch));
     }
     grid.sync();
-    table_steps<false>(P, grid);
-    // C: the warps' miss queues live in the staging memory of phase A
-    static_assert(sizeof(MissQueue<false>) * (kBatchThreads / 32) <= sizeof(Entry) * kStageEntries,
-                  "miss queues fit the staging memory");
-    query_items<ALIGNED, false, MODE>(
-        P, reinterpret_cast<MissQueue<false> *>(stage)[threadIdx.x >> 5]);
+    table_steps(P, grid, s_batch);
+    query_items<ALIGNED, MODE>(P, reinterpret_cast<MissQueue<true> *>(s_batch)[threadIdx.x >> 5]);
 }
 
-// Light index: block and micro-block tables only, light_smem() bytes of
-// dynamic shared memory.
-template <bool ALIGNED, uint32_t MODE>
-__global__ void __launch_bounds__(kBatchThreads, RMQ_BATCH_LIGHT_MINB)
-batch_kernel_light(BatchParams P) {
-    extern __shared__ __align__(128) unsigned char s_light[];
-    cg::grid_group grid = cg::this_grid();
+std::atomic<int> g_batch_per_sm[4];  // per key mode, of this unit's alignment
 
-    // A: tiles (micro-block minima, micro table, block minima)
-    for (int32_t it = (P.phases & 1u) ? blockIdx.x : P.nbuild; it < P.nbuild; it += gridDim.x) {
-        const uint2 w = P.build[it];
-        light_tile<ALIGNED, MODE>(P, P.arrays[w.x], w.y, s_light);
+template <bool ALIGNED, uint32_t MODE>
+cudaError_t pick_batch(const void **fn, int *per_sm) {
+    auto kern = batch_kernel<ALIGNED, MODE>;
+    if (g_batch_per_sm[MODE].load(std::memory_order_relaxed) == 0) {
+        const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     static_cast<int>(kBatchSmem));
+        if (err != cudaSuccess) return err;
     }
-    grid.sync();
-    table_steps<true>(P, grid);
-    query_items<ALIGNED, true, MODE>(
-        P, reinterpret_cast<MissQueue<true> *>(s_light)[threadIdx.x >> 5]);
+    *fn = reinterpret_cast<const void *>(kern);
+    return occupancy_cached(kern, kBatchThreads, g_batch_per_sm[MODE], *per_sm, kBatchSmem);
+}
+
+template <bool ALIGNED>
+cudaError_t batch_kernel_t(uint32_t mode, const void **fn, int *per_sm) {
+    switch (mode) {
+    case kFloatMax: return pick_batch<ALIGNED, kFloatMax>(fn, per_sm);
+    case kIntMin: return pick_batch<ALIGNED, kIntMin>(fn, per_sm);
+    case kIntMax: return pick_batch<ALIGNED, kIntMax>(fn, per_sm);
+    default: return pick_batch<ALIGNED, kFloatMin>(fn, per_sm);
+    }
 }
 
 }  // namespace

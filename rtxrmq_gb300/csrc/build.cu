@@ -9,6 +9,7 @@
 //   st[k][j] = leftmost minimum of blocks j .. j + 2^k - 1 (k = 0: block minima)
 #include "build_impl.cuh"
 #include "engine.h"
+#include "minima_impl.cuh"
 #include "tables_impl.cuh"
 
 // CTAs per SM the unit kernel is compiled for (a register bound).
@@ -39,102 +40,110 @@ void launch_units(const UnitJob &J, uint32_t nunits, uint32_t grid, cudaStream_t
     }
 }
 
-__global__ void st_level_kernel(Entry *st, uint32_t nb, uint32_t k) {
-    const Entry *prev = st + static_cast<size_t>(k - 1) * nb;
-    Entry *cur = st + static_cast<size_t>(k) * nb;
-    const uint32_t half = 1u << (k - 1);
-    const uint32_t cnt = nb - (1u << k) + 1;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt;
-         j += gridDim.x * blockDim.x)
-        if (rmq_chk(j + half < nb)) cur[j] = better(prev[j], prev[j + half]);
+// Micro-block minima and the micro table (build_run): a run of `units` units
+// of micro-blocks per CTA.
+#ifndef RMQ_TABLE_MINB
+#define RMQ_TABLE_MINB 4
+#endif
+template <bool ALIGNED, uint32_t MODE>
+__global__ void __launch_bounds__(kUnit, RMQ_TABLE_MINB)
+table_kernel(const float *__restrict__ A, int64_t limit, int64_t base, uint32_t n, uint32_t lead,
+             Entry *mst, MicroTable T, uint32_t units) {
+    extern __shared__ __align__(1024) unsigned char s_table[];
+    const uint32_t lo = blockIdx.x * units * kUnit;
+    build_run<ALIGNED, MODE>(A, limit, base, n, lead, mst, T, lo, min(lo + units * kUnit, T.nmicro),
+                             *reinterpret_cast<TableSmem *>(s_table));
 }
 
-constexpr int kTableThreads = 256;
+// Block minima: a thread per block of up to 16 micro-blocks, else a warp.
+constexpr int kBlockThreads = 256;
+__global__ void __launch_bounds__(kBlockThreads)
+block_minima_kernel(const Entry *__restrict__ mst, uint32_t nmicro, uint32_t pb, Entry *bmin,
+                    uint32_t nb, uint32_t per_cta) {
+    const uint32_t b0 = blockIdx.x * per_cta;
+    block_minima<kBlockThreads>(mst, nmicro, pb, b0, min(b0 + per_cta, nb), nb, bmin);
+}
 
-// The micro table (masks and offset rows) from the micro-block minima, one
-// tile of consecutive positions per CTA.
-__global__ void __launch_bounds__(kTableThreads)
-table_kernel(MicroTable T, uint32_t tile) {
+// The offset rows apart (split_rows), one tile of kRowTile positions per CTA.
+constexpr uint32_t kRowTile = 2048;
+__global__ void __launch_bounds__(512) rows_kernel(MicroTable T) {
     extern __shared__ __align__(16) unsigned char s_tile[];
-    const uint32_t t0 = blockIdx.x * tile;
-    table_tile_global<kTableThreads>(T, t0, min(tile, T.nmicro - t0), s_tile);
+    const uint32_t t0 = blockIdx.x * kRowTile;
+    rows_tile_global<512>(T, t0, min(kRowTile, T.nmicro - t0), s_tile);
 }
 
-// One pass over the values: the minimum of every 32-element
-// micro-block (level 0 of the micro table) and, folded in with a 64-bit
-// atomic minimum, of every block (level 0 of the block table, filled with
-// all-ones before; bs a multiple of 32, so every micro-block lies in one
-// block). A warp takes 16 consecutive micro-blocks per step: four 512-byte
-// rows, each lane 4 consecutive elements of every row, all four loads in
-// flight before any reduction; 8 lanes reduce one micro-block. When the 16
-// micro-blocks lie in one block (bs a multiple of 512, or away from block
-// edges) the warp folds them into that block with a single atomic.
+constexpr int kLevelThreads = 1024;
+constexpr uint32_t kSmallTable = 4096;
+__global__ void __launch_bounds__(kLevelThreads)
+small_levels_kernel(Entry *st, uint32_t nb, uint32_t levels) {
+    extern __shared__ Entry s_level[];
+    all_levels<kLevelThreads>(st, nb, levels, s_level);
+}
 
-template <uint32_t MODE>
-__global__ void __launch_bounds__(256)
-micro_min_kernel(const float *__restrict__ A, uint32_t n, uint32_t nmicro, uint32_t per_block,
-                 Entry *mst0, Entry *bmin, bool aligned) {
-    static_assert(kMicroElems == kMicro, "micro-block size");
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t sub = lane & 7u;
-    const uint32_t grp = lane >> 3;
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    const uint32_t nblocks = (nmicro + per_block - 1) / per_block;
-    for (uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-         w * kMicroPerWarp < nmicro; w += warps) {
-        const uint32_t j0 = w * kMicroPerWarp;
-        Entry m[4];  // micro-block j0 + 4i + grp, on all 8 lanes of the group
-        if (aligned && (j0 + kMicroPerWarp) * kMicro <= n)
-            micro_min_warp<MODE, true>(A, n, j0, nmicro, mst0, 0u, m);
-        else
-            micro_min_warp<MODE, false>(A, n, j0, nmicro, mst0, 0u, m);
-        const uint32_t jl = min(j0 + kMicroPerWarp, nmicro) - 1u;
-        if (j0 / per_block == jl / per_block) {
-            // one block: micro-blocks past nmicro hold kEntryNone, the identity
-            Entry v = better(better(m[0], m[1]), better(m[2], m[3]));
-            v = better(v, __shfl_xor_sync(0xffffffffu, v, 8));
-            v = better(v, __shfl_xor_sync(0xffffffffu, v, 16));
-            const uint32_t blk = j0 / per_block;
-            if (lane == 0u && rmq_chk(blk < nblocks))
-                atomicMin(reinterpret_cast<unsigned long long *>(bmin + blk),
-                          static_cast<unsigned long long>(v));
-        } else if (sub == 0u) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const uint32_t j = j0 + 4u * i + grp;
-                const uint32_t blk = j / per_block;
-                if (j < nmicro && rmq_chk(blk < nblocks))
-                    atomicMin(reinterpret_cast<unsigned long long *>(bmin + blk),
-                              static_cast<unsigned long long>(m[i]));
-            }
-        }
-    }
+// Levels k0 + 1 .. k0 + g of a larger block table.
+__global__ void __launch_bounds__(256) level_group_kernel(Entry *st, uint32_t nb, uint32_t k0, uint32_t g) {
+    const uint32_t first = blockIdx.x * 256u;
+    level_group<256>(st, nb, k0, g, first, min(256u, nb - first));
 }
 
 std::atomic<int> g_units_per_sm[2];
 
-cudaError_t launch_levels(Entry *st, uint32_t nb, uint32_t levels, const DeviceInfo &dev,
-                          cudaStream_t s) {
-    for (uint32_t k = 1; k < levels; ++k) {
-        const uint32_t cnt = nb - (1u << k) + 1;
-        uint32_t g = (cnt + 255) / 256;
-        const uint32_t cap = static_cast<uint32_t>(dev.sms) * 8u;
-        if (g > cap) g = cap;
-        st_level_kernel<<<g, 256, 0, s>>>(st, nb, k);
-        cudaError_t err = cudaGetLastError();
+cudaError_t launch_levels(Entry *st, uint32_t nb, uint32_t levels, cudaStream_t s) {
+    if (levels <= 1) return cudaSuccess;
+    if (nb <= kSmallTable) {
+        static std::atomic<bool> ready{false};
+        if (!ready.load(std::memory_order_relaxed)) {
+            const cudaError_t err =
+                cudaFuncSetAttribute(small_levels_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(2 * sizeof(Entry) * kSmallTable));
+            if (err != cudaSuccess) return err;
+            ready.store(true, std::memory_order_relaxed);
+        }
+        small_levels_kernel<<<1, kLevelThreads, 2 * sizeof(Entry) * nb, s>>>(st, nb, levels);
+        return cudaGetLastError();
+    }
+    for (uint32_t k = 0; k + 1 < levels; k += kLevelGroup) {
+        const uint32_t g = levels - 1 - k < kLevelGroup ? levels - 1 - k : kLevelGroup;
+        level_group_kernel<<<(nb + 255) / 256, 256, 0, s>>>(st, nb, k, g);
+        const cudaError_t err = cudaGetLastError();
         if (err != cudaSuccess) return err;
     }
     return cudaSuccess;
 }
 
-// Positions per table tile: 1024, 2048 where the halo is about as long (rows
-// up to level 9 and 10), 256 while a tile per SM is not to be had.
-uint32_t table_tile_size(const BuildPlan &p, const DeviceInfo &dev) {
-    if (p.mlevels >= 10) return 2048u;
-    return p.nmicro >= 1024u * static_cast<uint32_t>(dev.sms) ? 1024u : 256u;
+template <bool ALIGNED, uint32_t MODE>
+cudaError_t launch_runs_t(const BuildPlan &p, const MicroTable &T, const DeviceInfo &dev,
+                          cudaStream_t s) {
+    static std::atomic<int> per_sm_cache{0};
+    auto kern = table_kernel<ALIGNED, MODE>;
+    if (per_sm_cache.load(std::memory_order_relaxed) == 0) {
+        const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     static_cast<int>(sizeof(TableSmem)));
+        if (err != cudaSuccess) return err;
+    }
+    int per_sm;
+    const cudaError_t err = occupancy_cached(kern, kUnit, per_sm_cache, per_sm, sizeof(TableSmem));
+    if (err != cudaSuccess) return err;
+    if (per_sm < 1) per_sm = 1;
+    const uint32_t cap = static_cast<uint32_t>(dev.sms) * static_cast<uint32_t>(per_sm);
+    const uint32_t all = (p.nmicro + kUnit - 1) / kUnit, units = (all + cap - 1) / cap;
+    kern<<<(all + units - 1) / units, kUnit, sizeof(TableSmem), s>>>(
+        p.A, p.limit, p.off, p.n, p.lead, p.mst, T, units);
+    return cudaGetLastError();
 }
 
-cudaError_t launch_table(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s) {
+template <bool ALIGNED>
+cudaError_t launch_runs(const BuildPlan &p, const MicroTable &T, const DeviceInfo &dev,
+                        cudaStream_t s) {
+    switch (p.kmode) {
+    case kFloatMax: return launch_runs_t<ALIGNED, kFloatMax>(p, T, dev, s);
+    case kIntMin: return launch_runs_t<ALIGNED, kIntMin>(p, T, dev, s);
+    case kIntMax: return launch_runs_t<ALIGNED, kIntMax>(p, T, dev, s);
+    default: return launch_runs_t<ALIGNED, kFloatMin>(p, T, dev, s);
+    }
+}
+
+cudaError_t launch_build_tables(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s) {
     MicroTable T;
     T.mst = p.mst;
     T.mask = p.mask;
@@ -142,19 +151,28 @@ cudaError_t launch_table(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t
     T.moff_bytes = p.moff_bytes;
     T.nmicro = p.nmicro;
     T.mlevels = p.mlevels;
-    const uint32_t tile = table_tile_size(p, dev);
-    const size_t smem = table_smem((tile + table_halo(p.mlevels) + 1u) & ~1u);
-    static std::atomic<bool> ready{false};
-    if (!ready.load(std::memory_order_relaxed)) {
-        // the largest tile: 2048 positions and a halo of 1023
-        const cudaError_t err = cudaFuncSetAttribute(
-            table_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            static_cast<int>(table_smem(2048u + 1024u)));
+    cudaError_t err = p.aligned ? launch_runs<true>(p, T, dev, s) : launch_runs<false>(p, T, dev, s);
+    if (err != cudaSuccess) return err;
+    if (split_rows(p.mlevels)) {
+        const size_t smem = 2 * sizeof(Entry) * ((kRowTile + table_halo(p.mlevels) + 1u) & ~1u);
+        static std::atomic<bool> ready{false};
+        if (!ready.load(std::memory_order_relaxed)) {
+            // the longest halo: 1023
+            err = cudaFuncSetAttribute(rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(2 * sizeof(Entry) * (kRowTile + 1024u)));
+            if (err != cudaSuccess) return err;
+            ready.store(true, std::memory_order_relaxed);
+        }
+        rows_kernel<<<(p.nmicro + kRowTile - 1) / kRowTile, 512, smem, s>>>(T);
+        err = cudaGetLastError();
         if (err != cudaSuccess) return err;
-        ready.store(true, std::memory_order_relaxed);
     }
-    table_kernel<<<(p.nmicro + tile - 1) / tile, kTableThreads, smem, s>>>(T, tile);
-    return cudaGetLastError();
+    const uint32_t pb = p.tbs / kMicro, per_cta = pb <= 16u ? kBlockThreads : kBlockThreads / 32;
+    block_minima_kernel<<<(p.nb + per_cta - 1) / per_cta, kBlockThreads, 0, s>>>(p.mst, p.nmicro, pb,
+                                                                               p.st, p.nb, per_cta);
+    err = cudaGetLastError();
+    if (err != cudaSuccess) return err;
+    return launch_levels(p.st, p.nb, p.levels, s);
 }
 
 }  // namespace
@@ -182,6 +200,9 @@ Offsets offsets_of(const BuildPlan &p) {
 }  // namespace
 
 size_t plan_index(BuildPlan &p, bool no_micro) {
+    p.off = 0;
+    p.limit = p.n;
+    p.lead = 0;
     p.micro = !no_micro;
     p.tbs = p.micro ? table_block(p.bs) : p.bs;
     p.nb = (p.n + p.tbs - 1) / p.tbs;
@@ -232,39 +253,6 @@ uint32_t micro_levels(uint32_t bs) {
     return st_levels(touched);
 }
 
-static cudaError_t launch_build_tables(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s) {
-    cudaError_t err = cudaMemsetAsync(p.st, 0xff, sizeof(Entry) * static_cast<size_t>(p.nb), s);
-    if (err != cudaSuccess) return err;
-    // 8 warps per CTA, kMicroPerWarp micro-blocks per warp step
-    uint32_t g = (p.nmicro + 8 * kMicroPerWarp - 1) / (8 * kMicroPerWarp);
-    const uint32_t cap = static_cast<uint32_t>(dev.sms) * 8u;
-    if (g > cap) g = cap;
-    const uint32_t per_block = p.tbs / kMicro;
-    switch (p.kmode) {
-    case kFloatMax:
-        micro_min_kernel<kFloatMax><<<g, 256, 0, s>>>(p.A, p.n, p.nmicro, per_block, p.mst, p.st,
-                                                      p.aligned);
-        break;
-    case kIntMin:
-        micro_min_kernel<kIntMin><<<g, 256, 0, s>>>(p.A, p.n, p.nmicro, per_block, p.mst, p.st,
-                                                    p.aligned);
-        break;
-    case kIntMax:
-        micro_min_kernel<kIntMax><<<g, 256, 0, s>>>(p.A, p.n, p.nmicro, per_block, p.mst, p.st,
-                                                    p.aligned);
-        break;
-    default:
-        micro_min_kernel<kFloatMin><<<g, 256, 0, s>>>(p.A, p.n, p.nmicro, per_block, p.mst, p.st,
-                                                      p.aligned);
-        break;
-    }
-    err = cudaGetLastError();
-    if (err != cudaSuccess) return err;
-    err = launch_levels(p.st, p.nb, p.levels, dev, s);
-    if (err != cudaSuccess) return err;
-    return launch_table(p, dev, s);
-}
-
 cudaError_t launch_build_entries(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s) {
     UnitJob J;
     J.A = p.A;
@@ -306,7 +294,7 @@ cudaError_t launch_build(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t
     if (p.micro) return launch_build_tables(p, dev, s);
     const cudaError_t err = launch_build_entries(p, dev, s);
     if (err != cudaSuccess) return err;
-    return launch_levels(p.st, p.nb, p.levels, dev, s);
+    return launch_levels(p.st, p.nb, p.levels, s);
 }
 
 RMQ_VIOLATIONS_READER(violations_build)

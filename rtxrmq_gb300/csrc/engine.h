@@ -70,12 +70,16 @@ cudaError_t occupancy_cached(K kernel, int threads, std::atomic<int> &cache, int
 unsigned long long violations_build();
 unsigned long long violations_query();
 unsigned long long violations_batch();
-unsigned long long violations_batch_light();
+unsigned long long violations_query_lead();
+unsigned long long violations_batch_unaligned();
 unsigned long long violations_persist();
 
 // ---- plain index (build.cu) ----
 struct BuildPlan {
-    const float *A;
+    const float *A;   // buffer; element i of the array is A[off + i]
+    int64_t off;      // table index only; 0 but for an array of a batch
+    int64_t limit;    // one past the buffer's last value
+    uint32_t lead;    // elements before the array's first (of n), 0 but in a batch
     uint32_t n;
     uint32_t bs;      // block size asked for
     bool aligned;

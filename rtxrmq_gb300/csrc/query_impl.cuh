@@ -30,17 +30,23 @@
 #pragma once
 
 #include "common.cuh"
+#include "lines.cuh"
 #include "tables_impl.cuh"
 
 namespace rmq {
 
 // One built array: values A[off .. off + n) of the buffer A (loads never go
-// past A[limit - 1]); structure arrays are array-relative.
+// past A[limit - 1]); structure arrays are array-relative. A batched array
+// that starts off a 128-byte boundary is built from that boundary on, with
+// `lead` elements before its first that no query reaches (LEAD): positions
+// here count from the boundary, queries and answers from the array's first
+// element.
 struct V1View {
     const float *A;
     int64_t off;
     int64_t limit;
     uint32_t n;
+    uint32_t lead;  // elements before the array's first (LEAD launches)
     uint32_t bs;
     uint32_t nb;
     Div31 dv;
@@ -138,8 +144,9 @@ __device__ __forceinline__ void put_bits_idx(const QueryOut &o, int64_t i, uint3
     if (o.idx) __stcs(o.idx + i, static_cast<int32_t>(idx));
 }
 
-__device__ __forceinline__ void put_result(const QueryOut &o, int64_t i, Entry e, uint32_t mode) {
-    put_bits_idx(o, i, o.val ? entry_bits(e, mode) : 0u, entry_idx(e));
+__device__ __forceinline__ void put_result(const QueryOut &o, int64_t i, Entry e, uint32_t mode,
+                                           uint32_t lead = 0u) {
+    put_bits_idx(o, i, o.val ? entry_bits(e, mode) : 0u, entry_idx(e) - lead);
 }
 
 __device__ __forceinline__ void put_invalid(const QueryOut &o, int64_t i) {
@@ -347,45 +354,6 @@ constexpr int kStageLines = 16;
 constexpr int kLanesPerLine = 32 / kStageLines;
 constexpr int kChunksPerLane = 8 / kLanesPerLine;
 
-// What a key mode compares: IEEE minimum / maximum, which skips NaN (ordered
-// last) and equates the zeros, or signed minimum / maximum. `fill` stands for
-// an element outside the request: it never beats one inside.
-template <uint32_t MODE>
-struct Best {
-    using T = float;
-    static __device__ __forceinline__ T of(uint32_t b) { return __uint_as_float(b); }
-    static __device__ __forceinline__ uint32_t bits(T x) { return __float_as_uint(x); }
-    static __device__ __forceinline__ T fill() { return __uint_as_float(0x7fc00000u); }
-    static __device__ __forceinline__ T best(T a, T b) { return MODE == kFloatMin ? fminf(a, b) : fmaxf(a, b); }
-};
-template <>
-struct Best<kIntMin> {
-    using T = int32_t;
-    static __device__ __forceinline__ T of(uint32_t b) { return static_cast<int32_t>(b); }
-    static __device__ __forceinline__ uint32_t bits(T x) { return static_cast<uint32_t>(x); }
-    static __device__ __forceinline__ T fill() { return 0x7fffffff; }
-    static __device__ __forceinline__ T best(T a, T b) { return min(a, b); }
-};
-template <>
-struct Best<kIntMax> {
-    using T = int32_t;
-    static __device__ __forceinline__ T of(uint32_t b) { return static_cast<int32_t>(b); }
-    static __device__ __forceinline__ uint32_t bits(T x) { return static_cast<uint32_t>(x); }
-    static __device__ __forceinline__ T fill() { return -0x7fffffff - 1; }
-    static __device__ __forceinline__ T best(T a, T b) { return max(a, b); }
-};
-
-// Shared-memory address of chunk 0 of a staged line; chunk c is at ^ (c << 4).
-__device__ __forceinline__ uint32_t staged_line(uint32_t stage, uint32_t slot) {
-    return stage + slot * 128u + ((slot & 7u) << 4);
-}
-__device__ __forceinline__ uint4 lds_chunk(uint32_t addr) {
-    uint4 f;
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(f.x), "=r"(f.y), "=r"(f.z), "=r"(f.w) : "r"(addr));
-    return f;
-}
-
 // Starts copying the chunks holding a set bit of the requests of lanes
 // h .. h + kStageLines - 1 into the warp's stage. Bytes past the end of the
 // buffer are not read.
@@ -473,10 +441,8 @@ __device__ __forceinline__ Entry reduce_lines(uint32_t line, uint32_t bits, uint
 #pragma unroll
     for (int c = kChunksPerLane - 1; c >= 0; --c) cs = m[c] == mm ? c : cs;
     const uint4 f = lds_chunk(base ^ (cs << 4));
-    uint32_t pos = 3u, wb = f.w;
-    if (B::of(f.z) == mm) pos = 2u, wb = f.z;
-    if (B::of(f.y) == mm) pos = 1u, wb = f.y;
-    if (B::of(f.x) == mm) pos = 0u, wb = f.x;
+    uint32_t wb;
+    const uint32_t pos = first_in_chunk<MODE>(f, mm, wb);
     // no number, or nothing above the fill: every element of the request has
     // the largest key, and the first of them is the best
     const bool last = !(mm == mm) || mm == B::fill();
@@ -591,7 +557,7 @@ struct StepMap {
 // rarely, it joins the queue again, for the units between both ends and its
 // part at the other end: few lanes in a warp need that, so doing it at once
 // would cost every drain a second pass.
-template <bool ALIGNED, bool MICRO, uint32_t MODE, bool STATS, int THREADS, int QPT>
+template <bool ALIGNED, bool MICRO, uint32_t MODE, bool STATS, bool LEAD, int THREADS, int QPT>
 __device__ __forceinline__ void drain_misses(const V1View &v, const QueryOut &o,
                                              const StepMap &map, MissQueue<MICRO> &mq,
                                              uint32_t &count, uint64_t pol, QStats &s) {
@@ -644,7 +610,7 @@ __device__ __forceinline__ void drain_misses(const V1View &v, const QueryOut &o,
             res = better(res, reduce_lines<MODE>(line, bits, stage, h));
         }
     }
-    if (act && !again) put_result(o, map.query(id, THREADS * QPT), res, MODE);
+    if (act && !again) put_result(o, map.query(id, THREADS * QPT), res, MODE, LEAD ? v.lead : 0u);
     if constexpr (MICRO) {
         const unsigned mask = __ballot_sync(0xffffffffu, again);
         if (again) {
@@ -707,11 +673,11 @@ __device__ __forceinline__ Entry superset_probe(const V1View &v, uint32_t l, uin
 // block table serves longer ones). Queries left open join the warp's queue, whose length `count`
 // carries from step to step (`last` empties it); `id0` is the step's first
 // query in the CTA's numbering.
-template <bool ALIGNED, bool MICRO, uint32_t MODE, int THREADS, int QPT, bool STATS>
+template <bool ALIGNED, bool MICRO, uint32_t MODE, int THREADS, int QPT, bool STATS, bool LEAD>
 __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryOut &o,
                                                    const StepMap &map, int64_t base, uint32_t cnt,
                                                    uint32_t id0, bool last,
-                                                   const int2 (&qq)[QPT], QStats &s,
+                                                   const int2 (&in)[QPT], QStats &s,
                                                    MissQueue<MICRO> &mq, uint32_t &count) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t pol = l2_keep_policy();
@@ -719,10 +685,15 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
     int32_t *const is = o.idx ? o.idx + base : nullptr;
     Entry res[QPT];
     bool ok[QPT], scan[QPT];
+    const uint32_t lead = LEAD ? v.lead : 0u;
+    int2 qq[QPT];
+#pragma unroll
+    for (int k = 0; k < QPT; ++k)  // unsigned: an end past 2^31 - 1 stays past n
+        qq[k] = make_int2(static_cast<int>(in[k].x + lead), static_cast<int>(in[k].y + lead));
 #pragma unroll
     for (int k = 0; k < QPT; ++k) {
         const uint32_t l = static_cast<uint32_t>(qq[k].x), r = static_cast<uint32_t>(qq[k].y);
-        ok[k] = qq[k].x >= 0 && l <= r && r < v.n;
+        ok[k] = in[k].x >= 0 && l <= r && r < v.n;
         scan[k] = MICRO && (l >> 5) == (r >> 5);
         res[k] = kEntryNone;
         if (ok[k]) {
@@ -762,7 +733,7 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
         // drain (same warp, after __syncwarp) or the warp scan (same thread)
         // overwrites it, and whole-warp stores keep the output lines whole
         if (vs) __stcs(reinterpret_cast<unsigned int *>(vs) + j, decode_bits<MODE>(res[k]));
-        if (is) __stcs(is + j, static_cast<int32_t>(entry_idx(res[k])));
+        if (is) __stcs(is + j, static_cast<int32_t>(entry_idx(res[k]) - lead));
     }
     if constexpr (!MICRO) {
 #pragma unroll
@@ -822,7 +793,7 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
         const uint32_t drain_at = last && k == QPT - 1 ? 1u : 32u;
 #pragma unroll 1
         while (count >= drain_at)
-            drain_misses<ALIGNED, MICRO, MODE, STATS, THREADS, QPT>(v, o, map, mq, count, pol, s);
+            drain_misses<ALIGNED, MICRO, MODE, STATS, LEAD, THREADS, QPT>(v, o, map, mq, count, pol, s);
     }
 }
 
@@ -841,7 +812,7 @@ __device__ __forceinline__ void flush_stats(const QStats &s, unsigned long long 
 // Answer queries [q0, q1) of one array with the whole CTA (THREADS
 // threads) in the queued form, QPT queries per thread per step; `mq` is the
 // calling warp's queue, empty on entry and on return.
-template <bool ALIGNED, bool MICRO, uint32_t MODE, int THREADS, int QPT>
+template <bool ALIGNED, bool MICRO, uint32_t MODE, bool LEAD, int THREADS, int QPT>
 __device__ __forceinline__ void answer_range_queued(const V1View &v, const QueryOut &o,
                                                     int64_t q0, int64_t q1, MissQueue<MICRO> &mq) {
     constexpr int64_t step = static_cast<int64_t>(THREADS) * QPT;
@@ -851,7 +822,7 @@ __device__ __forceinline__ void answer_range_queued(const V1View &v, const Query
     for (int64_t base = q0; base < q1; base += step, id0 += step) {
         int2 qq[QPT];
         load_queries<QPT>(o, base, q1, qq);
-        answer_step_queued<ALIGNED, MICRO, MODE, THREADS, QPT, false>(
+        answer_step_queued<ALIGNED, MICRO, MODE, THREADS, QPT, false, LEAD>(
             v, o, map, base, static_cast<uint32_t>(min(step, q1 - base)), id0, base + step >= q1, qq,
             s, mq, waiting);
     }

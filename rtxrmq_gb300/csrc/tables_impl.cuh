@@ -18,6 +18,8 @@
 #pragma once
 
 #include "common.cuh"
+#include "lines.cuh"
+#include "minima_impl.cuh"
 
 namespace rmq {
 
@@ -54,40 +56,22 @@ struct MicroTable {
     uint32_t mlevels;
 };
 
-// Shared memory of a tile of `entries` minima (its positions and halo, an
-// even number): two buffers of composites, the keys alone padded for 16-byte
-// reads past the last one, and the 32-bit half masks.
-constexpr uint32_t kKeyPad = 32;
-RMQ_HD constexpr uint32_t key_words(uint32_t entries) { return (entries + 3) / 4 * 4 + kKeyPad; }
-constexpr size_t table_smem(uint32_t entries) {
-    return 2 * sizeof(Entry) * static_cast<size_t>(entries) +
-           2 * sizeof(uint32_t) * static_cast<size_t>(key_words(entries));
+// One step of a record mask: bit d of `bits` when k beats `run`, which
+// becomes the smaller of both. Three instructions; the compiler's form of the
+// same takes four to five.
+template <int D>
+__device__ __forceinline__ void record_step(uint32_t k, uint32_t &run, uint32_t &bits) {
+    asm("{\n\t.reg .pred p;\n\t"
+        "setp.lt.u32 p, %2, %0;\n\t"
+        "min.u32 %0, %0, %2;\n\t"
+        "@p or.b32 %1, %1, %3;\n\t}"
+        : "+r"(run), "+r"(bits) : "r"(k), "n"(1u << D));
 }
-
-// Masks of the windows of 32 at positions i0 .. i0 + 3 from their keys. Every key
-// is read once into registers (9 16-byte reads without bank conflicts); per
-// position and distance a compare and two predicated moves. ALU-bound, about
-// 100 instructions per micro-block of 32 elements.
-__device__ __forceinline__ void mask4(const uint32_t *keys, uint32_t i0, uint32_t (&m)[4]) {
-    uint32_t k[36];
-#pragma unroll
-    for (int c = 0; c < 9; ++c) {
-        const uint4 f = *reinterpret_cast<const uint4 *>(keys + i0 + 4 * c);
-        k[4 * c] = f.x;
-        k[4 * c + 1] = f.y;
-        k[4 * c + 2] = f.z;
-        k[4 * c + 3] = f.w;
-    }
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-        uint32_t run = k[p], bits = 1u;
-#pragma unroll
-        for (int d = 1; d < 32; ++d)
-            if (k[p + d] < run) {
-                run = k[p + d];
-                bits |= 1u << d;
-            }
-        m[p] = bits;
+template <int D>
+__device__ __forceinline__ void record_steps(const uint32_t *k, uint32_t &run, uint32_t &bits) {
+    if constexpr (D < 32) {
+        record_step<D>(k[D], run, bits);
+        record_steps<D + 1>(k, run, bits);
     }
 }
 
@@ -115,79 +99,248 @@ __device__ __forceinline__ void tile_rows(const MicroTable &T, uint32_t t0, uint
     }
 }
 
-// Masks and offset rows at positions [t0, t0 + count) from the minima a[0 ..
-// e) of micro-blocks [t0, t0 + e) in shared memory. b: a second buffer of as
-// many entries; keys, half: key_words(e) words each, keys[i] the key of a[i]
-// and the largest key from e on. The CTA calls it after a barrier; it ends
-// with the buffers still in use by other threads.
+// The offset rows of positions [t0, t0 + count) from the masks and minima in
+// global memory (written by an earlier launch or phase), for tables with rows
+// up to windows of 512 and 1024 (split_rows). smem: two buffers of count +
+// halo entries.
 template <int THREADS>
-__device__ __forceinline__ void table_tile(const MicroTable &T, uint32_t t0, uint32_t count,
-                                           uint32_t e, Entry *a, Entry *b, const uint32_t *keys,
-                                           uint32_t *half) {
+__device__ __forceinline__ void rows_tile_global(const MicroTable &T, uint32_t t0, uint32_t count,
+                                                 unsigned char *smem) {
     const bool wide = wide_masks(T.nmicro);
     const uint32_t k0 = mask_levels(wide), span = 1u << (k0 - 1u);
-    const bool rows = T.mlevels > k0 && e >= 2u * span;
-    // the rows' first level needs the best of every mask's window that lies in
-    // the loaded range, also past the tile's own positions; a 64-bit mask
-    // needs the half mask 32 further on
-    const uint32_t npos = rows ? max(count, e - span + 1u) : count;
-    const uint32_t nhalf = wide ? min(npos + 32u, e) : npos;
-    for (uint32_t i0 = 4u * threadIdx.x; i0 < nhalf; i0 += 4u * THREADS) {
-        uint32_t m[4];
-        mask4(keys, i0, m);
-        *reinterpret_cast<uint4 *>(half + i0) = make_uint4(m[0], m[1], m[2], m[3]);
+    const uint32_t e = min(count + table_halo(T.mlevels), T.nmicro - t0);
+    if (e < 2u * span) return;  // no window of the first row starts here
+    Entry *a = reinterpret_cast<Entry *>(smem);
+    Entry *b = a + ((count + table_halo(T.mlevels) + 1u) & ~1u);
+    for (uint32_t i = threadIdx.x; i + span <= e; i += THREADS) {
+        const uint32_t j = t0 + i;
+        const uint32_t d = wide ? 63u - __clzll(static_cast<const uint64_t *>(T.mask)[j])
+                                : 31u - __clz(static_cast<const uint32_t *>(T.mask)[j]);
+        if (rmq_chk(j + d < T.nmicro)) b[i] = T.mst[j + d];
     }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < npos; i += THREADS) {
-        const uint32_t lo = half[i];
-        uint32_t d = 31u - __clz(lo);
-        const bool mine = i < count && rmq_chk(t0 + i < T.nmicro);
-        if (wide) {
-            // the second half's new bests (their keys fall strictly) from the
-            // first that beats the first half's best on
-            uint32_t hi = i + 32u < e ? half[i + 32u] : 0u;
-            const uint32_t best = keys[i + d];
-            while (hi && keys[i + 31u + __ffs(hi)] >= best) hi &= hi - 1u;
-            if (mine) static_cast<uint64_t *>(T.mask)[t0 + i] = (static_cast<uint64_t>(hi) << 32) | lo;
-            if (hi) d = 63u - __clz(hi);
-        } else if (mine) {
-            static_cast<uint32_t *>(T.mask)[t0 + i] = lo;
-        }
-        if (rows) b[i] = a[min(i + d, e - 1u)];
-    }
-    if (!rows) return;
     __syncthreads();
     if (T.moff_bytes == 1u)
         tile_rows<uint8_t, THREADS>(T, t0, count, e, b, a, k0);
     else
         tile_rows<uint16_t, THREADS>(T, t0, count, e, b, a, k0);
+    __syncthreads();
 }
 
-// The keys of a[0 .. e) and the padding behind them.
-template <int THREADS>
-__device__ __forceinline__ void tile_keys(const Entry *a, uint32_t e, uint32_t *keys) {
-    for (uint32_t i = threadIdx.x; i < key_words(e); i += THREADS)
-        keys[i] = i < e ? static_cast<uint32_t>(a[i] >> 32) : 0xffffffffu;
+// Whether rows are made apart from the masks: windows of 512 and 1024 reach
+// further than the fused builder's ring.
+RMQ_HD bool split_rows(uint32_t mlevels) { return mlevels >= 10u; }
+
+// ---- minima and micro table in one pass over the values ---------------------
+//
+// A CTA takes a run of consecutive micro-blocks, from its right end to its
+// left, in units of 256: copies of the next unit's values are in flight while
+// the masks of the current one are made, and the minima to its right that its
+// windows reach are still in shared memory (a ring of 512 positions, indexed
+// by micro-block mod 512) from the unit before. So the values are read once
+// plus 63 to 255 micro-blocks per run, and the masks' arithmetic (about 200
+// instructions per micro-block) hides behind the stream. As two launches,
+// minima and then tables, 10^8 values took 63 + 38 us.
+constexpr uint32_t kUnit = 256;         // micro-blocks per unit = threads
+constexpr uint32_t kRing = 512;
+constexpr uint32_t kMirror = 64;        // ring positions 0 .. 63 again behind its end
+struct TableSmem {
+    uint4 stage[kUnit * 8];             // the unit's values, 4 KB per warp
+    Entry a[kRing + kMirror];           // minima
+    Entry c[kRing];                     // best of the whole mask's window
+    uint32_t key[kRing + kMirror];
+    uint32_t half[kRing + kMirror];     // masks of windows of 32, 0 past the array
+};
+
+// Micro-blocks [lo, hi) (multiples of kUnit, or hi the array's last) of the
+// array whose element 0 is value `base`; the CTA of kUnit threads. With `T`'s
+// rows only when they are not split.
+template <bool ALIGNED, uint32_t MODE>
+__device__ __forceinline__ void build_run(const float *__restrict__ A, int64_t limit, int64_t base,
+                                          uint32_t n, uint32_t lead, Entry *mst, const MicroTable &T,
+                                          uint32_t lo, uint32_t hi, TableSmem &sm) {
+    const uint32_t t = threadIdx.x, warp = t >> 5;
+    const uint32_t stage = static_cast<uint32_t>(__cvta_generic_to_shared(sm.stage)) + 4096u * warp;
+    const bool wide = wide_masks(T.nmicro);
+    const uint32_t k0 = mask_levels(wide), span = 1u << (k0 - 1u);
+    const bool rows = T.mlevels > k0 && !split_rows(T.mlevels);
+    const uint32_t reach = rows ? (1u << (T.mlevels - 1u)) - 1u : 63u;
+    LineStep step;
+    auto issue = [&](uint32_t s, uint32_t cnt) {
+        const uint32_t w0 = 32u * warp;
+        step = LineStep{base, n, lead, s + w0, cnt > w0 ? min(kStepLines, cnt - w0) : 0u, mst};
+        if (step.cnt) copy_step<ALIGNED>(A, limit, step, stage);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // first what lies right of the run (no output), then its units
+    uint32_t s = hi, cnt = min(reach, T.nmicro - hi);
+    bool out = false;
+    issue(s, cnt);
+    for (uint32_t i = t; i < kRing + kMirror; i += kUnit) {
+        sm.a[i] = kEntryNone;
+        sm.key[i] = 0xffffffffu;
+        sm.half[i] = 0u;
+        if (i < kRing) sm.c[i] = kEntryNone;
+    }
+    for (;;) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+        const Entry m = reduce_step<MODE>(step, stage);
+        const uint32_t j = s + t, r = j & (kRing - 1u);
+        const bool have = t < cnt;
+        __syncthreads();  // the slots written next were the last unit's right neighbours
+        if (have) {
+            const uint32_t key = static_cast<uint32_t>(m >> 32);
+            sm.a[r] = m;
+            sm.key[r] = key;
+            if (r < kMirror) {
+                sm.a[r + kRing] = m;
+                sm.key[r + kRing] = key;
+            }
+            if (out && rmq_chk(j < T.nmicro)) mst[j] = m;
+        }
+        __syncthreads();
+        const uint32_t next = out ? s - kUnit : (hi - 1u) / kUnit * kUnit;
+        const bool more = out ? s > lo : true;
+        if (more) issue(next, min(hi - next, kUnit));
+
+        uint32_t bits = 1u;
+        {
+            uint32_t run = sm.key[r];
+            const uint32_t *k = sm.key + r;
+            record_steps<1>(k, run, bits);
+        }
+        if (have) {
+            sm.half[r] = bits;
+            if (r < kMirror) sm.half[r + kRing] = bits;
+        }
+        __syncthreads();
+        uint32_t d = 31u - __clz(bits);
+        uint32_t top = 0u;
+        if (wide) {
+            // the second half's new bests (their keys fall strictly) from the
+            // first that beats the first half's best on: none when its last
+            // does not, else by bisection (a loop over the bests to drop costs
+            // a warp its longest one, twice as much)
+            top = sm.half[r + 32u];
+            const uint32_t best = sm.key[r + d];
+            const uint32_t *k2 = sm.key + r + 32u;
+            if (top != 0u && k2[31u - __clz(top)] >= best) top = 0u;
+            uint32_t from = 0u;
+#pragma unroll
+            for (uint32_t w = 16u; w > 0u; w >>= 1) {
+                const uint32_t sub = (top >> from) & ((1u << w) - 1u);
+                if (sub == 0u || k2[from + 31u - __clz(sub)] >= best) from += w;
+            }
+            top &= 0xffffffffu << from;
+            if (top) d = 63u - __clz(top);
+        }
+        const bool store = out && have && rmq_chk(j < T.nmicro);
+        if (store) {
+            if (wide)
+                static_cast<uint64_t *>(T.mask)[j] = (static_cast<uint64_t>(top) << 32) | bits;
+            else
+                static_cast<uint32_t *>(T.mask)[j] = bits;
+        }
+        if (rows) {
+            if (have) sm.c[r] = sm.a[r + d];
+            __syncthreads();
+            if (store) {
+                Entry acc = sm.c[r];
+                for (uint32_t k = k0; k < T.mlevels; ++k) {
+                    const uint32_t parts = 1u << (k - k0);
+                    for (uint32_t i = parts; i < 2u * parts; ++i)
+                        acc = better(acc, sm.c[(r + i * span) & (kRing - 1u)]);
+                    if (j + (1u << k) <= T.nmicro) {
+                        const size_t at = static_cast<size_t>(k - k0) * T.nmicro + j;
+                        const uint32_t off = (entry_idx(acc) >> 5) - j;
+                        if (T.moff_bytes == 1u)
+                            static_cast<uint8_t *>(T.moff)[at] = static_cast<uint8_t>(off);
+                        else
+                            static_cast<uint16_t *>(T.moff)[at] = static_cast<uint16_t>(off);
+                    }
+                }
+            }
+        }
+        if (!more) break;
+        s = next;
+        cnt = min(hi - next, kUnit);
+        out = true;
+    }
+    __syncthreads();  // a further run clears the ring
 }
 
-// A tile whose minima are read from global memory (tile positions [t0, t0 +
-// count), smem: table_smem of count + halo rounded up to an even number,
-// 16-byte aligned).
+// Minima of blocks [b0, b1) of `pb` micro-blocks each, from the micro-block
+// minima: a thread per block for small blocks, a warp per block otherwise.
 template <int THREADS>
-__device__ __forceinline__ void table_tile_global(const MicroTable &T, uint32_t t0, uint32_t count,
-                                                  unsigned char *smem) {
-    const uint32_t e = min(count + table_halo(T.mlevels), T.nmicro - t0);
-    const uint32_t cap = (count + table_halo(T.mlevels) + 1u) & ~1u;
-    Entry *a = reinterpret_cast<Entry *>(smem);
-    Entry *b = a + cap;
-    uint32_t *keys = reinterpret_cast<uint32_t *>(b + cap);
-    for (uint32_t i = threadIdx.x; i < e; i += THREADS)
-        a[i] = rmq_chk(t0 + i < T.nmicro) ? T.mst[t0 + i] : kEntryNone;
+__device__ __forceinline__ void block_minima(const Entry *mst, uint32_t nmicro, uint32_t pb,
+                                             uint32_t b0, uint32_t b1, uint32_t nb, Entry *bmin) {
+    if (pb <= 16u) {
+        for (uint32_t b = b0 + threadIdx.x; b < b1; b += THREADS) {
+            Entry m = kEntryNone;
+            const uint32_t j1 = min(b * pb + pb, nmicro);
+            for (uint32_t j = b * pb; j < j1; ++j) m = better(m, mst[j]);
+            if (rmq_chk(b < nb)) bmin[b] = m;
+        }
+        return;
+    }
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t b = b0 + (threadIdx.x >> 5); b < b1; b += THREADS / 32) {
+        Entry m = kEntryNone;
+        const uint32_t j1 = min(b * pb + pb, nmicro);
+        for (uint32_t j = b * pb + lane; j < j1; j += 32u) m = better(m, mst[j]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = better(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane == 0u && rmq_chk(b < nb)) bmin[b] = m;
+    }
+}
+
+// Every level of a block table st[levels][nb] from its block minima, by one
+// CTA: two buffers of nb entries in shared memory, one barrier per level.
+template <int THREADS>
+__device__ __forceinline__ void all_levels(Entry *st, uint32_t nb, uint32_t levels, Entry *buf) {
+    Entry *src = buf, *dst = buf + nb;
+    for (uint32_t i = threadIdx.x; i < nb; i += THREADS) src[i] = st[i];
     __syncthreads();
-    tile_keys<THREADS>(a, e, keys);
-    __syncthreads();
-    table_tile<THREADS>(T, t0, count, e, a, b, keys, keys + key_words(cap));
-    __syncthreads();  // a further tile overwrites the buffers
+    for (uint32_t k = 1; k < levels; ++k) {
+        const uint32_t half = 1u << (k - 1), cnt = nb - (1u << k) + 1;
+        Entry *row = st + static_cast<size_t>(k) * nb;
+        for (uint32_t i = threadIdx.x; i < cnt; i += THREADS) {
+            const Entry m = better(src[i], src[i + half]);
+            dst[i] = m;
+            row[i] = m;
+        }
+        __syncthreads();
+        Entry *t = src;
+        src = dst;
+        dst = t;
+    }
+    __syncthreads();  // a further table overwrites the buffers
+}
+
+// Levels k0 + 1 .. k0 + g (g <= kLevelGroup) of a block table st[levels][nb]
+// at positions [first, first + count), from level k0: a level's entry is the
+// best of 2^g entries of level k0, 2^k0 apart, so several levels need no
+// synchronisation between them.
+constexpr uint32_t kLevelGroup = 3;
+template <int THREADS>
+__device__ __forceinline__ void level_group(Entry *st, uint32_t nb, uint32_t k0, uint32_t g,
+                                            uint32_t first, uint32_t count) {
+    const Entry *__restrict__ src = st + static_cast<size_t>(k0) * nb;
+    for (uint32_t j = first + threadIdx.x; j < first + count; j += THREADS) {
+        Entry x[1 << kLevelGroup];
+#pragma unroll
+        for (uint32_t i = 0; i < (1u << kLevelGroup); ++i) {
+            const uint64_t at = j + (static_cast<uint64_t>(i) << k0);
+            x[i] = i < (1u << g) && at < nb ? src[at] : kEntryNone;
+        }
+#pragma unroll
+        for (uint32_t t = 1; t <= kLevelGroup; ++t) {
+#pragma unroll
+            for (uint32_t i = 0; i < (1u << (kLevelGroup - t)); ++i)
+                x[i] = better(x[2 * i], x[2 * i + 1]);
+            if (t <= g && j + (1ull << (k0 + t)) <= nb) st[static_cast<size_t>(k0 + t) * nb + j] = x[0];
+        }
+    }
 }
 
 #endif  // __CUDACC__
