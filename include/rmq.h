@@ -99,7 +99,8 @@ typedef struct rmq_info {
  * sparse table over the block minima.
  * The handle owns its structure memory; it does not own or copy d_vals,
  * which must stay valid and unchanged while the handle is used.
- * Allocates (cudaMalloc); not for use under stream capture.
+ * Allocates (in stream order from the library's pool, see rmq_trim, or by
+ * cudaMalloc); not for use under stream capture.
  */
 int rmq_build(const float *d_vals, int64_t n, int64_t bs, rmq_stream_t stream,
               rmq_handle_t **out);
@@ -202,8 +203,25 @@ int rmq_save(const rmq_handle_t *h, const char *path, rmq_stream_t stream);
 int rmq_load(const float *d_vals, int64_t n, const char *path,
              rmq_stream_t stream, rmq_handle_t **out);
 
-/* Release everything the handle owns. NULL is accepted. */
+/* Release everything the handle owns, after all work of the device. NULL is
+ * accepted. */
 int rmq_free(rmq_handle_t *h);
+
+/*
+ * rmq_free in stream order, without waiting: the handle's memory is released
+ * when the work enqueued on `stream` so far is done. All work that uses the
+ * handle must precede that point (it was enqueued on `stream`, or `stream`
+ * waits for it). Falls back to rmq_free where that cannot be known or done:
+ * a query of the handle was captured in a graph, `stream` is capturing, the
+ * handle came from rmq_load, has host staging or probe entries, or is larger
+ * than the pool keeps.
+ */
+int rmq_free_async(rmq_handle_t *h, rmq_stream_t stream);
+
+/* Indexes of up to 256 MB come from a pool per device that keeps at most
+ * 256 MB of freed memory for the next index. Gives back to the device what
+ * the current device's pool holds unused; RMQ_OK also without a pool. */
+int rmq_trim(void);
 
 /* Describe a built handle. */
 int rmq_info(const rmq_handle_t *h, rmq_info_t *info);

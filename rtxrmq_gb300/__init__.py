@@ -44,6 +44,18 @@ def _stream_handle(stream) -> Optional[int]:
     return stream.cuda_stream
 
 
+def _durable_stream(stream):
+    """(handle, object or None): the object when the stream outlives its
+    Python wrapper (the default stream and torch's pool streams are never
+    destroyed), None for a raw handle or an external stream."""
+    import torch
+    s = torch.cuda.current_stream() if stream is None else stream
+    if isinstance(s, int):
+        return s, None
+    sid = getattr(s, "stream_id", None)  # torch: 0 default, odd pool, else external
+    return s.cuda_stream, (s if sid is not None and (sid == 0 or sid & 1) else None)
+
+
 def _dptr(t) -> Optional[int]:
     if t is None:
         return None
@@ -87,10 +99,19 @@ class RMQIndex:
         self._values = values
         self._vdtype = values.dtype
         self._h = C.c_void_p()
+        s, self._keep = _durable_stream(stream)
+        self._one_stream = s  # the only stream this index was used on, or None
         flags = ((0 if micro else 1) | (2 if op == "max" else 0) |
                  (4 if values.dtype == torch.int32 else 0) | (8 if light else 0))  # RMQ_BUILD_*
-        check(lib.rmq_build_ex(_dptr(values), values.numel(), int(bs), flags,
-                               _stream_handle(stream), C.byref(self._h)))
+        check(lib.rmq_build_ex(_dptr(values), values.numel(), int(bs), flags, s,
+                               C.byref(self._h)))
+
+    def _use(self, stream) -> int:
+        """Handle of the stream a call runs on (remembered for close)."""
+        s = _stream_handle(stream)
+        if s != self._one_stream:
+            self._one_stream = None
+        return s
 
     def info(self) -> dict:
         inf = rmq_info_t()
@@ -102,17 +123,18 @@ class RMQIndex:
         """Answer int32 [q, 2] queries; returns (val, idx), either may be None."""
         import torch
         q = _check_queries(queries)
-        dev = queries.device
-        if values and out_val is None:
-            out_val = torch.empty(q, dtype=getattr(self, "_vdtype", torch.float32), device=dev)
-        if indices and out_idx is None:
-            out_idx = torch.empty(q, dtype=torch.int32, device=dev)
         if not values:
             out_val = None
+        elif out_val is None:
+            out_val = torch.empty(q, dtype=self._vdtype, device=queries.device)
         if not indices:
             out_idx = None
-        check(load().rmq_query(self._h, _dptr(queries), q, _dptr(out_val), _dptr(out_idx),
-                               _stream_handle(stream)))
+        elif out_idx is None:
+            out_idx = torch.empty(q, dtype=torch.int32, device=queries.device)
+        s = torch.cuda.current_stream().cuda_stream if stream is None else _stream_handle(stream)
+        if s != self._one_stream:
+            self._one_stream = None
+        check(load().rmq_query(self._h, _dptr(queries), q, _dptr(out_val), _dptr(out_idx), s))
         return out_val, out_idx
 
     def query_host(self, queries, out_val=None, out_idx=None, stream=None) -> None:
@@ -135,7 +157,7 @@ class RMQIndex:
         if tuple(queries.shape[1:]) != (2,):
             raise ValueError("queries must have shape [q, 2]")
         check(load().rmq_query_host(self._h, hptr(queries), q, hptr(out_val), hptr(out_idx),
-                                    _stream_handle(stream)))
+                                    self._use(stream)))
 
     def probe_gather(self, queries, out_val=None, out_idx=None, stream=None) -> Tuple:
         """rmq_probe_gather: the two-lookup random-access ceiling of query()
@@ -148,7 +170,7 @@ class RMQIndex:
         if out_idx is None:
             out_idx = torch.empty(q, dtype=torch.int32, device=queries.device)
         check(load().rmq_probe_gather(self._h, _dptr(queries), q, _dptr(out_val), _dptr(out_idx),
-                                      _stream_handle(stream)))
+                                      self._use(stream)))
         return out_val, out_idx
 
     STATS_FIELDS = ("first_probe", "second_probe", "full", "micro_scan", "block_edge",
@@ -162,12 +184,12 @@ class RMQIndex:
         q = _check_queries(queries)
         counts = (C.c_int64 * len(self.STATS_FIELDS))()
         check(load().rmq_query_stats(self._h, _dptr(queries), q, _dptr(out_val), _dptr(out_idx),
-                                     counts, _stream_handle(stream)))
+                                     counts, self._use(stream)))
         return dict(zip(self.STATS_FIELDS, (int(x) for x in counts)))
 
     def save(self, path, stream=None) -> None:
         """Write the index (not the values) to ``path`` (rmq_save)."""
-        check(load().rmq_save(self._h, str(path).encode(), _stream_handle(stream)))
+        check(load().rmq_save(self._h, str(path).encode(), self._use(stream)))
 
     @classmethod
     def load(cls, values, path, stream=None) -> "RMQIndex":
@@ -180,13 +202,14 @@ class RMQIndex:
         self._values = values
         self._vdtype = values.dtype
         self._h = C.c_void_p()
+        self._keep = self._one_stream = None
         check(load().rmq_load(_dptr(values), values.numel(), str(path).encode(),
                               _stream_handle(stream), C.byref(self._h)))
         return self
 
     def invalid_count(self, stream=None) -> int:
         v = C.c_int64()
-        check(load().rmq_invalid_count(self._h, _stream_handle(stream), C.byref(v)))
+        check(load().rmq_invalid_count(self._h, self._use(stream), C.byref(v)))
         return v.value
 
     @property
@@ -194,9 +217,14 @@ class RMQIndex:
         return self._h.value or 0
 
     def close(self) -> None:
+        """Release the index: in stream order when every call on it ran on one
+        stream that still exists, else after all work of the device."""
         if getattr(self, "_h", None) is not None and self._h.value:
-            check(load().rmq_free(self._h))
-            self._h = C.c_void_p()
+            h, self._h = self._h, C.c_void_p()
+            if self._keep is not None and self._one_stream is not None:
+                check(load().rmq_free_async(h, self._one_stream))
+            else:
+                check(load().rmq_free(h))
 
     def __enter__(self):
         return self

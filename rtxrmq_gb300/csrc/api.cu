@@ -12,6 +12,8 @@
 #include <mutex>
 
 #include "../../include/rmq.h"
+#include <cuda.h>  // cuuint64_t
+
 #include "engine.h"
 #include "tables_impl.cuh"
 
@@ -21,6 +23,8 @@ struct rmq_handle {
     void *mem;                      // single allocation holding everything below
     size_t mem_bytes;
     unsigned long long *invalid;    // device counter of rejected queries
+    bool pooled;                    // mem comes from the library's pool
+    bool captured;                  // a query was captured: a graph may still replay it
     int64_t table_bytes;
     // rmq_probe_gather on a table index: the per-element entries it looks up
     // (pre, suf, then block minima), allocated and built by its first call
@@ -76,6 +80,70 @@ int cuda_fail(cudaError_t err, const char *what) {
 }
 
 int device_info(DeviceInfo *out) {
+static std::mutex g_pool_mu;
+static cudaMemPool_t g_pool[64] = {nullptr};
+
+// The device's pool, made on first use; null when it cannot be.
+static cudaMemPool_t device_pool(int device) {
+    if (device < 0 || device >= 64) return nullptr;
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    if (!g_pool[device]) {
+        cudaMemPoolProps props;
+        std::memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t pool = nullptr;
+        cuuint64_t keep = kPoolKeep;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaGetLastError();
+            cudaMemPoolDestroy(pool);
+            return nullptr;
+        }
+        g_pool[device] = pool;
+    }
+    return g_pool[device];
+}
+
+static bool fail_alloc() {
+    const char *f = std::getenv("RTXRMQ_FAIL_ALLOC");
+    return f && f[0] == '1';
+}
+
+cudaError_t pool_malloc(void **p, size_t bytes, int device, cudaStream_t s, bool *pooled) {
+    *pooled = false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!fail_alloc() && bytes <= kPoolKeep && cudaStreamIsCapturing(s, &cap) == cudaSuccess &&
+        cap == cudaStreamCaptureStatusNone) {
+        cudaMemPool_t pool = device_pool(device);
+        if (pool && cudaMallocFromPoolAsync(p, bytes, pool, s) == cudaSuccess) {
+            *pooled = true;
+            return cudaSuccess;
+        }
+    }
+    cudaGetLastError();
+    cudaError_t err = dev_malloc(p, bytes);
+    if (err == cudaErrorMemoryAllocation && !fail_alloc()) {
+        // what the pool keeps may be what is missing
+        cudaGetLastError();
+        if (pool_trim(device) == cudaSuccess) err = dev_malloc(p, bytes);
+    }
+    return err;
+}
+
+cudaError_t pool_trim(int device) {
+    cudaMemPool_t pool = nullptr;
+    if (device >= 0 && device < 64) {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        pool = g_pool[device];
+    }
+    return pool ? cudaMemPoolTrimTo(pool, 0) : cudaSuccess;
+}
+
     static std::mutex mu;
     static DeviceInfo cache[64];
     static bool have[64] = {false};
@@ -216,7 +284,7 @@ int rmq_build_ex(const float *d_vals, int64_t n, int64_t bs, uint32_t flags, rmq
         return set_error(RMQ_ENOMEM, "rmq_build: host allocation failed");
     }
     h->device = dev.device;
-    cudaError_t err = dev_malloc(&h->mem, total);
+    cudaError_t err = pool_malloc(&h->mem, total, dev.device, stream, &h->pooled);
     if (err != cudaSuccess) {
         delete h->host_mu;
         delete h;
@@ -233,7 +301,10 @@ int rmq_build_ex(const float *d_vals, int64_t n, int64_t bs, uint32_t flags, rmq
     if (err == cudaSuccess) err = launch_build(p, dev, stream);
     if (err != cudaSuccess) {
         rc = cuda_fail(err, "rmq_build: launch");
-        cudaFree(h->mem);
+        if (h->pooled)
+            cudaFreeAsync(h->mem, stream);
+        else
+            cudaFree(h->mem);
         delete h->host_mu;
         delete h;
         return rc;
@@ -243,6 +314,14 @@ int rmq_build_ex(const float *d_vals, int64_t n, int64_t bs, uint32_t flags, rmq
 }
 
 int rmq_query(const rmq_handle_t *h, const int32_t *d_queries, int64_t q, float *d_val,
+// Remembers that a graph may replay work on the handle at any time.
+static void note_capture(const rmq_handle_t *h, cudaStream_t stream) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!h->pooled) return;
+    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+        const_cast<rmq_handle_t *>(h)->captured = true;
+}
+
               int32_t *d_idx, rmq_stream_t stream) {
     NvtxRange nvtx_range("rmq_query");
     g_err[0] = '\0';
@@ -271,6 +350,7 @@ int rmq_query(const rmq_handle_t *h, const int32_t *d_queries, int64_t q, float 
     cudaError_t err = launch_query(h->plan, a, dev, stream);
     if (err != cudaSuccess) return cuda_fail(err, "rmq_query: launch");
     return RMQ_OK;
+    note_capture(h, stream);
 }
 
 // The plan of a handle with pre / suf present. A table index has none: the
@@ -594,7 +674,16 @@ int rmq_free(rmq_handle_t *h) {
     g_err[0] = '\0';
     if (!h) return RMQ_OK;
     cudaError_t err = release_staging(h);
-    cudaError_t e2 = cudaFree(h->mem);
+    cudaError_t e2 = cudaSuccess;
+    if (h->pooled) {
+        // cudaFree does not wait for the uses of pool memory
+        int cur = 0;
+        e2 = cudaGetDevice(&cur);
+        if (e2 == cudaSuccess && cur != h->device) e2 = cudaSetDevice(h->device);
+        if (e2 == cudaSuccess) e2 = cudaDeviceSynchronize();
+        if (cur != h->device) cudaSetDevice(cur);
+    }
+    if (e2 == cudaSuccess) e2 = cudaFree(h->mem);
     if (err == cudaSuccess) err = e2;
     e2 = cudaFree(h->entries);
     if (err == cudaSuccess) err = e2;
@@ -605,6 +694,34 @@ int rmq_free(rmq_handle_t *h) {
 }
 
 int rmq_info(const rmq_handle_t *h, rmq_info_t *info) {
+int rmq_free_async(rmq_handle_t *h, rmq_stream_t stream) {
+    NvtxRange nvtx_range("rmq_free_async");
+    g_err[0] = '\0';
+    if (!h) return RMQ_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!h->pooled || h->captured || h->stage || h->entries ||
+        cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return rmq_free(h);
+    }
+    const cudaError_t err = cudaFreeAsync(h->mem, stream);
+    release_staging(h);
+    delete h->host_mu;
+    delete h;
+    if (err != cudaSuccess) return cuda_fail(err, "rmq_free_async");
+    return RMQ_OK;
+}
+
+int rmq_trim(void) {
+    g_err[0] = '\0';
+    DeviceInfo dev;
+    const int rc = device_info(&dev);
+    if (rc) return rc;
+    const cudaError_t err = pool_trim(dev.device);
+    if (err != cudaSuccess) return cuda_fail(err, "rmq_trim");
+    return RMQ_OK;
+}
+
     g_err[0] = '\0';
     if (!h || !info) return set_error(RMQ_EINVAL, "rmq_info: NULL argument");
     info->n = h->plan.n;
