@@ -5,15 +5,16 @@
 // OPTIX_CHECK print and carry on (common/common.h:57-69) and HRMQ calls
 // exit() (hrmq/RMQRMM64.cpp:237-240); here every failure is a status code
 // plus a per-thread message.
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
 
-#include "../../include/rmq.h"
 #include <cuda.h>  // cuuint64_t
 
+#include "../../include/rmq.h"
 #include "engine.h"
 #include "tables_impl.cuh"
 
@@ -22,9 +23,9 @@ struct rmq_handle {
     int device;
     void *mem;                      // single allocation holding everything below
     size_t mem_bytes;
-    unsigned long long *invalid;    // device counter of rejected queries
     bool pooled;                    // mem comes from the library's pool
     bool captured;                  // a query was captured: a graph may still replay it
+    unsigned long long *invalid;    // device counter of rejected queries
     int64_t table_bytes;
     // rmq_probe_gather on a table index: the per-element entries it looks up
     // (pre, suf, then block minima), allocated and built by its first call
@@ -79,7 +80,6 @@ int cuda_fail(cudaError_t err, const char *what) {
                      what, cudaGetErrorName(err), cudaGetErrorString(err));
 }
 
-int device_info(DeviceInfo *out) {
 static std::mutex g_pool_mu;
 static cudaMemPool_t g_pool[64] = {nullptr};
 
@@ -144,6 +144,7 @@ cudaError_t pool_trim(int device) {
     return pool ? cudaMemPoolTrimTo(pool, 0) : cudaSuccess;
 }
 
+int device_info(DeviceInfo *out) {
     static std::mutex mu;
     static DeviceInfo cache[64];
     static bool have[64] = {false};
@@ -313,7 +314,6 @@ int rmq_build_ex(const float *d_vals, int64_t n, int64_t bs, uint32_t flags, rmq
     return RMQ_OK;
 }
 
-int rmq_query(const rmq_handle_t *h, const int32_t *d_queries, int64_t q, float *d_val,
 // Remembers that a graph may replay work on the handle at any time.
 static void note_capture(const rmq_handle_t *h, cudaStream_t stream) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -322,6 +322,7 @@ static void note_capture(const rmq_handle_t *h, cudaStream_t stream) {
         const_cast<rmq_handle_t *>(h)->captured = true;
 }
 
+int rmq_query(const rmq_handle_t *h, const int32_t *d_queries, int64_t q, float *d_val,
               int32_t *d_idx, rmq_stream_t stream) {
     NvtxRange nvtx_range("rmq_query");
     g_err[0] = '\0';
@@ -349,8 +350,8 @@ static void note_capture(const rmq_handle_t *h, cudaStream_t stream) {
     a.invalid = h->invalid;
     cudaError_t err = launch_query(h->plan, a, dev, stream);
     if (err != cudaSuccess) return cuda_fail(err, "rmq_query: launch");
-    return RMQ_OK;
     note_capture(h, stream);
+    return RMQ_OK;
 }
 
 // The plan of a handle with pre / suf present. A table index has none: the
@@ -693,7 +694,6 @@ int rmq_free(rmq_handle_t *h) {
     return RMQ_OK;
 }
 
-int rmq_info(const rmq_handle_t *h, rmq_info_t *info) {
 int rmq_free_async(rmq_handle_t *h, rmq_stream_t stream) {
     NvtxRange nvtx_range("rmq_free_async");
     g_err[0] = '\0';
@@ -722,6 +722,7 @@ int rmq_trim(void) {
     return RMQ_OK;
 }
 
+int rmq_info(const rmq_handle_t *h, rmq_info_t *info) {
     g_err[0] = '\0';
     if (!h || !info) return set_error(RMQ_EINVAL, "rmq_info: NULL argument");
     info->n = h->plan.n;
@@ -732,8 +733,10 @@ int rmq_trim(void) {
     info->aligned = h->plan.aligned ? 1 : 0;
     info->table_bytes = h->table_bytes;
     info->struct_bytes = static_cast<int64_t>(h->mem_bytes);
-    info->micro_levels = h->plan.micro ? static_cast<int32_t>(micro_levels(
-                                             h->plan.bs < 64u ? 64u : h->plan.bs)) : 0;
+    // above 2^15: of the micro table that blocks of bs would need
+    info->micro_levels = static_cast<int32_t>(
+        h->plan.micro && h->plan.bs > (1u << 15) ? std::max(micro_levels(h->plan.bs), h->plan.mlevels)
+                                                 : h->plan.mlevels);
     info->light = h->plan.light ? 1 : 0;
     info->micro_table_bytes =
         h->plan.micro ? static_cast<int64_t>(static_cast<size_t>(h->plan.nmicro) *

@@ -306,12 +306,14 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
         a.qoff = qs;
         a.n = static_cast<uint32_t>(n) + lead;
         a.lead = lead;
-        a.bs = table_block(static_cast<uint32_t>(std::min<int64_t>(bs, std::max<int64_t>(n, 1))));
+        const TableShape shape = table_shape(
+            a.n, static_cast<uint32_t>(std::min<int64_t>(bs, std::max<int64_t>(n, 1))), 32u);
+        a.bs = shape.tbs;
         a.nb = (a.n + a.bs - 1) / a.bs;
         a.levels = a.nb > 0 ? st_levels(a.nb) : 0u;
         a.dv = make_div31(a.bs);
         a.nmicro = (a.n + kMicro - 1) / kMicro;
-        a.mlevels = a.n > 0 ? micro_levels(a.bs) : 0u;
+        a.mlevels = a.n > 0 ? shape.mlevels : 0u;
         a.moff_bytes = a.mlevels ? micro_offset_bytes(a.mlevels) : 0u;
         a.st = ws_entries;
         ws_entries += static_cast<int64_t>(a.nb) * a.levels;
@@ -331,13 +333,15 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
             const uint32_t units = (a.nmicro + kUnit - 1) / kUnit;
             for (uint32_t u = 0; u < units; u += kRunUnits)
                 runs.push_back(make_uint4(i, u, std::min(kRunUnits, units - u), 0));
-            add_items(1, i, kItemBlockMinima, 0, a.nb, std::max<uint32_t>(8u, lchunk / (a.bs / kMicro)));
+            if (!fused_blocks(a.bs / kMicro))
+                add_items(1, i, kItemBlockMinima, 0, a.nb, std::max<uint32_t>(8u, lchunk / (a.bs / kMicro)));
             if (split_rows(a.mlevels)) add_items(1, i, kItemRows, 0, a.nmicro, kBatchRowTile);
+            const int level_step = fused_blocks(a.bs / kMicro) ? 1 : 2;
             if (a.nb <= kOneItemTable) {
-                if (a.levels > 1) add_items(2, i, kItemTable, 0, a.nb, a.nb);
+                if (a.levels > 1) add_items(level_step, i, kItemTable, 0, a.nb, a.nb);
             } else {
                 for (uint32_t k = 0; k + 1 < a.levels; k += kLevelGroup)
-                    add_items(2 + static_cast<int>(k / kLevelGroup), i, kItemLevels, k, a.nb, lchunk);
+                    add_items(level_step + static_cast<int>(k / kLevelGroup), i, kItemLevels, k, a.nb, lchunk);
             }
         }
         for (int64_t j = 0; j < qc; j += qchunk)
@@ -358,6 +362,8 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
         if (!steps[k].empty()) P.steps = k + 1;
     }
     P.step_start[kMaxSteps] = static_cast<int32_t>(tables.size());
+    // the longest runs first, so that the short ones even out the end
+    std::stable_sort(runs.begin(), runs.end(), [](const uint4 &x, const uint4 &y) { return x.z > y.z; });
     P.nruns = static_cast<int32_t>(runs.size());
     P.nqitems = static_cast<int32_t>(b->h_qitems.size());
     P.total_q = b->total_q;
@@ -403,6 +409,7 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
     P.qitems = reinterpret_cast<const uint4 *>(base + o_q);
     P.invalid = reinterpret_cast<unsigned long long *>(base + o_cnt);
     P.ws = reinterpret_cast<Entry *>(base + o_ws);
+    P.next = reinterpret_cast<uint32_t *>(P.invalid + 1);  // cleared with it
     P.limit = b->limit;
     *out = b;
     return RMQ_OK;

@@ -6,8 +6,8 @@
 //   A  run items (array, first unit, units): micro-block minima and micro
 //      table, the plain builder's CTA body (build_run, tables_impl.cuh);
 //   B  table items (array, kind | level, first, count), one step per barrier:
-//      the block minima and the rows made apart from the masks at step 1, the
-//      block table's levels after them;
+//      the block minima and the rows not made in the runs at step 1, the block
+//      table's levels after them;
 //   C  query items (array, first query, count), query_impl.cuh's queued form.
 // Work lists are built on the host once per plan, so a run allocates nothing
 // and can be captured in a CUDA graph.
@@ -34,7 +34,7 @@ constexpr int kBatchThreads = kUnit;  // phase A runs the table builder
 constexpr int kBatchQPT = 2;
 // default tile schedule: queries per query item, table entries per level
 // item (a plan can set both per size bucket, rmq_batch_create_ex)
-constexpr uint32_t kQueryChunk = 2048;
+constexpr uint32_t kQueryChunk = 4096;
 constexpr uint32_t kLevelChunk = 4096;
 constexpr int kMaxSteps = 16;
 // units (of 256 micro-blocks) per run item: 512 KB of values, so that the 63
@@ -85,6 +85,7 @@ struct BatchParams {
     const uint4 *qitems;
     int32_t nqitems;
     int64_t total_q;      // one past the last query any array owns
+    uint32_t *next;       // work counters: runs, query items (0 between launches)
     uint32_t phases;      // bit 0 runs, bit 1 table steps, bit 2 queries
 };
 
@@ -143,6 +144,16 @@ __device__ __forceinline__ MicroTable batch_table(const BatchParams &P, const Ba
     return T;
 }
 
+// The next item of a work list for this CTA: items go to CTAs as they come
+// free (their costs differ by more than ten times). Called by the whole CTA;
+// a barrier on either side of the shared word.
+__device__ __forceinline__ int32_t next_item(uint32_t *counter, int32_t *s_item) {
+    __syncthreads();
+    if (threadIdx.x == 0) *s_item = static_cast<int32_t>(atomicAdd(counter, 1u));
+    __syncthreads();
+    return *s_item;
+}
+
 // Phase B: table steps 1 .. steps - 1, a grid barrier after each.
 __device__ __forceinline__ void table_steps(const BatchParams &P, cg::grid_group &grid,
                                             unsigned char *smem) {
@@ -167,8 +178,9 @@ __device__ __forceinline__ void table_steps(const BatchParams &P, cg::grid_group
 
 // Phase C: the query items, in the queued form.
 template <bool ALIGNED, uint32_t MODE>
-__device__ __forceinline__ void query_items(const BatchParams &P, MissQueue<true> &mq) {
-    for (int32_t it = (P.phases & 4u) ? blockIdx.x : P.nqitems; it < P.nqitems; it += gridDim.x) {
+__device__ __forceinline__ void query_items(const BatchParams &P, MissQueue<true> &mq, int32_t *s_item) {
+    if (!(P.phases & 4u)) return;
+    for (int32_t it; (it = next_item(P.next + 1, s_item)) < P.nqitems;) {
         const uint4 w = P.qitems[it];
         const BatchArray a = P.arrays[w.x];
         const V1View v = batch_view<MODE>(P, a);
@@ -186,17 +198,22 @@ __device__ __forceinline__ void query_items(const BatchParams &P, MissQueue<true
 template <bool ALIGNED, uint32_t MODE>
 __global__ void __launch_bounds__(kBatchThreads, RMQ_BATCH_MINB) batch_kernel(BatchParams P) {
     extern __shared__ __align__(1024) unsigned char s_batch[];
+    __shared__ int32_t s_item;
     cg::grid_group grid = cg::this_grid();
-    for (int32_t it = (P.phases & 1u) ? blockIdx.x : P.nruns; it < P.nruns; it += gridDim.x) {
+    // each counter is cleared in the phase that does not use it
+    if (blockIdx.x == 0 && threadIdx.x == 0) P.next[1] = 0u;
+    for (int32_t it; (P.phases & 1u) && (it = next_item(P.next, &s_item)) < P.nruns;) {
         const uint4 w = P.runs[it];
         const BatchArray &a = P.arrays[w.x];
         const uint32_t lo = w.y * kUnit;
         build_run<ALIGNED, MODE>(P.A, P.limit, a.off, a.n, a.lead, P.ws + a.mst, batch_table(P, a), lo,
-                                 min(lo + w.z * kUnit, a.nmicro), *reinterpret_cast<TableSmem *>(s_batch));
+                                 min(lo + w.z * kUnit, a.nmicro), P.ws + a.st, a.bs / 32u,
+                                 *reinterpret_cast<TableSmem *>(s_batch));
     }
     grid.sync();
+    if (blockIdx.x == 0 && threadIdx.x == 0) P.next[0] = 0u;
     table_steps(P, grid, s_batch);
-    query_items<ALIGNED, MODE>(P, reinterpret_cast<MissQueue<true> *>(s_batch)[threadIdx.x >> 5]);
+    query_items<ALIGNED, MODE>(P, reinterpret_cast<MissQueue<true> *>(s_batch)[threadIdx.x >> 5], &s_item);
 }
 
 std::atomic<int> g_batch_per_sm[4];  // per key mode, of this unit's alignment

@@ -48,11 +48,11 @@ void launch_units(const UnitJob &J, uint32_t nunits, uint32_t grid, cudaStream_t
 template <bool ALIGNED, uint32_t MODE>
 __global__ void __launch_bounds__(kUnit, RMQ_TABLE_MINB)
 table_kernel(const float *__restrict__ A, int64_t limit, int64_t base, uint32_t n, uint32_t lead,
-             Entry *mst, MicroTable T, uint32_t units) {
+             Entry *mst, MicroTable T, uint32_t units, Entry *bmin, uint32_t pb) {
     extern __shared__ __align__(1024) unsigned char s_table[];
     const uint32_t lo = blockIdx.x * units * kUnit;
     build_run<ALIGNED, MODE>(A, limit, base, n, lead, mst, T, lo, min(lo + units * kUnit, T.nmicro),
-                             *reinterpret_cast<TableSmem *>(s_table));
+                             bmin, pb, *reinterpret_cast<TableSmem *>(s_table));
 }
 
 // Block minima: a thread per block of up to 16 micro-blocks, else a warp.
@@ -128,7 +128,7 @@ cudaError_t launch_runs_t(const BuildPlan &p, const MicroTable &T, const DeviceI
     const uint32_t cap = static_cast<uint32_t>(dev.sms) * static_cast<uint32_t>(per_sm);
     const uint32_t all = (p.nmicro + kUnit - 1) / kUnit, units = (all + cap - 1) / cap;
     kern<<<(all + units - 1) / units, kUnit, sizeof(TableSmem), s>>>(
-        p.A, p.limit, p.off, p.n, p.lead, p.mst, T, units);
+        p.A, p.limit, p.off, p.n, p.lead, p.mst, T, units, p.st, p.tbs / kMicro);
     return cudaGetLastError();
 }
 
@@ -168,10 +168,12 @@ cudaError_t launch_build_tables(const BuildPlan &p, const DeviceInfo &dev, cudaS
         if (err != cudaSuccess) return err;
     }
     const uint32_t pb = p.tbs / kMicro, per_cta = pb <= 16u ? kBlockThreads : kBlockThreads / 32;
-    block_minima_kernel<<<(p.nb + per_cta - 1) / per_cta, kBlockThreads, 0, s>>>(p.mst, p.nmicro, pb,
-                                                                               p.st, p.nb, per_cta);
-    err = cudaGetLastError();
-    if (err != cudaSuccess) return err;
+    if (!fused_blocks(pb)) {
+        block_minima_kernel<<<(p.nb + per_cta - 1) / per_cta, kBlockThreads, 0, s>>>(
+            p.mst, p.nmicro, pb, p.st, p.nb, per_cta);
+        err = cudaGetLastError();
+        if (err != cudaSuccess) return err;
+    }
     return launch_levels(p.st, p.nb, p.levels, s);
 }
 
@@ -204,10 +206,11 @@ size_t plan_index(BuildPlan &p, bool no_micro) {
     p.limit = p.n;
     p.lead = 0;
     p.micro = !no_micro;
-    p.tbs = p.micro ? table_block(p.bs) : p.bs;
+    const TableShape shape = table_shape(p.n, p.bs, 128u);
+    p.tbs = p.micro ? shape.tbs : p.bs;
     p.nb = (p.n + p.tbs - 1) / p.tbs;
     p.levels = st_levels(p.nb);
-    p.mlevels = p.micro ? micro_levels(p.tbs) : 0u;
+    p.mlevels = p.micro ? shape.mlevels : 0u;
     p.nmicro = p.micro ? (p.n + kMicro - 1) / kMicro : 0u;
     p.moff_bytes = p.micro ? micro_offset_bytes(p.mlevels) : 0u;
     p.aligned = reinterpret_cast<uintptr_t>(p.A) % 16 == 0;

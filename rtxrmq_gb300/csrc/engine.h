@@ -11,6 +11,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include "common.cuh"
+#include "tables_impl.cuh"
 
 namespace rmq {
 
@@ -49,7 +50,6 @@ inline cudaError_t dev_malloc(void **p, size_t bytes) {
     return cudaMalloc(p, bytes);
 }
 
-// Resident CTAs per SM of `kernel` at `threads` threads and `dynamic_smem`
 // Device memory of an index, in stream order: from a pool of the library (one
 // per device) that keeps at most kPoolKeep bytes of freed memory; the rest
 // goes back to the device at the next synchronisation, all of it by
@@ -60,6 +60,7 @@ constexpr size_t kPoolKeep = size_t(256) << 20;
 cudaError_t pool_malloc(void **p, size_t bytes, int device, cudaStream_t s, bool *pooled);
 cudaError_t pool_trim(int device);
 
+// Resident CTAs per SM of `kernel` at `threads` threads and `dynamic_smem`
 // bytes of dynamic shared memory, computed once per cache slot; concurrent
 // first callers compute and store the same value.
 template <class K>
@@ -123,15 +124,37 @@ uint32_t micro_levels(uint32_t bs);
 inline uint32_t micro_offset_bytes(uint32_t mlevels) {
     return mlevels <= 9 ? 1u : (mlevels <= 17 ? 2u : 4u);
 }
-// Block size of the block table of a table index asked for with block size
-// bs. Multiples of 32 (blocks hold whole micro-blocks), at least 64. Above
-// 2^15 the micro table would be 13 rows and more of 2-byte offsets, too large
-// for L2 and read twice per query: queries inside such blocks go through
-// blocks of 4096 instead (n = 1e8, 2^26 queries, lr=-2, bs 195312: 0.83 ms
-// with the rows, 0.48 with blocks of 4096).
-inline uint32_t table_block(uint32_t bs) {
-    if (bs > (1u << 15)) return 4096u;
-    return bs <= 64u ? 64u : (bs + 31u) / 32u * 32u;
+// Shape of a table index over n elements asked for with block size bs: the
+// blocks of its block table (multiples of 32, so that blocks hold whole
+// micro-blocks, at least 64) and the levels of its micro table.
+struct TableShape {
+    uint32_t tbs, mlevels;
+};
+// - Blocks above 2^15: the micro table would be 13 rows and more of 2-byte
+//   offsets, too large for L2 and read twice per query; 4096 instead (n = 1e8,
+//   2^26 queries, lr=-2, bs 195312: 0.83 ms with the rows, 0.58 with 4096).
+// - Fewer than `least_blocks`: a range of a few blocks is open as often as the
+//   blocks at its ends are larger than it, so the blocks shrink until there
+//   are that many, and windows of up to 511 micro-blocks do (rows up to level
+//   8 are made in the run of the minima, longer ones take another launch).
+//   Plain index: 128 (n = 3e5, bs 2^15, uniform lengths, 2^25 queries: 0.318 ms
+//   with 10 blocks, 0.291 with 128). Batch: 32; with 128 the ragged benchmark's
+//   build takes 1.83 ms in place of 1.67 for its many small block tables, and
+//   its queries gain nothing.
+// - The masks answer windows of up to 63 (127) micro-blocks whatever the
+//   block size: 6 or 7 levels cost nothing.
+inline TableShape table_shape(uint32_t n, uint32_t bs, uint32_t least_blocks) {
+    TableShape s;
+    s.tbs = bs > (1u << 15) ? 4096u : bs <= 64u ? 64u : (bs + 31u) / 32u * 32u;
+    const uint32_t least = mask_levels(wide_masks((n + kMicro - 1) / kMicro));
+    s.mlevels = micro_levels(s.tbs);
+    if (s.mlevels < least) s.mlevels = least;
+    const uint32_t few = (n / least_blocks + 31u) / 32u * 32u;
+    if (few < s.tbs) {
+        s.tbs = few < 64u ? 64u : few;
+        if (s.mlevels > 9u) s.mlevels = 9u;
+    }
+    return s;
 }
 
 // Fill the size fields of a plan (A, n, bs and light given; the table index

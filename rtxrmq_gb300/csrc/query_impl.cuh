@@ -371,6 +371,9 @@ __device__ __forceinline__ void stage_lines(const V1View &v, uint32_t line, uint
         // slot 4 t + grp: its swizzle depends on t's parity alone
         const uint32_t d0 = staged_line(stage, grp) ^ (sub << 4);
         const uint32_t d1 = staged_line(stage, 4u + grp) ^ (sub << 4);
+        // through L1 (.ca): of a small array thousands of warps want the same
+        // few lines, which queue up at the L2 (n = 1335, 2^25 ranges of 20: 0.92
+        // ms, 1.78 with .cg; n = 1e8, lr=-3: 0.798 and 0.787)
 #pragma unroll
         for (uint32_t t = 0; t < kStageLines / 4; ++t) {
             const uint32_t ln = __shfl_sync(0xffffffffu, line, h + 4u * t + grp);
@@ -378,7 +381,7 @@ __device__ __forceinline__ void stage_lines(const V1View &v, uint32_t line, uint
             const float *src = base + static_cast<size_t>(ln) * 32;
             const uint32_t dst = ((t & 1u) ? d1 : d0) + (t / 2u) * 1024u;
             if ((bt >> (4u * sub)) & 15u && rmq_chk(v.off + static_cast<int64_t>(ln) * 32 + 32 <= v.limit))
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
         }
     } else {
 #pragma unroll 1
@@ -523,22 +526,65 @@ __device__ __forceinline__ Entry finish_entries(const V1View &v, bool left, uint
     return better(better(e1, other), mid);
 }
 
+// Leftmost best of l .. r inside one micro-block and within kShortChunks
+// 16-byte chunks, by the lane alone. More chunks cost more L1 lookups than
+// the warp's staged copy of the line does (one). 2^25 ranges of 8 in an array
+// of 3e5: 0.99 ms all staged, 1.06 with two chunks, 0.74 with three.
+constexpr uint32_t kShortChunks = 3;
+template <bool ALIGNED, uint32_t MODE>
+__device__ __forceinline__ Entry short_range(const V1View &v, uint32_t l, uint32_t r) {
+    const uint32_t c = l & ~3u;
+    const int64_t g = v.off + c;
+    uint32_t w[4 * kShortChunks];
+    if (ALIGNED && (v.off & 3) == 0 && g + 4 * kShortChunks <= v.limit) {
+#pragma unroll
+        for (uint32_t k = 0; k < kShortChunks; ++k) {
+            // past r the first chunk again: no further line
+            const uint4 x = ld_elem4(v, c + 4u * k <= r ? g + 4 * k : g);
+            w[4 * k] = x.x, w[4 * k + 1] = x.y, w[4 * k + 2] = x.z, w[4 * k + 3] = x.w;
+        }
+    } else {
+#pragma unroll
+        for (uint32_t k = 0; k < 4 * kShortChunks; ++k)
+            w[k] = c + k >= l && c + k <= r ? ld_elem(v, g + k) : 0u;
+    }
+    using B = Best<MODE>;
+    typename B::T best = B::fill();
+#pragma unroll
+    for (uint32_t k = 0; k < 4 * kShortChunks; ++k)
+        if (c + k >= l && c + k <= r) best = B::best(best, B::of(w[k]));
+    // the first element holding it; l when none does or only the fill
+    uint32_t pos = l, wb = 0u;
+#pragma unroll
+    for (int k = 4 * kShortChunks - 1; k >= 0; --k)
+        if (c + k >= l && c + k <= r && B::of(w[k]) == best) pos = c + k, wb = w[k];
+    const bool last = !(best == best) || best == B::fill();
+    return (static_cast<uint64_t>(last ? 0xffffffffu : key_of(wb, MODE)) << 32) |
+           ((last ? l : pos) << 1) | (last ? 0u : negzero_of(wb, MODE));
+}
+
 // One warp's queue (up to 31 waiting queries plus the 32 that one query slot
-// of a step can add, 12 bytes each) and its line stage: what they take from
-// the L1 matters, the block table's upper levels live there. `id` numbers the
-// queries of the CTA in the order it takes them: step * step size + place in
-// the step.
+// of a step can add, 16 bytes each) and its line stage. What they take from
+// the L1 matters, the block table's upper levels live there: 3 KB per warp
+// are 100 KB per SM, with 256 bytes more the next carve-out is 132 KB (n =
+// 1e8, uniform lengths, bs 2^14: 0.36 and 0.45 ms). `id` numbers the queries
+// of the CTA in the order it takes them: step * step size + place in the
+// step.
 template <bool MICRO>
 struct MissQueue {
     static constexpr int kCap = 64;
     uint4 stage[MICRO ? kStageLines * 8 : 1];
-    Entry part[MICRO ? kCap : 1];  // kSecond: the best of what is settled so far
-    uint32_t l[kCap];   // kMissLeft set: the probe's best lay left of l
-    uint32_t r[kCap];   // kSecond set: back for its other end
-    uint32_t id[kCap];
+    uint32_t l[kCap];    // kMissLeft set: the probe's best lay left of l
+    uint32_t r[kCap];    // kSecond set: back for its other end
+    uint32_t id[kCap];   // below 2^30
+    uint32_t key[MICRO ? kCap : 1];
 };
-constexpr uint32_t kSecond = 0x80000000u;  // above every index
 constexpr uint32_t kMissLeft = 0x80000000u;  // above every index
+// A query back for its other end has the best of the end that is settled in
+// its entry: its key, its index in place of that end's position (it lies in
+// the same unit), its -0.0 flag, and which table's units are meant.
+constexpr uint32_t kSecond = 0x80000000u;
+constexpr uint32_t kPartNegzero = 0x80000000u, kPartMicro = 0x40000000u;  // in id
 
 // The queries a CTA takes: steps of `chunk` consecutive ones, `stride` apart.
 struct StepMap {
@@ -568,38 +614,40 @@ __device__ __forceinline__ void drain_misses(const V1View &v, const QueryOut &o,
     const uint32_t e = count + lane;
     const bool act = lane < take;
     const uint32_t lq = act ? mq.l[e] : 0u, rq = act ? mq.r[e] : 0u;
-    const uint32_t id = act ? mq.id[e] : 0u;
+    const uint32_t iq = act ? mq.id[e] : 0u;
     const uint32_t l = lq & ~kMissLeft, r = rq & ~kSecond;
+    const uint32_t id = iq & ~(kPartNegzero | kPartMicro);
     const bool left = (lq & kMissLeft) != 0u;
     Entry res = kEntryNone;
-    bool again = false;
+    bool again = false, micro = false;
     if constexpr (!MICRO) {
         if (act) res = finish_entries<STATS>(v, left, l, r, pol, s);
     } else {
         const uint32_t stage = static_cast<uint32_t>(__cvta_generic_to_shared(mq.stage));
         const bool second = (rq & kSecond) != 0u;
         const bool side = left != second;  // the end whose line is wanted
-        const bool scan = (l >> 5) == (r >> 5);
+        const bool scan = !second && (l >> 5) == (r >> 5);
         const uint32_t line = (side ? l : r) >> 5;
         // the left end's unit lies before the right end's, so its line is whole
         uint32_t bits = scan ? bit_range(l & 31u, r & 31u)
                         : side ? 0xffffffffu << (l & 31u) : 0xffffffffu >> (31u - (r & 31u));
         if (!act) bits = 0u;
         stage_lines<ALIGNED>(v, line, bits, stage, 0u);
-        if (second) res = mq.part[e];
         // the probes run while the lines arrive
-        Entry e2 = kEntryNone;
         if (act && !scan) {
-            const bool micro = (r >> 5) - (l >> 5) < v.micro_span;
+            micro = second ? (iq & kPartMicro) != 0u : (r >> 5) - (l >> 5) < v.micro_span;
             const uint32_t a = micro ? (l >> 5) : div31_ge2(l, v.dv);
             const uint32_t b = micro ? (r >> 5) : div31_ge2(r, v.dv);
             const uint32_t lo = a + (left || second), hi = b - (!left || second);
+            Entry e2 = kEntryNone;
             if (lo <= hi)
                 e2 = micro ? micro_probe<STATS>(v, lo, hi, pol, s) : st_probe<STATS>(v, lo, hi, pol, s);
-            res = better(res, end_rest<STATS>(v, micro, side, a, b, l, r, pol, s));
+            res = end_rest<STATS>(v, micro, side, a, b, l, r, pol, s);
             const uint32_t m2 = entry_idx(e2);
             again = !second && (left ? m2 > r : m2 < l);
             if (!again) res = better(res, e2);
+            if (second)
+                res = better(res, (static_cast<uint64_t>(mq.key[e]) << 32) | ((left ? l : r) << 1) | (iq >> 31));
             if constexpr (STATS)
                 if (!second) s.c[again ? kStatFull : kStatSecond] += 1u;
         }
@@ -615,10 +663,11 @@ __device__ __forceinline__ void drain_misses(const V1View &v, const QueryOut &o,
         const unsigned mask = __ballot_sync(0xffffffffu, again);
         if (again) {
             const uint32_t w = count + __popc(mask & ((1u << lane) - 1u));
-            mq.l[w] = lq;
-            mq.r[w] = r | kSecond;
-            mq.id[w] = id;
-            mq.part[w] = res;
+            const uint32_t at = entry_idx(res);
+            mq.l[w] = left ? at | kMissLeft : l;
+            mq.r[w] = (left ? r : at) | kSecond;
+            mq.id[w] = id | (static_cast<uint32_t>(res) << 31) | (micro ? kPartMicro : 0u);
+            mq.key[w] = static_cast<uint32_t>(res >> 32);
         }
         count += __popc(mask);
     }
@@ -672,8 +721,10 @@ __device__ __forceinline__ Entry superset_probe(const V1View &v, uint32_t l, uin
 // block spans few enough micro-blocks for the micro table, and only the
 // block table serves longer ones). Queries left open join the warp's queue, whose length `count`
 // carries from step to step (`last` empties it); `id0` is the step's first
-// query in the CTA's numbering.
-template <bool ALIGNED, bool MICRO, uint32_t MODE, int THREADS, int QPT, bool STATS, bool LEAD>
+// query in the CTA's numbering. SHORT: the lanes settle the shortest ranges
+// themselves.
+template <bool ALIGNED, bool MICRO, uint32_t MODE, int THREADS, int QPT, bool STATS, bool LEAD,
+          bool SHORT>
 __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryOut &o,
                                                    const StepMap &map, int64_t base, uint32_t cnt,
                                                    uint32_t id0, bool last,
@@ -696,15 +747,10 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
         ok[k] = in[k].x >= 0 && l <= r && r < v.n;
         scan[k] = MICRO && (l >> 5) == (r >> 5);
         res[k] = kEntryNone;
-        if (ok[k]) {
-            if (!scan[k])
-                res[k] = superset_probe<MICRO, STATS>(v, l, r, pol, s);
-            else if (l == r)
-                res[k] = make_entry(ld_elem(v, v.off + l), l, MODE);
-        }
+        if (ok[k] && !scan[k]) res[k] = superset_probe<MICRO, STATS>(v, l, r, pol, s);
     }
     bool miss[QPT];
-    bool any_miss = false;
+    bool any_miss = false, any_scan = false;
 #pragma unroll
     for (int k = 0; k < QPT; ++k) {
         const uint32_t j = threadIdx.x + k * THREADS;
@@ -717,10 +763,11 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
             }
             continue;
         }
-        // a query inside one micro-block (of more than one element) still
-        // holds kEntryNone here, whose index lies outside [l, r]
+        // a query inside one micro-block still holds kEntryNone here, whose
+        // index lies outside [l, r]
         miss[k] = entry_idx(res[k]) - l > r - l;
         any_miss |= miss[k];
+        any_scan |= scan[k];
         if constexpr (STATS) {
             if (MICRO && scan[k]) {
                 s.c[kStatMicroScan] += 1u;
@@ -769,6 +816,7 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
     // queue what is open, slot by slot, and drain: one copy of the drain's
     // code (every copy costs instruction fetches)
     if (!last && !__any_sync(0xffffffffu, any_miss)) return;
+    const bool scans = MICRO && SHORT && __any_sync(0xffffffffu, any_scan);
 #pragma unroll 1
     for (int k = 0; k < QPT; ++k) {
         int2 lr = qq[0];
@@ -781,6 +829,13 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
                 open = miss[j];
                 at = entry_idx(res[j]);
             }
+        if (scans) {
+            const uint32_t l = static_cast<uint32_t>(lr.x), r = static_cast<uint32_t>(lr.y);
+            if (open && (l >> 5) == (r >> 5) && (r >> 2) - (l >> 2) < kShortChunks) {
+                put_result(o, base + threadIdx.x + k * THREADS, short_range<ALIGNED, MODE>(v, l, r), MODE, lead);
+                open = false;
+            }
+        }
         const unsigned mask = __ballot_sync(0xffffffffu, open);
         if (open) {
             const uint32_t l = static_cast<uint32_t>(lr.x);
@@ -819,12 +874,16 @@ __device__ __forceinline__ void answer_range_queued(const V1View &v, const Query
     const StepMap map{q0, step};
     QStats s;
     uint32_t waiting = 0, id0 = 0;
+    int2 qq[QPT];
+    load_queries<QPT>(o, q0, q1, qq);
     for (int64_t base = q0; base < q1; base += step, id0 += step) {
-        int2 qq[QPT];
-        load_queries<QPT>(o, base, q1, qq);
-        answer_step_queued<ALIGNED, MICRO, MODE, THREADS, QPT, false, LEAD>(
+        int2 nxt[QPT];
+        load_queries<QPT>(o, base + step, q1, nxt);  // in flight while this step is answered
+        answer_step_queued<ALIGNED, MICRO, MODE, THREADS, QPT, false, LEAD, false>(
             v, o, map, base, static_cast<uint32_t>(min(step, q1 - base)), id0, base + step >= q1, qq,
             s, mq, waiting);
+#pragma unroll
+        for (int k = 0; k < QPT; ++k) qq[k] = nxt[k];
     }
 }
 

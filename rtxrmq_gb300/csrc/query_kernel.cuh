@@ -59,7 +59,7 @@ query_kernel(V1View v, QueryOut o, int64_t q, unsigned long long *stats) {
             load_full(o, c1, nxt);
         else if (c1 < q)
             load_queries<kQPT>(o, c1, q, nxt);
-        answer_step_queued<ALIGNED, MICRO, MODE, kThreads, kQPT, STATS, LEAD>(
+        answer_step_queued<ALIGNED, MICRO, MODE, kThreads, kQPT, STATS, LEAD, true>(
             v, o, map, c0, static_cast<uint32_t>(min(chunk, q - c0)), id0, c1 >= q, cur, s, mq, waiting);
 #pragma unroll
         for (int k = 0; k < kQPT; ++k) cur[k] = nxt[k];
@@ -75,8 +75,9 @@ cudaError_t occupancy(K kernel, std::atomic<int> *cache, int *per_sm) {
 }
 
 // `bytes` of shared memory per SM (the runtime's 1 KB per CTA included) as a
-// percentage of the largest carve-out, 228 KB.
-int carveout_percent(size_t bytes) { return static_cast<int>((bytes * 100 + 228 * 1024 - 1) / (228 * 1024)); }
+// percentage of the largest carve-out, 228 KB. Rounded down: a hint above one
+// of the supported sizes takes the next one.
+int carveout_percent(size_t bytes) { return static_cast<int>(bytes * 100 / (228 * 1024)); }
 
 uint32_t grid_size(int64_t q, int64_t per_block, int per_sm, const DeviceInfo &dev) {
     const int64_t need = (q + per_block - 1) / per_block;

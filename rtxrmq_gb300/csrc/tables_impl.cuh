@@ -149,21 +149,29 @@ struct TableSmem {
     Entry c[kRing];                     // best of the whole mask's window
     uint32_t key[kRing + kMirror];
     uint32_t half[kRing + kMirror];     // masks of windows of 32, 0 past the array
+    Entry warp[kUnit / 32];             // each warp's best
 };
+
+// Whether the run also reduces its blocks' minima: blocks of pb micro-blocks
+// tile a unit. (Read again from the micro-block minima, they cost the ragged
+// benchmark 0.44 GB and a grid barrier.)
+RMQ_HD bool fused_blocks(uint32_t pb) { return pb <= kUnit && (pb & (pb - 1u)) == 0u; }
 
 // Micro-blocks [lo, hi) (multiples of kUnit, or hi the array's last) of the
 // array whose element 0 is value `base`; the CTA of kUnit threads. With `T`'s
-// rows only when they are not split.
+// rows only when they are not split, the block minima only when they are fused.
 template <bool ALIGNED, uint32_t MODE>
 __device__ __forceinline__ void build_run(const float *__restrict__ A, int64_t limit, int64_t base,
                                           uint32_t n, uint32_t lead, Entry *mst, const MicroTable &T,
-                                          uint32_t lo, uint32_t hi, TableSmem &sm) {
+                                          uint32_t lo, uint32_t hi, Entry *bmin, uint32_t pb,
+                                          TableSmem &sm) {
     const uint32_t t = threadIdx.x, warp = t >> 5;
     const uint32_t stage = static_cast<uint32_t>(__cvta_generic_to_shared(sm.stage)) + 4096u * warp;
     const bool wide = wide_masks(T.nmicro);
     const uint32_t k0 = mask_levels(wide), span = 1u << (k0 - 1u);
     const bool rows = T.mlevels > k0 && !split_rows(T.mlevels);
     const uint32_t reach = rows ? (1u << (T.mlevels - 1u)) - 1u : 63u;
+    const bool blocks = fused_blocks(pb);
     LineStep step;
     auto issue = [&](uint32_t s, uint32_t cnt) {
         const uint32_t w0 = 32u * warp;
@@ -198,7 +206,25 @@ __device__ __forceinline__ void build_run(const float *__restrict__ A, int64_t l
             }
             if (out && rmq_chk(j < T.nmicro)) mst[j] = m;
         }
+        if (blocks) {
+            // the best of min(pb, 32) lanes; of more, the warps' bests below
+            Entry best = have ? m : kEntryNone;
+            if (pb >= 32u) {
+                const uint32_t k = __reduce_min_sync(0xffffffffu, static_cast<uint32_t>(best >> 32));
+                const uint32_t l = __reduce_min_sync(
+                    0xffffffffu, static_cast<uint32_t>(best >> 32) == k ? static_cast<uint32_t>(best) : 0xffffffffu);
+                if ((t & 31u) == 0u) sm.warp[warp] = (static_cast<uint64_t>(k) << 32) | l;
+            } else {
+                for (uint32_t o = pb >> 1; o > 0u; o >>= 1) best = better(best, __shfl_xor_sync(0xffffffffu, best, o));
+                if (out && have && (t & (pb - 1u)) == 0u) bmin[j / pb] = best;
+            }
+        }
         __syncthreads();
+        if (blocks && out && pb >= 32u && t < kUnit / pb && t * pb < cnt) {
+            Entry best = sm.warp[t * (pb / 32u)];
+            for (uint32_t i = 1; i < pb / 32u; ++i) best = better(best, sm.warp[t * (pb / 32u) + i]);
+            bmin[s / pb + t] = best;
+        }
         const uint32_t next = out ? s - kUnit : (hi - 1u) / kUnit * kUnit;
         const bool more = out ? s > lo : true;
         if (more) issue(next, min(hi - next, kUnit));
