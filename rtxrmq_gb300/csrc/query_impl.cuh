@@ -102,8 +102,18 @@ __device__ __forceinline__ Entry ld_entry_keep(const Entry *t, uint64_t i, uint6
     return v;
 }
 
-// Mask of micro-block j, and offset i of the micro table's rows. Width is the
-// same for every query of an index, so the branches on it do not diverge.
+// Mask of micro-block j, its low 32 bits, and offset i of the micro table's
+// rows. Width is the same for every query of an index, so the branches on it
+// do not diverge. The low word serves windows of up to 32 micro-blocks of
+// either width, with 32-bit shifts (n = 1e8, lr = -3, with the queue's one
+// drain site: 0.795 and 0.771 ms).
+__device__ __forceinline__ uint32_t ld_mask_low(const V1View &v, uint32_t j, uint64_t pol) {
+    if (!rmq_chk(j < v.nmicro)) return 1u;
+    const uint32_t *at = static_cast<const uint32_t *>(v.mask) + (static_cast<uint64_t>(j) << (v.wide ? 1 : 0));
+    uint32_t r;
+    asm volatile("ld.global.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(r) : "l"(at), "l"(pol));
+    return r;
+}
 __device__ __forceinline__ uint64_t ld_mask(const V1View &v, uint32_t j, uint64_t pol) {
     if (!rmq_chk(j < v.nmicro)) return 1u;
     if (v.wide) {
@@ -276,12 +286,10 @@ __device__ __forceinline__ Entry micro_probe(const V1View &v, uint32_t a, uint32
     const uint32_t w = b - a + 1u;
     if (w <= (v.wide ? 64u : 32u)) {
         uint32_t x = a;
-        if (w > 1u) {
-            if (v.wide)
-                x += 63u - __clzll(ld_mask(v, a, pol) & (~0ull >> (64u - w)));
-            else
-                x += 31u - __clz(static_cast<uint32_t>(ld_mask(v, a, pol)) & (0xffffffffu >> (32u - w)));
-        }
+        if (w > 32u)
+            x += 63u - __clzll(ld_mask(v, a, pol) & (~0ull >> (64u - w)));
+        else if (w > 1u)
+            x += 31u - __clz(ld_mask_low(v, a, pol) & (0xffffffffu >> (32u - w)));
         if constexpr (STATS) s.c[kStatTable] += w > 1u ? 2u : 1u;
         return ld_entry_keep(v.mst, x, v.nmicro, pol);
     }
@@ -351,8 +359,6 @@ __device__ __forceinline__ uint32_t range_sectors(const V1View &v, uint32_t a, u
 // block tables live in (n = 1e8, 2^26 queries, uniform lengths, bs 2^15:
 // 0.33 ms with 16, 0.57 with 32; ranges of 32: 1.60 and 1.81).
 constexpr int kStageLines = 16;
-constexpr int kLanesPerLine = 32 / kStageLines;
-constexpr int kChunksPerLane = 8 / kLanesPerLine;
 
 // Starts copying the chunks holding a set bit of the requests of lanes
 // h .. h + kStageLines - 1 into the warp's stage. Bytes past the end of the
@@ -402,21 +408,28 @@ __device__ __forceinline__ void stage_lines(const V1View &v, uint32_t line, uint
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-// Waits for the staged lines and returns, on lanes h .. h + kStageLines - 1
-// with bits != 0, the leftmost best of their requests; kEntryNone elsewhere.
-// The set bits of a request are consecutive.
+// What a request's lane knows of its line before it forms the entry: the bits
+// of the best element and its position, or that every element of the request
+// has the largest key (no number, or the fill), when the first of them is it.
+struct LineBest {
+    uint32_t bits, pos;
+    bool last;
+};
+
+// Waits for the staged lines and gives lanes h .. h + kStageLines - 1 the best
+// of their requests (leftmost; meaningless without a set bit). Two lanes
+// reduce a line, four consecutive chunks each; they meet on the value, and a
+// request's key is formed once, by its own lane. The set bits of a request
+// are consecutive.
 template <uint32_t MODE>
-__device__ __forceinline__ Entry reduce_lines(uint32_t line, uint32_t bits, uint32_t stage,
-                                              uint32_t h) {
+__device__ __forceinline__ void reduce_lines(uint32_t bits, uint32_t stage, uint32_t h, LineBest &out) {
     using B = Best<MODE>;
-    constexpr uint32_t kBits = 4u * kChunksPerLane;
+    static_assert(kStageLines == 16, "two lanes per line");
     const uint32_t lane = threadIdx.x & 31u;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncwarp();
-    // kLanesPerLine lanes per line, kChunksPerLane consecutive chunks each
-    const uint32_t slot = lane / kLanesPerLine, c0 = (lane % kLanesPerLine) * kChunksPerLane;
-    const uint32_t all = kLanesPerLine == 1 ? bits : __shfl_sync(0xffffffffu, bits, h + slot);
-    const uint32_t mine = kBits == 32u ? all : (all >> (4u * c0)) & ((1u << (kBits % 32u)) - 1u);
+    const uint32_t slot = lane >> 1, c0 = (lane & 1u) * 4u;
+    const uint32_t mine = (__shfl_sync(0xffffffffu, bits, h + slot) >> (4u * c0)) & 0xffffu;
     const uint32_t base = staged_line(stage, slot) ^ (c0 << 4);
     // the elements outside the request in its first and last chunk are
     // overwritten with the fill, so that only whole chunks are selected below
@@ -429,42 +442,35 @@ __device__ __forceinline__ Entry reduce_lines(uint32_t line, uint32_t bits, uint
         if (3u - k > (end & 3u))
             asm volatile("st.shared.u32 [%0], %1;" :: "r"((base ^ ((end >> 2) << 4)) + 12u - 4u * k), "r"(fill) : "memory");
     }
-    typename B::T m[kChunksPerLane];
+    typename B::T m[4];
 #pragma unroll
-    for (int c = 0; c < kChunksPerLane; ++c) {
+    for (int c = 0; c < 4; ++c) {
         const uint4 f = lds_chunk(base ^ (c << 4));
         m[c] = B::best(B::best(B::best(B::of(f.x), B::of(f.y)), B::of(f.z)), B::of(f.w));
         m[c] = mine & (15u << (4 * c)) ? m[c] : B::fill();
     }
-    typename B::T mm = m[0];
-#pragma unroll
-    for (int c = 1; c < kChunksPerLane; ++c) mm = B::best(mm, m[c]);
-    // the first chunk holding it, and in that chunk the first element
-    uint32_t cs = 0u;
-#pragma unroll
-    for (int c = kChunksPerLane - 1; c >= 0; --c) cs = m[c] == mm ? c : cs;
-    const uint4 f = lds_chunk(base ^ (cs << 4));
+    typename B::T mm = B::best(B::best(m[0], m[1]), B::best(m[2], m[3]));
+    const typename B::T both = B::best(mm, B::of(__shfl_xor_sync(0xffffffffu, B::bits(mm), 1)));
+    // the half that holds the best (the left one when both do), in it the
+    // first chunk and the first element
+    const uint32_t holds = __ballot_sync(0xffffffffu, mm == both);
+    const uint32_t cs = m[0] == mm ? 0u : m[1] == mm ? 1u : m[2] == mm ? 2u : 3u;
     uint32_t wb;
-    const uint32_t pos = first_in_chunk<MODE>(f, mm, wb);
-    // no number, or nothing above the fill: every element of the request has
-    // the largest key, and the first of them is the best
-    const bool last = !(mm == mm) || mm == B::fill();
-    uint32_t hi = last ? 0xffffffffu : key_of(wb, MODE);
-    uint32_t lo = (4u * c0 + (last ? first : 4u * cs + pos)) << 1 | (last ? 0u : negzero_of(wb, MODE));
-    if (kLanesPerLine > 1) {
-        if (mine == 0u) lo = 0xffffffffu;
-#pragma unroll
-        for (int o = 1; o < kLanesPerLine; o <<= 1) {
-            const uint32_t th = __shfl_xor_sync(0xffffffffu, hi, o), tl = __shfl_xor_sync(0xffffffffu, lo, o);
-            if (th < hi || (th == hi && tl < lo)) hi = th, lo = tl;
-        }
-        const uint32_t from = ((lane - h) * kLanesPerLine) & 31u;
-        hi = __shfl_sync(0xffffffffu, hi, from);
-        lo = __shfl_sync(0xffffffffu, lo, from);
-    }
+    const uint32_t pos = 4u * (c0 + cs) + first_in_chunk<MODE>(lds_chunk(base ^ (cs << 4)), mm, wb);
+    const uint32_t me = (lane - h) & 15u;
+    const uint32_t from = 2u * me + ((holds >> (2u * me)) & 1u ^ 1u);
+    const uint32_t rb = __shfl_sync(0xffffffffu, wb, from), rp = __shfl_sync(0xffffffffu, pos, from);
+    const uint32_t rl = __shfl_sync(0xffffffffu, !(both == both) || both == B::fill() ? 1u : 0u, from);
+    if (lane - h < kStageLines) out = LineBest{rb, rp, rl != 0u};
     __syncwarp();  // the stage may be written again
-    return bits != 0u && lane - h < kStageLines
-               ? (static_cast<uint64_t>(hi) << 32) | ((line << 6) + lo) : kEntryNone;
+}
+
+template <uint32_t MODE>
+__device__ __forceinline__ Entry line_entry(const LineBest &x, uint32_t line, uint32_t bits) {
+    if (bits == 0u) return kEntryNone;
+    const uint32_t key = x.last ? 0xffffffffu : key_of(x.bits, MODE);
+    const uint32_t lo = x.last ? (__ffs(bits) - 1u) << 1 : (x.pos << 1) | negzero_of(x.bits, MODE);
+    return (static_cast<uint64_t>(key) << 32) | ((line << 6) + lo);
 }
 
 // Bits lo .. hi (inclusive, 0 <= lo <= hi <= 31)
@@ -651,12 +657,13 @@ __device__ __forceinline__ void drain_misses(const V1View &v, const QueryOut &o,
             if constexpr (STATS)
                 if (!second) s.c[again ? kStatFull : kStatSecond] += 1u;
         }
-        res = better(res, reduce_lines<MODE>(line, bits, stage, 0u));
-#pragma unroll 1
-        for (uint32_t h = kStageLines; h < 32u; h += kStageLines) {
-            stage_lines<ALIGNED>(v, line, bits, stage, h);
-            res = better(res, reduce_lines<MODE>(line, bits, stage, h));
+        LineBest best;
+        reduce_lines<MODE>(bits, stage, 0u, best);
+        if (take > kStageLines) {
+            stage_lines<ALIGNED>(v, line, bits, stage, kStageLines);
+            reduce_lines<MODE>(bits, stage, kStageLines, best);
         }
+        res = better(res, line_entry<MODE>(best, line, bits));
     }
     if (act && !again) put_result(o, map.query(id, THREADS * QPT), res, MODE, LEAD ? v.lead : 0u);
     if constexpr (MICRO) {
@@ -750,7 +757,7 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
         if (ok[k] && !scan[k]) res[k] = superset_probe<MICRO, STATS>(v, l, r, pol, s);
     }
     bool miss[QPT];
-    bool any_miss = false, any_scan = false;
+    bool any_scan = false;
 #pragma unroll
     for (int k = 0; k < QPT; ++k) {
         const uint32_t j = threadIdx.x + k * THREADS;
@@ -766,7 +773,6 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
         // a query inside one micro-block still holds kEntryNone here, whose
         // index lies outside [l, r]
         miss[k] = entry_idx(res[k]) - l > r - l;
-        any_miss |= miss[k];
         any_scan |= scan[k];
         if constexpr (STATS) {
             if (MICRO && scan[k]) {
@@ -813,42 +819,57 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
             }
         }
     }
-    // queue what is open, slot by slot, and drain: one copy of the drain's
-    // code (every copy costs instruction fetches)
-    if (!last && !__any_sync(0xffffffffu, any_miss)) return;
-    const bool scans = MICRO && SHORT && __any_sync(0xffffffffu, any_scan);
-#pragma unroll 1
-    for (int k = 0; k < QPT; ++k) {
-        int2 lr = qq[0];
-        bool open = miss[0];
-        uint32_t at = entry_idx(res[0]);
+    // what is open joins the queue, up to 32 queries at a time: both slots
+    // together when they fit (about always: a few lanes in a hundred miss), else
+    // one after the other. One site for the drain, whose code is large: before
+    // each, and after the last step until the queue is empty (n = 1e8, lr = -2,
+    // 2^26 queries: 0.586 and 0.565 ms slot by slot and so)
+    static_assert(QPT == 2, "two slots");
+    const uint32_t below = (1u << lane) - 1u;
+    uint32_t m0 = __ballot_sync(0xffffffffu, miss[0]), m1 = __ballot_sync(0xffffffffu, miss[1]);
+    if ((m0 | m1) == 0u && !last) return;
+    bool tiny[2] = {false, false};
+    if (MICRO && SHORT && __any_sync(0xffffffffu, any_scan))
 #pragma unroll
-        for (int j = 1; j < QPT; ++j)
-            if (k == j) {
-                lr = qq[j];
-                open = miss[j];
-                at = entry_idx(res[j]);
-            }
-        if (scans) {
-            const uint32_t l = static_cast<uint32_t>(lr.x), r = static_cast<uint32_t>(lr.y);
-            if (open && (l >> 5) == (r >> 5) && (r >> 2) - (l >> 2) < kShortChunks) {
+        for (int k = 0; k < 2; ++k)
+            tiny[k] = scan[k] && miss[k] &&
+                      (static_cast<uint32_t>(qq[k].y) >> 2) - (static_cast<uint32_t>(qq[k].x) >> 2) < kShortChunks;
+    if (MICRO && SHORT && __any_sync(0xffffffffu, tiny[0] || tiny[1])) {
+#pragma unroll 1
+        for (int k = 0; k < 2; ++k) {
+            const uint32_t l = static_cast<uint32_t>(k ? qq[1].x : qq[0].x);
+            const uint32_t r = static_cast<uint32_t>(k ? qq[1].y : qq[0].y);
+            if (k ? tiny[1] : tiny[0])
                 put_result(o, base + threadIdx.x + k * THREADS, short_range<ALIGNED, MODE>(v, l, r), MODE, lead);
-                open = false;
-            }
         }
-        const unsigned mask = __ballot_sync(0xffffffffu, open);
-        if (open) {
-            const uint32_t l = static_cast<uint32_t>(lr.x);
-            const uint32_t e = count + __popc(mask & ((1u << lane) - 1u));
-            mq.l[e] = l | (at < l ? kMissLeft : 0u);
-            mq.r[e] = static_cast<uint32_t>(lr.y);
-            mq.id[e] = id0 + threadIdx.x + k * THREADS;
-        }
-        count += __popc(mask);
-        const uint32_t drain_at = last && k == QPT - 1 ? 1u : 32u;
+        miss[0] = miss[0] && !tiny[0];
+        miss[1] = miss[1] && !tiny[1];
+        m0 = __ballot_sync(0xffffffffu, miss[0]);
+        m1 = __ballot_sync(0xffffffffu, miss[1]);
+    }
+    const uint32_t n0 = __popc(m0), n1 = __popc(m1);
+    const bool both = n0 + n1 <= 32u;
+#pragma unroll 1
+    for (uint32_t k = both ? 1u : 0u; k < 2u + (last ? 1u : 0u); ++k) {
+        const uint32_t drain_at = k == 2u ? 1u : 32u;
 #pragma unroll 1
         while (count >= drain_at)
             drain_misses<ALIGNED, MICRO, MODE, STATS, LEAD, THREADS, QPT>(v, o, map, mq, count, pol, s);
+        if (k == 2u) break;
+        const uint32_t first = both || k == 0u ? n0 : 0u;
+        if (miss[0] && (both || k == 0u)) {
+            const uint32_t l = static_cast<uint32_t>(qq[0].x), e = count + __popc(m0 & below);
+            mq.l[e] = l | (entry_idx(res[0]) < l ? kMissLeft : 0u);
+            mq.r[e] = static_cast<uint32_t>(qq[0].y);
+            mq.id[e] = id0 + threadIdx.x;
+        }
+        if (miss[1] && k == 1u) {
+            const uint32_t l = static_cast<uint32_t>(qq[1].x), e = count + first + __popc(m1 & below);
+            mq.l[e] = l | (entry_idx(res[1]) < l ? kMissLeft : 0u);
+            mq.r[e] = static_cast<uint32_t>(qq[1].y);
+            mq.id[e] = id0 + threadIdx.x + THREADS;
+        }
+        count += first + (k == 1u ? n1 : 0u);
     }
 }
 
