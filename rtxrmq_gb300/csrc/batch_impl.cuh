@@ -37,9 +37,11 @@ constexpr int kBatchQPT = 2;
 constexpr uint32_t kQueryChunk = 4096;
 constexpr uint32_t kLevelChunk = 4096;
 constexpr int kMaxSteps = 16;
-// units (of 256 micro-blocks) per run item: 512 KB of values, so that the 63
-// to 255 micro-blocks a run reads beyond its end stay below a few percent
-constexpr uint32_t kRunUnits = 16;
+// units (of 256 micro-blocks) per run item: 1 MB of values, so that the 63 to
+// 255 micro-blocks a run reads beyond its end stay below a few percent (ragged
+// benchmark's build: 1.25 ms with 8 units, 1.20 with 16, 1.18 with 32; with 64
+// 1.17, but a few arrays of 2e7 leave SMs idle: 0.14 and 0.23 ms)
+constexpr uint32_t kRunUnits = 32;
 // positions per item of rows made apart, and the largest block table that one
 // item takes through all its levels: both fit the run's shared memory
 constexpr uint32_t kBatchRowTile = 1024;
@@ -170,7 +172,8 @@ __device__ __forceinline__ void table_steps(const BatchParams &P, cg::grid_group
             else if (kind == kItemTable)
                 all_levels<kBatchThreads>(st, a.nb, a.levels, reinterpret_cast<Entry *>(smem));
             else
-                level_group<kBatchThreads>(st, a.nb, k, min(kLevelGroup, a.levels - 1u - k), w.z, w.w);
+                level_group<kBatchThreads>(st + static_cast<size_t>(k) * a.nb, st, a.nb, k,
+                                           min(kLevelGroup, a.levels - 1u - k), w.z, w.w, nullptr);
         }
         grid.sync();
     }

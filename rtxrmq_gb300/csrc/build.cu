@@ -55,21 +55,23 @@ table_kernel(const float *__restrict__ A, int64_t limit, int64_t base, uint32_t 
                              bmin, pb, *reinterpret_cast<TableSmem *>(s_table));
 }
 
-// Block minima: a thread per block of up to 16 micro-blocks, else a warp.
-constexpr int kBlockThreads = 256;
-__global__ void __launch_bounds__(kBlockThreads)
-block_minima_kernel(const Entry *__restrict__ mst, uint32_t nmicro, uint32_t pb, Entry *bmin,
-                    uint32_t nb, uint32_t per_cta) {
-    const uint32_t b0 = blockIdx.x * per_cta;
-    block_minima<kBlockThreads>(mst, nmicro, pb, b0, min(b0 + per_cta, nb), nb, bmin);
-}
-
-// The offset rows apart (split_rows), one tile of kRowTile positions per CTA.
+// What the runs left out, from the micro-block minima (and masks): the offset
+// rows of split_rows, one tile of kRowTile positions per CTA, and in the CTAs
+// before them the block minima of blocks that do not tile a unit, a thread
+// per block of up to 16 micro-blocks, else a warp. One launch: the block
+// minima are few and slow (n = 1e8, bs 2^15: 11 us beside the rows' 26).
 constexpr uint32_t kRowTile = 2048;
-__global__ void __launch_bounds__(512) rows_kernel(MicroTable T) {
+constexpr int kRestThreads = 512;
+__global__ void __launch_bounds__(kRestThreads)
+rest_kernel(MicroTable T, uint32_t pb, Entry *bmin, uint32_t nb, uint32_t per_cta, uint32_t block_ctas) {
     extern __shared__ __align__(16) unsigned char s_tile[];
-    const uint32_t t0 = blockIdx.x * kRowTile;
-    rows_tile_global<512>(T, t0, min(kRowTile, T.nmicro - t0), s_tile);
+    if (blockIdx.x < block_ctas) {
+        const uint32_t b0 = blockIdx.x * per_cta;
+        block_minima<kRestThreads>(T.mst, T.nmicro, pb, b0, min(b0 + per_cta, nb), nb, bmin);
+    } else {
+        const uint32_t t0 = (blockIdx.x - block_ctas) * kRowTile;
+        rows_tile_global<kRestThreads>(T, t0, min(kRowTile, T.nmicro - t0), s_tile);
+    }
 }
 
 constexpr int kLevelThreads = 1024;
@@ -83,7 +85,7 @@ small_levels_kernel(Entry *st, uint32_t nb, uint32_t levels) {
 // Levels k0 + 1 .. k0 + g of a larger block table.
 __global__ void __launch_bounds__(256) level_group_kernel(Entry *st, uint32_t nb, uint32_t k0, uint32_t g) {
     const uint32_t first = blockIdx.x * 256u;
-    level_group<256>(st, nb, k0, g, first, min(256u, nb - first));
+    level_group<256>(st + static_cast<size_t>(k0) * nb, st, nb, k0, g, first, min(256u, nb - first), nullptr);
 }
 
 std::atomic<int> g_units_per_sm[2];
@@ -153,24 +155,21 @@ cudaError_t launch_build_tables(const BuildPlan &p, const DeviceInfo &dev, cudaS
     T.mlevels = p.mlevels;
     cudaError_t err = p.aligned ? launch_runs<true>(p, T, dev, s) : launch_runs<false>(p, T, dev, s);
     if (err != cudaSuccess) return err;
-    if (split_rows(p.mlevels)) {
-        const size_t smem = 2 * sizeof(Entry) * ((kRowTile + table_halo(p.mlevels) + 1u) & ~1u);
+    const uint32_t pb = p.tbs / kMicro;
+    const uint32_t per_cta = pb <= 16u ? kRestThreads : kRestThreads / 32;
+    const uint32_t block_ctas = fused_blocks(pb) ? 0u : (p.nb + per_cta - 1) / per_cta;
+    const uint32_t row_ctas = split_rows(p.mlevels) ? (p.nmicro + kRowTile - 1) / kRowTile : 0u;
+    if (block_ctas + row_ctas > 0u) {
+        const size_t smem = row_ctas ? 2 * sizeof(Entry) * ((kRowTile + table_halo(p.mlevels) + 1u) & ~1u) : 0;
         static std::atomic<bool> ready{false};
         if (!ready.load(std::memory_order_relaxed)) {
             // the longest halo: 1023
-            err = cudaFuncSetAttribute(rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            err = cudaFuncSetAttribute(rest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(2 * sizeof(Entry) * (kRowTile + 1024u)));
             if (err != cudaSuccess) return err;
             ready.store(true, std::memory_order_relaxed);
         }
-        rows_kernel<<<(p.nmicro + kRowTile - 1) / kRowTile, 512, smem, s>>>(T);
-        err = cudaGetLastError();
-        if (err != cudaSuccess) return err;
-    }
-    const uint32_t pb = p.tbs / kMicro, per_cta = pb <= 16u ? kBlockThreads : kBlockThreads / 32;
-    if (!fused_blocks(pb)) {
-        block_minima_kernel<<<(p.nb + per_cta - 1) / per_cta, kBlockThreads, 0, s>>>(
-            p.mst, p.nmicro, pb, p.st, p.nb, per_cta);
+        rest_kernel<<<block_ctas + row_ctas, kRestThreads, smem, s>>>(T, pb, p.st, p.nb, per_cta, block_ctas);
         err = cudaGetLastError();
         if (err != cudaSuccess) return err;
     }

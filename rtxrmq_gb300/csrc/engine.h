@@ -149,9 +149,10 @@ inline TableShape table_shape(uint32_t n, uint32_t bs, uint32_t least_blocks) {
     const uint32_t least = mask_levels(wide_masks((n + kMicro - 1) / kMicro));
     s.mlevels = micro_levels(s.tbs);
     if (s.mlevels < least) s.mlevels = least;
-    const uint32_t few = (n / least_blocks + 31u) / 32u * 32u;
+    uint32_t few = 64u;  // a power of two, so that the run reduces their minima
+    while (few <= n / least_blocks / 2u) few *= 2u;
     if (few < s.tbs) {
-        s.tbs = few < 64u ? 64u : few;
+        s.tbs = few;
         if (s.mlevels > 9u) s.mlevels = 9u;
     }
     return s;

@@ -320,38 +320,14 @@ __device__ __forceinline__ void block_minima(const Entry *mst, uint32_t nmicro, 
     }
 }
 
-// Every level of a block table st[levels][nb] from its block minima, by one
-// CTA: two buffers of nb entries in shared memory, one barrier per level.
-template <int THREADS>
-__device__ __forceinline__ void all_levels(Entry *st, uint32_t nb, uint32_t levels, Entry *buf) {
-    Entry *src = buf, *dst = buf + nb;
-    for (uint32_t i = threadIdx.x; i < nb; i += THREADS) src[i] = st[i];
-    __syncthreads();
-    for (uint32_t k = 1; k < levels; ++k) {
-        const uint32_t half = 1u << (k - 1), cnt = nb - (1u << k) + 1;
-        Entry *row = st + static_cast<size_t>(k) * nb;
-        for (uint32_t i = threadIdx.x; i < cnt; i += THREADS) {
-            const Entry m = better(src[i], src[i + half]);
-            dst[i] = m;
-            row[i] = m;
-        }
-        __syncthreads();
-        Entry *t = src;
-        src = dst;
-        dst = t;
-    }
-    __syncthreads();  // a further table overwrites the buffers
-}
-
 // Levels k0 + 1 .. k0 + g (g <= kLevelGroup) of a block table st[levels][nb]
-// at positions [first, first + count), from level k0: a level's entry is the
-// best of 2^g entries of level k0, 2^k0 apart, so several levels need no
-// synchronisation between them.
+// at positions [first, first + count), from level k0 (`src`): a level's entry is
+// the best of 2^g entries of level k0, 2^k0 apart, so several levels need no
+// synchronisation between them. The last one also goes to `top`, if any.
 constexpr uint32_t kLevelGroup = 3;
 template <int THREADS>
-__device__ __forceinline__ void level_group(Entry *st, uint32_t nb, uint32_t k0, uint32_t g,
-                                            uint32_t first, uint32_t count) {
-    const Entry *__restrict__ src = st + static_cast<size_t>(k0) * nb;
+__device__ __forceinline__ void level_group(const Entry *src, Entry *st, uint32_t nb, uint32_t k0,
+                                            uint32_t g, uint32_t first, uint32_t count, Entry *top) {
     for (uint32_t j = first + threadIdx.x; j < first + count; j += THREADS) {
         Entry x[1 << kLevelGroup];
 #pragma unroll
@@ -364,9 +340,30 @@ __device__ __forceinline__ void level_group(Entry *st, uint32_t nb, uint32_t k0,
 #pragma unroll
             for (uint32_t i = 0; i < (1u << (kLevelGroup - t)); ++i)
                 x[i] = better(x[2 * i], x[2 * i + 1]);
-            if (t <= g && j + (1ull << (k0 + t)) <= nb) st[static_cast<size_t>(k0 + t) * nb + j] = x[0];
+            if (t <= g && j + (1ull << (k0 + t)) <= nb) {
+                st[static_cast<size_t>(k0 + t) * nb + j] = x[0];
+                if (top && t == g) top[j] = x[0];
+            }
         }
     }
+}
+
+// Every level of a block table st[levels][nb] from its block minima, by one
+// CTA: a group of levels per step between two buffers of nb entries in shared
+// memory (nb = 3052, 12 levels: 11 us with a step per level).
+template <int THREADS>
+__device__ __forceinline__ void all_levels(Entry *st, uint32_t nb, uint32_t levels, Entry *buf) {
+    Entry *src = buf, *dst = buf + nb;
+    for (uint32_t i = threadIdx.x; i < nb; i += THREADS) src[i] = st[i];
+    __syncthreads();
+    for (uint32_t k = 0; k + 1u < levels; k += kLevelGroup) {
+        level_group<THREADS>(src, st, nb, k, min(kLevelGroup, levels - 1u - k), 0u, nb, dst);
+        __syncthreads();
+        Entry *t = src;
+        src = dst;
+        dst = t;
+    }
+    __syncthreads();  // a further table overwrites the buffers
 }
 
 #endif  // __CUDACC__
