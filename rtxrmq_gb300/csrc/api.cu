@@ -441,6 +441,18 @@ int rmq_query_stats(const rmq_handle_t *h, const int32_t *d_queries, int64_t q, 
     if (dev.device != h->device)
         return set_error(RMQ_EINVAL, "rmq_query_stats: handle built on device %d, current is %d",
                          h->device, dev.device);
+    // A table index is counted on tables in blocks of its bs, made for the
+    // call: the counts describe the decomposition asked for, while rmq_query
+    // takes its own block sizes.
+    BuildPlan plan = h->plan;
+    void *tables = nullptr;
+    cudaError_t err = cudaSuccess;
+    if (plan.micro) {
+        err = dev_malloc(&tables, plan_index(plan, false, true));
+        if (err != cudaSuccess) return cuda_fail(err, "rmq_query_stats: tables");
+        place_index(plan, tables);
+        err = launch_build(plan, dev, stream);
+    }
     // the counters sit in the handle's counter block, after the invalid-query
     // counter (kStatsSlot words in, RMQ_QUERY_STATS_FIELDS words)
     unsigned long long *dst = h->invalid + kStatsSlot;
@@ -452,10 +464,11 @@ int rmq_query_stats(const rmq_handle_t *h, const int32_t *d_queries, int64_t q, 
     a.invalid = h->invalid;
     a.stats = dst;
     unsigned long long host[RMQ_QUERY_STATS_FIELDS];
-    cudaError_t err = cudaMemsetAsync(dst, 0, sizeof(host), stream);
-    if (err == cudaSuccess) err = launch_query(h->plan, a, dev, stream);
+    if (err == cudaSuccess) err = cudaMemsetAsync(dst, 0, sizeof(host), stream);
+    if (err == cudaSuccess) err = launch_query(plan, a, dev, stream);
     if (err == cudaSuccess) err = cudaMemcpyAsync(host, dst, sizeof(host), cudaMemcpyDeviceToHost, stream);
     if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
+    if (tables) cudaFree(tables);
     if (err != cudaSuccess) return cuda_fail(err, "rmq_query_stats");
     for (int c = 0; c < RMQ_QUERY_STATS_FIELDS; ++c) h_counts[c] = static_cast<int64_t>(host[c]);
     return RMQ_OK;
@@ -733,10 +746,9 @@ int rmq_info(const rmq_handle_t *h, rmq_info_t *info) {
     info->aligned = h->plan.aligned ? 1 : 0;
     info->table_bytes = h->table_bytes;
     info->struct_bytes = static_cast<int64_t>(h->mem_bytes);
-    // above 2^15: of the micro table that blocks of bs would need
+    // at least those of the micro table that blocks of bs would need
     info->micro_levels = static_cast<int32_t>(
-        h->plan.micro && h->plan.bs > (1u << 15) ? std::max(micro_levels(h->plan.bs), h->plan.mlevels)
-                                                 : h->plan.mlevels);
+        h->plan.micro ? std::max(micro_levels(h->plan.bs), h->plan.mlevels) : 0u);
     info->light = h->plan.light ? 1 : 0;
     info->micro_table_bytes =
         h->plan.micro ? static_cast<int64_t>(static_cast<size_t>(h->plan.nmicro) *

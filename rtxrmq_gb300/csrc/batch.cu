@@ -307,7 +307,7 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
         a.n = static_cast<uint32_t>(n) + lead;
         a.lead = lead;
         const TableShape shape = table_shape(
-            a.n, static_cast<uint32_t>(std::min<int64_t>(bs, std::max<int64_t>(n, 1))), 32u);
+            a.n, static_cast<uint32_t>(std::min<int64_t>(bs, std::max<int64_t>(n, 1))));
         a.bs = shape.tbs;
         a.nb = (a.n + a.bs - 1) / a.bs;
         a.levels = a.nb > 0 ? st_levels(a.nb) : 0u;
@@ -518,6 +518,7 @@ int rmq_batch_run_per_array(rmq_batch_t *b, const float *d_vals, const int32_t *
         p.micro = true;
         p.nmicro = a.nmicro;
         p.mlevels = a.mlevels;
+        p.micro_span = (1u << a.mlevels) - 1u;
         p.moff_bytes = a.moff_bytes;
         p.st = ws + a.st;
         p.mst = ws + a.mst;

@@ -119,6 +119,7 @@ __device__ __forceinline__ V1View batch_view(const BatchParams &P, const BatchAr
     v.nb = a.nb;
     v.dv = a.dv;
     v.st = P.ws + a.st;
+    v.coarse_from = 0xffffffffu;
     v.mst = P.ws + a.mst;
     v.mask = P.ws + a.mask;
     v.wide = wide_masks(a.nmicro);

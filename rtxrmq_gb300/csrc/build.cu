@@ -82,17 +82,21 @@ small_levels_kernel(Entry *st, uint32_t nb, uint32_t levels) {
     all_levels<kLevelThreads>(st, nb, levels, s_level);
 }
 
-// Levels k0 + 1 .. k0 + g of a larger block table.
-__global__ void __launch_bounds__(256) level_group_kernel(Entry *st, uint32_t nb, uint32_t k0, uint32_t g) {
+// Levels k0 + 1 .. k0 + g of a larger block table, and of the table C of larger
+// blocks.
+template <bool COARSE>
+__global__ void __launch_bounds__(256)
+level_group_kernel(Entry *st, uint32_t nb, uint32_t levels, uint32_t k0, uint32_t g, CoarseTable C) {
     const uint32_t first = blockIdx.x * 256u;
-    level_group<256>(st + static_cast<size_t>(k0) * nb, st, nb, k0, g, first, min(256u, nb - first), nullptr);
+    level_group<256, COARSE>(st + static_cast<size_t>(k0) * nb, st, nb, k0, g, first,
+                             min(256u, nb - first), nullptr, levels, C);
 }
 
 std::atomic<int> g_units_per_sm[2];
 
-cudaError_t launch_levels(Entry *st, uint32_t nb, uint32_t levels, cudaStream_t s) {
+cudaError_t launch_levels(Entry *st, uint32_t nb, uint32_t levels, const CoarseTable &C, cudaStream_t s) {
     if (levels <= 1) return cudaSuccess;
-    if (nb <= kSmallTable) {
+    if (nb <= kSmallTable && !C.st) {
         static std::atomic<bool> ready{false};
         if (!ready.load(std::memory_order_relaxed)) {
             const cudaError_t err =
@@ -104,9 +108,13 @@ cudaError_t launch_levels(Entry *st, uint32_t nb, uint32_t levels, cudaStream_t 
         small_levels_kernel<<<1, kLevelThreads, 2 * sizeof(Entry) * nb, s>>>(st, nb, levels);
         return cudaGetLastError();
     }
-    for (uint32_t k = 0; k + 1 < levels; k += kLevelGroup) {
-        const uint32_t g = levels - 1 - k < kLevelGroup ? levels - 1 - k : kLevelGroup;
-        level_group_kernel<<<(nb + 255) / 256, 256, 0, s>>>(st, nb, k, g);
+    const uint32_t all = C.st && C.levels + C.shift > levels ? C.levels + C.shift : levels;
+    for (uint32_t k = 0; k + 1 < all; k += kLevelGroup) {
+        const uint32_t g = all - 1 - k < kLevelGroup ? all - 1 - k : kLevelGroup;
+        if (C.st)
+            level_group_kernel<true><<<(nb + 255) / 256, 256, 0, s>>>(st, nb, levels, k, g, C);
+        else
+            level_group_kernel<false><<<(nb + 255) / 256, 256, 0, s>>>(st, nb, levels, k, g, C);
         const cudaError_t err = cudaGetLastError();
         if (err != cudaSuccess) return err;
     }
@@ -173,7 +181,9 @@ cudaError_t launch_build_tables(const BuildPlan &p, const DeviceInfo &dev, cudaS
         err = cudaGetLastError();
         if (err != cudaSuccess) return err;
     }
-    return launch_levels(p.st, p.nb, p.levels, s);
+    CoarseTable C;
+    if (p.cbs) C = CoarseTable{p.cst, p.cnb, p.clevels, static_cast<uint32_t>(ilog2(p.cbs / p.tbs))};
+    return launch_levels(p.st, p.nb, p.levels, C, s);
 }
 
 }  // namespace
@@ -183,7 +193,7 @@ uint32_t st_levels(uint32_t nb) { return nb ? static_cast<uint32_t>(ilog2(nb)) +
 namespace {
 size_t a256(size_t x) { return (x + 255) / 256 * 256; }
 struct Offsets {
-    size_t pre, suf, st, mst, mask, moff, counter, total;
+    size_t pre, suf, st, cst, mst, mask, moff, counter, total;
 };
 Offsets offsets_of(const BuildPlan &p) {
     Offsets o;
@@ -191,7 +201,8 @@ Offsets offsets_of(const BuildPlan &p) {
     o.pre = 0;
     o.suf = nent;
     o.st = 2 * nent;
-    o.mst = o.st + a256(sizeof(Entry) * static_cast<size_t>(p.nb) * p.levels);
+    o.cst = o.st + a256(sizeof(Entry) * static_cast<size_t>(p.nb) * p.levels);
+    o.mst = o.cst + a256(sizeof(Entry) * static_cast<size_t>(p.cnb) * p.clevels);
     o.mask = o.mst + a256(sizeof(Entry) * static_cast<size_t>(p.nmicro));
     o.moff = o.mask + a256((wide_masks(p.nmicro) ? 8 : 4) * static_cast<size_t>(p.nmicro));
     o.counter = o.moff + a256(static_cast<size_t>(p.moff_bytes) * p.nmicro * moff_rows(p.mlevels, wide_masks(p.nmicro)));
@@ -200,16 +211,24 @@ Offsets offsets_of(const BuildPlan &p) {
 }
 }  // namespace
 
-size_t plan_index(BuildPlan &p, bool no_micro) {
+size_t plan_index(BuildPlan &p, bool no_micro, bool asked) {
     p.off = 0;
     p.limit = p.n;
     p.lead = 0;
     p.micro = !no_micro;
-    const TableShape shape = table_shape(p.n, p.bs, 128u);
+    IndexShape shape = index_shape(p.n);
+    if (asked) {
+        const TableShape t = table_shape(p.n, p.bs);
+        shape = IndexShape{t.tbs, t.mlevels, (1u << t.mlevels) - 1u, 0u};
+    }
     p.tbs = p.micro ? shape.tbs : p.bs;
     p.nb = (p.n + p.tbs - 1) / p.tbs;
     p.levels = st_levels(p.nb);
+    p.cbs = p.micro ? shape.cbs : 0u;
+    p.cnb = p.cbs ? (p.n + p.cbs - 1) / p.cbs : 0u;
+    p.clevels = st_levels(p.cnb);
     p.mlevels = p.micro ? shape.mlevels : 0u;
+    p.micro_span = p.micro ? shape.micro_span : 0u;
     p.nmicro = p.micro ? (p.n + kMicro - 1) / kMicro : 0u;
     p.moff_bytes = p.micro ? micro_offset_bytes(p.mlevels) : 0u;
     p.aligned = reinterpret_cast<uintptr_t>(p.A) % 16 == 0;
@@ -222,6 +241,7 @@ unsigned long long *place_index(BuildPlan &p, void *base_v) {
     p.pre = p.micro ? nullptr : reinterpret_cast<Entry *>(base + o.pre);
     p.suf = p.micro ? nullptr : reinterpret_cast<Entry *>(base + o.suf);
     p.st = reinterpret_cast<Entry *>(base + o.st);
+    p.cst = p.cbs ? reinterpret_cast<Entry *>(base + o.cst) : nullptr;
     p.mst = p.micro ? reinterpret_cast<Entry *>(base + o.mst) : nullptr;
     p.mask = p.micro ? static_cast<void *>(base + o.mask) : nullptr;
     p.moff = p.micro ? static_cast<void *>(base + o.moff) : nullptr;
@@ -296,7 +316,7 @@ cudaError_t launch_build(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t
     if (p.micro) return launch_build_tables(p, dev, s);
     const cudaError_t err = launch_build_entries(p, dev, s);
     if (err != cudaSuccess) return err;
-    return launch_levels(p.st, p.nb, p.levels, s);
+    return launch_levels(p.st, p.nb, p.levels, CoarseTable(), s);
 }
 
 RMQ_VIOLATIONS_READER(violations_build)

@@ -106,9 +106,15 @@ struct BuildPlan {
     uint32_t nb;      // blocks of tbs elements
     uint32_t levels;
     Entry *st;        // [levels * nb], level 0 = block minima
+    // block table of larger blocks for longer ranges (cbs 0: none)
+    uint32_t cbs, cnb, clevels;
+    Entry *cst;       // [clevels * cnb]
     uint32_t nmicro;  // ceil(n / 32)
     uint32_t mlevels;
     uint32_t moff_bytes;
+    // queries whose end micro-blocks are fewer than this apart go through the
+    // micro table
+    uint32_t micro_span;
     Entry *mst;       // [nmicro] micro-block minima
     void *mask;       // [nmicro] (tables_impl.cuh)
     void *moff;       // [moff_rows * nmicro]
@@ -124,33 +130,33 @@ uint32_t micro_levels(uint32_t bs);
 inline uint32_t micro_offset_bytes(uint32_t mlevels) {
     return mlevels <= 9 ? 1u : (mlevels <= 17 ? 2u : 4u);
 }
-// Shape of a table index over n elements asked for with block size bs: the
-// blocks of its block table (multiples of 32, so that blocks hold whole
-// micro-blocks, at least 64) and the levels of its micro table.
+// Shape of a table index with blocks of about bs elements (arrays of a batch;
+// rmq_query_stats): the blocks of its block table (multiples of 32, so that
+// blocks hold whole micro-blocks, at least 64) and the levels of its micro
+// table, which answers every query inside a block.
 struct TableShape {
     uint32_t tbs, mlevels;
 };
 // - Blocks above 2^15: the micro table would be 13 rows and more of 2-byte
 //   offsets, too large for L2 and read twice per query; 4096 instead (n = 1e8,
 //   2^26 queries, lr=-2, bs 195312: 0.83 ms with the rows, 0.58 with 4096).
-// - Fewer than `least_blocks`: a range of a few blocks is open as often as the
-//   blocks at its ends are larger than it, so the blocks shrink until there
-//   are that many, and windows of up to 511 micro-blocks do (rows up to level
-//   8 are made in the run of the minima, longer ones take another launch).
-//   Plain index: 128 (n = 3e5, bs 2^15, uniform lengths, 2^25 queries: 0.318 ms
-//   with 10 blocks, 0.291 with 128). Batch: 32; with 128 the ragged benchmark's
-//   build takes 1.83 ms in place of 1.67 for its many small block tables, and
-//   its queries gain nothing.
+// - Fewer than 32: a range of a few blocks is open as often as the blocks at
+//   its ends are larger than it, so the blocks shrink until there are that
+//   many, and windows of up to 511 micro-blocks do (rows up to level 8 are
+//   made in the run of the minima, longer ones take another step). With 128
+//   the ragged benchmark's build takes 1.83 ms in place of 1.67 for its many
+//   small block tables, and its queries gain nothing.
 // - The masks answer windows of up to 63 (127) micro-blocks whatever the
 //   block size: 6 or 7 levels cost nothing.
-inline TableShape table_shape(uint32_t n, uint32_t bs, uint32_t least_blocks) {
+constexpr uint32_t kLeastBlocks = 32;
+inline TableShape table_shape(uint32_t n, uint32_t bs) {
     TableShape s;
     s.tbs = bs > (1u << 15) ? 4096u : bs <= 64u ? 64u : (bs + 31u) / 32u * 32u;
     const uint32_t least = mask_levels(wide_masks((n + kMicro - 1) / kMicro));
     s.mlevels = micro_levels(s.tbs);
     if (s.mlevels < least) s.mlevels = least;
     uint32_t few = 64u;  // a power of two, so that the run reduces their minima
-    while (few <= n / least_blocks / 2u) few *= 2u;
+    while (few <= n / kLeastBlocks / 2u) few *= 2u;
     if (few < s.tbs) {
         s.tbs = few;
         if (s.mlevels > 9u) s.mlevels = 9u;
@@ -158,10 +164,36 @@ inline TableShape table_shape(uint32_t n, uint32_t bs, uint32_t least_blocks) {
     return s;
 }
 
+// Shape of the plain table index: of n alone, whatever block size is asked for.
+// - Windows of up to 64 (32) micro-blocks, one mask, are answered by the micro
+//   table; twice as many by two masks would be, but four scattered loads cost
+//   more than the block table's two, if its blocks are small (n = 1e8, ranges
+//   of 3000, 2^26 queries: 0.94 ms by masks, 0.77 by blocks of 512). So the
+//   micro table needs no offset rows.
+// - Blocks: small ones leave fewer queries open, large ones make rows that fit
+//   L1. 2^13 to 2^14 of them up to 512 elements each (n = 4e6, lr=-2: 0.51 ms
+//   with 512, 0.49 with 256, 0.56 with 64; n = 1e7: 0.54 with 1024, 0.52, 0.56
+//   with 256).
+// - From 2^13 blocks on a second table over larger ones, 2^12 to 2^13 of them,
+//   for ranges of kCoarseFrom and more of those: rows of 64 KB (n = 1e8, uniform
+//   lengths: 0.57 ms by blocks of 4096, 0.34 by blocks of 16384).
+struct IndexShape {
+    uint32_t tbs, mlevels, micro_span, cbs;
+};
+constexpr uint32_t kIndexBlocks = 1u << 13, kCoarseFrom = 64;
+inline IndexShape index_shape(uint32_t n) {
+    const bool wide = wide_masks((n + kMicro - 1) / kMicro);
+    IndexShape s{64u, mask_levels(wide), wide ? 64u : 32u, 0u};
+    while (s.tbs < 512u && n / (2u * s.tbs) >= kIndexBlocks) s.tbs *= 2u;
+    if (n / s.tbs >= kIndexBlocks)
+        for (s.cbs = 2u * s.tbs; n / s.cbs >= kIndexBlocks; s.cbs *= 2u) {}
+    return s;
+}
+
 // Fill the size fields of a plan (A, n, bs and light given; the table index
-// unless `no_micro`); returns the bytes of the single allocation holding the
-// index and its invalid-query counter.
-size_t plan_index(BuildPlan &p, bool no_micro);
+// unless `no_micro`, in blocks of bs where `asked`); returns the bytes of the
+// single allocation holding the index and its invalid-query counter.
+size_t plan_index(BuildPlan &p, bool no_micro, bool asked = false);
 // Point the plan's arrays into that allocation; returns the counter.
 unsigned long long *place_index(BuildPlan &p, void *base);
 uint32_t st_levels(uint32_t nb);

@@ -117,6 +117,11 @@ V1View view_of(const BuildPlan &p) {
     v.nb = p.nb;
     v.dv = make_div31(p.tbs);
     v.st = p.st;
+    v.cst = p.cst;
+    v.cnb = p.cnb;
+    v.clevels = p.clevels;
+    v.cdiv = p.cbs ? make_div31(p.cbs).m : 0u;
+    v.coarse_from = p.cbs ? kCoarseFrom * (p.cbs / kMicro) : 0xffffffffu;
     v.mst = p.mst;
     v.mask = p.mask;
     v.wide = wide_masks(p.nmicro);
@@ -128,7 +133,7 @@ V1View view_of(const BuildPlan &p) {
     v.kmode = p.kmode;
     v.levels = p.levels;
     v.mlevels = p.mlevels;
-    v.micro_span = p.micro ? (1u << p.mlevels) - 1u : 0u;
+    v.micro_span = p.micro_span;
     v.light = p.light;
     return v;
 }

@@ -51,6 +51,11 @@ struct V1View {
     uint32_t nb;
     Div31 dv;
     const Entry *st;
+    // block table of larger blocks (2^k elements, cdiv the multiplier of their
+    // Div31), for queries whose end micro-blocks are coarse_from or more apart
+    const Entry *cst;
+    uint32_t cnb, clevels, cdiv;
+    uint32_t coarse_from;  // 2^32 - 1: none
     // table index: 32-element micro-blocks (local index / 32) and the micro
     // table over their minima (tables_impl.cuh); blocks hold whole
     // micro-blocks. Null when the index has none: per-element entries then
@@ -704,16 +709,18 @@ __device__ __forceinline__ uint32_t decode_bits(Entry e) {
 // micro-block: through the micro table when the query's micro-blocks fit
 // it (`mic`), else through the block table (two entries, one straight
 // sequence).
-template <bool MICRO, bool STATS>
+template <bool MICRO, bool COARSE, bool STATS>
 __device__ __forceinline__ Entry superset_probe(const V1View &v, uint32_t l, uint32_t r,
                                                 uint64_t pol, QStats &s) {
     const uint32_t ml = l >> 5, mr = r >> 5;
     if (MICRO && mr - ml < v.micro_span) return micro_probe<STATS>(v, ml, mr, pol, s);
-    const uint32_t a = MICRO ? div31_ge2(l, v.dv) : div31(l, v.dv);
-    const uint32_t b = MICRO ? div31_ge2(r, v.dv) : div31(r, v.dv);
+    const bool coarse = COARSE && mr - ml >= v.coarse_from;
+    const uint32_t m = coarse ? v.cdiv : v.dv.m, sh = coarse ? 0u : v.dv.shift, nb = coarse ? v.cnb : v.nb;
+    const uint32_t a = MICRO ? __umulhi(l, m) >> sh : div31(l, v.dv);
+    const uint32_t b = MICRO ? __umulhi(r, m) >> sh : div31(r, v.dv);
     const int lev = ilog2(b - a + 1u);
-    const Entry *t = v.st + static_cast<uint64_t>(lev) * v.nb;
-    const uint64_t size = static_cast<uint64_t>(v.levels - lev) * v.nb;
+    const Entry *t = (coarse ? v.cst : v.st) + static_cast<uint64_t>(lev) * nb;
+    const uint64_t size = static_cast<uint64_t>((coarse ? v.clevels : v.levels) - lev) * nb;
     const Entry e1 = ld_entry_keep(t, a, size, pol);
     const Entry e2 = ld_entry_keep(t, b + 1u - (1u << lev), size, pol);
     if constexpr (STATS) s.c[kStatTable] += 2u;
@@ -754,7 +761,7 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
         ok[k] = in[k].x >= 0 && l <= r && r < v.n;
         scan[k] = MICRO && (l >> 5) == (r >> 5);
         res[k] = kEntryNone;
-        if (ok[k] && !scan[k]) res[k] = superset_probe<MICRO, STATS>(v, l, r, pol, s);
+        if (ok[k] && !scan[k]) res[k] = superset_probe<MICRO, MICRO && SHORT, STATS>(v, l, r, pol, s);
     }
     bool miss[QPT];
     bool any_scan = false;

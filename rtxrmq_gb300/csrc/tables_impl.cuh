@@ -324,10 +324,20 @@ __device__ __forceinline__ void block_minima(const Entry *mst, uint32_t nmicro, 
 // at positions [first, first + count), from level k0 (`src`): a level's entry is
 // the best of 2^g entries of level k0, 2^k0 apart, so several levels need no
 // synchronisation between them. The last one also goes to `top`, if any.
+// COARSE: a second table C is written as well, and windows that reach past the
+// last block are entries too, of what there is.
 constexpr uint32_t kLevelGroup = 3;
-template <int THREADS>
+
+// A second block table st[levels][nb] over blocks 2^shift times as large: row
+// k holds every 2^shift-th entry of row k + shift.
+struct CoarseTable {
+    Entry *st = nullptr;
+    uint32_t nb = 0, levels = 0, shift = 1;
+};
+template <int THREADS, bool COARSE = false>
 __device__ __forceinline__ void level_group(const Entry *src, Entry *st, uint32_t nb, uint32_t k0,
-                                            uint32_t g, uint32_t first, uint32_t count, Entry *top) {
+                                            uint32_t g, uint32_t first, uint32_t count, Entry *top,
+                                            uint32_t levels = 0u, const CoarseTable C = CoarseTable()) {
     for (uint32_t j = first + threadIdx.x; j < first + count; j += THREADS) {
         Entry x[1 << kLevelGroup];
 #pragma unroll
@@ -340,7 +350,12 @@ __device__ __forceinline__ void level_group(const Entry *src, Entry *st, uint32_
 #pragma unroll
             for (uint32_t i = 0; i < (1u << (kLevelGroup - t)); ++i)
                 x[i] = better(x[2 * i], x[2 * i + 1]);
-            if (t <= g && j + (1ull << (k0 + t)) <= nb) {
+            if constexpr (COARSE) {
+                if (t <= g && k0 + t < levels) st[static_cast<size_t>(k0 + t) * nb + j] = x[0];
+                const uint32_t c = k0 + t - C.shift;  // wraps below its levels
+                if (t <= g && c < C.levels && (j & ((1u << C.shift) - 1u)) == 0u)
+                    C.st[static_cast<size_t>(c) * C.nb + (j >> C.shift)] = x[0];
+            } else if (t <= g && j + (1ull << (k0 + t)) <= nb) {
                 st[static_cast<size_t>(k0 + t) * nb + j] = x[0];
                 if (top && t == g) top[j] = x[0];
             }
