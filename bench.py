@@ -21,8 +21,8 @@ e2e        -- the same step through the C ABI with host buffers
               NVLink-C2C, all inside the timed region.
 roofline   -- algorithmic HBM bytes per launch / kernel time against the
               measured copy bandwidth. The bytes are the query read and the
-              result write (16 B per query) plus 32 B per per-element entry and
-              per 32-byte sector of values the kernel must read, counted for
+              result write (16 B per query) plus 32 B per end part and per
+              32-byte sector of values the kernel must read, counted for
               this query set by rmq_query_stats (the kernel's counting
               instantiation). The small-table probes are L2-resident and
               reported apart, as is the un-pruned 80 B/query figure.
@@ -63,8 +63,8 @@ BS_BELOW = [1 << 7, 1 << 8, 1 << 9]              # extra: short ranges over smal
 TIE_N = 1 << 27
 TIE_LENGTHS = [1, 32, 1 << 10, 1 << 16, 1 << 22]
 PUBLISHED_LR1 = 3.52e8  # RTXRMQ alg 5, RTX 6000 Ada (csv-to-plot/perf-RTX6000ADA-ALG5.csv:1586-1601)
-L2_NOTE = ("no flush: the per-step working set (values, index entries, queries, outputs; "
-           "2.9 GB at n=1e8) is larger than L2")
+L2_NOTE = ("no flush: the per-step working set (values, index tables, queries, outputs; "
+           "1.5 GB at n=1e8) is larger than L2")
 
 
 def parse():
@@ -197,8 +197,8 @@ class ClockSampler:
 def stats_bytes(st: dict, q: int, out_bytes: int = 8) -> dict:
     """Algorithmic bytes of one query launch from the kernel's own counts
     (rmq_query_stats): the query read and result write, plus one 32-byte
-    sector per per-element entry and per scanned sector of values (random
-    HBM); the small-table words are L2-resident and reported apart."""
+    sector per end part and per scanned sector of values (random HBM); the
+    small-table words are L2-resident and reported apart."""
     hbm = q * (8 + out_bytes) + 32 * (st["entries"] + st["scan_sectors"])
     valid = max(1, q - st["invalid"])
     return {"alg_bytes": float(hbm), "alg_bytes_per_query": hbm / q,
@@ -271,7 +271,8 @@ CPU_KIND = ("HRMQ restated (oracle/hrmq_port.c: balanced-parentheses RMQ of the 
 TRAFFIC_PROFILE = ROOT / "profiles" / "query_kernel_plain_n1e8_q2e26_lr1.md"
 # the sources query_kernel is compiled from; a traffic capture holds their digest
 QUERY_SOURCES = tuple(ROOT / "rtxrmq_gb300" / "csrc" / f
-                      for f in ("query.cu", "query_impl.cuh", "common.cuh", "engine.h"))
+                      for f in ("query.cu", "query_kernel.cuh", "query_impl.cuh", "lines.cuh",
+                                "tables_impl.cuh", "common.cuh", "engine.h"))
 
 
 def query_sources_digest():
@@ -464,8 +465,8 @@ def bench_plain_mode(R, dA, n, Q, out_v, out_i, args, stream, barrier, world, de
            "achieved_gbs": acc["alg_bytes"] / (ms / 1e3) / 1e9,
            "unpruned_achieved_gbs": acc["unpruned_alg_bytes"] / (ms / 1e3) / 1e9,
            "info": ix.info()}
-    # the light index (RMQ_BUILD_LIGHT) at the same block size: tables only,
-    # its construction, size and query time beside the full index's
+    # the light index (RMQ_BUILD_LIGHT) at the same block size: its
+    # construction, size and query time beside the full index's
     if bs % 32 == 0 and bs >= 64:
         lix, lc_ms = timed_build(lambda: R.RMQIndex(dA, bs, light=True))
         lfn = lambda: lix.query(dQ, out_val=out_v, out_idx=out_i)  # noqa: E731
@@ -681,8 +682,7 @@ def bench_batched(args, dev, stream, barrier):
         dms = time_steps(lambda: b.run(dV, dQ, ov, oi), args.steps, 1, stream, barrier)
     from rtxrmq_gb300.replicas import job_rate, world
     q, nr = w.total_q, world()[1]
-    # the light index on the same workload: block and micro-block tables only,
-    # its own tuned tiles; answers compared bit for bit with the full plan's
+    # the light index on the same workload, its own tuned tiles; answers compared bit for bit with the full plan's
     t = time.perf_counter()
     lcfg = ([(max(64, args.batch_bs // 32 * 32), 0, 0)] * 32 if args.batch_bs else
             autotune(w.starts, w.lengths, w.qstarts, w.qcounts, dV, dQ, reps=2,
@@ -725,10 +725,10 @@ def bench_batched(args, dev, stream, barrier):
                 "per_array_matches_batched": match,
                 "build_only_ms": bms, "query_only_ms": qms,
                 "query_only_rmq_s": job_rate(q, nr, qms),
-                # algorithmic bytes of one step: the build reads each value once and
-                # writes its prefix / suffix entries (4 + 16 B per element); each
-                # query reads its pair and writes 8 B, plus at most two random 32-B
-                # entry sectors (the un-pruned bound); against the graph-launched step
+                # bytes of one step of the un-pruned design: the build reads each
+                # value once and writes its prefix / suffix entries (4 + 16 B per
+                # element); each query reads its pair and writes 8 B, plus two random
+                # 32-B entry sectors; against the graph-launched step
                 "alg_bytes_per_step_unpruned": int(w.lengths.sum()) * 20 + q * 80,
                 "alg_gbs_unpruned": (int(w.lengths.sum()) * 20 + q * 80) / (gms / 1e3) / 1e9,
                 "launches_per_step": {"batched": 1, "per_array": "one build + level + query "
@@ -926,7 +926,7 @@ def main():
                      "kernel": "query_kernel",
                      "alg_bytes_per_launch": h["accounting"]["alg_bytes"],
                      "alg_bytes_basis": "16 B per query (query read, value + index write) + 32 B "
-                                        "per per-element entry read and per 32-B sector of values "
+                                        "per end part read and per 32-B sector of values "
                                         "scanned, counted by rmq_query_stats on this query set",
                      "l2_table_words_per_query": h["accounting"]["l2_table_words_per_query"],
                      "unpruned_alg_bytes_per_launch": h["accounting"]["unpruned_alg_bytes"],

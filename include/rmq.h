@@ -57,11 +57,12 @@ typedef struct rmq_info {
     int64_t nb;           /* blocks = ceil(n / bs)  (src/rtx.h:42)      */
     int32_t levels;       /* sparse-table levels over the block minima  */
     int32_t aligned;      /* 1 when d_vals is 16-byte aligned           */
-    int64_t table_bytes;  /* sparse table (block minima and levels)     */
+    int64_t table_bytes;  /* sparse table over the index's own blocks   */
     int64_t struct_bytes; /* all device memory owned by the handle      */
-    int32_t micro_levels; /* levels of the sub-block table (0 = none)   */
+    int32_t micro_levels; /* levels of a sub-block table that answers
+                             every query inside a block (0 = none)     */
     int32_t light;        /* 1: light index (RMQ_BUILD_LIGHT)           */
-    int64_t micro_table_bytes; /* micro-block minima + table offsets     */
+    int64_t micro_table_bytes; /* micro-block minima + masks             */
     int32_t is_max;       /* 1: range maximum (RMQ_BUILD_MAX)           */
     int32_t is_int32;     /* 1: int32 elements (RMQ_BUILD_INT32)        */
 } rmq_info_t;
@@ -77,16 +78,14 @@ typedef struct rmq_info {
                                   bits (pass an int32 buffer cast to float *).
                                   The role of HRMQ's integer constructors,
                                   hrmq/includes/RMQRMM64.h:175-178 */
-#define RMQ_BUILD_LIGHT    8u  /* light index: the block and micro-block
-                                  tables only, no per-element prefix /
-                                  suffix entries (about 1.3 instead of 32
-                                  bytes per element, a build that reads the
-                                  values once and writes ~1/25 as much); a
-                                  query the table probe leaves open scans
-                                  one 128-byte line of values per end
-                                  instead of reading an entry. Needs the
-                                  sub-block level and bs a multiple of 32,
-                                  >= 64 (bs > n is rounded up to one block).
+#define RMQ_BUILD_LIGHT    8u  /* light index. Every index but a NO_MICRO
+                                  one holds tables only (about 0.8 bytes per
+                                  element) and reads a 128-byte line of
+                                  values for an open end, so this changes no
+                                  structure; it is reported by rmq_info and
+                                  kept in files. Needs the sub-block level
+                                  and bs a multiple of 32, >= 64 (bs > n is
+                                  rounded up to one block).
                                   No counterpart in the reference. */
 
 /*
@@ -95,8 +94,9 @@ typedef struct rmq_info {
  * per-block minimum (kernel_min_blocks, src/device_tools.cuh:243-253), the
  * per-block leftmost argmin (compute_min_blocks, src/rtx.h:3-22) and the
  * geometry + BVH build (src/device_tools.cuh:139-169, 378-389,
- * src/rtx_functions.h:289-379) become in-block prefix/suffix minima and a
- * sparse table over the block minima.
+ * src/rtx_functions.h:289-379) become tables over the minima of 32-element
+ * micro-blocks and of blocks whose size follows from n; bs is the size of
+ * the blocks an RMQ_BUILD_NO_MICRO index is made of.
  * The handle owns its structure memory; it does not own or copy d_vals,
  * which must stay valid and unchanged while the handle is used.
  * Allocates (in stream order from the library's pool, see rmq_trim, or by
@@ -106,16 +106,13 @@ int rmq_build(const float *d_vals, int64_t n, int64_t bs, rmq_stream_t stream,
               rmq_handle_t **out);
 
 /*
- * rmq_build with options. When bs >= 64 the index
- * also gets a sub-block level -- prefix and suffix minima inside 32-element
- * micro-blocks (16 more bytes per element) and a sparse table over the
- * micro-block minima, truncated to windows no longer than one block and
- * stored as 1-4 byte offsets to each window's best micro-block (small
- * enough to stay in L2). A query spanning at most about two blocks is then
- * answered from that table: usually from its table words alone, otherwise
- * with one or two per-element entries (one 128-byte line of values if it
- * lies inside one micro-block), never by scanning A[l..r].
- * RMQ_BUILD_NO_MICRO leaves it out.
+ * rmq_build with options. The index has a sub-block level: the minima of
+ * 32-element micro-blocks and, per micro-block, a mask from which the best
+ * of up to 64 (32 in large arrays) micro-blocks is read. A query is answered
+ * from two or three table words, otherwise with a few more and one or two
+ * 128-byte lines of values, never by scanning A[l..r].
+ * RMQ_BUILD_NO_MICRO: blocks of bs, prefix and suffix minima per element (16
+ * bytes each element) and a sparse table over the block minima instead.
  * rmq_build(...) is rmq_build_ex(..., 0, ...).
  */
 int rmq_build_ex(const float *d_vals, int64_t n, int64_t bs, uint32_t flags,
@@ -260,8 +257,10 @@ int rmq_query_scan(const float *d_vals, int64_t n, const int32_t *d_queries,
  * stream and output stores, but per query only the two random 8-byte
  * lookups of its cross-block case (suffix minimum at l, prefix minimum at r)
  * and no other work. The outputs are better(suf[l], pre[r]), which is the
- * range minimum only when l and r lie in the same or in adjacent blocks;
- * out-of-range l / r are clamped into the array. A benchmark times it
+ * range minimum only when l and r lie in the same or in adjacent blocks of
+ * bs; out-of-range l / r are clamped into the array. An index that holds no
+ * such entries gets them (16 bytes per element) on its first call here. A
+ * benchmark times it
  * beside rmq_query to state the fraction of this ceiling a query reaches.
  */
 int rmq_probe_gather(const rmq_handle_t *h, const int32_t *d_queries, int64_t q,
@@ -271,18 +270,23 @@ int rmq_probe_gather(const rmq_handle_t *h, const int32_t *d_queries, int64_t q,
  * Measurement helper, no reference counterpart: rmq_query (same arguments,
  * same results; d_val and d_idx may both be NULL here) through an
  * instantiation of the query kernel that also counts how every query was
- * settled and what it read, into h_counts[RMQ_QUERY_STATS_FIELDS]:
+ * settled and what it read, into h_counts[RMQ_QUERY_STATS_FIELDS]. With the
+ * sub-block level it counts on tables in blocks of the index's bs (4096 above
+ * 2^15, smaller ones in arrays of fewer than 32 blocks), which it makes for
+ * the call and frees:
  *   [0] settled by the probe of the small table over every unit (block or
  *       32-element micro-block) the query touches: the best of that
  *       superset lay inside [l, r]
- *   [1] settled by a narrower probe plus one per-element entry
- *   [2] the three-part decomposition (two entries, probe of the middle)
+ *   [1] settled by a narrower probe plus one end part
+ *   [2] the three-part decomposition (two end parts, probe of the middle)
  *   [3] inside one micro-block: its line of values is scanned
  *   [4] inside one block without the sub-block level: an edge entry
  *   [5] inside one block without the sub-block level: warp scan
- *   [6] per-element entries read (random 8-byte HBM lookups)
+ *   [6] end parts read: per-element entries (random 8-byte HBM lookups), or
+ *       with the sub-block level a line of values; 0 for a light index
  *   [7] small-table words read (L2-resident probes)
- *   [8] 32-byte sectors of the values read by scans
+ *   [8] 32-byte sectors of the values read by scans (of a light index: end
+ *       parts too)
  *   [9] invalid queries
  * Synchronises `stream`. Uses the handle's counter block, so concurrent
  * rmq_query_stats calls on one handle race (rmq_query does not).
@@ -328,8 +332,8 @@ int rmq_checked_violations(int64_t *count);
  * the bits 0x7fc00000 in an int32 plan, counted by rmq_batch_invalid_count).
  * Arrays are grouped into size buckets floor(log2 length);
  * h_bucket_bs[bucket] (RMQ_BATCH_BUCKETS entries, or NULL; <= 0 means the
- * default: 64 below 2^17 elements, 256 above; 4096 for a light plan) is
- * the block size of that bucket, as chosen by rmq_batch_autotune.
+ * default: 4096) is the block size of that bucket, as chosen by
+ * rmq_batch_autotune.
  * ---------------------------------------------------------------------- */
 #define RMQ_BATCH_BUCKETS 32
 
@@ -340,7 +344,7 @@ typedef struct rmq_batch_info {
     int32_t max_levels;
     int64_t values_span;      /* one past the last value any array uses   */
     int64_t queries_span;     /* one past the last query any array owns   */
-    int64_t workspace_bytes;  /* prefix/suffix minima and sparse tables   */
+    int64_t workspace_bytes;  /* minima, masks and sparse tables          */
     int64_t device_bytes;     /* all device memory owned by the plan      */
     int32_t build_items;
     int32_t query_items;
@@ -359,7 +363,7 @@ int rmq_batch_create(int32_t narrays, const int64_t *h_starts,
  * of the bucket into query items of query_chunk queries (the unit of work a
  * CTA takes in the query phase) and each sparse-table level into items of
  * level_chunk entries (the unit of the table phase). Values <= 0 mean the
- * defaults (bs as rmq_batch_create, 2048 queries, 4096 entries). The
+ * defaults (bs as rmq_batch_create, 4096 queries, 4096 entries). The
  * reference has no batched form, so no counterpart.
  */
 typedef struct rmq_batch_tile {
@@ -372,9 +376,8 @@ typedef struct rmq_batch_tile {
 /* rmq_batch_create with a tile per bucket (h_bucket_tiles: RMQ_BATCH_BUCKETS
  * entries, or NULL for the defaults) and build flags for every array of the
  * plan: RMQ_BUILD_INT32 (d_vals holds int32 and the value outputs are int32),
- * RMQ_BUILD_MAX (range maximum), RMQ_BUILD_LIGHT (light index per array:
- * block and micro-block tables only; block sizes multiples of 32 and >= 64,
- * default 4096; an array shorter than its block size gets one block of its
+ * RMQ_BUILD_MAX (range maximum), RMQ_BUILD_LIGHT (reported; the same tables;
+ * block sizes multiples of 32 and >= 64; an array shorter than its block size gets one block of its
  * length rounded up to a multiple of 32, at least 64). Other flags:
  * RMQ_EINVAL. rmq_batch_create(..., bs, out) is this call with tiles
  * {bs[b], 0, 0, 0} and flags 0. */

@@ -88,8 +88,8 @@ class RMQIndex:
                  light: bool = False):
         """values: 1-D float32 or int32 CUDA tensor; op: "min" (the
         reference's semantics) or "max"; ties resolve to the leftmost index.
-        light=True builds the light index (RMQ_BUILD_LIGHT: tables only, no
-        per-element entries; bs a multiple of 32, >= 64)."""
+        light=True gives the light flag (RMQ_BUILD_LIGHT; every index but a
+        micro=False one holds tables only; bs a multiple of 32, >= 64)."""
         import torch
         if values.dim() != 1 or values.dtype not in (torch.float32, torch.int32):
             raise TypeError("values must be a 1-D float32 or int32 CUDA tensor")

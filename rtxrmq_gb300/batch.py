@@ -2,9 +2,8 @@
 
 Thousands of independent float32 (or int32) arrays of uneven length, each
 with its own (l, r) queries, are built and answered by one persistent
-cooperative kernel launch, for range minimum or maximum, with the full index
-(prefix / suffix entries per element) or the light one (block and
-micro-block tables only). ``run_per_array`` produces the same results
+cooperative kernel launch, for range minimum or maximum.
+``run_per_array`` produces the same results
 through the plain path (one build + one query launch sequence per array)
 for comparison.
 ``autotune`` picks the block size of every size bucket (floor(log2 length))
@@ -68,7 +67,7 @@ def _vals(t, int32: bool = False):
 
 def plan_flags(op: str = "min", dtype="float32", light: bool = False) -> int:
     """rmq_batch_create_ex flags: range minimum or maximum, float32 or int32
-    values, full or light index."""
+    values, light flag."""
     if op not in ("min", "max"):
         raise ValueError("op must be 'min' or 'max'")
     name = str(dtype).split(".")[-1]
@@ -102,8 +101,8 @@ class RMQBatch:
     int32 (l, r) pairs). ``bucket_bs`` maps size bucket -> block size, or
     -> (block size, queries per query item, entries per level item) as
     ``autotune(..., tiles=True)`` returns. ``op`` ("min" / "max"),
-    ``dtype`` (float32 / int32 values) and ``light`` (block and micro-block
-    tables only) hold for every array of the plan."""
+    ``dtype`` (float32 / int32 values) and ``light`` (the flag; every plan holds
+    block and micro-block tables only) hold for every array of the plan."""
 
     def __init__(self, starts: Sequence[int], lengths: Sequence[int], qstarts: Sequence[int],
                  qcounts: Sequence[int], bucket_bs: Optional[Sequence] = None, *,

@@ -4,9 +4,11 @@
 // per block minimum and hands them to the OptiX BVH builder
 // (src/device_tools.cuh:139-169, 243-253, src/rtx.h:3-22, 39-99). GB300 has
 // no RT cores, so the search structure is rebuilt as arrays a query indexes
-// directly: in-block prefix / suffix minima (build_impl.cuh) and a sparse
-// table over the block minima:
+// directly: micro-block minima and the micro table over them
+// (tables_impl.cuh) and sparse tables over block minima:
 //   st[k][j] = leftmost minimum of blocks j .. j + 2^k - 1 (k = 0: block minima)
+// Without the sub-block level: in-block prefix / suffix minima per element
+// (build_impl.cuh) and one sparse table.
 #include "build_impl.cuh"
 #include "engine.h"
 #include "minima_impl.cuh"
@@ -55,7 +57,8 @@ table_kernel(const float *__restrict__ A, int64_t limit, int64_t base, uint32_t 
                              bmin, pb, *reinterpret_cast<TableSmem *>(s_table));
 }
 
-// What the runs left out, from the micro-block minima (and masks): the offset
+// Tables in blocks of bs (arrays of a batch, rmq_query_stats; an index's own
+// blocks leave nothing): what the runs left out, from the micro-block minima, the offset
 // rows of split_rows, one tile of kRowTile positions per CTA, and in the CTAs
 // before them the block minima of blocks that do not tile a unit, a thread
 // per block of up to 16 micro-blocks, else a warp. One launch: the block

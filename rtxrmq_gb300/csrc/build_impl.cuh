@@ -1,5 +1,6 @@
-// build_impl.cuh -- the CTA-level unit builder shared by the plain build
-// kernel (build.cu) and the persistent batch kernel (batch.cu).
+// build_impl.cuh -- the CTA-level builder of per-element entries (build.cu):
+// indexes without the sub-block level, and the entries rmq_probe_gather
+// looks up.
 //
 // For one array A[0..n) cut into blocks of bs it produces
 //   pre[i]  = leftmost minimum of A[blockstart(i) .. i]
@@ -38,7 +39,6 @@
 #pragma once
 
 #include "common.cuh"
-#include "lane_min.cuh"
 
 namespace rmq {
 
@@ -732,119 +732,6 @@ __device__ __forceinline__ void build_unit(const UnitJob &J, uint32_t u, Entry *
         build_unit_stream<ALIGNED, MODE>(J, u, stage, s_warp);
     } else {
         build_unit_tiles<ALIGNED, MODE>(J, u, stage, s_warp);
-    }
-}
-
-// ---- table index: micro-block minima ----
-
-constexpr uint32_t kMicroElems = 32;    // elements per micro-block
-constexpr uint32_t kMicroPerWarp = 16;  // micro-blocks a warp reduces per step
-
-// The composite minimum of one micro-block whose 32 elements lie 4 per lane
-// on the 8 lanes of group `grp` (this lane's first element at e = base +
-// 4 sub). Composites order by (key, index), so the 32-bit keys are reduced
-// first: each lane keeps its smallest key and the first position holding
-// it (lane_best4), the group takes the minimum key, and the leftmost lane holding that
-// key owns the leftmost best element; its position and -0.0 flag come over
-// in one shuffle. Elements at or past n take the largest key; they lie to
-// the right of every valid element, so a tie never selects one.
-template <uint32_t MODE, bool FULL>
-__device__ __forceinline__ Entry micro_row_min(const uint32_t (&b)[4], uint32_t e, uint32_t n,
-                                               uint32_t grp, uint32_t sub) {
-    uint32_t km, info;  // the lane's best key; its position | (-0.0 flag << 2)
-    lane_best4<MODE>(b, FULL ? 4u : (e < n ? min(4u, n - e) : 0u), km, info);
-    uint32_t gk = km;
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) gk = min(gk, __shfl_xor_sync(0xffffffffu, gk, o, 8));
-    const uint32_t owners = (__ballot_sync(0xffffffffu, km == gk) >> (grp * 8u)) & 0xffu;
-    const uint32_t w = __ffs(owners) - 1u;
-    const uint32_t winfo = __shfl_sync(0xffffffffu, info, grp * 8u + w);
-    const uint32_t base = e - 4u * sub;
-    if (!FULL && base >= n) return kEntryNone;
-    const uint32_t idx = base + 4u * w + (winfo & 3u);
-    return (static_cast<uint64_t>(gk) << 32) | (idx << 1) | (winfo >> 2);
-}
-
-// Micro-block minima of micro-blocks [j0, j0 + 16) of one array (values
-// A[0 .. n)) with one whole warp: four 512-byte rows, each lane 4
-// consecutive elements of every row, all loads in flight before any
-// reduction (micro_row_min). VEC: 16-byte loads (A + j0 * 32 16-byte aligned
-// and all 512 elements inside the array). Writes dst[j - base] for j < jend
-// (jend <= ceil(n / 32)); returns the four minima of the lane's group
-// (micro-blocks j0 + 4i + lane / 8; kEntryNone past the array).
-template <uint32_t MODE, bool VEC>
-__device__ __forceinline__ void micro_min_warp(const float *__restrict__ A, uint32_t n,
-                                               uint32_t j0, uint32_t jend, Entry *dst,
-                                               uint32_t base, Entry (&m)[4]) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t sub = lane & 7u;
-    const uint32_t grp = lane >> 3;
-    const uint32_t e0 = j0 * kMicroElems + lane * 4u;  // row 0 of this lane
-    uint32_t b[4][4];
-    if (VEC) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint4 f = ld_u4(A + e0 + i * 128u);
-            b[i][0] = f.x;
-            b[i][1] = f.y;
-            b[i][2] = f.z;
-            b[i][3] = f.w;
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint32_t g = e0 + i * 128u + k;
-                b[i][k] = g < n ? ld_u1(A + g) : 0u;
-            }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) m[i] = micro_row_min<MODE, VEC>(b[i], e0 + i * 128u, n, grp, sub);
-    if (sub == 0u) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t j = j0 + 4u * i + grp;
-            if (j < jend) dst[j - base] = m[i];
-        }
-    }
-}
-
-// micro_min_warp over ROWS rows (4 * ROWS micro-blocks [j0, j0 + 4 ROWS)),
-// every row's loads in flight before any reduction, each row's minima
-// written (dst[j - base], j < jend) as soon as they are reduced, none kept.
-template <uint32_t MODE, bool VEC, int ROWS>
-__device__ __forceinline__ void micro_min_rows(const float *__restrict__ A, uint32_t n,
-                                               uint32_t j0, uint32_t jend, Entry *dst,
-                                               uint32_t base) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t sub = lane & 7u;
-    const uint32_t grp = lane >> 3;
-    const uint32_t e0 = j0 * kMicroElems + lane * 4u;
-    uint32_t b[ROWS][4];
-    if (VEC) {
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i) {
-            const uint4 f = ld_u4(A + e0 + i * 128u);
-            b[i][0] = f.x;
-            b[i][1] = f.y;
-            b[i][2] = f.z;
-            b[i][3] = f.w;
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint32_t g = e0 + i * 128u + k;
-                b[i][k] = g < n ? ld_u1(A + g) : 0u;
-            }
-    }
-#pragma unroll
-    for (int i = 0; i < ROWS; ++i) {
-        const Entry m = micro_row_min<MODE, VEC>(b[i], e0 + i * 128u, n, grp, sub);
-        const uint32_t j = j0 + 4u * i + grp;
-        if (sub == 0u && j < jend) dst[j - base] = m;
     }
 }
 

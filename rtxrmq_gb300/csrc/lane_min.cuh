@@ -1,6 +1,6 @@
 // lane_min.cuh -- the best of one lane's four consecutive values, as a key
-// (common.cuh) and a position, for the micro-block minima of the light
-// index. Host and device code, so that the host tests run it against the
+// (common.cuh) and a position: the comparison rule of lines.cuh for one lane,
+// spelt out. Host and device code, so that the host tests run it against the
 // definition (the smallest key, leftmost among equal keys).
 #pragma once
 

@@ -6,8 +6,8 @@
 // device memory through its own pool and forbids third-party cudaMalloc, or
 // a latency-critical loop that cannot take cudaMalloc / cudaFree's implicit
 // device-wide synchronisation. They pass their own input and output buffers;
-// the prefix/suffix minima, sparse tables and invalid-query counter are
-// written into g_noalloc_scratch below instead of memory from rmq_build.
+// the minima, tables and invalid-query counter are written into
+// g_noalloc_scratch below instead of memory from rmq_build.
 //
 // The array is a file-scope __device__ variable of kNoallocScratchBytes, so
 // every GPU that loads this library holds it until the process exits. In

@@ -3,7 +3,7 @@
 // The role of HRMQ's saveDS / loadDS (hrmq/RMQRMM64.cpp:1471-1659), which
 // write the structure's scalars and tables so it can be reused without a
 // rebuild. Here the file is a fixed header followed by the handle's single
-// device allocation (prefix/suffix minima, sparse tables, sub-block level).
+// device allocation (minima, tables).
 // The values are not stored (the index refers to the caller's array); the
 // header holds a 64-bit fingerprint of all values, computed on the GPU, and
 // rmq_load refuses an array whose fingerprint, length or layout differs.

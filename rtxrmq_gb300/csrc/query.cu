@@ -3,9 +3,10 @@
 // query_kernel: one CTA answers 256 * QPT consecutive queries at a time with
 // the queued body of query_impl.cuh (RTX_blocks' three-ray decomposition,
 // src/rtx_kernels.cu:85-193 and 350-465, needed only for the queries a
-// probe of the small tables over a superset of [l, r] does not settle). Queries and outputs may live in device memory or in pinned host
-// memory mapped into the device address space: on a Grace-Blackwell node the
-// kernel then streams them over NVLink-C2C while its random lookups hit HBM.
+// probe of the small tables over a superset of [l, r] does not settle).
+// Queries and outputs may live in device memory or in pinned host memory
+// mapped into the device address space: on a Grace-Blackwell node the kernel
+// then streams them over NVLink-C2C while its random lookups hit HBM.
 //
 // scan_kernel is the GPU brute force of alg 2 / 102
 // (src/cuda_methods.cuh:3-66): one thread per query, strict `<` from A[l].

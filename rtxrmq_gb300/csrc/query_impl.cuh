@@ -6,16 +6,17 @@
 // query: one through the fully covered blocks lB+1..rB-1, one through the
 // left partial block and one through the right partial block, and keeps the
 // closest hit. Here the same decomposition is answered from arrays:
-//   left partial block   -> suf[l]   (random HBM lookup)
-//   right partial block  -> pre[r]   (random HBM lookup)
+//   left partial block   -> a line of values and the micro-blocks after it
+//   right partial block  -> a line of values and the micro-blocks before it
 //   full blocks between  -> two sparse-table entries (L2-resident)
-// and it is needed only for the few queries a cheaper test does not settle:
-// every query first probes a small L2-resident table over all the units it
-// touches (blocks lB..rB, or with the sub-block level the 32-element
-// micro-blocks l/32..r/32), and when the leftmost best of that superset
-// lies inside [l, r] it is the answer without any per-element lookup. A
-// query inside one micro-block is settled by a scan of that 128-byte line,
-// 8 lanes per query; without the sub-block level a query inside one block that
+// (suf[l] and pre[r] for the partial blocks of an index without the sub-block
+// level), and it is needed only for the few queries a cheaper test does not
+// settle: every query first probes a small L2-resident table over all the
+// units it touches (blocks lB..rB, or the 32-element micro-blocks
+// l/32..r/32), and when the leftmost best of that superset lies inside [l, r]
+// it is the answer without a look at the values. A query inside one
+// micro-block is settled from that 128-byte line, copied to shared memory by
+// 8 lanes; without the sub-block level a query inside one block that
 // the probe does not settle reads pre / suf at a block edge, or is scanned
 // by the whole warp (__reduce_min_sync over the composites). All
 // comparisons are unsigned minima of the composites of common.cuh; only the
@@ -72,8 +73,8 @@ struct V1View {
     uint32_t levels;    // sparse-table levels (st holds levels * nb entries)
     uint32_t mlevels;   // micro-table levels (moff holds moff_rows(mlevels) rows of nmicro)
     bool light;         // counting launches: how the end parts are counted
-    // 2^mlevels - 1: a query whose end micro-blocks ml < mr have
-    // mr - ml < micro_span is probed through the micro table (0: no micro level)
+    // a query whose end micro-blocks ml < mr have mr - ml < micro_span is probed
+    // through the micro table (at most 2^mlevels - 1; 0: no micro level)
     uint32_t micro_span;
 };
 
@@ -213,10 +214,6 @@ __device__ __forceinline__ Entry warp_scan_range(const V1View &v, uint32_t l, ui
     return (static_cast<uint64_t>(kmin) << 32) | lo;
 }
 
-// Answer queries [q0, q1) of one array with the whole CTA. The loop is
-// uniform across the CTA (warp-cooperative scans need full warps).
-// QPT queries per thread per iteration keep several independent lookups in
-// flight per thread.
 // Queries base + threadIdx.x + k * blockDim.x (k < QPT) of [.., q1), loaded
 // ahead of use (the query stream may come from host memory over the host
 // link, so a caller can issue the next step's loads before answering the
@@ -240,23 +237,23 @@ __device__ __forceinline__ void load_queries(const QueryOut &o, int64_t base, in
 // answer: it beats every element of the superset, and an equal element
 // further left inside [l, r] would have been chosen instead. Otherwise the
 // best lies outside on one side, say left of l in unit a; then the answer is
-// better(S[l], best of units a+1..b) when the latter falls at or before r
-// (S[l] covers [l, end of a]), and the three-part decomposition of the
-// reference (left partial, units between, right partial) only when it does
-// not. The per-element entries S / P, the random HBM lookups, are read only
-// on those two fallbacks.
+// better(part, best of units a+1..b) when the latter falls at or before r
+// (`part` is the best of [l, end of a]), and the three-part decomposition of
+// the reference (left partial, units between, right partial) only when it
+// does not. The parts, the random HBM lookups, are read only on those two
+// fallbacks.
 
 // Query counters of a measurement launch (rmq_query_stats); the normal
 // kernels compile them out.
 enum QStat : int {
     kStatFirst = 0,   // settled by the superset probe
-    kStatSecond,      // settled by the second probe and one per-element entry
-    kStatFull,        // three-part decomposition: two entries and a middle probe
+    kStatSecond,      // settled by the second probe and one end part
+    kStatFull,        // three-part decomposition: two end parts and a middle probe
     kStatMicroScan,   // inside one micro-block: its line of values is scanned
     kStatBlockEdge,   // one block, no sub-block level: pre / suf at a block edge
     kStatWarpScan,    // one block, no sub-block level: warp-cooperative scan
-    kStatEntries,     // per-element entries read (pre, suf, mpre, msuf)
-    kStatTable,       // small-table words read (sparse table, micro offsets and minima)
+    kStatEntries,     // end parts read (pre / suf entries, or lines of values)
+    kStatTable,       // small-table words read (sparse table, masks, offsets and minima)
     kStatSectors,     // 32-byte sectors of A read by scans
     kStatInvalid,     // invalid queries
     kStatCount
@@ -707,8 +704,11 @@ __device__ __forceinline__ uint32_t decode_bits(Entry e) {
 
 // The superset probe of the queued form for a valid query not inside one
 // micro-block: through the micro table when the query's micro-blocks fit
-// it (`mic`), else through the block table (two entries, one straight
-// sequence).
+// it, else through a block table (two entries, one straight sequence), with
+// COARSE that of the larger blocks for long queries. What the larger blocks
+// leave open is drained with the smaller ones. For shorter ranges they leave
+// too much open, also with a second probe before the queue (n = 1e7, lr=-2,
+// blocks of 2048 and 1024: 0.67 ms so, 0.54 by the smaller ones at once).
 template <bool MICRO, bool COARSE, bool STATS>
 __device__ __forceinline__ Entry superset_probe(const V1View &v, uint32_t l, uint32_t r,
                                                 uint64_t pol, QStats &s) {
