@@ -165,11 +165,11 @@ inline TableShape table_shape(uint32_t n, uint32_t bs) {
 }
 
 // Shape of the plain table index: of n alone, whatever block size is asked for.
-// - Windows of up to 64 (32) micro-blocks, one mask, are answered by the micro
-//   table; twice as many by two masks would be, but four scattered loads cost
-//   more than the block table's two, if its blocks are small (n = 1e8, ranges
-//   of 3000, 2^26 queries: 0.94 ms by masks, 0.77 by blocks of 512). So the
-//   micro table needs no offset rows.
+// - Windows of up to 64 micro-blocks are answered by the micro table, from one
+//   64-bit mask or two of 32. Twice as many by two masks of 64 would be, but
+//   four scattered loads cost more than the block table's two, if its blocks
+//   are small (n = 1e8, ranges of 3000, 2^26 queries: 0.94 ms by masks, 0.77
+//   by blocks of 512). So the micro table needs no offset rows.
 // - Blocks: small ones leave fewer queries open, large ones make rows that fit
 //   L1. 2^13 to 2^14 of them up to 512 elements each (n = 4e6, lr=-2: 0.51 ms
 //   with 512, 0.49 with 256, 0.56 with 64; n = 1e7: 0.54 with 1024, 0.52, 0.56
@@ -183,7 +183,7 @@ struct IndexShape {
 constexpr uint32_t kIndexBlocks = 1u << 13, kCoarseFrom = 64;
 inline IndexShape index_shape(uint32_t n) {
     const bool wide = wide_masks((n + kMicro - 1) / kMicro);
-    IndexShape s{64u, mask_levels(wide), wide ? 64u : 32u, 0u};
+    IndexShape s{64u, mask_levels(wide), wide ? 64u : 63u, 0u};
     while (s.tbs < 512u && n / (2u * s.tbs) >= kIndexBlocks) s.tbs *= 2u;
     if (n / s.tbs >= kIndexBlocks)
         for (s.cbs = 2u * s.tbs; n / s.cbs >= kIndexBlocks; s.cbs *= 2u) {}

@@ -534,6 +534,21 @@ __device__ __forceinline__ Entry finish_entries(const V1View &v, bool left, uint
     return better(better(e1, other), mid);
 }
 
+// Ties. Where the least value of a range repeats all over the array, its first
+// place in l's block nearly always lies before l, and every query of the block
+// tables is open. The best of the micro-blocks from l's on that one mask
+// covers answers such a query when it has the value that the probe found and
+// lies at or after l. A warp looks for it when many of its 64 queries are open:
+// of distinct values few are, and none of those is answered this way (n = 2^27,
+// values of 256, 2^26 ranges of 2^16: 2.70 ms, so 0.94; n = 4.5e7, 2^23 ranges of
+// uniform length: 0.33 and 0.14).
+constexpr uint32_t kManyOpen = 16;
+template <bool STATS>
+__device__ __forceinline__ Entry tied_entry(const V1View &v, uint32_t l, uint64_t pol, QStats &s) {
+    if constexpr (STATS) s.c[kStatTable] += 2u;
+    return ld_entry_keep(v.mst, (l >> 5) + 63u - __clzll(ld_mask(v, l >> 5, pol)), v.nmicro, pol);
+}
+
 // Leftmost best of l .. r inside one micro-block and within kShortChunks
 // 16-byte chunks, by the lane alone. More chunks cost more L1 lookups than
 // the warp's staged copy of the line does (one). 2^25 ranges of 8 in an array
@@ -851,6 +866,29 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
         }
         miss[0] = miss[0] && !tiny[0];
         miss[1] = miss[1] && !tiny[1];
+        m0 = __ballot_sync(0xffffffffu, miss[0]);
+        m1 = __ballot_sync(0xffffffffu, miss[1]);
+    }
+    if (MICRO && __popc(m0) + __popc(m1) >= kManyOpen &&
+        __any_sync(0xffffffffu, miss[0] && static_cast<uint32_t>((qq[0].y >> 5) - (qq[0].x >> 5)) >= v.micro_span)) {
+#pragma unroll 1
+        for (int k = 0; k < 2; ++k) {
+            const uint32_t l = static_cast<uint32_t>(k ? qq[1].x : qq[0].x);
+            const uint32_t r = static_cast<uint32_t>(k ? qq[1].y : qq[0].y);
+            const Entry e = k ? res[1] : res[0];
+            if ((k ? miss[1] : miss[0]) && entry_idx(e) < l && (r >> 5) - (l >> 5) >= v.micro_span) {
+                const Entry x = tied_entry<STATS>(v, l, pol, s);
+                if ((x >> 32) == (e >> 32) && entry_idx(x) >= l) {
+                    put_result(o, base + threadIdx.x + k * THREADS, x, MODE, lead);
+                    if (k) miss[1] = false;
+                    else miss[0] = false;
+                    if constexpr (STATS) {
+                        s.c[kStatSecond] += 1u;
+                        if (!v.light) s.c[kStatEntries] += 1u;
+                    }
+                }
+            }
+        }
         m0 = __ballot_sync(0xffffffffu, miss[0]);
         m1 = __ballot_sync(0xffffffffu, miss[1]);
     }

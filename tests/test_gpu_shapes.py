@@ -66,3 +66,29 @@ def test_index_shapes(cuda, native, n, kind):
             np.testing.assert_array_equal(i.cpu().numpy(), ei)
             np.testing.assert_array_equal(v.cpu().numpy(), A[ei])
             assert sum(st[k] for k in ("first_probe", "second_probe", "full", "micro_scan")) == len(Q)
+
+
+@pytest.mark.parametrize("n", [8192 * 512 + 1, 1 << 23])
+@pytest.mark.parametrize("levels", [2, 256, 4096])
+@pytest.mark.parametrize("op", ["min", "max"])
+def test_long_ranges_of_few_values(cuda, native, n, levels, op):
+    """Nearly every probe finds the best value left of the range: answered by
+    the micro-blocks from l's on, or not when the value only comes later."""
+    import torch
+
+    import rtxrmq_gb300 as R
+    rng = np.random.default_rng(levels)
+    A = rng.integers(0, levels, n).astype(np.float32)
+    A[n // 2:n // 2 + 300_000] = np.where(rng.random(300_000) < 1e-4, 0.0, 5.0)  # rare least values
+    size = np.exp(rng.uniform(np.log(2000), np.log(n), 40_000)).astype(np.int64)
+    l = (rng.random(40_000) * (n - size + 1)).astype(np.int64)
+    l[::3] = n // 2 + rng.integers(0, 200_000, len(l[::3]))
+    size = np.minimum(size, n - l)
+    Q = np.stack([l, l + size - 1], 1)
+    B = A if op == "min" else -A  # the leftmost largest is the leftmost least of -A
+    m = range_min(composites(B + 0.0), Q[:, 0], Q[:, 1])
+    ei = (m & np.uint64(0xffffffff)).astype(np.int64) >> 1
+    with R.RMQIndex(torch.from_numpy(A).to(cuda), op=op) as ix:
+        v, i = ix.query(torch.from_numpy(Q.astype(np.int32)).to(cuda))
+        np.testing.assert_array_equal(i.cpu().numpy(), ei)
+        np.testing.assert_array_equal(v.cpu().numpy(), A[ei])
