@@ -806,7 +806,10 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
         }
         // the probe's answer is stored even for a query it leaves open: the
         // drain (same warp, after __syncwarp) or the warp scan (same thread)
-        // overwrites it, and whole-warp stores keep the output lines whole
+        // overwrites it, and whole-warp stores keep the output lines whole. A
+        // query inside one micro-block has none (results in host memory,
+        // ranges of 1: stored twice 0.38 ms per 3.8e6 queries, 0.22 once)
+        if (MICRO && scan[k]) continue;
         if (vs) __stcs(reinterpret_cast<unsigned int *>(vs) + j, decode_bits<MODE>(res[k]));
         if (is) __stcs(is + j, static_cast<int32_t>(entry_idx(res[k]) - lead));
     }
