@@ -363,7 +363,8 @@ int rmq_batch_create(int32_t narrays, const int64_t *h_starts,
  * of the bucket into query items of query_chunk queries (the unit of work a
  * CTA takes in the query phase) and each sparse-table level into items of
  * level_chunk entries (the unit of the table phase). Values <= 0 mean the
- * defaults (bs as rmq_batch_create, 4096 queries, 4096 entries). The
+ * defaults (bs as rmq_batch_create, 4096 queries, fewer in a plan that has
+ * not that many for every CTA, 4096 entries). The
  * reference has no batched form, so no counterpart.
  */
 typedef struct rmq_batch_tile {

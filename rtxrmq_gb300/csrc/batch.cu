@@ -277,6 +277,17 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
         for (uint32_t j = 0; j < cnt; j += chunk)
             steps[step].push_back(make_uint4(i, (kind << 16) | k, j, std::min(chunk, cnt - j)));
     };
+    // items small enough for every CTA to get one
+    int64_t all_units = 0, all_q = 0;
+    for (int32_t i = 0; i < narrays; ++i) {
+        if (h_lengths[i] > 0) all_units += h_lengths[i] / (kUnit * static_cast<int64_t>(kMicro)) + 1;
+        if (h_qcounts[i] > 0 && h_qcounts[i] <= 0xffffffffLL) all_q += h_qcounts[i];
+    }
+    const int64_t ctas = static_cast<int64_t>(dev.sms) * RMQ_BATCH_MINB;
+    const uint32_t run_units =
+        static_cast<uint32_t>(std::clamp<int64_t>(all_units / ctas, 1, kRunUnits));
+    const uint32_t default_chunk = static_cast<uint32_t>(
+        std::clamp<int64_t>(all_q / ctas, kLeastQueryChunk, kQueryChunk));
     for (int32_t i = 0; i < narrays; ++i) {
         const int64_t n = h_lengths[i], s = h_starts[i];
         const int64_t qs = h_qstarts[i], qc = h_qcounts[i];
@@ -291,7 +302,8 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
         const int bk = n > 0 ? bucket_of(n) : 0;
         int64_t bs = n > 0 ? b->bucket_bs[bk] : 1;
         if (bs <= 0) bs = kDefaultBatchBs;
-        const uint32_t qchunk = static_cast<uint32_t>(b->tiles[bk].query_chunk);
+        const bool chunk_set = h_bucket_tiles && h_bucket_tiles[bk].query_chunk > 0;
+        const uint32_t qchunk = chunk_set ? static_cast<uint32_t>(b->tiles[bk].query_chunk) : default_chunk;
         const uint32_t lchunk = static_cast<uint32_t>(b->tiles[bk].level_chunk);
         BatchArray &a = b->h_arrays[i];
         std::memset(&a, 0, sizeof(a));
@@ -331,8 +343,8 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
             // A: runs of units. B, step 1: block minima, rows made apart;
             // then the block table's levels
             const uint32_t units = (a.nmicro + kUnit - 1) / kUnit;
-            for (uint32_t u = 0; u < units; u += kRunUnits)
-                runs.push_back(make_uint4(i, u, std::min(kRunUnits, units - u), 0));
+            for (uint32_t u = 0; u < units; u += run_units)
+                runs.push_back(make_uint4(i, u, std::min(run_units, units - u), 0));
             if (!fused_blocks(a.bs / kMicro))
                 add_items(1, i, kItemBlockMinima, 0, a.nb, std::max<uint32_t>(8u, lchunk / (a.bs / kMicro)));
             if (split_rows(a.mlevels)) add_items(1, i, kItemRows, 0, a.nmicro, kBatchRowTile);

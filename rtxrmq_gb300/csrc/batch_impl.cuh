@@ -32,16 +32,22 @@ namespace rmq {
 
 constexpr int kBatchThreads = kUnit;  // phase A runs the table builder
 constexpr int kBatchQPT = 2;
-// default tile schedule: queries per query item, table entries per level
-// item (a plan can set both per size bucket, rmq_batch_create_ex)
+// default tile schedule: queries per query item (at most, see kRunUnits), table
+// entries per level item (a plan can set both per size bucket,
+// rmq_batch_create_ex)
 constexpr uint32_t kQueryChunk = 4096;
 constexpr uint32_t kLevelChunk = 4096;
 constexpr int kMaxSteps = 16;
-// units (of 256 micro-blocks) per run item: 1 MB of values, so that the 63 to
-// 255 micro-blocks a run reads beyond its end stay below a few percent (ragged
-// benchmark's build: 1.25 ms with 8 units, 1.20 with 16, 1.18 with 32; with 64
-// 1.17, but a few arrays of 2e7 leave SMs idle: 0.14 and 0.23 ms)
+// units (of 256 micro-blocks) per run item, at most: 1 MB of values, so that
+// the 63 to 255 micro-blocks a run reads beyond its end stay below a few
+// percent (ragged benchmark's build: 1.25 ms with 8 units, 1.20 with 16, 1.18
+// with 32; with 64 1.17, but a few arrays of 2e7 leave SMs idle: 0.14 and 0.23
+// ms). Fewer where a plan has not that many for every CTA, and the same for
+// the queries of an item where the tile does not set them (29 arrays of up to
+// 2.6e5 values, 26 thousand queries: 101 us with the most, 43 so; 100 of up to
+// 1e6, 1 million queries: 160 and 66).
 constexpr uint32_t kRunUnits = 32;
+constexpr uint32_t kLeastQueryChunk = 512;  // one step of a CTA
 // positions per item of rows made apart, and the largest block table that one
 // item takes through all its levels: both fit the run's shared memory
 constexpr uint32_t kBatchRowTile = 1024;
