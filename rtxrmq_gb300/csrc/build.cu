@@ -191,8 +191,6 @@ cudaError_t launch_build_tables(const BuildPlan &p, const DeviceInfo &dev, cudaS
 
 }  // namespace
 
-uint32_t st_levels(uint32_t nb) { return nb ? static_cast<uint32_t>(ilog2(nb)) + 1u : 0u; }
-
 namespace {
 size_t a256(size_t x) { return (x + 255) / 256 * 256; }
 struct Offsets {
@@ -263,19 +261,6 @@ size_t layout_v5(uint32_t n, uint32_t bs, bool light, bool no_micro, LayoutV5 *o
                  a256(static_cast<size_t>(micro_offset_bytes(out->mlevels)) * out->nmicro *
                       (out->mlevels - 1));
     return total;
-}
-
-// The micro table works on 32-element micro-blocks aligned in the array,
-// whatever the block size. A query first probes it over every micro-block it
-// touches (a superset of [l, r]; two windows of 2^k micro-blocks cover up to
-// 2^(k+1) - 1 of them), so it holds windows long enough for any query inside
-// one block: a block touches bs/32 micro-blocks when blocks start on
-// micro-block boundaries (bs a multiple of 32, as in every table index), at
-// most floor((bs + 30) / 32) + 1 otherwise.
-uint32_t micro_levels(uint32_t bs) {
-    if (bs < 2 * kMicro) return 0;
-    const uint32_t touched = (bs % kMicro == 0) ? bs / kMicro : (bs + kMicro - 2) / kMicro + 1;
-    return st_levels(touched);
 }
 
 cudaError_t launch_build_entries(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s) {

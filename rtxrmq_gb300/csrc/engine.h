@@ -122,9 +122,20 @@ struct BuildPlan {
     Entry *suf;       // [n]
 };
 constexpr uint32_t kMicro = 32;
+// levels of a sparse table over nb blocks
+inline uint32_t st_levels(uint32_t nb) { return nb ? static_cast<uint32_t>(ilog2(nb)) + 1u : 0u; }
 // levels of a micro table that answers every query inside one block of bs
-// elements (0 below 64)
-uint32_t micro_levels(uint32_t bs);
+// elements (0 below 64). The micro table works on 32-element micro-blocks
+// aligned in the array, whatever the block size. A query first probes it over
+// every micro-block it touches (a superset of [l, r]; two windows of 2^k
+// micro-blocks cover up to 2^(k+1) - 1 of them), so it holds windows long
+// enough for any query inside one block: a block touches bs/32 micro-blocks
+// when blocks start on micro-block boundaries (bs a multiple of 32, as in
+// every table index), at most floor((bs + 30) / 32) + 1 otherwise.
+inline uint32_t micro_levels(uint32_t bs) {
+    if (bs < 2u * 32u) return 0;
+    return st_levels(bs % 32u == 0 ? bs / 32u : (bs + 30u) / 32u + 1u);
+}
 // bytes of one micro-table offset for a table of `mlevels` levels: the
 // largest offset is 2^(mlevels - 1) - 1
 inline uint32_t micro_offset_bytes(uint32_t mlevels) {
@@ -142,10 +153,11 @@ struct TableShape {
 //   2^26 queries, lr=-2, bs 195312: 0.83 ms with the rows, 0.58 with 4096).
 // - Fewer than 32: a range of a few blocks is open as often as the blocks at
 //   its ends are larger than it, so the blocks shrink until there are that
-//   many, and windows of up to 511 micro-blocks do (rows up to level 8 are
-//   made in the run of the minima, longer ones take another step). With 128
-//   the ragged benchmark's build takes 1.83 ms in place of 1.67 for its many
-//   small block tables, and its queries gain nothing.
+//   many, and windows of up to 511 micro-blocks do for blocks of no more than
+//   that (rows up to level 8 are made in the run of the minima, longer ones
+//   take another step); blocks of 2^14 elements hold 512 and need the next
+//   level. With 128 the ragged benchmark's build takes 1.83 ms in place of 1.67
+//   for its many small block tables, and its queries gain nothing.
 // - The masks answer windows of up to 63 (127) micro-blocks whatever the
 //   block size: 6 or 7 levels cost nothing.
 constexpr uint32_t kLeastBlocks = 32;
@@ -159,7 +171,8 @@ inline TableShape table_shape(uint32_t n, uint32_t bs) {
     while (few <= n / kLeastBlocks / 2u) few *= 2u;
     if (few < s.tbs) {
         s.tbs = few;
-        if (s.mlevels > 9u) s.mlevels = 9u;
+        const uint32_t most = few > 511u * kMicro ? micro_levels(few) : 9u;
+        if (s.mlevels > most) s.mlevels = most;
     }
     return s;
 }
@@ -196,7 +209,6 @@ inline IndexShape index_shape(uint32_t n) {
 size_t plan_index(BuildPlan &p, bool no_micro, bool asked = false);
 // Point the plan's arrays into that allocation; returns the counter.
 unsigned long long *place_index(BuildPlan &p, void *base);
-uint32_t st_levels(uint32_t nb);
 cudaError_t launch_build(const BuildPlan &p, const DeviceInfo &dev, cudaStream_t s);
 // Per-element prefix / suffix minima over blocks of p.bs elements into p.pre
 // and p.suf, block minima into p.st[0 .. ceil(n / bs)).
