@@ -400,11 +400,12 @@ int rmq_batch_run(rmq_batch_t *b, const float *d_vals,
  * The two halves of rmq_batch_run, for arrays that stay the same while the
  * queries change: rmq_batch_build builds every array's index in the plan's
  * workspace (one cooperative launch, phases build + tables);
- * rmq_batch_query answers the plan's queries from that index (one
- * cooperative launch, query phase only). rmq_batch_query needs a build
- * (rmq_batch_build or rmq_batch_run) enqueued earlier on the same d_vals
- * (RMQ_EINVAL otherwise); the values must not change in between. Both
- * allocate nothing and can be captured in a CUDA graph.
+ * rmq_batch_query answers the plan's queries from that index (one launch,
+ * query phase only). rmq_batch_query needs a build (rmq_batch_build or
+ * rmq_batch_run) enqueued earlier on the same d_vals (RMQ_EINVAL otherwise);
+ * the values must not change in between. Both allocate nothing and can be
+ * captured in a CUDA graph. Once a plan is built, calls on it with the same
+ * d_vals and outputs of their own may run on several streams at a time.
  */
 int rmq_batch_build(rmq_batch_t *b, const float *d_vals, rmq_stream_t stream);
 int rmq_batch_query(rmq_batch_t *b, const float *d_vals, const int32_t *d_queries,

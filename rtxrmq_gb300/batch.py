@@ -147,7 +147,7 @@ class RMQBatch:
     def query(self, vals, queries, out_val=None, out_idx=None, *, values=True, indices=True,
               stream=None):
         """Answer the plan's queries from the last build on ``vals``
-        (rmq_batch_query), one cooperative launch."""
+        (rmq_batch_query), one launch."""
         v, i = self._out(queries, out_val, out_idx, values, indices)
         check(load().rmq_batch_query(self._h, _vals(vals, self._int32), _queries(queries),
                                      _dptr(v), _dptr(i), _stream(stream)))

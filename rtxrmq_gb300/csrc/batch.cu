@@ -8,6 +8,7 @@
 // The reference has no batched form: rtx_rmq<T> (src/rtx.h:24-177) builds one
 // structure for one array and launches one optixLaunch per batch of queries.
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <new>
 #include <vector>
@@ -41,8 +42,8 @@ size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 }  // namespace
 
-cudaError_t batch_kernel_aligned(uint32_t mode, const void **fn, int *per_sm) {
-    return batch_kernel_t<true>(mode, fn, per_sm);
+cudaError_t batch_kernel_aligned(uint32_t mode, bool build, const void **fn, int *per_sm) {
+    return batch_kernel_t<true>(mode, build, fn, per_sm);
 }
 
 RMQ_VIOLATIONS_READER(violations_batch)
@@ -69,6 +70,8 @@ struct rmq_batch {
     int32_t bucket_bs[RMQ_BATCH_BUCKETS];
     rmq_batch_tile_t tiles[RMQ_BATCH_BUCKETS];  // block size and tile schedule per bucket
     const float *built_vals;  // values of the last build enqueued on this plan
+    // building launches so far: enqueued ones, captured ones (their work counters)
+    std::atomic<uint32_t> enqueued{0}, captured{0};
 };
 
 namespace {
@@ -380,13 +383,14 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
     P.nqitems = static_cast<int32_t>(b->h_qitems.size());
     P.total_q = b->total_q;
 
-    // one allocation: arrays | runs | tables | qitems | counter | workspace
+    // one allocation: arrays | runs | tables | qitems | counters | workspace
     const size_t o_arr = 0;
     const size_t o_runs = align_up(o_arr + sizeof(BatchArray) * narrays, 256);
     const size_t o_tables = align_up(o_runs + sizeof(uint4) * runs.size(), 256);
     const size_t o_q = align_up(o_tables + sizeof(uint4) * tables.size(), 256);
     const size_t o_cnt = align_up(o_q + sizeof(uint4) * b->h_qitems.size(), 256);
-    const size_t o_ws = align_up(o_cnt + 256, 256);
+    const size_t cnt_bytes = align_up(sizeof(unsigned long long) + kCounterPairs * 2 * sizeof(uint32_t), 256);
+    const size_t o_ws = o_cnt + cnt_bytes;
     b->ws_bytes = sizeof(Entry) * static_cast<size_t>(ws_entries);
     b->mem_bytes = o_ws + b->ws_bytes;
     cudaError_t err = dev_malloc(&b->mem, b->mem_bytes);
@@ -408,7 +412,7 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
     if (err == cudaSuccess && !b->h_qitems.empty())
         err = cudaMemcpy(base + o_q, b->h_qitems.data(), sizeof(uint4) * b->h_qitems.size(),
                          cudaMemcpyHostToDevice);
-    if (err == cudaSuccess) err = cudaMemset(base + o_cnt, 0, 256);
+    if (err == cudaSuccess) err = cudaMemset(base + o_cnt, 0, cnt_bytes);
     if (err != cudaSuccess) {
         rc = cuda_fail(err, "rmq_batch_create: upload");
         cudaFree(b->mem);
@@ -421,7 +425,7 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
     P.qitems = reinterpret_cast<const uint4 *>(base + o_q);
     P.invalid = reinterpret_cast<unsigned long long *>(base + o_cnt);
     P.ws = reinterpret_cast<Entry *>(base + o_ws);
-    P.next = reinterpret_cast<uint32_t *>(P.invalid + 1);  // cleared with it
+    P.next = reinterpret_cast<uint32_t *>(P.invalid + 1);  // cleared with it; a pair per launch
     P.limit = b->limit;
     *out = b;
     return RMQ_OK;
@@ -445,9 +449,11 @@ static int batch_args(const rmq_batch_t *b, const float *d_vals, const int32_t *
     return RMQ_OK;
 }
 
-// One cooperative launch of batch_kernel running the given phases.
+// One launch: batch_kernel (cooperative, with work counters of its own) with the
+// phases up to the tables, or up to the queries; batch_query_kernel for the
+// queries alone.
 static int launch_batch(rmq_batch_t *b, const float *d_vals, const int32_t *d_queries,
-                        float *d_val, int32_t *d_idx, rmq_stream_t stream, uint32_t phases,
+                        float *d_val, int32_t *d_idx, rmq_stream_t stream, bool build, bool queries,
                         const char *who) {
     DeviceInfo dev;
     int rc = device_info(&dev);
@@ -457,20 +463,31 @@ static int launch_batch(rmq_batch_t *b, const float *d_vals, const int32_t *d_qu
     P.Q = reinterpret_cast<const int2 *>(d_queries);
     P.val = d_val;
     P.idx = d_idx;
-    P.phases = phases;
+    P.queries = queries;
     const bool aligned = reinterpret_cast<uintptr_t>(d_vals) % 16 == 0 && !b->unaligned;
     const void *kern = nullptr;
     int per_sm = 0;
-    cudaError_t err = aligned ? batch_kernel_aligned(b->kmode, &kern, &per_sm)
-                              : batch_kernel_unaligned(b->kmode, &kern, &per_sm);
+    cudaError_t err = aligned ? batch_kernel_aligned(b->kmode, build, &kern, &per_sm)
+                              : batch_kernel_unaligned(b->kmode, build, &kern, &per_sm);
     if (err != cudaSuccess) return cuda_fail(err, who);
+    void *args[] = {&P};
+    if (!build) {
+        if (P.nqitems > 0)
+            err = cudaLaunchKernel(kern, dim3(static_cast<unsigned>(P.nqitems)), dim3(kThreads), args, 0, stream);
+        return err == cudaSuccess ? RMQ_OK : cuda_fail(err, who);
+    }
     // a cooperative launch needs every CTA resident
     if (per_sm < 1) return set_error(RMQ_ENOTSUP, "%s: kernel cannot be resident", who);
+    constexpr uint32_t half = kCounterPairs / 2;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) cudaGetLastError();  // the launch will tell
+    const uint32_t pair = cap == cudaStreamCaptureStatusNone ? b->enqueued.fetch_add(1) % half
+                                                             : half + b->captured.fetch_add(1) % half;
+    P.next += 2 * pair;
     const unsigned grid = static_cast<unsigned>(dev.sms * per_sm);
-    void *args[] = {&P};
     err = cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kThreads), args, kBatchSmem, stream);
     if (err != cudaSuccess) return cuda_fail(err, who);
-    if (phases & 1u) b->built_vals = d_vals;
+    b->built_vals = d_vals;
     return RMQ_OK;
 }
 
@@ -479,14 +496,14 @@ int rmq_batch_run(rmq_batch_t *b, const float *d_vals, const int32_t *d_queries,
     NvtxRange nvtx_range("rmq_batch_run");
     const int rc = batch_args(b, d_vals, d_queries, d_val, d_idx, "rmq_batch_run");
     if (rc) return rc;
-    return launch_batch(b, d_vals, d_queries, d_val, d_idx, stream, 7u, "rmq_batch_run");
+    return launch_batch(b, d_vals, d_queries, d_val, d_idx, stream, true, true, "rmq_batch_run");
 }
 
 int rmq_batch_build(rmq_batch_t *b, const float *d_vals, rmq_stream_t stream) {
     NvtxRange nvtx_range("rmq_batch_build");
     const int rc = batch_args(b, d_vals, nullptr, nullptr, nullptr, "rmq_batch_build", false);
     if (rc) return rc;
-    return launch_batch(b, d_vals, nullptr, nullptr, nullptr, stream, 3u, "rmq_batch_build");
+    return launch_batch(b, d_vals, nullptr, nullptr, nullptr, stream, true, false, "rmq_batch_build");
 }
 
 int rmq_batch_query(rmq_batch_t *b, const float *d_vals, const int32_t *d_queries, float *d_val,
@@ -497,7 +514,7 @@ int rmq_batch_query(rmq_batch_t *b, const float *d_vals, const int32_t *d_querie
     if (b->built_vals != d_vals)
         return set_error(RMQ_EINVAL, "rmq_batch_query: the plan was not built (rmq_batch_build or "
                                      "rmq_batch_run) on these values");
-    return launch_batch(b, d_vals, d_queries, d_val, d_idx, stream, 4u, "rmq_batch_query");
+    return launch_batch(b, d_vals, d_queries, d_val, d_idx, stream, false, true, "rmq_batch_query");
 }
 
 int rmq_batch_run_per_array(rmq_batch_t *b, const float *d_vals, const int32_t *d_queries,

@@ -10,7 +10,13 @@
 //      table's levels after them;
 //   C  query items (array, first query, count), query_impl.cuh's queued form.
 // Work lists are built on the host once per plan, so a run allocates nothing
-// and can be captured in a CUDA graph.
+// and can be captured in a CUDA graph. A launch of phase C alone needs no
+// barrier: it is an ordinary launch of a kernel of its own.
+//
+// Launches of one plan may overlap, at their ends, when they are on different
+// streams. So a launch shares no state with the next but the index: the two
+// counters from which a building launch's CTAs take items are its own (a pair
+// out of kCounterPairs), and a query launch has none.
 //
 // An array is built from the 128-byte boundary (32 values) at or before its
 // first element on: its micro-blocks are whole 128-byte lines whatever its
@@ -93,9 +99,15 @@ struct BatchParams {
     const uint4 *qitems;
     int32_t nqitems;
     int64_t total_q;      // one past the last query any array owns
-    uint32_t *next;       // work counters: runs, query items (0 between launches)
-    uint32_t phases;      // bit 0 runs, bit 1 table steps, bit 2 queries
+    uint32_t *next;       // the launch's work counters: runs, query items (0 when it starts)
+    bool queries;         // batch_kernel: phase C too
 };
+
+// Pairs of work counters of a plan: launches take them in turn, captured ones
+// from a half of their own. A building launch fills the GPU and its CTAs wait for
+// one another, so no more than two can overlap. Captured launches keep their
+// pair for every replay.
+constexpr uint32_t kCounterPairs = 64;
 
 // Dynamic shared memory of a CTA: the run's buffers in phase A, buffers of
 // two halves in phase B, the warps' miss queues in phase C.
@@ -104,10 +116,11 @@ static_assert(2 * sizeof(Entry) * (kBatchRowTile + 1024) <= kBatchSmem, "row til
 static_assert(2 * sizeof(Entry) * kOneItemTable <= kBatchSmem, "small tables fit");
 static_assert(sizeof(MissQueue<true>) * (kBatchThreads / 32) <= kBatchSmem, "miss queues fit");
 
-// The instantiation for (aligned, key mode) and its CTAs per SM (its limit of
-// dynamic shared memory set).
-cudaError_t batch_kernel_aligned(uint32_t mode, const void **fn, int *per_sm);
-cudaError_t batch_kernel_unaligned(uint32_t mode, const void **fn, int *per_sm);
+// The instantiation for (aligned, key mode): of batch_kernel and its CTAs per SM
+// (its limit of dynamic shared memory set), or without `build` of
+// batch_query_kernel.
+cudaError_t batch_kernel_aligned(uint32_t mode, bool build, const void **fn, int *per_sm);
+cudaError_t batch_kernel_unaligned(uint32_t mode, bool build, const void **fn, int *per_sm);
 
 namespace {
 
@@ -166,7 +179,7 @@ __device__ __forceinline__ int32_t next_item(uint32_t *counter, int32_t *s_item)
 // Phase B: table steps 1 .. steps - 1, a grid barrier after each.
 __device__ __forceinline__ void table_steps(const BatchParams &P, cg::grid_group &grid,
                                             unsigned char *smem) {
-    for (int s = 1; (P.phases & 2u) && s < P.steps; ++s) {
+    for (int s = 1; s < P.steps; ++s) {
         for (int32_t it = P.step_start[s] + blockIdx.x; it < P.step_start[s + 1]; it += gridDim.x) {
             const uint4 w = P.tables[it];
             const BatchArray &a = P.arrays[w.x];
@@ -186,23 +199,20 @@ __device__ __forceinline__ void table_steps(const BatchParams &P, cg::grid_group
     }
 }
 
-// Phase C: the query items, in the queued form.
+// Phase C, one query item by the CTA, in the queued form.
 template <bool ALIGNED, uint32_t MODE>
-__device__ __forceinline__ void query_items(const BatchParams &P, MissQueue<true> &mq, int32_t *s_item) {
-    if (!(P.phases & 4u)) return;
-    for (int32_t it; (it = next_item(P.next + 1, s_item)) < P.nqitems;) {
-        const uint4 w = P.qitems[it];
-        const BatchArray a = P.arrays[w.x];
-        const V1View v = batch_view<MODE>(P, a);
-        QueryOut o;
-        o.Q = P.Q + a.qoff;
-        o.val = P.val ? P.val + a.qoff : nullptr;
-        o.idx = P.idx ? P.idx + a.qoff : nullptr;
-        o.invalid = P.invalid;
-        o.span = P.total_q - a.qoff;
-        answer_range_queued<ALIGNED, true, MODE, true, kBatchThreads, kBatchQPT>(
-            v, o, w.y, static_cast<int64_t>(w.y) + w.z, mq);
-    }
+__device__ __forceinline__ void query_item(const BatchParams &P, int32_t it, MissQueue<true> &mq) {
+    const uint4 w = P.qitems[it];
+    const BatchArray a = P.arrays[w.x];
+    const V1View v = batch_view<MODE>(P, a);
+    QueryOut o;
+    o.Q = P.Q + a.qoff;
+    o.val = P.val ? P.val + a.qoff : nullptr;
+    o.idx = P.idx ? P.idx + a.qoff : nullptr;
+    o.invalid = P.invalid;
+    o.span = P.total_q - a.qoff;
+    answer_range_queued<ALIGNED, true, MODE, true, kBatchThreads, kBatchQPT>(
+        v, o, w.y, static_cast<int64_t>(w.y) + w.z, mq);
 }
 
 template <bool ALIGNED, uint32_t MODE>
@@ -212,7 +222,7 @@ __global__ void __launch_bounds__(kBatchThreads, RMQ_BATCH_MINB) batch_kernel(Ba
     cg::grid_group grid = cg::this_grid();
     // each counter is cleared in the phase that does not use it
     if (blockIdx.x == 0 && threadIdx.x == 0) P.next[1] = 0u;
-    for (int32_t it; (P.phases & 1u) && (it = next_item(P.next, &s_item)) < P.nruns;) {
+    for (int32_t it; (it = next_item(P.next, &s_item)) < P.nruns;) {
         const uint4 w = P.runs[it];
         const BatchArray &a = P.arrays[w.x];
         const uint32_t lo = w.y * kUnit;
@@ -223,13 +233,26 @@ __global__ void __launch_bounds__(kBatchThreads, RMQ_BATCH_MINB) batch_kernel(Ba
     grid.sync();
     if (blockIdx.x == 0 && threadIdx.x == 0) P.next[0] = 0u;
     table_steps(P, grid, s_batch);
-    query_items<ALIGNED, MODE>(P, reinterpret_cast<MissQueue<true> *>(s_batch)[threadIdx.x >> 5], &s_item);
+    MissQueue<true> &mq = reinterpret_cast<MissQueue<true> *>(s_batch)[threadIdx.x >> 5];
+    for (int32_t it; P.queries && (it = next_item(P.next + 1, &s_item)) < P.nqitems;)
+        query_item<ALIGNED, MODE>(P, it, mq);
+}
+
+// Phase C alone (rmq_batch_query): a CTA per item.
+template <bool ALIGNED, uint32_t MODE>
+__global__ void __launch_bounds__(kBatchThreads, RMQ_BATCH_MINB) batch_query_kernel(BatchParams P) {
+    __shared__ __align__(1024) MissQueue<true> s_mq[kBatchThreads / 32];
+    query_item<ALIGNED, MODE>(P, static_cast<int32_t>(blockIdx.x), s_mq[threadIdx.x >> 5]);
 }
 
 std::atomic<int> g_batch_per_sm[4];  // per key mode, of this unit's alignment
 
 template <bool ALIGNED, uint32_t MODE>
-cudaError_t pick_batch(const void **fn, int *per_sm) {
+cudaError_t pick_batch(bool build, const void **fn, int *per_sm) {
+    if (!build) {
+        *fn = reinterpret_cast<const void *>(batch_query_kernel<ALIGNED, MODE>);
+        return cudaSuccess;
+    }
     auto kern = batch_kernel<ALIGNED, MODE>;
     if (g_batch_per_sm[MODE].load(std::memory_order_relaxed) == 0) {
         const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -241,12 +264,12 @@ cudaError_t pick_batch(const void **fn, int *per_sm) {
 }
 
 template <bool ALIGNED>
-cudaError_t batch_kernel_t(uint32_t mode, const void **fn, int *per_sm) {
+cudaError_t batch_kernel_t(uint32_t mode, bool build, const void **fn, int *per_sm) {
     switch (mode) {
-    case kFloatMax: return pick_batch<ALIGNED, kFloatMax>(fn, per_sm);
-    case kIntMin: return pick_batch<ALIGNED, kIntMin>(fn, per_sm);
-    case kIntMax: return pick_batch<ALIGNED, kIntMax>(fn, per_sm);
-    default: return pick_batch<ALIGNED, kFloatMin>(fn, per_sm);
+    case kFloatMax: return pick_batch<ALIGNED, kFloatMax>(build, fn, per_sm);
+    case kIntMin: return pick_batch<ALIGNED, kIntMin>(build, fn, per_sm);
+    case kIntMax: return pick_batch<ALIGNED, kIntMax>(build, fn, per_sm);
+    default: return pick_batch<ALIGNED, kFloatMin>(build, fn, per_sm);
     }
 }
 

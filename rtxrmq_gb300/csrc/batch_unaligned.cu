@@ -5,8 +5,8 @@
 
 namespace rmq {
 
-cudaError_t batch_kernel_unaligned(uint32_t mode, const void **fn, int *per_sm) {
-    return batch_kernel_t<false>(mode, fn, per_sm);
+cudaError_t batch_kernel_unaligned(uint32_t mode, bool build, const void **fn, int *per_sm) {
+    return batch_kernel_t<false>(mode, build, fn, per_sm);
 }
 
 RMQ_VIOLATIONS_READER(violations_batch_unaligned)
