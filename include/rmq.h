@@ -210,8 +210,8 @@ int rmq_free(rmq_handle_t *h);
  * handle must precede that point (it was enqueued on `stream`, or `stream`
  * waits for it). Falls back to rmq_free where that cannot be known or done:
  * a query of the handle was captured in a graph, `stream` is capturing, the
- * handle came from rmq_load, has host staging or probe entries, or is larger
- * than the pool keeps.
+ * current device is not the handle's, the handle came from rmq_load, has host
+ * staging or probe entries, or is larger than the pool keeps.
  */
 int rmq_free_async(rmq_handle_t *h, rmq_stream_t stream);
 

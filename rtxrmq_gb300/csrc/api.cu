@@ -711,9 +711,12 @@ int rmq_free_async(rmq_handle_t *h, rmq_stream_t stream) {
     NvtxRange nvtx_range("rmq_free_async");
     g_err[0] = '\0';
     if (!h) return RMQ_OK;
+    // the order of another device's default stream would be no order at all
+    int cur = -1;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (!h->pooled || h->captured || h->stage || h->entries ||
-        cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    if (!h->pooled || h->captured || h->stage || h->entries || cudaGetDevice(&cur) != cudaSuccess ||
+        cur != h->device || cudaStreamIsCapturing(stream, &cap) != cudaSuccess ||
+        cap != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
         return rmq_free(h);
     }

@@ -1,0 +1,49 @@
+"""CPU: the rules of api.cu about index memory, run against a CUDA runtime on the
+host (fake_cuda.h): which device's order a release follows."""
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+HEAD = '#include "fake_cuda.h"\n#include "api.cu"\n'
+INDEX = r"""
+static float values[100000];
+static rmq_handle_t *index_of(int device, rmq_stream_t s = nullptr, int64_t n = 100000) {
+    fake::device = device;
+    rmq_handle_t *h = nullptr;
+    return rmq_build(values, n, 0, s, &h) == RMQ_OK ? h : nullptr;
+}
+"""
+
+
+def run(tmp_path, body):
+    src = tmp_path / "rules.cpp"
+    src.write_text(HEAD + INDEX + "int main() {\n" + body + '    std::printf("ok\\n");\n    return 0;\n}\n')
+    exe = tmp_path / "rules"
+    csrc = ROOT / "rtxrmq_gb300" / "csrc"
+    r = subprocess.run(["g++", "-std=c++17", "-x", "c++", f"-I{ROOT / 'tests'}", f"-I{csrc}",
+                        "-I/usr/local/cuda/include", str(src), "-o", str(exe), "-ldl", "-lpthread",
+                        "-Wl,--unresolved-symbols=ignore-all"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0 and r.stdout == "ok\n", r.stdout + r.stderr
+
+
+def test_release_follows_the_index_device(tmp_path):
+    """In stream order on the index's own device; on another current device the
+    default stream is that device's, so the release waits for the index's."""
+    run(tmp_path, r"""
+    rmq_handle_t *h = index_of(0);
+    EXPECT(h && fake::take() == "create0 pool0 ");
+    EXPECT(rmq_free_async(h, nullptr) == RMQ_OK && fake::take() == "free-async0 ");
+    h = index_of(1);
+    EXPECT(h && fake::take() == "create1 pool1 ");
+    fake::device = 0;
+    EXPECT(rmq_free_async(h, nullptr) == RMQ_OK);
+    EXPECT(fake::log == "wait1 free0 " && fake::device == 0 && fake::held.empty());
+    fake::take();
+    h = index_of(1);
+    fake::take();
+    EXPECT(rmq_free_async(h, nullptr) == RMQ_OK && fake::take() == "free-async1 ");
+""")
