@@ -684,6 +684,19 @@ int rmq_query_host(const rmq_handle_t *h, const int32_t *h_queries, int64_t q, f
     return RMQ_OK;
 }
 
+// Waits for all work of the current device as a cudaFree of the memory would,
+// which a capture in relaxed or thread-local mode allows. cudaDeviceSynchronize
+// fails while any stream of the device captures, and ends that capture.
+static cudaError_t wait_for_device() {
+    void *p = nullptr;
+    const cudaError_t err = cudaMalloc(&p, sizeof(unsigned long long));
+    if (err == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return cudaDeviceSynchronize();
+    }
+    return err == cudaSuccess ? cudaFree(p) : err;
+}
+
 int rmq_free(rmq_handle_t *h) {
     g_err[0] = '\0';
     if (!h) return RMQ_OK;
@@ -694,7 +707,7 @@ int rmq_free(rmq_handle_t *h) {
         int cur = 0;
         e2 = cudaGetDevice(&cur);
         if (e2 == cudaSuccess && cur != h->device) e2 = cudaSetDevice(h->device);
-        if (e2 == cudaSuccess) e2 = cudaDeviceSynchronize();
+        if (e2 == cudaSuccess) e2 = wait_for_device();
         if (cur != h->device) cudaSetDevice(cur);
     }
     if (e2 == cudaSuccess) e2 = cudaFree(h->mem);

@@ -1,5 +1,6 @@
 """CPU: the rules of api.cu about index memory, run against a CUDA runtime on the
-host (fake_cuda.h): which device's order a release follows."""
+host (fake_cuda.h): whose order a release follows, and that a waiting one leaves
+captures alone."""
 import subprocess
 from pathlib import Path
 
@@ -46,4 +47,25 @@ def test_release_follows_the_index_device(tmp_path):
     h = index_of(1);
     fake::take();
     EXPECT(rmq_free_async(h, nullptr) == RMQ_OK && fake::take() == "free-async1 ");
+""")
+
+
+def test_waiting_release_leaves_captures_alone(tmp_path):
+    """rmq_free waits by calls that a relaxed or thread-local capture allows, as
+    the release of memory from cudaMalloc does; under a global one it fails, as
+    that does."""
+    run(tmp_path, r"""
+    rmq_handle_t *h = index_of(0), *g = index_of(0);
+    fake::take();
+    fake::capture = 1;
+    EXPECT(rmq_free(h) == RMQ_OK && fake::take() == "wait0 free0 " && !fake::broken);
+    fake::capturing_stream = true;
+    EXPECT(rmq_free_async(g, nullptr) == RMQ_OK && fake::take() == "wait0 free0 " && !fake::broken);
+    fake::capturing_stream = false;
+    fake::capture = 0;
+    h = index_of(0);
+    fake::left = 0;  // not even a word for the wait
+    fake::take();
+    EXPECT(rmq_free(h) == RMQ_OK && fake::take() == "wait0 free0 ");
+    EXPECT(fake::held.empty());
 """)
