@@ -12,7 +12,7 @@
 #include <cstring>
 #include <mutex>
 
-#include <cuda.h>  // cuuint64_t
+#include <cuda.h>  // driver types only; the driver is reached through the runtime
 
 #include "../../include/rmq.h"
 #include "engine.h"
@@ -23,7 +23,7 @@ struct rmq_handle {
     int device;
     void *mem;                      // single allocation holding everything below
     size_t mem_bytes;
-    bool pooled;                    // mem comes from the library's pool
+    unsigned long long pool_context;  // mem comes from the library's pool in this context, 0: it does not
     bool captured;                  // a query was captured: a graph may still replay it
     unsigned long long *invalid;    // device counter of rejected queries
     int64_t table_bytes;
@@ -80,33 +80,79 @@ int cuda_fail(cudaError_t err, const char *what) {
                      what, cudaGetErrorName(err), cudaGetErrorString(err));
 }
 
-static std::mutex g_pool_mu;
-static cudaMemPool_t g_pool[64] = {nullptr};
+// Unique id of the calling thread's current context (cuCtxGetId), 0 when
+// there is none or the driver cannot tell. Context handles may be reused
+// after a reset; the ids are not.
+unsigned long long current_context_id() {
+    using GetCurrent = CUresult (*)(CUcontext *);
+    using GetId = CUresult (*)(CUcontext, unsigned long long *);
+    static std::once_flag once;
+    static GetCurrent get_current = nullptr;
+    static GetId get_id = nullptr;
+    std::call_once(once, [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult st;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &st) ==
+                cudaSuccess && st == cudaDriverEntryPointSuccess)
+            get_current = reinterpret_cast<GetCurrent>(f);
+        f = nullptr;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &st) ==
+                cudaSuccess && st == cudaDriverEntryPointSuccess)
+            get_id = reinterpret_cast<GetId>(f);
+        cudaGetLastError();
+    });
+    CUcontext c = nullptr;
+    unsigned long long id = 0;
+    if (!get_current || !get_id || get_current(&c) != CUDA_SUCCESS || !c ||
+        get_id(c, &id) != CUDA_SUCCESS)
+        return 0;
+    return id;
+}
 
-// The device's pool, made on first use; null when it cannot be.
-static cudaMemPool_t device_pool(int device) {
-    if (device < 0 || device >= 64) return nullptr;
+// The id with the primary context of `device` (the current one) brought up when
+// the thread has none yet.
+static unsigned long long device_context_id(int device) {
+    unsigned long long id = current_context_id();
+    if (!id && cudaSetDevice(device) == cudaSuccess) id = current_context_id();
+    return id;
+}
+
+// The pools made so far, each for one context: a device reset ends the context,
+// its pool and its memory, and the next context takes a pool of its own.
+struct Pool {
+    unsigned long long context;
+    int device;
+    cudaMemPool_t pool;
+};
+static std::mutex g_pool_mu;
+static Pool g_pools[64];
+static int g_npools = 0;
+
+// The pool of `device` in `context`, made on first use where `make`; null when
+// there is none.
+static cudaMemPool_t device_pool(int device, unsigned long long context, bool make) {
     std::lock_guard<std::mutex> lock(g_pool_mu);
-    if (!g_pool[device]) {
-        cudaMemPoolProps props;
-        std::memset(&props, 0, sizeof(props));
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
-        cudaMemPool_t pool = nullptr;
-        cuuint64_t keep = kPoolKeep;
-        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-            cudaGetLastError();
-            cudaMemPoolDestroy(pool);
-            return nullptr;
-        }
-        g_pool[device] = pool;
+    for (int i = 0; i < g_npools; ++i)
+        if (g_pools[i].context == context && g_pools[i].device == device) return g_pools[i].pool;
+    if (!make || !context || g_npools == 64) return nullptr;
+    cudaMemPoolProps props;
+    std::memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t pool = nullptr;
+    cuuint64_t keep = kPoolKeep;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
     }
-    return g_pool[device];
+    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaGetLastError();
+        cudaMemPoolDestroy(pool);
+        return nullptr;
+    }
+    g_pools[g_npools++] = Pool{context, device, pool};
+    return pool;
 }
 
 static bool fail_alloc() {
@@ -114,14 +160,16 @@ static bool fail_alloc() {
     return f && f[0] == '1';
 }
 
-cudaError_t pool_malloc(void **p, size_t bytes, int device, cudaStream_t s, bool *pooled) {
-    *pooled = false;
+cudaError_t pool_malloc(void **p, size_t bytes, int device, cudaStream_t s,
+                        unsigned long long *pool_context) {
+    *pool_context = 0;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (!fail_alloc() && bytes <= kPoolKeep && cudaStreamIsCapturing(s, &cap) == cudaSuccess &&
         cap == cudaStreamCaptureStatusNone) {
-        cudaMemPool_t pool = device_pool(device);
+        const unsigned long long context = device_context_id(device);
+        cudaMemPool_t pool = device_pool(device, context, true);
         if (pool && cudaMallocFromPoolAsync(p, bytes, pool, s) == cudaSuccess) {
-            *pooled = true;
+            *pool_context = context;
             return cudaSuccess;
         }
     }
@@ -136,11 +184,7 @@ cudaError_t pool_malloc(void **p, size_t bytes, int device, cudaStream_t s, bool
 }
 
 cudaError_t pool_trim(int device) {
-    cudaMemPool_t pool = nullptr;
-    if (device >= 0 && device < 64) {
-        std::lock_guard<std::mutex> lock(g_pool_mu);
-        pool = g_pool[device];
-    }
+    cudaMemPool_t pool = device_pool(device, device_context_id(device), false);
     return pool ? cudaMemPoolTrimTo(pool, 0) : cudaSuccess;
 }
 
@@ -285,7 +329,7 @@ int rmq_build_ex(const float *d_vals, int64_t n, int64_t bs, uint32_t flags, rmq
         return set_error(RMQ_ENOMEM, "rmq_build: host allocation failed");
     }
     h->device = dev.device;
-    cudaError_t err = pool_malloc(&h->mem, total, dev.device, stream, &h->pooled);
+    cudaError_t err = pool_malloc(&h->mem, total, dev.device, stream, &h->pool_context);
     if (err != cudaSuccess) {
         delete h->host_mu;
         delete h;
@@ -302,7 +346,7 @@ int rmq_build_ex(const float *d_vals, int64_t n, int64_t bs, uint32_t flags, rmq
     if (err == cudaSuccess) err = launch_build(p, dev, stream);
     if (err != cudaSuccess) {
         rc = cuda_fail(err, "rmq_build: launch");
-        if (h->pooled)
+        if (h->pool_context)
             cudaFreeAsync(h->mem, stream);
         else
             cudaFree(h->mem);
@@ -317,7 +361,7 @@ int rmq_build_ex(const float *d_vals, int64_t n, int64_t bs, uint32_t flags, rmq
 // Remembers that a graph may replay work on the handle at any time.
 static void note_capture(const rmq_handle_t *h, cudaStream_t stream) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (!h->pooled) return;
+    if (!h->pool_context) return;
     if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
         const_cast<rmq_handle_t *>(h)->captured = true;
 }
@@ -702,15 +746,18 @@ int rmq_free(rmq_handle_t *h) {
     if (!h) return RMQ_OK;
     cudaError_t err = release_staging(h);
     cudaError_t e2 = cudaSuccess;
-    if (h->pooled) {
+    bool gone = false;
+    if (h->pool_context) {
         // cudaFree does not wait for the uses of pool memory
         int cur = 0;
         e2 = cudaGetDevice(&cur);
         if (e2 == cudaSuccess && cur != h->device) e2 = cudaSetDevice(h->device);
-        if (e2 == cudaSuccess) e2 = wait_for_device();
+        // a reset of the device took the memory with it
+        if (e2 == cudaSuccess) gone = device_context_id(h->device) != h->pool_context;
+        if (e2 == cudaSuccess && !gone) e2 = wait_for_device();
         if (cur != h->device) cudaSetDevice(cur);
     }
-    if (e2 == cudaSuccess) e2 = cudaFree(h->mem);
+    if (e2 == cudaSuccess && !gone) e2 = cudaFree(h->mem);
     if (err == cudaSuccess) err = e2;
     e2 = cudaFree(h->entries);
     if (err == cudaSuccess) err = e2;
@@ -727,9 +774,9 @@ int rmq_free_async(rmq_handle_t *h, rmq_stream_t stream) {
     // the order of another device's default stream would be no order at all
     int cur = -1;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (!h->pooled || h->captured || h->stage || h->entries || cudaGetDevice(&cur) != cudaSuccess ||
-        cur != h->device || cudaStreamIsCapturing(stream, &cap) != cudaSuccess ||
-        cap != cudaStreamCaptureStatusNone) {
+    if (!h->pool_context || h->captured || h->stage || h->entries || cudaGetDevice(&cur) != cudaSuccess ||
+        cur != h->device || device_context_id(cur) != h->pool_context ||
+        cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
         return rmq_free(h);
     }

@@ -50,14 +50,20 @@ inline cudaError_t dev_malloc(void **p, size_t bytes) {
     return cudaMalloc(p, bytes);
 }
 
+// Id of the calling thread's current context, 0 when there is none or the
+// driver cannot tell.
+unsigned long long current_context_id();
+
 // Device memory of an index, in stream order: from a pool of the library (one
-// per device) that keeps at most kPoolKeep bytes of freed memory; the rest
-// goes back to the device at the next synchronisation, all of it by
-// pool_trim(). Larger requests, and requests while `s` is capturing, take
-// cudaMalloc (*pooled false). cudaMalloc + cudaFree cost 0.2 ms a call,
-// cudaFree waits for the device: a build + query of 10^5 values took 0.24 ms.
+// per device and context) that keeps at most kPoolKeep bytes of freed memory;
+// the rest goes back to the device at the next synchronisation, all of it by
+// pool_trim(). *pool_context is the context whose pool it came from. Larger
+// requests, and requests while `s` is capturing, take cudaMalloc (0). cudaMalloc
+// + cudaFree cost 0.2 ms a call, cudaFree waits for the device: a build + query
+// of 10^5 values took 0.24 ms.
 constexpr size_t kPoolKeep = size_t(256) << 20;
-cudaError_t pool_malloc(void **p, size_t bytes, int device, cudaStream_t s, bool *pooled);
+cudaError_t pool_malloc(void **p, size_t bytes, int device, cudaStream_t s,
+                        unsigned long long *pool_context);
 cudaError_t pool_trim(int device);
 
 // Resident CTAs per SM of `kernel` at `threads` threads and `dynamic_smem`

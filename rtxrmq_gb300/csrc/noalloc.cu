@@ -23,8 +23,6 @@
 #include <cstring>
 #include <mutex>
 
-#include <cuda.h>  // driver types only; the driver is reached through the runtime
-
 #include "../../include/rmq.h"
 #include "engine.h"
 
@@ -39,35 +37,6 @@ constexpr int kMaxDevices = 64;
 std::mutex g_noalloc_mu;
 void *g_noalloc_ptr[kMaxDevices] = {nullptr};
 unsigned long long g_noalloc_ctx[kMaxDevices] = {0};
-
-// Unique id of the calling thread's current context (cuCtxGetId), 0 when
-// there is none or the driver cannot tell. Context handles may be reused
-// after a reset; the ids are not.
-unsigned long long current_context_id() {
-    using GetCurrent = CUresult (*)(CUcontext *);
-    using GetId = CUresult (*)(CUcontext, unsigned long long *);
-    static std::once_flag once;
-    static GetCurrent get_current = nullptr;
-    static GetId get_id = nullptr;
-    std::call_once(once, [] {
-        void *f = nullptr;
-        cudaDriverEntryPointQueryResult st;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &st) ==
-                cudaSuccess && st == cudaDriverEntryPointSuccess)
-            get_current = reinterpret_cast<GetCurrent>(f);
-        f = nullptr;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &st) ==
-                cudaSuccess && st == cudaDriverEntryPointSuccess)
-            get_id = reinterpret_cast<GetId>(f);
-        cudaGetLastError();
-    });
-    CUcontext c = nullptr;
-    unsigned long long id = 0;
-    if (!get_current || !get_id || get_current(&c) != CUDA_SUCCESS || !c ||
-        get_id(c, &id) != CUDA_SUCCESS)
-        return 0;
-    return id;
-}
 
 // Device address of the scratch array on the current device (set-up on the
 // first call per device, repeated when the context is not the one the

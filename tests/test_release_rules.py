@@ -1,6 +1,6 @@
 """CPU: the rules of api.cu about index memory, run against a CUDA runtime on the
-host (fake_cuda.h): whose order a release follows, and that a waiting one leaves
-captures alone."""
+host (fake_cuda.h): whose order a release follows, that a waiting one leaves
+captures alone, and that a pool ends with its context."""
 import subprocess
 from pathlib import Path
 
@@ -68,4 +68,25 @@ def test_waiting_release_leaves_captures_alone(tmp_path):
     fake::take();
     EXPECT(rmq_free(h) == RMQ_OK && fake::take() == "wait0 free0 ");
     EXPECT(fake::held.empty());
+""")
+
+
+def test_pool_ends_with_its_context(tmp_path):
+    """A device reset ends the pool and what came from it: the next index takes a
+    new pool, a handle of before releases nothing, the other device keeps its
+    own."""
+    run(tmp_path, r"""
+    rmq_handle_t *a = index_of(0), *b = index_of(0), *c = index_of(1);
+    EXPECT(fake::take() == "create0 pool0 pool0 create1 pool1 ");
+    fake::device = 0;
+    fake::context[0] = 21;
+    EXPECT(rmq_trim() == RMQ_OK && fake::take() == "");
+    rmq_handle_t *d = index_of(0);
+    EXPECT(d && fake::take() == "create0 pool0 ");
+    EXPECT(rmq_free(a) == RMQ_OK && rmq_free_async(b, nullptr) == RMQ_OK && fake::take() == "");
+    EXPECT(rmq_free_async(d, nullptr) == RMQ_OK && fake::take() == "free-async0 ");
+    EXPECT(rmq_trim() == RMQ_OK && fake::take() == "trim0 ");
+    EXPECT(index_of(0) && fake::take() == "pool0 ");
+    fake::device = 1;
+    EXPECT(rmq_free_async(c, nullptr) == RMQ_OK && fake::take() == "free-async1 ");
 """)
