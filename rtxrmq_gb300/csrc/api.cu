@@ -190,12 +190,12 @@ cudaError_t pool_trim(int device) {
 
 int device_info(DeviceInfo *out) {
     static std::mutex mu;
-    static DeviceInfo cache[64];
-    static bool have[64] = {false};
+    static DeviceInfo cache[kMaxDevices];
+    static bool have[kMaxDevices] = {false};
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess) return cuda_fail(err, "cudaGetDevice");
-    if (dev < 0 || dev >= 64) return set_error(RMQ_ENOTSUP, "device ordinal %d unsupported", dev);
+    if (dev < 0 || dev >= kMaxDevices) return set_error(RMQ_ENOTSUP, "device ordinal %d unsupported", dev);
     std::lock_guard<std::mutex> lock(mu);
     if (!have[dev]) {
         DeviceInfo d;

@@ -112,13 +112,13 @@ constexpr uint32_t kCounterPairs = 64;
 // Dynamic shared memory of a CTA: the run's buffers in phase A, buffers of
 // two halves in phase B, the warps' miss queues in phase C.
 constexpr size_t kBatchSmem = sizeof(TableSmem);
+static_assert(kBatchSmem <= kDefaultSmem, "no attribute needed");
 static_assert(2 * sizeof(Entry) * (kBatchRowTile + 1024) <= kBatchSmem, "row tiles fit");
 static_assert(2 * sizeof(Entry) * kOneItemTable <= kBatchSmem, "small tables fit");
 static_assert(sizeof(MissQueue<true>) * (kBatchThreads / 32) <= kBatchSmem, "miss queues fit");
 
-// The instantiation for (aligned, key mode): of batch_kernel and its CTAs per SM
-// (its limit of dynamic shared memory set), or without `build` of
-// batch_query_kernel.
+// The instantiation for (aligned, key mode): of batch_kernel and its CTAs per SM,
+// or without `build` of batch_query_kernel.
 cudaError_t batch_kernel_aligned(uint32_t mode, bool build, const void **fn, int *per_sm);
 cudaError_t batch_kernel_unaligned(uint32_t mode, bool build, const void **fn, int *per_sm);
 
@@ -254,11 +254,6 @@ cudaError_t pick_batch(bool build, const void **fn, int *per_sm) {
         return cudaSuccess;
     }
     auto kern = batch_kernel<ALIGNED, MODE>;
-    if (g_batch_per_sm[MODE].load(std::memory_order_relaxed) == 0) {
-        const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     static_cast<int>(kBatchSmem));
-        if (err != cudaSuccess) return err;
-    }
     *fn = reinterpret_cast<const void *>(kern);
     return occupancy_cached(kern, kBatchThreads, g_batch_per_sm[MODE], *per_sm, kBatchSmem);
 }

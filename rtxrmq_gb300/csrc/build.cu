@@ -100,15 +100,14 @@ std::atomic<int> g_units_per_sm[2];
 cudaError_t launch_levels(Entry *st, uint32_t nb, uint32_t levels, const CoarseTable &C, cudaStream_t s) {
     if (levels <= 1) return cudaSuccess;
     if (nb <= kSmallTable && !C.st) {
-        static std::atomic<bool> ready{false};
-        if (!ready.load(std::memory_order_relaxed)) {
-            const cudaError_t err =
-                cudaFuncSetAttribute(small_levels_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(2 * sizeof(Entry) * kSmallTable));
+        const size_t smem = 2 * sizeof(Entry) * nb;
+        if (smem > kDefaultSmem) {
+            // belongs to the current device, so it is set at each launch (0.2 us)
+            const cudaError_t err = cudaFuncSetAttribute(
+                small_levels_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
             if (err != cudaSuccess) return err;
-            ready.store(true, std::memory_order_relaxed);
         }
-        small_levels_kernel<<<1, kLevelThreads, 2 * sizeof(Entry) * nb, s>>>(st, nb, levels);
+        small_levels_kernel<<<1, kLevelThreads, smem, s>>>(st, nb, levels);
         return cudaGetLastError();
     }
     const uint32_t all = C.st && C.levels + C.shift > levels ? C.levels + C.shift : levels;
@@ -129,11 +128,7 @@ cudaError_t launch_runs_t(const BuildPlan &p, const MicroTable &T, const DeviceI
                           cudaStream_t s) {
     static std::atomic<int> per_sm_cache{0};
     auto kern = table_kernel<ALIGNED, MODE>;
-    if (per_sm_cache.load(std::memory_order_relaxed) == 0) {
-        const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     static_cast<int>(sizeof(TableSmem)));
-        if (err != cudaSuccess) return err;
-    }
+    static_assert(sizeof(TableSmem) <= kDefaultSmem, "no attribute needed");
     int per_sm;
     const cudaError_t err = occupancy_cached(kern, kUnit, per_sm_cache, per_sm, sizeof(TableSmem));
     if (err != cudaSuccess) return err;
@@ -172,14 +167,8 @@ cudaError_t launch_build_tables(const BuildPlan &p, const DeviceInfo &dev, cudaS
     const uint32_t row_ctas = split_rows(p.mlevels) ? (p.nmicro + kRowTile - 1) / kRowTile : 0u;
     if (block_ctas + row_ctas > 0u) {
         const size_t smem = row_ctas ? 2 * sizeof(Entry) * ((kRowTile + table_halo(p.mlevels) + 1u) & ~1u) : 0;
-        static std::atomic<bool> ready{false};
-        if (!ready.load(std::memory_order_relaxed)) {
-            // the longest halo: 1023
-            err = cudaFuncSetAttribute(rest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(2 * sizeof(Entry) * (kRowTile + 1024u)));
-            if (err != cudaSuccess) return err;
-            ready.store(true, std::memory_order_relaxed);
-        }
+        // the longest halo: 1023
+        static_assert(2 * sizeof(Entry) * (kRowTile + 1024u) <= kDefaultSmem, "no attribute needed");
         rest_kernel<<<block_ctas + row_ctas, kRestThreads, smem, s>>>(T, pb, p.st, p.nb, per_cta, block_ctas);
         err = cudaGetLastError();
         if (err != cudaSuccess) return err;

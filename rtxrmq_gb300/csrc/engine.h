@@ -66,6 +66,12 @@ cudaError_t pool_malloc(void **p, size_t bytes, int device, cudaStream_t s,
                         unsigned long long *pool_context);
 cudaError_t pool_trim(int device);
 
+// Dynamic shared memory that a launch may ask for without
+// cudaFuncAttributeMaxDynamicSharedMemorySize. Function attributes belong to a
+// device: what one device was told does not hold on the next.
+constexpr size_t kDefaultSmem = 48 * 1024;
+constexpr int kMaxDevices = 64;  // device_info refuses higher ordinals
+
 // Resident CTAs per SM of `kernel` at `threads` threads and `dynamic_smem`
 // bytes of dynamic shared memory, computed once per cache slot; concurrent
 // first callers compute and store the same value.

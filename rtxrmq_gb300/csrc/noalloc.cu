@@ -33,7 +33,6 @@ namespace {
 
 constexpr size_t kNoallocScratchBytes = static_cast<size_t>(RMQ_NOALLOC_SCRATCH_BYTES);
 
-constexpr int kMaxDevices = 64;
 std::mutex g_noalloc_mu;
 void *g_noalloc_ptr[kMaxDevices] = {nullptr};
 unsigned long long g_noalloc_ctx[kMaxDevices] = {0};

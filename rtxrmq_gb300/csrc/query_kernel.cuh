@@ -88,9 +88,9 @@ uint32_t grid_size(int64_t q, int64_t per_block, int per_sm, const DeviceInfo &d
 template <bool ALIGNED, bool MICRO, uint32_t MODE, bool STATS, bool LEAD>
 cudaError_t launch_query_t(const V1View &v, const QueryOut &o, int64_t q,
                            unsigned long long *stats, const DeviceInfo &dev, cudaStream_t s) {
-    static std::atomic<int> per_sm_cache{0};
+    static std::atomic<int> per_sm_cache[kMaxDevices] = {};  // the carve-out is set per device
     auto kern = query_kernel<ALIGNED, MICRO, MODE, STATS, LEAD>;
-    int per_sm = per_sm_cache.load(std::memory_order_relaxed);
+    int per_sm = per_sm_cache[dev.device].load(std::memory_order_relaxed);
     if (per_sm == 0) {
         cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, 0);
         if (err != cudaSuccess) return err;
@@ -102,7 +102,7 @@ cudaError_t launch_query_t(const V1View &v, const QueryOut &o, int64_t q,
         err = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                                    carveout_percent(per_sm * (sizeof(MissQueue<MICRO>) * (kThreads / 32) + 1024)));
         if (err != cudaSuccess) return err;
-        per_sm_cache.store(per_sm, std::memory_order_relaxed);
+        per_sm_cache[dev.device].store(per_sm, std::memory_order_relaxed);
     }
     kern<<<grid_size(q, kThreads * kQPT, per_sm, dev), kThreads, 0, s>>>(v, o, q, stats);
     return cudaGetLastError();
