@@ -44,6 +44,13 @@ def _stream_handle(stream) -> Optional[int]:
     return stream.cuda_stream
 
 
+def _current_handle(device: int) -> int:
+    """Handle of a device's current stream, CUDA being initialised (0.06 us;
+    torch.cuda.current_stream() takes 2.9 to make an object of it)."""
+    import torch
+    return torch._C._cuda_getCurrentRawStream(device)
+
+
 def _durable_stream(stream):
     """(handle, object or None): the object when the stream outlives its
     Python wrapper (the default stream and torch's pool streams are never
@@ -131,7 +138,7 @@ class RMQIndex:
             out_idx = None
         elif out_idx is None:
             out_idx = torch.empty(q, dtype=torch.int32, device=queries.device)
-        s = torch.cuda.current_stream().cuda_stream if stream is None else _stream_handle(stream)
+        s = _current_handle(torch.cuda.current_device()) if stream is None else _stream_handle(stream)
         if s != self._one_stream:
             self._one_stream = None
         check(load().rmq_query(self._h, _dptr(queries), q, _dptr(out_val), _dptr(out_idx), s))
@@ -156,6 +163,7 @@ class RMQIndex:
         q = len(queries)
         if tuple(queries.shape[1:]) != (2,):
             raise ValueError("queries must have shape [q, 2]")
+        self._keep = None  # the host reads the results: close() waits
         check(load().rmq_query_host(self._h, hptr(queries), q, hptr(out_val), hptr(out_idx),
                                     self._use(stream)))
 
@@ -217,14 +225,28 @@ class RMQIndex:
         return self._h.value or 0
 
     def close(self) -> None:
-        """Release the index: in stream order when every call on it ran on one
-        stream that still exists, else after all work of the device."""
+        """Release the index. Without waiting, in the order of the stream that is
+        current now, when every call on the index ran on that stream, none wrote
+        to the host, and ``values`` is torch's own memory, which is then kept
+        from reuse until the stream's work so far is done. Else after all work of
+        the device. Queries and outputs follow torch's rules for tensors used on
+        another stream than their own."""
         if getattr(self, "_h", None) is not None and self._h.value:
             h, self._h = self._h, C.c_void_p()
-            if self._keep is not None and self._one_stream is not None:
+            if self._in_stream_order():
+                self._values.record_stream(self._keep)
                 check(load().rmq_free_async(h, self._one_stream))
             else:
                 check(load().rmq_free(h))
+
+    def _in_stream_order(self) -> bool:
+        if self._keep is None or self._one_stream is None:
+            return False
+        # another current device is rmq_free_async's to see. Memory that is not
+        # torch's (a storage of a foreign buffer cannot be resized) is given back by
+        # its owner as soon as the tensor is gone.
+        return (_current_handle(self._keep.device_index) == self._one_stream and
+                self._values.untyped_storage().resizable())
 
     def __enter__(self):
         return self
