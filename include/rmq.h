@@ -364,8 +364,8 @@ int rmq_batch_create(int32_t narrays, const int64_t *h_starts,
  * CTA takes in the query phase) and each sparse-table level into items of
  * level_chunk entries (the unit of the table phase). Values <= 0 mean the
  * defaults (bs as rmq_batch_create, 4096 queries, fewer in a plan that has
- * not that many for every CTA, 4096 entries). The
- * reference has no batched form, so no counterpart.
+ * not that many for every CTA, 4096 entries), a query_chunk above 2^29 means
+ * 2^29. The reference has no batched form, so no counterpart.
  */
 typedef struct rmq_batch_tile {
     int32_t bs;

@@ -264,7 +264,9 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
         const rmq_batch_tile_t t = h_bucket_tiles ? h_bucket_tiles[i] : rmq_batch_tile_t{0, 0, 0, 0};
         b->bucket_bs[i] = t.bs > 0 ? t.bs : 0;
         b->tiles[i].bs = b->bucket_bs[i];
-        b->tiles[i].query_chunk = t.query_chunk > 0 ? t.query_chunk : static_cast<int32_t>(kQueryChunk);
+        // items are numbered query by query below 2^30 (MissQueue)
+        b->tiles[i].query_chunk = t.query_chunk > 0 ? std::min(t.query_chunk, kMostQueryChunk)
+                                                    : static_cast<int32_t>(kQueryChunk);
         b->tiles[i].level_chunk = t.level_chunk > 0 ? t.level_chunk : static_cast<int32_t>(kLevelChunk);
         b->tiles[i].reserved = 0;
     }

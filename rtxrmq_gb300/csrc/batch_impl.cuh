@@ -54,6 +54,7 @@ constexpr int kMaxSteps = 16;
 // 1e6, 1 million queries: 160 and 66).
 constexpr uint32_t kRunUnits = 32;
 constexpr uint32_t kLeastQueryChunk = 512;  // one step of a CTA
+constexpr int32_t kMostQueryChunk = 1 << 29;
 // positions per item of rows made apart, and the largest block table that one
 // item takes through all its levels: both fit the run's shared memory
 constexpr uint32_t kBatchRowTile = 1024;
