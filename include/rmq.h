@@ -388,7 +388,8 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts,
                         const rmq_batch_tile_t *h_bucket_tiles, uint32_t flags,
                         rmq_batch_t **out);
 
-/* The plan's tile per bucket (RMQ_BATCH_BUCKETS entries, defaults filled in). */
+/* The plan's tile per bucket (RMQ_BATCH_BUCKETS entries): chunks as the plan was
+ * cut, defaults filled in; bs as asked for, 0 for the default. */
 int rmq_batch_tiles(const rmq_batch_t *b, rmq_batch_tile_t *h_bucket_tiles);
 
 /* Build every array and answer every query: one cooperative launch. */

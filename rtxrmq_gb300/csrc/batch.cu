@@ -265,8 +265,7 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
         b->bucket_bs[i] = t.bs > 0 ? t.bs : 0;
         b->tiles[i].bs = b->bucket_bs[i];
         // items are numbered query by query below 2^30 (MissQueue)
-        b->tiles[i].query_chunk = t.query_chunk > 0 ? std::min(t.query_chunk, kMostQueryChunk)
-                                                    : static_cast<int32_t>(kQueryChunk);
+        b->tiles[i].query_chunk = std::min(t.query_chunk, kMostQueryChunk);  // 0: below, from the plan's queries
         b->tiles[i].level_chunk = t.level_chunk > 0 ? t.level_chunk : static_cast<int32_t>(kLevelChunk);
         b->tiles[i].reserved = 0;
     }
@@ -293,6 +292,9 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
         static_cast<uint32_t>(std::clamp<int64_t>(all_units / ctas, 1, kRunUnits));
     const uint32_t default_chunk = static_cast<uint32_t>(
         std::clamp<int64_t>(all_q / ctas, kLeastQueryChunk, kQueryChunk));
+    for (int i = 0; i < RMQ_BATCH_BUCKETS; ++i)
+        if (!h_bucket_tiles || h_bucket_tiles[i].query_chunk <= 0)
+            b->tiles[i].query_chunk = static_cast<int32_t>(default_chunk);
     for (int32_t i = 0; i < narrays; ++i) {
         const int64_t n = h_lengths[i], s = h_starts[i];
         const int64_t qs = h_qstarts[i], qc = h_qcounts[i];
@@ -307,8 +309,7 @@ int rmq_batch_create_ex(int32_t narrays, const int64_t *h_starts, const int64_t 
         const int bk = n > 0 ? bucket_of(n) : 0;
         int64_t bs = n > 0 ? b->bucket_bs[bk] : 1;
         if (bs <= 0) bs = kDefaultBatchBs;
-        const bool chunk_set = h_bucket_tiles && h_bucket_tiles[bk].query_chunk > 0;
-        const uint32_t qchunk = chunk_set ? static_cast<uint32_t>(b->tiles[bk].query_chunk) : default_chunk;
+        const uint32_t qchunk = static_cast<uint32_t>(b->tiles[bk].query_chunk);
         const uint32_t lchunk = static_cast<uint32_t>(b->tiles[bk].level_chunk);
         BatchArray &a = b->h_arrays[i];
         std::memset(&a, 0, sizeof(a));
