@@ -174,18 +174,42 @@ cudaError_t pool_malloc(void **p, size_t bytes, int device, cudaStream_t s,
         }
     }
     cudaGetLastError();
-    cudaError_t err = dev_malloc(p, bytes);
-    if (err == cudaErrorMemoryAllocation && !fail_alloc()) {
-        // what the pool keeps may be what is missing
-        cudaGetLastError();
-        if (pool_trim(device) == cudaSuccess) err = dev_malloc(p, bytes);
-    }
-    return err;
+    return dev_malloc(p, bytes);
 }
 
 cudaError_t pool_trim(int device) {
     cudaMemPool_t pool = device_pool(device, device_context_id(device), false);
     return pool ? cudaMemPoolTrimTo(pool, 0) : cudaSuccess;
+}
+
+// Waits for all work of the current device as a cudaFree of the memory would,
+// which a capture in relaxed or thread-local mode allows. cudaDeviceSynchronize
+// fails while any stream of the device captures, and ends that capture.
+static cudaError_t wait_for_device() {
+    void *p = nullptr;
+    const cudaError_t err = cudaMalloc(&p, sizeof(unsigned long long));
+    if (err == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return cudaDeviceSynchronize();
+    }
+    return err == cudaSuccess ? cudaFree(p) : err;
+}
+
+cudaError_t dev_malloc(void **p, size_t bytes) {
+    *p = nullptr;
+    if (fail_alloc()) return cudaErrorMemoryAllocation;
+    cudaError_t err = cudaMalloc(p, bytes);
+    int device = 0;
+    if (err != cudaErrorMemoryAllocation || cudaGetDevice(&device) != cudaSuccess ||
+        !device_pool(device, device_context_id(device), false))
+        return err;
+    cudaGetLastError();
+    // what was freed in stream order can go back when the work before it is done;
+    // waited for as in wait_for_device, which must not end a capture here
+    void *word = nullptr;
+    if (cudaMalloc(&word, sizeof(unsigned long long)) == cudaSuccess) cudaFree(word);
+    cudaGetLastError();
+    return pool_trim(device) == cudaSuccess ? cudaMalloc(p, bytes) : err;
 }
 
 int device_info(DeviceInfo *out) {
@@ -726,19 +750,6 @@ int rmq_query_host(const rmq_handle_t *h, const int32_t *h_queries, int64_t q, f
     if (err == cudaSuccess) err = cudaStreamWaitEvent(stream, hm->ev_end, 0);
     if (err != cudaSuccess) return cuda_fail(err, "rmq_query_host");
     return RMQ_OK;
-}
-
-// Waits for all work of the current device as a cudaFree of the memory would,
-// which a capture in relaxed or thread-local mode allows. cudaDeviceSynchronize
-// fails while any stream of the device captures, and ends that capture.
-static cudaError_t wait_for_device() {
-    void *p = nullptr;
-    const cudaError_t err = cudaMalloc(&p, sizeof(unsigned long long));
-    if (err == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        return cudaDeviceSynchronize();
-    }
-    return err == cudaSuccess ? cudaFree(p) : err;
 }
 
 int rmq_free(rmq_handle_t *h) {

@@ -38,17 +38,12 @@ struct NvtxRange {
     NvtxRange &operator=(const NvtxRange &) = delete;
 };
 
-// Every device allocation of the library goes through here. Fault
-// injection for tests: with RTXRMQ_FAIL_ALLOC=1 in the environment it
-// fails as an out-of-memory would, without touching the device.
-inline cudaError_t dev_malloc(void **p, size_t bytes) {
-    const char *f = std::getenv("RTXRMQ_FAIL_ALLOC");
-    if (f && f[0] == '1') {
-        *p = nullptr;
-        return cudaErrorMemoryAllocation;
-    }
-    return cudaMalloc(p, bytes);
-}
+// Every device allocation of the library goes through here. Memory that the
+// pool below keeps counts as free: when there is no other, it is given back
+// and the allocation tried again. Fault injection for tests: with
+// RTXRMQ_FAIL_ALLOC=1 in the environment it fails as an out-of-memory would,
+// without touching the device.
+cudaError_t dev_malloc(void **p, size_t bytes);
 
 // Id of the calling thread's current context, 0 when there is none or the
 // driver cannot tell.

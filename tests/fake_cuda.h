@@ -24,6 +24,7 @@ size_t left = ~size_t(0);  // bytes that cudaMalloc still has
 unsigned long long context[2] = {11, 12};  // ids of the devices' contexts
 std::map<void *, size_t> held;
 struct Pool { int device; unsigned long long context; size_t keeps; };
+std::map<void *, Pool *> pooled;
 inline void note(const std::string &s) { log += s + " "; }
 inline std::string take() { std::string s; s.swap(log); return s; }
 inline cudaError_t unsafe(const char *) {  // potentially unsafe under a global capture
@@ -62,6 +63,8 @@ cudaError_t cudaMallocFromPoolAsync(void **p, size_t n, cudaMemPool_t pool, cuda
     if (n > fake::left) return cudaErrorMemoryAllocation;
     fake::note("pool" + std::to_string(f->device));
     fake::held[*p = std::calloc(1, n)] = n;
+    fake::left -= n;
+    fake::pooled[*p] = reinterpret_cast<fake::Pool *>(pool);
     return cudaSuccess;
 }
 cudaError_t cudaMemPoolTrimTo(cudaMemPool_t pool, size_t) {
@@ -80,6 +83,7 @@ cudaError_t cudaMalloc(void **p, size_t n) {
     if (n > fake::left) return cudaErrorMemoryAllocation;
     if (n > 4096) fake::note("malloc" + std::to_string(fake::device));
     fake::held[*p = std::calloc(1, n)] = n;
+    fake::left -= n;
     return cudaSuccess;
 }
 cudaError_t cudaFree(void *p) {  // waits for the device, in any capture but a global one
@@ -91,12 +95,16 @@ cudaError_t cudaFree(void *p) {  // waits for the device, in any capture but a g
         return cudaErrorInvalidValue;
     }
     fake::note((it->second > 4096 ? "free" : "wait") + std::to_string(fake::device));
+    (fake::pooled.count(p) ? fake::pooled[p]->keeps : fake::left) += it->second;
+    fake::pooled.erase(p);
     fake::held.erase(it);
     std::free(p);
     return cudaSuccess;
 }
 cudaError_t cudaFreeAsync(void *p, cudaStream_t s) {
     fake::note("free-async" + std::to_string(fake::device) + (s ? "s" : ""));
+    fake::pooled[p]->keeps += fake::held[p];
+    fake::pooled.erase(p);
     fake::held.erase(p);
     std::free(p);
     return cudaSuccess;
@@ -109,6 +117,7 @@ cudaError_t cudaDeviceSynchronize(void) {
     fake::note("wait" + std::to_string(fake::device));
     return cudaSuccess;
 }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void *, int, size_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaGetDriverEntryPointByVersion(const char *name, void **f, unsigned, unsigned long long,
                                              cudaDriverEntryPointQueryResult *st) {
@@ -120,9 +129,14 @@ cudaError_t cudaGetDriverEntryPointByVersion(const char *name, void **f, unsigne
 }
 
 namespace rmq {
-size_t plan_index(BuildPlan &p, bool, bool) { return size_t(p.n) * 4; }
+size_t plan_index(BuildPlan &p, bool no_micro, bool) {
+    p.micro = !no_micro;
+    return size_t(p.n) * 4;
+}
 unsigned long long *place_index(BuildPlan &, void *base) { return static_cast<unsigned long long *>(base); }
 cudaError_t launch_build(const BuildPlan &, const DeviceInfo &, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_build_entries(const BuildPlan &, const DeviceInfo &, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_probe_gather(const BuildPlan &, const QueryArgs &, const DeviceInfo &, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_query(const BuildPlan &, const QueryArgs &, const DeviceInfo &, cudaStream_t) { return cudaSuccess; }
 }  // namespace rmq
 

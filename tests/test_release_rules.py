@@ -1,6 +1,7 @@
 """CPU: the rules of api.cu about index memory, run against a CUDA runtime on the
 host (fake_cuda.h): whose order a release follows, that a waiting one leaves
-captures alone, and that a pool ends with its context."""
+captures alone, that a pool ends with its context, and that what it keeps counts as
+free."""
 import subprocess
 from pathlib import Path
 
@@ -89,4 +90,23 @@ def test_pool_ends_with_its_context(tmp_path):
     EXPECT(index_of(0) && fake::take() == "pool0 ");
     fake::device = 1;
     EXPECT(rmq_free_async(c, nullptr) == RMQ_OK && fake::take() == "free-async1 ");
+""")
+
+
+def test_kept_memory_counts_as_free(tmp_path):
+    """Memory that the pool keeps from released indexes goes to any allocation of
+    the library that finds no other, after the work before the release; injected
+    failures stay failures."""
+    run(tmp_path, r"""
+    static int32_t queries[2], out[1];
+    fake::left = 2100000;
+    rmq_handle_t *a = index_of(0), *b = index_of(0);  // 400 kB each
+    EXPECT(a && b && rmq_free_async(a, nullptr) == RMQ_OK);
+    EXPECT(fake::left < 1600000 && fake::take() == "create0 pool0 pool0 free-async0 ");
+    EXPECT(rmq_probe_gather(b, queries, 1, nullptr, out, nullptr) == RMQ_OK);  // entries of 1.6 MB
+    EXPECT(fake::take() == "wait0 trim0 malloc0 ");
+    EXPECT(rmq_free(b) == RMQ_OK);
+    fake::take();
+    setenv("RTXRMQ_FAIL_ALLOC", "1", 1);
+    EXPECT(!index_of(0) && fake::take() == "");
 """)
