@@ -277,7 +277,8 @@ int rmq_probe_gather(const rmq_handle_t *h, const int32_t *d_queries, int64_t q,
  *   [0] settled by the probe of the small table over every unit (block or
  *       32-element micro-block) the query touches: the best of that
  *       superset lay inside [l, r]
- *   [1] settled by a narrower probe plus one end part
+ *   [1] settled by a narrower probe plus one end part, or, where many queries
+ *       are tied with the start of l's block, by one mask and no end part
  *   [2] the three-part decomposition (two end parts, probe of the middle)
  *   [3] inside one micro-block: its line of values is scanned
  *   [4] inside one block without the sub-block level: an edge entry

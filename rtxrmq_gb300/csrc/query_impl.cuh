@@ -247,7 +247,7 @@ __device__ __forceinline__ void load_queries(const QueryOut &o, int64_t base, in
 // kernels compile them out.
 enum QStat : int {
     kStatFirst = 0,   // settled by the superset probe
-    kStatSecond,      // settled by the second probe and one end part
+    kStatSecond,      // settled by a second probe and one end part, or by one mask (tied_entry)
     kStatFull,        // three-part decomposition: two end parts and a middle probe
     kStatMicroScan,   // inside one micro-block: its line of values is scanned
     kStatBlockEdge,   // one block, no sub-block level: pre / suf at a block edge
@@ -538,7 +538,7 @@ __device__ __forceinline__ Entry finish_entries(const V1View &v, bool left, uint
 // place in l's block nearly always lies before l, and every query of the block
 // tables is open. The best of the micro-blocks from l's on that one mask
 // covers answers such a query when it has the value that the probe found and
-// lies at or after l. A warp looks for it when many of its 64 queries are open:
+// lies at or after l; no end part is read. A warp looks for it when many of its 64 queries are open:
 // of distinct values few are, and none of those is answered this way (n = 2^27,
 // values of 256, 2^26 ranges of 2^16: 2.70 ms, so 0.94; n = 4.5e7, 2^23 ranges of
 // uniform length: 0.33 and 0.14).
@@ -885,10 +885,7 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
                     put_result(o, base + threadIdx.x + k * THREADS, x, MODE, lead);
                     if (k) miss[1] = false;
                     else miss[0] = false;
-                    if constexpr (STATS) {
-                        s.c[kStatSecond] += 1u;
-                        if (!v.light) s.c[kStatEntries] += 1u;
-                    }
+                    if constexpr (STATS) s.c[kStatSecond] += 1u;
                 }
             }
         }
