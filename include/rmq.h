@@ -298,6 +298,17 @@ int rmq_query_stats(const rmq_handle_t *h, const int32_t *d_queries, int64_t q,
                     rmq_stream_t stream);
 
 /*
+ * rmq_query_stats with options. RMQ_STATS_OWN_TABLES: with the sub-block level,
+ * counts on the tables that rmq_query reads, in place of ones in blocks of bs, and
+ * end parts by the 32-byte sectors of their lines ([8]; [6] stays 0): what the
+ * launch of rmq_query on the same queries reads. flags 0: rmq_query_stats.
+ */
+#define RMQ_STATS_OWN_TABLES 1u
+int rmq_query_stats_ex(const rmq_handle_t *h, const int32_t *d_queries, int64_t q,
+                       float *d_val, int32_t *d_idx, int64_t *h_counts,
+                       uint32_t flags, rmq_stream_t stream);
+
+/*
  * Measurement helper, no reference counterpart: the random-access rate of
  * the GPU for this query stream, independent of any index layout. One
  * launch with rmq_query's grid, query stream and output stores, and per

@@ -184,15 +184,18 @@ class RMQIndex:
     STATS_FIELDS = ("first_probe", "second_probe", "full", "micro_scan", "block_edge",
                     "warp_scan", "entries", "table_words", "scan_sectors", "invalid")
 
-    def query_stats(self, queries, out_val=None, out_idx=None, stream=None) -> dict:
+    def query_stats(self, queries, out_val=None, out_idx=None, stream=None,
+                    own: bool = False) -> dict:
         """rmq_query_stats: the same answers as query() (into out_val /
         out_idx when given) from the counting instantiation of the query
         kernel, and how every query was settled and what it read (field
-        names in STATS_FIELDS). Synchronises the stream."""
+        names in STATS_FIELDS), on tables in blocks of the bs asked for, or with
+        own=True (RMQ_STATS_OWN_TABLES) on the ones that query() reads.
+        Synchronises the stream."""
         q = _check_queries(queries)
         counts = (C.c_int64 * len(self.STATS_FIELDS))()
-        check(load().rmq_query_stats(self._h, _dptr(queries), q, _dptr(out_val), _dptr(out_idx),
-                                     counts, self._use(stream)))
+        check(load().rmq_query_stats_ex(self._h, _dptr(queries), q, _dptr(out_val), _dptr(out_idx),
+                                        counts, int(bool(own)), self._use(stream)))
         return dict(zip(self.STATS_FIELDS, (int(x) for x in counts)))
 
     def save(self, path, stream=None) -> None:

@@ -79,6 +79,7 @@ SIGNATURES = {
     "rmq_query_scan": (C.c_int, [_vp, _i64, _vp, _i64, _vp, _vp, _vp]),
     "rmq_probe_gather": (C.c_int, [_vp, _vp, _i64, _vp, _vp, _vp]),
     "rmq_query_stats": (C.c_int, [_vp, _vp, _i64, _vp, _vp, C.POINTER(_i64), _vp]),
+    "rmq_query_stats_ex": (C.c_int, [_vp, _vp, _i64, _vp, _vp, _vp, C.c_uint32, _vp]),
     "rmq_probe_random": (C.c_int, [_vp, _i64, _vp, _i64, _vp, _vp, _vp]),
     "rmq_checked_violations": (C.c_int, [C.POINTER(_i64)]),
     "rmq_batch_create": (C.c_int, [_i32, _vp, _vp, _vp, _vp, _vp, C.POINTER(_vp)]),

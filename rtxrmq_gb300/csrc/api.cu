@@ -492,8 +492,15 @@ int rmq_probe_gather(const rmq_handle_t *h, const int32_t *d_queries, int64_t q,
 
 int rmq_query_stats(const rmq_handle_t *h, const int32_t *d_queries, int64_t q, float *d_val,
                     int32_t *d_idx, int64_t *h_counts, rmq_stream_t stream) {
+    return rmq_query_stats_ex(h, d_queries, q, d_val, d_idx, h_counts, 0u, stream);
+}
+
+int rmq_query_stats_ex(const rmq_handle_t *h, const int32_t *d_queries, int64_t q, float *d_val,
+                       int32_t *d_idx, int64_t *h_counts, uint32_t flags, rmq_stream_t stream) {
     NvtxRange nvtx_range("rmq_query_stats");
     g_err[0] = '\0';
+    if (flags & ~RMQ_STATS_OWN_TABLES)
+        return set_error(RMQ_EINVAL, "rmq_query_stats_ex: unknown flags 0x%x", flags);
     if (!h || !h_counts) return set_error(RMQ_EINVAL, "rmq_query_stats: NULL argument");
     if (q < 0) return set_error(RMQ_EINVAL, "rmq_query_stats: q=%lld < 0", (long long)q);
     for (int c = 0; c < RMQ_QUERY_STATS_FIELDS; ++c) h_counts[c] = 0;
@@ -511,11 +518,13 @@ int rmq_query_stats(const rmq_handle_t *h, const int32_t *d_queries, int64_t q, 
                          h->device, dev.device);
     // A table index is counted on tables in blocks of its bs, made for the
     // call: the counts describe the decomposition asked for, while rmq_query
-    // takes its own block sizes.
+    // takes its own block sizes (counted with RMQ_STATS_OWN_TABLES).
     BuildPlan plan = h->plan;
     void *tables = nullptr;
     cudaError_t err = cudaSuccess;
-    if (plan.micro) {
+    if (plan.micro && (flags & RMQ_STATS_OWN_TABLES)) {
+        plan.light = true;  // end parts by their sectors
+    } else if (plan.micro) {
         err = dev_malloc(&tables, plan_index(plan, false, true));
         if (err != cudaSuccess) return cuda_fail(err, "rmq_query_stats: tables");
         place_index(plan, tables);
