@@ -5,10 +5,10 @@ plain RMQ over n = 1e8 float32 values uniform in [0,1) (seed 1321) with
 q = 2^26 inclusive (l, r) queries, values and leftmost indices both returned.
 The headline step is one rmq_query over the uniform-length queries (lr=-1);
 the other length modes of the same configuration (lr=-2, lr=-3, fixed
-len 2^10) are timed the same way and reported under "modes". Each mode's
-block size is the fastest of a sweep over every power of two in 2^10..2^16
-(the workload's range); the sweep also covers 2^7..2^9, reported apart as
-"best_below_2^10".
+len 2^10) are timed the same way and reported under "modes". The index takes
+its blocks from the number of elements, so the block size it is asked for (the
+default, or --bs) makes no difference; "bs_sweep_rmq_s" shows that over the
+workload's range 2^10..2^16, and nothing is chosen from it.
 
 Inputs are generated here with numpy (same seeds for both arms), so the
 reference arm never loads this package.
@@ -21,11 +21,11 @@ e2e        -- the same step through the C ABI with host buffers
               NVLink-C2C, all inside the timed region.
 roofline   -- algorithmic HBM bytes per launch / kernel time against the
               measured copy bandwidth. The bytes are the query read and the
-              result write (16 B per query) plus 32 B per end part and per
-              32-byte sector of values the kernel must read, counted for
-              this query set by rmq_query_stats (the kernel's counting
-              instantiation). The small-table probes are L2-resident and
-              reported apart, as is the un-pruned 80 B/query figure.
+              result write (16 B per query) plus 32 B per sector of values
+              that the launch reads, counted for this query set on the
+              index's own tables (rmq_query_stats_ex). The small-table
+              probes are L2-resident and reported apart, as is the
+              un-pruned 80 B/query figure.
 cpu_baseline -- the reference's CPU comparator HRMQ (restated in the
               oracle, hrmq_port.c) on this host's cores, on a bounded sample
               of the same queries.
@@ -59,7 +59,6 @@ N_QUERIES = 1 << 26
 SEED = 1321
 MODES = [("lr=-1", -1), ("lr=-2", -2), ("lr=-3", -3), ("len=2^10", 1024)]
 BS_RANGE = [1 << k for k in range(10, 17)]       # the workload's block-size range
-BS_BELOW = [1 << 7, 1 << 8, 1 << 9]              # extra: short ranges over small blocks
 TIE_N = 1 << 27
 TIE_LENGTHS = [1, 32, 1 << 10, 1 << 16, 1 << 22]
 PUBLISHED_LR1 = 3.52e8  # RTXRMQ alg 5, RTX 6000 Ada (csv-to-plot/perf-RTX6000ADA-ALG5.csv:1586-1601)
@@ -77,7 +76,7 @@ def parse():
     ap.add_argument("--q", type=int, default=N_QUERIES)
     ap.add_argument("--modes", default="all", help="comma list of lr values or 'all'")
     ap.add_argument("--no-cpu", action="store_true", help="skip the CPU baseline sample")
-    ap.add_argument("--bs", type=int, default=0, help="fixed block size (skips the sweep)")
+    ap.add_argument("--bs", type=int, default=0, help="block size the indexes are asked for (default 2^15; skips the sweep)")
     ap.add_argument("--no-e2e", action="store_true", help="skip the host-buffer end-to-end step")
     ap.add_argument("--skip-plain", action="store_true", help="skip the plain modes (headline)")
     ap.add_argument("--skip-tie", action="store_true", help="skip the tie-heavy configuration")
@@ -196,8 +195,8 @@ class ClockSampler:
 
 def stats_bytes(st: dict, q: int, out_bytes: int = 8) -> dict:
     """Algorithmic bytes of one query launch from the kernel's own counts
-    (rmq_query_stats): the query read and result write, plus one 32-byte
-    sector per end part and per scanned sector of values (random HBM); the
+    (query_stats(own=True)): the query read and result write, plus the 32-byte
+    sectors of values read, one for a per-element entry (random HBM); the
     small-table words are L2-resident and reported apart."""
     hbm = q * (8 + out_bytes) + 32 * (st["entries"] + st["scan_sectors"])
     valid = max(1, q - st["invalid"])
@@ -403,16 +402,14 @@ def graph_of(fn, stream):
     return g
 
 
-def sweep_block_sizes(R, dA, dQ, out_v, out_i, bs_list, stream, barrier, q, world):
-    """RMQ/s of every block size in bs_list (3 timed steps each)."""
+def sweep_block_sizes(R, dA, dQ, out_v, out_i, stream, barrier, q, world):
+    """RMQ/s at every block size of the workload's range (3 timed steps each)."""
     sweep = {}
-    for bs in bs_list:
-        if bs > dA.numel():
-            continue
+    for bs in BS_RANGE:
         with R.RMQIndex(dA, bs) as ix:
             fn = lambda: ix.query(dQ, out_val=out_v, out_idx=out_i)  # noqa: E731
             ms = time_steps(fn, 3, 1, stream, barrier)
-        sweep[bs] = q * world / (ms / 1e3)
+        sweep[str(bs)] = q * world / (ms / 1e3)
     return sweep
 
 
@@ -433,53 +430,30 @@ def timed_build(make, reps: int = 5):
     return ix, statistics.median(times)
 
 
-def pick(sweep, lo, hi):
-    cand = [(k, v) for k, v in sweep.items() if lo <= k <= hi]
-    return max(cand, key=lambda kv: kv[1]) if cand else None
-
-
 def bench_plain_mode(R, dA, n, Q, out_v, out_i, args, stream, barrier, world, dev, rbuf):
-    """One length mode of the headline configuration: block-size sweep, the
-    timed steps at the best block size of the workload's range, the kernel's
-    own counts, and the two random-access probes."""
+    """One length mode of the headline configuration: construction, the timed
+    steps, the counts of the same launch, and the two random-access probes."""
     import torch
 
     from rtxrmq_gb300.replicas import job_rate
     q = len(Q)
     dQ = torch.from_numpy(Q).to(dev)
-    if args.bs:
-        sweep, bs = {}, args.bs
-    else:
-        sweep = sweep_block_sizes(R, dA, dQ, out_v, out_i, BS_BELOW + BS_RANGE, stream, barrier,
-                                  q, world)
-        bs = pick(sweep, BS_RANGE[0], BS_RANGE[-1])[0]
+    sweep = None if args.bs else sweep_block_sizes(R, dA, dQ, out_v, out_i, stream, barrier, q, world)
+    bs = args.bs or R.DEFAULT_BS
     ix, construction_ms = timed_build(lambda: R.RMQIndex(dA, bs))
     fn = lambda: ix.query(dQ, out_val=out_v, out_idx=out_i)  # noqa: E731
     ms = time_steps(fn, args.steps, args.warmup, stream, barrier)
-    st = ix.query_stats(dQ)
+    st = ix.query_stats(dQ, own=True)
     acc = stats_bytes(st, q)
     res = {"value": job_rate(q, world, ms), "ms_per_step": ms, "ms_per_step_min": STEP_MIN[id(fn)],
-           "bs": bs, "bs_sweep_rmq_s": {str(k): v for k, v in sweep.items()},
-           "best_below_2^10": pick(sweep, 1, BS_RANGE[0] - 1),
-           "construction_ms": construction_ms, "query_stats": st, "accounting": acc,
+           "bs": bs, "bs_sweep_rmq_s": sweep, "construction_ms": construction_ms, "query_stats": st, "accounting": acc,
            "achieved_gbs": acc["alg_bytes"] / (ms / 1e3) / 1e9,
            "unpruned_achieved_gbs": acc["unpruned_alg_bytes"] / (ms / 1e3) / 1e9,
            "info": ix.info()}
-    # the light index (RMQ_BUILD_LIGHT) at the same block size: its
-    # construction, size and query time beside the full index's
-    if bs % 32 == 0 and bs >= 64:
-        lix, lc_ms = timed_build(lambda: R.RMQIndex(dA, bs, light=True))
-        lfn = lambda: lix.query(dQ, out_val=out_v, out_idx=out_i)  # noqa: E731
-        lms = time_steps(lfn, args.steps, args.warmup, stream, barrier)
-        res["light_index"] = {"rmq_s": job_rate(q, world, lms), "ms_per_step": lms,
-                              "construction_ms": lc_ms,
-                              "index_gb": lix.info()["struct_bytes"] / 1e9,
-                              "full_index_gb": res["info"]["struct_bytes"] / 1e9}
-        lix.close()
     # random-access probes with the query kernel's grid and query stream:
-    # two random 8-B lookups per query into this index's prefix / suffix
-    # tables (rmq_probe_gather), and into a 4 GiB buffer (rmq_probe_random,
-    # independent of the index layout)
+    # two random 8-B lookups per query into prefix / suffix minima per element
+    # in blocks of bs (rmq_probe_gather, which makes them), and into a 4 GiB
+    # buffer (rmq_probe_random, independent of the index layout)
     gfn = lambda: ix.probe_gather(dQ, out_val=out_v, out_idx=out_i)  # noqa: E731
     gms = time_steps(gfn, args.steps, args.warmup, stream, barrier)
     rfn = lambda: R.probe_random(rbuf, dQ, out_val=out_v, out_idx=out_i)  # noqa: E731
@@ -492,7 +466,7 @@ def bench_plain_mode(R, dA, n, Q, out_v, out_i, args, stream, barrier, world, de
         "probe_gather_ms": gms, "query_vs_probe_gather": gms / ms,
         "pattern": "per query: 8-B query read, two random 8-B loads, 8-B result write; "
                    "probe_random over a 4 GiB buffer (hashed positions), probe_gather at "
-                   "suf[l] / pre[r] of this index"}
+                   "suf[l] / pre[r]"}
     return res, ix, dQ
 
 
@@ -566,9 +540,8 @@ def bench_energy(fn, ms, q, local):
 
 def bench_tie_heavy(R, args, stream, barrier, world, rank, dev):
     """Tie-heavy configuration: n = 2^27 floats holding integers uniform in
-    [0, 256), q = 2^26 queries of each fixed length; bs swept over the
-    workload's range (2^10..2^16) per length. Bit-exactness at this size is
-    asserted by tests/test_gpu_fullscale.py."""
+    [0, 256), q = 2^26 queries of each fixed length. Bit-exactness at this size
+    is asserted by tests/test_gpu_fullscale.py."""
     import torch
 
     from rtxrmq_gb300.replicas import job_rate
@@ -581,15 +554,12 @@ def bench_tie_heavy(R, args, stream, barrier, world, rank, dev):
     for length in TIE_LENGTHS:
         Q = np_queries(q, n, length, query_seed(rank, length) + 5)
         dQ = torch.from_numpy(Q).to(dev)
-        sweep = sweep_block_sizes(R, dA, dQ, out_v, out_i, BS_RANGE, stream, barrier, q, world)
-        bs = pick(sweep, BS_RANGE[0], BS_RANGE[-1])[0]
-        with R.RMQIndex(dA, bs) as ix:
+        with R.RMQIndex(dA, args.bs) as ix:
             fn = lambda: ix.query(dQ, out_val=out_v, out_idx=out_i)  # noqa: E731
             ms = time_steps(fn, args.steps, args.warmup, stream, barrier)
-            st = ix.query_stats(dQ)
+            st = ix.query_stats(dQ, own=True)
         acc = stats_bytes(st, q)
-        res[f"len={length}"] = {"rmq_s": job_rate(q, world, ms), "ms_per_step": ms, "bs": bs,
-                                "bs_sweep_rmq_s": {str(k): v for k, v in sweep.items()},
+        res[f"len={length}"] = {"rmq_s": job_rate(q, world, ms), "ms_per_step": ms,
                                 "settled": acc["settled"],
                                 "alg_bytes_per_query": acc["alg_bytes_per_query"],
                                 "achieved_gbs": acc["alg_bytes"] / (ms / 1e3) / 1e9}
@@ -602,7 +572,7 @@ def bench_tie_heavy(R, args, stream, barrier, world, rank, dev):
 def bench_small(R, args, stream, barrier, world, rank, dev):
     """CPU-runnable configuration: n = 1e6 U[0,1), q = 2^20, lr=-3. Its
     working set fits in L2, so L2 is flushed (a 512 MB write) before every
-    timed step; bs swept over 2^7..2^16."""
+    timed step."""
     import torch
 
     from rtxrmq_gb300.replicas import job_rate
@@ -613,24 +583,16 @@ def bench_small(R, args, stream, barrier, world, rank, dev):
     out_v = torch.empty(q, dtype=torch.float32, device=dev)
     out_i = torch.empty(q, dtype=torch.int32, device=dev)
     flush = torch.empty(1 << 27, dtype=torch.float32, device=dev)
-    sweep = {}
-    for bs in BS_BELOW + BS_RANGE:
-        with R.RMQIndex(dA, bs) as ix:
-            fn = lambda: ix.query(dQ, out_val=out_v, out_idx=out_i)  # noqa: E731
-            ms, _ = time_steps_flushed(fn, 5, 1, stream, barrier, flush)
-        sweep[bs] = job_rate(q, world, ms)
-    bs = max(sweep.items(), key=lambda kv: kv[1])[0]
-    with R.RMQIndex(dA, bs) as ix:
+    with R.RMQIndex(dA, args.bs) as ix:
         fn = lambda: ix.query(dQ, out_val=out_v, out_idx=out_i)  # noqa: E731
         ms, best = time_steps_flushed(fn, args.steps, args.warmup, stream, barrier, flush)
-        st = ix.query_stats(dQ)
+        st = ix.query_stats(dQ, own=True)
     acc = stats_bytes(st, q)
     del dA, dQ, out_v, out_i, flush
     torch.cuda.empty_cache()
     return {"workload": "n=1e6 U[0,1), q=2^20, lr=-3 (lognormal 0.3 ln n), values+indices",
             "l2": "flushed (512 MB write) before every timed step: the working set fits in L2",
             "rmq_s": job_rate(q, world, ms), "ms_per_step": ms, "ms_per_step_min": best,
-            "bs": bs, "bs_sweep_rmq_s": {str(k): v for k, v in sweep.items()},
             "settled": acc["settled"], "alg_bytes_per_query": acc["alg_bytes_per_query"]}
 
 
@@ -682,41 +644,6 @@ def bench_batched(args, dev, stream, barrier):
         dms = time_steps(lambda: b.run(dV, dQ, ov, oi), args.steps, 1, stream, barrier)
     from rtxrmq_gb300.replicas import job_rate, world
     q, nr = w.total_q, world()[1]
-    # the light index on the same workload, its own tuned tiles; answers compared bit for bit with the full plan's
-    t = time.perf_counter()
-    lcfg = ([(max(64, args.batch_bs // 32 * 32), 0, 0)] * 32 if args.batch_bs else
-            autotune(w.starts, w.lengths, w.qstarts, w.qcounts, dV, dQ, reps=2,
-                     queries_host=w.queries, cache=None, tiles=True, light=True))
-    ltune_s = time.perf_counter() - t
-    with RMQBatch(w.starts, w.lengths, w.qstarts, w.qcounts, lcfg, light=True) as b:
-        linfo = b.info()
-        lfn = lambda: b.run(dV, dQ, ov, oi)  # noqa: E731
-        lms = time_steps(lfn, args.steps, args.warmup, stream, barrier)
-        lg = graph_of(lfn, stream)
-        lgms = time_steps(lg.replay, args.steps, args.warmup, stream, barrier)
-        lbms = time_steps(lambda: b.build(dV), args.steps, args.warmup, stream, barrier)
-        lqms = time_steps(lambda: b.query(dV, dQ, ov, oi), args.steps, args.warmup, stream,
-                          barrier)
-        lmatch = bool(torch.equal(i1, oi) and torch.equal(v1.view(torch.int32),
-                                                          ov.view(torch.int32)))
-        del lg
-    res["light_index"] = {
-        "batched_graph_rmq_s": job_rate(q, nr, lgms), "batched_graph_ms": lgms,
-        "batched_rmq_s": job_rate(q, nr, lms), "batched_ms": lms,
-        "build_only_ms": lbms, "query_only_ms": lqms, "autotune_s": ltune_s,
-        "workspace_gb": linfo["workspace_bytes"] / 1e9,
-        "matches_full_index": lmatch,
-        "speedup_vs_per_array": pms / lgms,
-        "bucket_tiles": {str(k): {"bs": v[0], "query_chunk": v[1], "level_chunk": v[2]}
-                         for k, v in enumerate(lcfg) if v[0]},
-        # one read of the values, 8 B per 32 elements of micro-block minima
-        "build_alg_bytes": int(w.lengths.sum()) * 4 + int(w.lengths.sum()) // 32 * 8}
-    # the faster plan of the two (same answers, checked above)
-    best_light = lgms < gms and lmatch
-    res["best"] = {"index": "light" if best_light else "full",
-                   "batched_graph_rmq_s": job_rate(q, nr, lgms if best_light else gms),
-                   "batched_graph_ms": lgms if best_light else gms,
-                   "speedup_vs_per_array": pms / (lgms if best_light else gms)}
     res.update({"batched_graph_rmq_s": job_rate(q, nr, gms), "batched_graph_ms": gms,
                 "batched_rmq_s": job_rate(q, nr, ms), "batched_ms": ms,
                 "per_array_rmq_s": job_rate(q, nr, pms), "per_array_ms": pms,
@@ -725,12 +652,10 @@ def bench_batched(args, dev, stream, barrier):
                 "per_array_matches_batched": match,
                 "build_only_ms": bms, "query_only_ms": qms,
                 "query_only_rmq_s": job_rate(q, nr, qms),
-                # bytes of one step of the un-pruned design: the build reads each
-                # value once and writes its prefix / suffix entries (4 + 16 B per
-                # element); each query reads its pair and writes 8 B, plus two random
-                # 32-B entry sectors; against the graph-launched step
-                "alg_bytes_per_step_unpruned": int(w.lengths.sum()) * 20 + q * 80,
-                "alg_gbs_unpruned": (int(w.lengths.sum()) * 20 + q * 80) / (gms / 1e3) / 1e9,
+                # bytes that one step cannot do without (each value read once, a query's
+                # pair read and 8 B written) against the graph-launched step
+                "alg_bytes_per_step": int(w.lengths.sum()) * 4 + q * 16,
+                "alg_gbs": (int(w.lengths.sum()) * 4 + q * 16) / (gms / 1e3) / 1e9,
                 "launches_per_step": {"batched": 1, "per_array": "one build + level + query "
                                       "launch sequence per array"}})
     del dV, dQ, ov, oi
@@ -833,7 +758,6 @@ def main():
 
     results = {}
     headline = None
-    ref_nb = {}
     tie = small = batched = autograd = None
     A = None
     sampler = ClockSampler(local)
@@ -860,19 +784,6 @@ def main():
                 results[name] = res
                 del dQ
             del rbuf
-            # the reference's own block sizes: its benchmark scripts pass --nb 512
-            # (lr=-1, -2) and --nb 8192 (lr=-3), bs = n / nb
-            # (scripts/perf-fulltest.sh:49-58, src/tools.h:129-132)
-            if not args.bs and args.modes == "all":
-                for name, lr, nb in (("lr=-1", -1, 512), ("lr=-2", -2, 512), ("lr=-3", -3, 8192)):
-                    bs = R.bs_from_nb(n, nb)
-                    dQ = torch.from_numpy(np_queries(q, n, lr, query_seed(rank, lr))).to(dev)
-                    with R.RMQIndex(dA, bs) as ix:
-                        fn = lambda: ix.query(dQ, out_val=out_v, out_idx=out_i)  # noqa: E731
-                        ms = time_steps(fn, max(3, args.steps // 2), 2, stream, barrier)
-                    ref_nb[name] = {"nb": nb, "bs": bs, "rmq_s": q * world / (ms / 1e3),
-                                    "ms_per_step": ms}
-                    del dQ
             del dA, out_v, out_i
             torch.cuda.empty_cache()
         if not args.skip_tie and args.modes == "all":
@@ -899,10 +810,6 @@ def main():
     achieved = h["achieved_gbs"]
     default, label, config = headline_config(n, q, lr)
     traffic, traffic_info = profiled_traffic(q) if default else (None, None)
-    if traffic_info and traffic_info.get("bs") not in (None, h["bs"]):
-        traffic_info["note"] = (f"captured at bs={traffic_info['bs']}; this run's bs={h['bs']} "
-                                "(lr=-1 traffic is the query stream and results at every bs "
-                                "in range)")
     line = {
         "metric": f"RMQ/s {label} (values+indices)",
         "value": h["value"], "unit": "RMQ/s", "n_gpus": world, "steps": args.steps,
@@ -926,8 +833,8 @@ def main():
                      "kernel": "query_kernel",
                      "alg_bytes_per_launch": h["accounting"]["alg_bytes"],
                      "alg_bytes_basis": "16 B per query (query read, value + index write) + 32 B "
-                                        "per end part read and per 32-B sector of values "
-                                        "scanned, counted by rmq_query_stats on this query set",
+                                        "per sector of values read, counted on this query set "
+                                        "and the launch's own tables (rmq_query_stats_ex)",
                      "l2_table_words_per_query": h["accounting"]["l2_table_words_per_query"],
                      "unpruned_alg_bytes_per_launch": h["accounting"]["unpruned_alg_bytes"],
                      "unpruned_achieved": h["unpruned_achieved_gbs"],
@@ -935,7 +842,6 @@ def main():
         "random_access_roofline": h.get("random_access"),
         "clocks": clocks,
         "modes": {k: {kk: vv for kk, vv in v.items() if kk not in ("info",)} for k, v in results.items()},
-        "modes_reference_nb": ref_nb,
         "energy": h.get("energy"),
         "tie_heavy": tie,
         "small_config": small,
