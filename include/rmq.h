@@ -53,14 +53,15 @@ typedef struct rmq_handle rmq_handle_t;
 
 typedef struct rmq_info {
     int64_t n;            /* elements                                   */
-    int64_t bs;           /* block size                                 */
-    int64_t nb;           /* blocks = ceil(n / bs)  (src/rtx.h:42)      */
-    int32_t levels;       /* sparse-table levels over the block minima  */
+    int64_t bs;           /* block size asked for                       */
+    int64_t nb;           /* ceil(n / bs) (src/rtx.h:42); an index with the
+                             sub-block level chooses its own blocks     */
+    int32_t levels;       /* sparse-table levels over nb blocks         */
     int32_t aligned;      /* 1 when d_vals is 16-byte aligned           */
-    int64_t table_bytes;  /* sparse table over the index's own blocks   */
+    int64_t table_bytes;  /* sparse tables over the index's own blocks  */
     int64_t struct_bytes; /* all device memory owned by the handle      */
     int32_t micro_levels; /* levels of a sub-block table that answers
-                             every query inside a block (0 = none)     */
+                             every query inside a block of bs (0 = none)*/
     int32_t light;        /* 1: light index (RMQ_BUILD_LIGHT)           */
     int64_t micro_table_bytes; /* micro-block minima + masks             */
     int32_t is_max;       /* 1: range maximum (RMQ_BUILD_MAX)           */

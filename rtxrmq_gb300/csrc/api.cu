@@ -26,7 +26,6 @@ struct rmq_handle {
     unsigned long long pool_context;  // mem comes from the library's pool in this context, 0: it does not
     bool captured;                  // a query was captured: a graph may still replay it
     unsigned long long *invalid;    // device counter of rejected queries
-    int64_t table_bytes;
     // rmq_probe_gather on a table index: the per-element entries it looks up
     // (pre, suf, then block minima), allocated and built by its first call
     // under host_mu
@@ -268,7 +267,6 @@ int handle_adopt(BuildPlan plan, void *mem, size_t bytes, cudaStream_t stream, r
     h->mem = mem;
     h->mem_bytes = bytes;
     h->invalid = place_index(plan, mem);
-    h->table_bytes = static_cast<int64_t>(sizeof(Entry) * static_cast<size_t>(plan.nb) * plan.levels);
     h->plan = plan;
     cudaError_t err = cudaMemsetAsync(h->invalid, 0, sizeof(unsigned long long), stream);
     if (err != cudaSuccess) {
@@ -363,7 +361,6 @@ int rmq_build_ex(const float *d_vals, int64_t n, int64_t bs, uint32_t flags, rmq
     }
     h->invalid = place_index(p, h->mem);
     h->mem_bytes = total;
-    h->table_bytes = static_cast<int64_t>(sizeof(Entry) * static_cast<size_t>(p.nb) * p.levels);
     h->plan = p;
 
     err = cudaMemsetAsync(h->invalid, 0, sizeof(unsigned long long), stream);
@@ -827,7 +824,9 @@ int rmq_info(const rmq_handle_t *h, rmq_info_t *info) {
     info->nb = nb;
     info->levels = static_cast<int32_t>(st_levels(nb));
     info->aligned = h->plan.aligned ? 1 : 0;
-    info->table_bytes = h->table_bytes;
+    info->table_bytes = static_cast<int64_t>(
+        sizeof(Entry) * (static_cast<size_t>(h->plan.nb) * h->plan.levels +
+                         static_cast<size_t>(h->plan.cnb) * h->plan.clevels));
     info->struct_bytes = static_cast<int64_t>(h->mem_bytes);
     // at least those of the micro table that blocks of bs would need
     info->micro_levels = static_cast<int32_t>(
