@@ -31,6 +31,11 @@ DEFAULT_CACHE = Path(os.environ.get("RTXRMQ_AUTOTUNE_CACHE",
                                     Path.home() / ".cache" / "rtxrmq_gb300" / "autotune.json"))
 
 
+# part of every cached choice's key: choices timed on another index structure or
+# another kernel do not hold
+_CACHE_VERSION = 2
+
+
 def _i64(a) -> np.ndarray:
     return np.ascontiguousarray(np.asarray(a, dtype=np.int64))
 
@@ -205,7 +210,7 @@ class RMQBatch:
 
 
 def _cache_keys(lengths, qstarts, qcounts, queries_host) -> dict:
-    """bucket -> key 'b<bucket>_q<log2 mean query length>'."""
+    """bucket -> key 'v<version>_b<bucket>_q<log2 mean query length>'."""
     keys = {}
     bk = bucket_of(lengths)
     for b in np.unique(bk):
@@ -221,7 +226,7 @@ def _cache_keys(lengths, qstarts, qcounts, queries_host) -> dict:
                     tot += float((q[:, 1] - q[:, 0] + 1).sum())
                     cnt += c
             qcls = str(int(round(np.log2(max(tot / max(cnt, 1), 1.0)))))
-        keys[int(b)] = f"b{int(b)}_q{qcls}"
+        keys[int(b)] = f"v{_CACHE_VERSION}_b{int(b)}_q{qcls}"
     return keys
 
 
@@ -233,7 +238,7 @@ def autotune(starts, lengths, qstarts, qcounts, vals, queries, *, reps: int = 3,
     entries per level item) triples (rmq_batch_autotune_ex), for plans with
     ``op`` and ``light`` (and the dtype of ``vals``).
 
-    Cached results (per GPU model and bucket/query-length key) are reused;
+    Cached results (per GPU model and version/bucket/query-length key) are reused;
     missing buckets are timed on the real data."""
     import torch
     starts, lengths = _i64(starts), _i64(lengths)
