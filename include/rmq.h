@@ -451,8 +451,9 @@ int rmq_batch_free(rmq_batch_t *b);
 /*
  * Per-size-bucket block-size autotuner: for every bucket present, times a
  * batch of that bucket's arrays and queries with each candidate block size
- * (64 .. 65536, up to twice the bucket's largest length) over `reps` runs
- * and writes the fastest to h_bucket_bs[bucket] (0 for absent buckets).
+ * (64 .. 16384, up to twice the bucket's largest length) over `reps` runs and
+ * writes the default, 4096, or one that is more than 3% faster, to
+ * h_bucket_bs[bucket] (0 for absent buckets).
  * Uses d_val / d_idx as scratch outputs; allocates and frees temporary plans.
  */
 int rmq_batch_autotune(int32_t narrays, const int64_t *h_starts,
@@ -464,12 +465,11 @@ int rmq_batch_autotune(int32_t narrays, const int64_t *h_starts,
 
 /*
  * rmq_batch_autotune over the whole tile: per bucket present, first the
- * block size (as rmq_batch_autotune; for a light plan 4096, 1024 or 16384,
- * another than 4096 only when it is more than 3% faster), then with it the
- * query-item size
+ * block size (as rmq_batch_autotune), then with it the query-item size
  * (512 .. 8192 queries) and then the level-item size (1024 .. 16384
- * entries), each the fastest over `reps` runs of a plan holding only that
- * bucket's arrays, built with `flags` (as rmq_batch_create_ex); absent
+ * entries), each over `reps` runs of a plan holding only that bucket's
+ * arrays, built with `flags` (as rmq_batch_create_ex), and another than the
+ * default (4096 each) only when it is more than 3% faster; absent
  * buckets get {0, 0, 0, 0}. Allocates and frees temporary plans; d_val /
  * d_idx are scratch outputs.
  */

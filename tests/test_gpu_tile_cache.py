@@ -32,3 +32,20 @@ def test_choices_of_another_version_are_timed_again(cuda, native, tmp_path):
     table[key] = [64, 7, 9]
     cache.write_text(json.dumps({dev: table}))
     assert autotune(*args, reps=1, cache=cache, tiles=True)[b] == (64, 7, 9)
+
+
+@pytest.mark.parametrize("light", [False, True])
+def test_candidates(cuda, native, light):
+    """One list of block sizes with and without the light flag, which changes no
+    structure, and none of them twice (above 2^15 the blocks are the default's)."""
+    import torch
+
+    from rtxrmq_gb300.batch import autotune
+    lengths = np.array([300, 5000, 90_000, 400_000, 700_000])
+    starts = np.cumsum(lengths) - lengths
+    qcounts = np.full(5, 300)
+    qstarts = np.cumsum(qcounts) - qcounts
+    A = torch.rand(int(lengths.sum()), device=cuda)
+    Q = torch.tensor([[10, 250]], dtype=torch.int32, device=cuda).repeat(1500, 1)
+    cfg = autotune(starts, lengths, qstarts, qcounts, A, Q, reps=1, cache=None, tiles=True, light=light)
+    assert {t[0] for t in cfg} <= {0, 64, 256, 1024, 4096, 16384}
