@@ -387,9 +387,8 @@ static void note_capture(const rmq_handle_t *h, cudaStream_t stream) {
         const_cast<rmq_handle_t *>(h)->captured = true;
 }
 
-int rmq_query(const rmq_handle_t *h, const int32_t *d_queries, int64_t q, float *d_val,
-              int32_t *d_idx, rmq_stream_t stream) {
-    NvtxRange nvtx_range("rmq_query");
+static int query_in_place(const rmq_handle_t *h, const int32_t *d_queries, int64_t q, float *d_val,
+                          int32_t *d_idx, bool host, rmq_stream_t stream) {
     g_err[0] = '\0';
     if (!h) return set_error(RMQ_EINVAL, "rmq_query: handle is NULL");
     if (q < 0) return set_error(RMQ_EINVAL, "rmq_query: q=%lld < 0", (long long)q);
@@ -413,10 +412,17 @@ int rmq_query(const rmq_handle_t *h, const int32_t *d_queries, int64_t q, float 
     a.val = d_val;
     a.idx = d_idx;
     a.invalid = h->invalid;
+    a.host = host;
     cudaError_t err = launch_query(h->plan, a, dev, stream);
     if (err != cudaSuccess) return cuda_fail(err, "rmq_query: launch");
     note_capture(h, stream);
     return RMQ_OK;
+}
+
+int rmq_query(const rmq_handle_t *h, const int32_t *d_queries, int64_t q, float *d_val,
+              int32_t *d_idx, rmq_stream_t stream) {
+    NvtxRange nvtx_range("rmq_query");
+    return query_in_place(h, d_queries, q, d_val, d_idx, false, stream);
 }
 
 // The plan of a handle with pre / suf present. A table index has none: the
@@ -669,7 +675,9 @@ int rmq_query_host(const rmq_handle_t *h, const int32_t *h_queries, int64_t q, f
     const bool v_stage = h_val && !vdev;
     const bool i_stage = h_idx && !idev;
     if (qdev && !v_stage && !i_stage)
-        return rmq_query(h, reinterpret_cast<const int32_t *>(qdev), q, vdev, idev, stream);
+        return query_in_place(h, reinterpret_cast<const int32_t *>(qdev), q, vdev, idev,
+                              (vdev && !is_device_memory(h_val)) || (idev && !is_device_memory(h_idx)),
+                              stream);
 
     DeviceInfo dev;
     int rc = device_info(&dev);
@@ -861,7 +869,7 @@ int rmq_checked_violations(int64_t *count) {
     if (!RMQ_CHECKED)
         return set_error(RMQ_ENOTSUP, "rmq_checked_violations: not a checked build (RMQ_CHECKED=1)");
     const unsigned long long parts[] = {violations_build(), violations_query(), violations_batch(),
-                                        violations_query_lead(), violations_batch_unaligned(),
+                                        violations_query_lead(), violations_query_host(), violations_batch_unaligned(),
                                         violations_persist()};
     for (unsigned long long v : parts) {
         if (v == ~0ull) return set_error(RMQ_ECUDA, "rmq_checked_violations: counter read failed");

@@ -89,6 +89,7 @@ unsigned long long violations_build();
 unsigned long long violations_query();
 unsigned long long violations_batch();
 unsigned long long violations_query_lead();
+unsigned long long violations_query_host();
 unsigned long long violations_batch_unaligned();
 unsigned long long violations_persist();
 
@@ -247,6 +248,7 @@ struct QueryArgs {
     // measurement launches only (rmq_query_stats): kStatCount device
     // counters of how each query was settled; null for every other launch
     unsigned long long *stats = nullptr;
+    bool host = false;  // val and idx, or one of them, are in host memory
 };
 cudaError_t launch_query(const BuildPlan &p, const QueryArgs &a, const DeviceInfo &dev,
                          cudaStream_t s);

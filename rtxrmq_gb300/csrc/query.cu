@@ -153,6 +153,10 @@ cudaError_t launch_query_s(const BuildPlan &p, const V1View &v, const QueryOut &
 cudaError_t launch_query_lead(const BuildPlan &p, const V1View &v, const QueryOut &o, int64_t q,
                               const DeviceInfo &dev, cudaStream_t s);
 
+// Results in host memory (query_host.cu).
+cudaError_t launch_query_host(const BuildPlan &p, const V1View &v, const QueryOut &o, int64_t q,
+                              const DeviceInfo &dev, cudaStream_t s);
+
 cudaError_t launch_query(const BuildPlan &p, const QueryArgs &a, const DeviceInfo &dev,
                          cudaStream_t s) {
     if (a.q <= 0) return cudaSuccess;
@@ -164,6 +168,7 @@ cudaError_t launch_query(const BuildPlan &p, const QueryArgs &a, const DeviceInf
     o.invalid = a.invalid;
     o.span = a.q;
     if (p.lead != 0u) return launch_query_lead(p, v, o, a.q, dev, s);
+    if (a.host && p.micro) return launch_query_host(p, v, o, a.q, dev, s);
     if (a.stats) return launch_query_s<true>(p, v, o, a.q, a.stats, dev, s);
     return launch_query_s<false>(p, v, o, a.q, nullptr, dev, s);
 }

@@ -593,15 +593,21 @@ __device__ __forceinline__ Entry short_range(const V1View &v, uint32_t l, uint32
 // 1e8, uniform lengths, bs 2^14: 0.36 and 0.45 ms). `id` numbers the queries
 // of the CTA in the order it takes them: step * step size + place in the
 // step.
-template <bool MICRO>
+template <bool MICRO, bool WHOLE = false>
 struct MissQueue {
     static constexpr int kCap = 64;
-    uint4 stage[MICRO ? kStageLines * 8 : 1];
+    uint4 stage[MICRO ? kStageLines * 8 : 1];  // on a 128-byte boundary (staged_line)
     uint32_t l[kCap];    // kMissLeft set: the probe's best lay left of l
     uint32_t r[kCap];    // kSecond set: back for its other end
     uint32_t id[kCap];   // below 2^30
     uint32_t key[MICRO ? kCap : 1];
 };
+template <>
+struct MissQueue<true, true> : MissQueue<true, false> {
+    Entry done[kCap];  // answers of the step's queued queries
+};
+static_assert(sizeof(MissQueue<true>) % 128 == 0 && sizeof(MissQueue<true, true>) % 128 == 0,
+              "the stages of all warps lie on 128-byte boundaries");
 constexpr uint32_t kMissLeft = 0x80000000u;  // above every index
 // A query back for its other end has the best of the end that is settled in
 // its entry: its key, its index in place of that end's position (it lies in
@@ -626,9 +632,10 @@ struct StepMap {
 // rarely, it joins the queue again, for the units between both ends and its
 // part at the other end: few lanes in a warp need that, so doing it at once
 // would cost every drain a second pass.
-template <bool ALIGNED, bool MICRO, uint32_t MODE, bool STATS, bool LEAD, int THREADS, int QPT>
+template <bool ALIGNED, bool MICRO, uint32_t MODE, bool STATS, bool LEAD, int THREADS, int QPT,
+          bool WHOLE>
 __device__ __forceinline__ void drain_misses(const V1View &v, const QueryOut &o,
-                                             const StepMap &map, MissQueue<MICRO> &mq,
+                                             const StepMap &map, MissQueue<MICRO, WHOLE> &mq,
                                              uint32_t &count, uint64_t pol, QStats &s) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t take = count < 32u ? count : 32u;
@@ -682,7 +689,12 @@ __device__ __forceinline__ void drain_misses(const V1View &v, const QueryOut &o,
         }
         res = better(res, line_entry<MODE>(best, line, bits));
     }
-    if (act && !again) put_result(o, map.query(id, THREADS * QPT), res, MODE, LEAD ? v.lead : 0u);
+    if (act && !again) {
+        if constexpr (WHOLE)
+            mq.done[id] = res;
+        else
+            put_result(o, map.query(id, THREADS * QPT), res, MODE, LEAD ? v.lead : 0u);
+    }
     if constexpr (MICRO) {
         const unsigned mask = __ballot_sync(0xffffffffu, again);
         if (again) {
@@ -752,13 +764,21 @@ __device__ __forceinline__ Entry superset_probe(const V1View &v, uint32_t l, uin
 // carries from step to step (`last` empties it); `id0` is the step's first
 // query in the CTA's numbering. SHORT: the lanes settle the shortest ranges
 // themselves.
+// WHOLE: the results go to host memory, where a store of part of a line travels
+// the link by itself. Every query of the step is settled before any is stored (the
+// queue is empty between steps, numbers are places in the warp's 64), and each slot
+// is stored once, by the whole warp. The drains are less full, which the link hides
+// (n = 1e6, 2^23 queries, 0.44 ms at the link's rate: ranges of 8 1.57 ms by the
+// device-memory form, 0.47 so; ranges of 40 1.30 and 0.46; uniform lengths 0.44 both).
+// In device memory L2 puts the parts together, and drains are worth more.
 template <bool ALIGNED, bool MICRO, uint32_t MODE, int THREADS, int QPT, bool STATS, bool LEAD,
-          bool SHORT>
+          bool SHORT, bool WHOLE = false>
 __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryOut &o,
                                                    const StepMap &map, int64_t base, uint32_t cnt,
                                                    uint32_t id0, bool last,
                                                    const int2 (&in)[QPT], QStats &s,
-                                                   MissQueue<MICRO> &mq, uint32_t &count) {
+                                                   MissQueue<MICRO, WHOLE> &mq, uint32_t &count) {
+    static_assert(!WHOLE || (MICRO && SHORT && !STATS && !LEAD), "plain queries of a table index");
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t pol = l2_keep_policy();
     float *const vs = o.val ? o.val + base : nullptr;
@@ -807,9 +827,8 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
         // the probe's answer is stored even for a query it leaves open: the
         // drain (same warp, after __syncwarp) or the warp scan (same thread)
         // overwrites it, and whole-warp stores keep the output lines whole. A
-        // query inside one micro-block has none (results in host memory,
-        // ranges of 1: stored twice 0.38 ms per 3.8e6 queries, 0.22 once)
-        if (MICRO && scan[k]) continue;
+        // query inside one micro-block has none
+        if (WHOLE || (MICRO && scan[k])) continue;
         if (vs) __stcs(reinterpret_cast<unsigned int *>(vs) + j, decode_bits<MODE>(res[k]));
         if (is) __stcs(is + j, static_cast<int32_t>(entry_idx(res[k]) - lead));
     }
@@ -852,7 +871,7 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
     static_assert(QPT == 2, "two slots");
     const uint32_t below = (1u << lane) - 1u;
     uint32_t m0 = __ballot_sync(0xffffffffu, miss[0]), m1 = __ballot_sync(0xffffffffu, miss[1]);
-    if ((m0 | m1) == 0u && !last) return;
+    if (!WHOLE && (m0 | m1) == 0u && !last) return;
     bool tiny[2] = {false, false};
     if (MICRO && SHORT && __any_sync(0xffffffffu, any_scan))
 #pragma unroll
@@ -864,8 +883,15 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
         for (int k = 0; k < 2; ++k) {
             const uint32_t l = static_cast<uint32_t>(k ? qq[1].x : qq[0].x);
             const uint32_t r = static_cast<uint32_t>(k ? qq[1].y : qq[0].y);
-            if (k ? tiny[1] : tiny[0])
-                put_result(o, base + threadIdx.x + k * THREADS, short_range<ALIGNED, MODE>(v, l, r), MODE, lead);
+            if (k ? tiny[1] : tiny[0]) {
+                const Entry x = short_range<ALIGNED, MODE>(v, l, r);
+                if constexpr (WHOLE) {
+                    if (k) res[1] = x;
+                    else res[0] = x;
+                } else {
+                    put_result(o, base + threadIdx.x + k * THREADS, x, MODE, lead);
+                }
+            }
         }
         miss[0] = miss[0] && !tiny[0];
         miss[1] = miss[1] && !tiny[1];
@@ -882,7 +908,12 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
             if ((k ? miss[1] : miss[0]) && entry_idx(e) < l && (r >> 5) - (l >> 5) >= v.micro_span) {
                 const Entry x = tied_entry<STATS>(v, l, pol, s);
                 if ((x >> 32) == (e >> 32) && entry_idx(x) >= l) {
-                    put_result(o, base + threadIdx.x + k * THREADS, x, MODE, lead);
+                    if constexpr (WHOLE) {
+                        if (k) res[1] = x;
+                        else res[0] = x;
+                    } else {
+                        put_result(o, base + threadIdx.x + k * THREADS, x, MODE, lead);
+                    }
                     if (k) miss[1] = false;
                     else miss[0] = false;
                     if constexpr (STATS) s.c[kStatSecond] += 1u;
@@ -893,6 +924,30 @@ __device__ __forceinline__ void answer_step_queued(const V1View &v, const QueryO
         m1 = __ballot_sync(0xffffffffu, miss[1]);
     }
     const uint32_t n0 = __popc(m0), n1 = __popc(m1);
+    if constexpr (WHOLE) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (!miss[k]) continue;
+            const uint32_t l = static_cast<uint32_t>(qq[k].x);
+            const uint32_t e = k ? n0 + __popc(m1 & below) : __popc(m0 & below);
+            mq.l[e] = l | (entry_idx(res[k]) < l ? kMissLeft : 0u);
+            mq.r[e] = static_cast<uint32_t>(qq[k].y);
+            mq.id[e] = lane + 32u * k;
+        }
+        count = n0 + n1;
+#pragma unroll 1
+        while (count > 0u)
+            drain_misses<ALIGNED, MICRO, MODE, STATS, LEAD, THREADS, QPT>(v, o, map, mq, count, pol, s);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const uint32_t j = threadIdx.x + k * THREADS;
+            const Entry x = miss[k] ? mq.done[lane + 32u * k] : res[k];
+            if (ok[k] && vs) __stcs(reinterpret_cast<unsigned int *>(vs) + j, decode_bits<MODE>(x));
+            if (ok[k] && is) __stcs(is + j, static_cast<int32_t>(entry_idx(x)));
+        }
+        __syncwarp();  // the next step's drains write the answers again
+        return;
+    }
     const bool both = n0 + n1 <= 32u;
 #pragma unroll 1
     for (uint32_t k = both ? 1u : 0u; k < 2u + (last ? 1u : 0u); ++k) {

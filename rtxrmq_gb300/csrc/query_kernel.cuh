@@ -1,6 +1,6 @@
 // query_kernel.cuh -- the plain query kernel and its launch, instantiated by
-// query.cu (plain indexes) and query_lead.cu (arrays of a batch that start
-// off a 128-byte boundary).
+// query.cu (plain indexes), query_lead.cu (arrays of a batch that start off a
+// 128-byte boundary) and query_host.cu (results in host memory).
 #pragma once
 
 #include "engine.h"
@@ -31,11 +31,12 @@ __device__ __forceinline__ void load_full(const QueryOut &o, int64_t base, int2 
 // rmq_query_host) overlaps the current step's lookups. Specialised on the
 // key mode and on whether the index has the sub-block level. STATS: the
 // measurement instantiation (rmq_query_stats), which also counts how each
-// query was settled and what it read into stats[kStatCount].
-template <bool ALIGNED, bool MICRO, uint32_t MODE, bool STATS, bool LEAD>
+// query was settled and what it read into stats[kStatCount]. WHOLE: results in
+// host memory (answer_step_queued).
+template <bool ALIGNED, bool MICRO, uint32_t MODE, bool STATS, bool LEAD, bool WHOLE>
 __global__ void __launch_bounds__(kThreads, RMQ_QUERY_MINB)
 query_kernel(V1View v, QueryOut o, int64_t q, unsigned long long *stats) {
-    __shared__ __align__(128) MissQueue<MICRO> s_mq[kThreads / 32];
+    __shared__ __align__(128) MissQueue<MICRO, WHOLE> s_mq[kThreads / 32];
     constexpr int64_t chunk = static_cast<int64_t>(kThreads) * kQPT;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * chunk;
     int64_t c0 = static_cast<int64_t>(blockIdx.x) * chunk;
@@ -44,7 +45,7 @@ query_kernel(V1View v, QueryOut o, int64_t q, unsigned long long *stats) {
     QStats s;
     if constexpr (STATS)
         for (int c = 0; c < kStatCount; ++c) s.c[c] = 0u;
-    MissQueue<MICRO> &mq = s_mq[threadIdx.x >> 5];
+    MissQueue<MICRO, WHOLE> &mq = s_mq[threadIdx.x >> 5];
     uint32_t waiting = 0;  // the warp's queue length (warp-uniform)
     int2 cur[kQPT];
     if (c0 <= last_full)
@@ -59,7 +60,7 @@ query_kernel(V1View v, QueryOut o, int64_t q, unsigned long long *stats) {
             load_full(o, c1, nxt);
         else if (c1 < q)
             load_queries<kQPT>(o, c1, q, nxt);
-        answer_step_queued<ALIGNED, MICRO, MODE, kThreads, kQPT, STATS, LEAD, true>(
+        answer_step_queued<ALIGNED, MICRO, MODE, kThreads, kQPT, STATS, LEAD, true, WHOLE>(
             v, o, map, c0, static_cast<uint32_t>(min(chunk, q - c0)), id0, c1 >= q, cur, s, mq, waiting);
 #pragma unroll
         for (int k = 0; k < kQPT; ++k) cur[k] = nxt[k];
@@ -85,11 +86,11 @@ uint32_t grid_size(int64_t q, int64_t per_block, int per_sm, const DeviceInfo &d
     return static_cast<uint32_t>(need < cap ? need : cap);
 }
 
-template <bool ALIGNED, bool MICRO, uint32_t MODE, bool STATS, bool LEAD>
+template <bool ALIGNED, bool MICRO, uint32_t MODE, bool STATS, bool LEAD, bool WHOLE>
 cudaError_t launch_query_t(const V1View &v, const QueryOut &o, int64_t q,
                            unsigned long long *stats, const DeviceInfo &dev, cudaStream_t s) {
     static std::atomic<int> per_sm_cache[kMaxDevices] = {};  // the carve-out is set per device
-    auto kern = query_kernel<ALIGNED, MICRO, MODE, STATS, LEAD>;
+    auto kern = query_kernel<ALIGNED, MICRO, MODE, STATS, LEAD, WHOLE>;
     int per_sm = per_sm_cache[dev.device].load(std::memory_order_relaxed);
     if (per_sm == 0) {
         cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, 0);
@@ -100,7 +101,7 @@ cudaError_t launch_query_t(const V1View &v, const QueryOut &o, int64_t q,
         // default split gives 100 KB for the 41 KB used (lr=-2, bs 4096,
         // n = 1e8: 0.52 ms, with this 0.48).
         err = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                   carveout_percent(per_sm * (sizeof(MissQueue<MICRO>) * (kThreads / 32) + 1024)));
+                                   carveout_percent(per_sm * (sizeof(MissQueue<MICRO, WHOLE>) * (kThreads / 32) + 1024)));
         if (err != cudaSuccess) return err;
         per_sm_cache[dev.device].store(per_sm, std::memory_order_relaxed);
     }
@@ -108,14 +109,14 @@ cudaError_t launch_query_t(const V1View &v, const QueryOut &o, int64_t q,
     return cudaGetLastError();
 }
 
-template <bool ALIGNED, bool MICRO, bool STATS, bool LEAD>
+template <bool ALIGNED, bool MICRO, bool STATS, bool LEAD, bool WHOLE = false>
 cudaError_t launch_query_m(const V1View &v, const QueryOut &o, int64_t q,
                            unsigned long long *stats, const DeviceInfo &dev, cudaStream_t s) {
     switch (v.kmode) {
-    case kFloatMax: return launch_query_t<ALIGNED, MICRO, kFloatMax, STATS, LEAD>(v, o, q, stats, dev, s);
-    case kIntMin: return launch_query_t<ALIGNED, MICRO, kIntMin, STATS, LEAD>(v, o, q, stats, dev, s);
-    case kIntMax: return launch_query_t<ALIGNED, MICRO, kIntMax, STATS, LEAD>(v, o, q, stats, dev, s);
-    default: return launch_query_t<ALIGNED, MICRO, kFloatMin, STATS, LEAD>(v, o, q, stats, dev, s);
+    case kFloatMax: return launch_query_t<ALIGNED, MICRO, kFloatMax, STATS, LEAD, WHOLE>(v, o, q, stats, dev, s);
+    case kIntMin: return launch_query_t<ALIGNED, MICRO, kIntMin, STATS, LEAD, WHOLE>(v, o, q, stats, dev, s);
+    case kIntMax: return launch_query_t<ALIGNED, MICRO, kIntMax, STATS, LEAD, WHOLE>(v, o, q, stats, dev, s);
+    default: return launch_query_t<ALIGNED, MICRO, kFloatMin, STATS, LEAD, WHOLE>(v, o, q, stats, dev, s);
     }
 }
 
