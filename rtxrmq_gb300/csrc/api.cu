@@ -524,11 +524,12 @@ int rmq_query_stats_ex(const rmq_handle_t *h, const int32_t *d_queries, int64_t 
     // takes its own block sizes (counted with RMQ_STATS_OWN_TABLES).
     BuildPlan plan = h->plan;
     void *tables = nullptr;
+    unsigned long long pooled = 0;
     cudaError_t err = cudaSuccess;
     if (plan.micro && (flags & RMQ_STATS_OWN_TABLES)) {
         plan.light = true;  // end parts by their sectors
     } else if (plan.micro) {
-        err = dev_malloc(&tables, plan_index(plan, false, true));
+        err = pool_malloc(&tables, plan_index(plan, false, true), dev.device, stream, &pooled);
         if (err != cudaSuccess) return cuda_fail(err, "rmq_query_stats: tables");
         place_index(plan, tables);
         err = launch_build(plan, dev, stream);
@@ -548,7 +549,10 @@ int rmq_query_stats_ex(const rmq_handle_t *h, const int32_t *d_queries, int64_t 
     if (err == cudaSuccess) err = launch_query(plan, a, dev, stream);
     if (err == cudaSuccess) err = cudaMemcpyAsync(host, dst, sizeof(host), cudaMemcpyDeviceToHost, stream);
     if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
-    if (tables) cudaFree(tables);
+    if (pooled)
+        cudaFreeAsync(tables, stream);
+    else if (tables)
+        cudaFree(tables);
     if (err != cudaSuccess) return cuda_fail(err, "rmq_query_stats");
     for (int c = 0; c < RMQ_QUERY_STATS_FIELDS; ++c) h_counts[c] = static_cast<int64_t>(host[c]);
     return RMQ_OK;

@@ -1,7 +1,7 @@
 """CPU: the rules of api.cu about index memory, run against a CUDA runtime on the
 host (fake_cuda.h): whose order a release follows, that a waiting one leaves
-captures alone, that a pool ends with its context, and that what it keeps counts as
-free."""
+captures alone, that a pool ends with its context, that what it keeps counts as free,
+and where tables made for one call come from."""
 import subprocess
 from pathlib import Path
 
@@ -109,4 +109,19 @@ def test_kept_memory_counts_as_free(tmp_path):
     fake::take();
     setenv("RTXRMQ_FAIL_ALLOC", "1", 1);
     EXPECT(!index_of(0) && fake::take() == "");
+""")
+
+
+def test_counting_takes_its_tables_from_the_pool(tmp_path):
+    """rmq_query_stats makes tables for the call: from the pool, and back to it in
+    stream order, with no allocation that waits for the device."""
+    run(tmp_path, r"""
+    static int32_t queries[2];
+    static int64_t counts[RMQ_QUERY_STATS_FIELDS];
+    rmq_handle_t *h = index_of(0);
+    fake::take();
+    EXPECT(rmq_query_stats(h, queries, 1, nullptr, nullptr, counts, nullptr) == RMQ_OK);
+    EXPECT(fake::take() == "pool0 free-async0 ");
+    setenv("RTXRMQ_FAIL_ALLOC", "1", 1);
+    EXPECT(rmq_query_stats(h, queries, 1, nullptr, nullptr, counts, nullptr) == RMQ_ENOMEM && fake::take() == "");
 """)
