@@ -44,13 +44,6 @@ def _stream_handle(stream) -> Optional[int]:
     return stream.cuda_stream
 
 
-def _current_handle(device: int) -> int:
-    """Handle of a device's current stream, CUDA being initialised (0.06 us;
-    torch.cuda.current_stream() takes 2.9 to make an object of it)."""
-    import torch
-    return torch._C._cuda_getCurrentRawStream(device)
-
-
 def _durable_stream(stream):
     """(handle, object or None): the object when the stream outlives its
     Python wrapper (the default stream and torch's pool streams are never
@@ -138,7 +131,10 @@ class RMQIndex:
             out_idx = None
         elif out_idx is None:
             out_idx = torch.empty(q, dtype=torch.int32, device=queries.device)
-        s = _current_handle(torch.cuda.current_device()) if stream is None else _stream_handle(stream)
+        if stream is None:  # 0.1 us; torch.cuda.current_stream() makes an object in 2.9
+            s = torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+        else:
+            s = _stream_handle(stream)
         if s != self._one_stream:
             self._one_stream = None
         check(load().rmq_query(self._h, _dptr(queries), q, _dptr(out_val), _dptr(out_idx), s))
@@ -236,19 +232,20 @@ class RMQIndex:
         another stream than their own."""
         if getattr(self, "_h", None) is not None and self._h.value:
             h, self._h = self._h, C.c_void_p()
-            if self._in_stream_order():
+            if self._one_stream is not None and self._in_stream_order():
                 self._values.record_stream(self._keep)
                 check(load().rmq_free_async(h, self._one_stream))
             else:
                 check(load().rmq_free(h))
 
     def _in_stream_order(self) -> bool:
-        if self._keep is None or self._one_stream is None:
-            return False
+        import torch
         # another current device is rmq_free_async's to see. Memory that is not
         # torch's (a storage of a foreign buffer cannot be resized) is given back by
         # its owner as soon as the tensor is gone.
-        return (_current_handle(self._keep.device_index) == self._one_stream and
+        s = self._keep
+        return (s is not None and
+                torch._C._cuda_getCurrentRawStream(s.device_index) == self._one_stream and
                 self._values.untyped_storage().resizable())
 
     def __enter__(self):
