@@ -1,7 +1,8 @@
-// lane_min.cuh -- the best of one lane's four consecutive values, as a key
-// (common.cuh) and a position: the comparison rule of lines.cuh for one lane,
-// spelt out. Host and device code, so that the host tests run it against the
-// definition (the smallest key, leftmost among equal keys).
+// lane_min.cuh -- the best of four consecutive values, as a key (common.cuh) and
+// a position: the comparison rule of lines.cuh spelt out for one lane. The
+// kernels reduce whole lines by that rule (minima_impl.cuh, query_impl.cuh); this
+// form of it is what the host tests run against the definition (the smallest
+// key, leftmost among equal keys).
 #pragma once
 
 #include <cmath>

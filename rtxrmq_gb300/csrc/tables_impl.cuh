@@ -12,9 +12,9 @@
 //
 // Two windows of level k cover 2^k .. 2^(k+1) - 1 micro-blocks. The masks
 // take the place of five or six rows of offsets, of which a query read two
-// entries. What bounds short queries is L1 tag lookups, one per scattered
-// load: two of them now (mask, minimum) for ranges of up to 1000 (2000)
-// elements, three to four before.
+// entries. What bounds short queries is scattered loads that miss the L1 (its
+// requests to the L2 are busy 78% of the time at lr = -3): two of them now (mask,
+// minimum) for ranges of up to 1000 (2000) elements, three to four before.
 #pragma once
 
 #include "common.cuh"
