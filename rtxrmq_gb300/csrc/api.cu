@@ -678,10 +678,10 @@ int rmq_query_host(const rmq_handle_t *h, const int32_t *h_queries, int64_t q, f
     if ((mode & 1) && h_idx && !is_device_memory(h_idx)) idev = nullptr;
     const bool v_stage = h_val && !vdev;
     const bool i_stage = h_idx && !idev;
+    // results that the kernel stores to host memory
+    const bool host = (vdev && !is_device_memory(h_val)) || (idev && !is_device_memory(h_idx));
     if (qdev && !v_stage && !i_stage)
-        return query_in_place(h, reinterpret_cast<const int32_t *>(qdev), q, vdev, idev,
-                              (vdev && !is_device_memory(h_val)) || (idev && !is_device_memory(h_idx)),
-                              stream);
+        return query_in_place(h, reinterpret_cast<const int32_t *>(qdev), q, vdev, idev, host, stream);
 
     DeviceInfo dev;
     int rc = device_info(&dev);
@@ -748,6 +748,7 @@ int rmq_query_host(const rmq_handle_t *h, const int32_t *h_queries, int64_t q, f
         a.val = dv;
         a.idx = di;
         a.invalid = h->invalid;
+        a.host = host;
         err = launch_query(h->plan, a, dev, hm->ks);
         if (err == cudaSuccess) err = cudaEventRecord(hm->k_done[b], hm->ks);
         if (err == cudaSuccess && (v_stage || i_stage)) {

@@ -66,3 +66,26 @@ def test_results_in_host_memory(cuda, native, n, kind, off, op):
             B = A if op == "min" else -A
             m = range_min(composites(B + 0.0), Q[~bad][:, 0], Q[~bad][:, 1])
             np.testing.assert_array_equal(di.numpy()[~bad], (m & np.uint64(0xffffffff)).astype(np.int64) >> 1)
+
+
+@pytest.mark.parametrize("mode", ["1", "2", "3"])
+def test_partly_staged(cuda, native, monkeypatch, mode):
+    """Queries staged and results in place, results staged, both."""
+    import torch
+
+    import rtxrmq_gb300 as R
+    rng = np.random.default_rng(int(mode))
+    A = rng.random(300_000).astype(np.float32)
+    Q, _ = mixed(len(A), 30_000, rng)
+    with R.RMQIndex(torch.from_numpy(A).to(cuda)) as ix:
+        dv, di = (x.cpu().numpy() for x in ix.query(torch.from_numpy(Q).to(cuda)))
+        monkeypatch.setenv("RTXRMQ_HOST_MODE", mode)
+        hv, hi = torch.zeros(len(Q)).pin_memory(), torch.zeros(len(Q), dtype=torch.int32).pin_memory()
+        for v, i in ((hv, hi), (hv, None), (None, hi)):
+            hv.fill_(7), hi.fill_(7)
+            ix.query_host(torch.from_numpy(Q).pin_memory(), v, i)
+            torch.cuda.synchronize()
+            if v is not None:
+                np.testing.assert_array_equal(hv.numpy().view(np.uint32), dv.view(np.uint32))
+            if i is not None:
+                np.testing.assert_array_equal(hi.numpy(), di)
