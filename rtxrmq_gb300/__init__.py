@@ -231,9 +231,11 @@ class RMQIndex:
         the device. Queries and outputs follow torch's rules for tensors used on
         another stream than their own."""
         if getattr(self, "_h", None) is not None and self._h.value:
-            h, self._h = self._h, C.c_void_p()
-            if self._one_stream is not None and self._in_stream_order():
+            in_order = self._one_stream is not None and self._in_stream_order()
+            if in_order:
                 self._values.record_stream(self._keep)
+            h, self._h = self._h, C.c_void_p()
+            if in_order:
                 check(load().rmq_free_async(h, self._one_stream))
             else:
                 check(load().rmq_free(h))

@@ -783,7 +783,10 @@ int rmq_free(rmq_handle_t *h) {
         e2 = cudaGetDevice(&cur);
         if (e2 == cudaSuccess && cur != h->device) e2 = cudaSetDevice(h->device);
         // a reset of the device took the memory with it
-        if (e2 == cudaSuccess) gone = device_context_id(h->device) != h->pool_context;
+        if (e2 == cudaSuccess) {
+            const unsigned long long now = device_context_id(h->device);
+            gone = now && now != h->pool_context;
+        }
         if (e2 == cudaSuccess && !gone) e2 = wait_for_device();
         if (cur != h->device) cudaSetDevice(cur);
     }

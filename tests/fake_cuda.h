@@ -11,7 +11,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
-#include "../../include/rmq.h"
+#include "../include/rmq.h"
 #include "engine.h"
 
 namespace fake {
