@@ -44,16 +44,27 @@ def _stream_handle(stream) -> Optional[int]:
     return stream.cuda_stream
 
 
+_durable = {}  # (device, handle) -> stream object: streams that live as long as the process
+
+
 def _durable_stream(stream):
     """(handle, object or None): the object when the stream outlives its
     Python wrapper (the default stream and torch's pool streams are never
     destroyed), None for a raw handle or an external stream."""
     import torch
-    s = torch.cuda.current_stream() if stream is None else stream
-    if isinstance(s, int):
-        return s, None
-    sid = getattr(s, "stream_id", None)  # torch: 0 default, odd pool, else external
-    return s.cuda_stream, (s if sid is not None and (sid == 0 or sid & 1) else None)
+    if stream is None:
+        device = torch.cuda.current_device()
+        s = torch._C._cuda_getCurrentRawStream(device)
+        if (device, s) in _durable:  # no new object for the current stream (2.9 us)
+            return s, _durable[device, s]
+        stream = torch.cuda.current_stream()
+    if isinstance(stream, int):
+        return stream, None
+    sid = getattr(stream, "stream_id", None)  # torch: 0 default, odd pool, else external
+    if sid is None or not (sid == 0 or sid & 1):
+        return stream.cuda_stream, None
+    _durable[stream.device_index, stream.cuda_stream] = stream
+    return stream.cuda_stream, stream
 
 
 def _dptr(t) -> Optional[int]:

@@ -49,6 +49,8 @@ def world(monkeypatch):
     lib, now = Calls(), [Stream(0)]
     monkeypatch.setattr(R, "load", lambda: lib)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: now[0])
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: now[0].device_index)
+    monkeypatch.setattr(R, "_durable", {})
     monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream",
                         lambda d: now[0].cuda_stream if d == now[0].device_index else 0, raising=False)
 
@@ -85,6 +87,12 @@ def test_rule(world):
     ix = index()
     ix._use(side)
     assert closed(ix) == waits
+    other = Stream(7)
+    other.stream_id = 0x7f00  # external: its handle may be gone at the close
+    now[0] = other
+    assert closed(index()) == waits
+    assert closed(index(other)) == waits and closed(index(7)) == waits
+    now[0] = Stream(0)
     ix = index()
     ix._values.own = False  # memory of another library
     assert closed(ix) == waits
